@@ -151,6 +151,7 @@ scw_status ensure_lanes(scw_batch b, int lanes) {
         // the tensor-core error flag is allocated here, never inside a capture
         if (cudaMalloc(&c->tc_err, sizeof(int)) != cudaSuccess) return fail(SCW_ERR_NOMEM, "cudaMalloc error flag");
         SCW_CUDA_TRY(cudaMemset(c->tc_err, 0, sizeof(int)));
+        c->tc_pending_check = true;        // and never cleared by a graph: scw_batch_wait reads it
         b->lane_ctx.push_back(c);
         b->lane_arena.push_back(nullptr);
         b->lane_bytes.push_back(0);
@@ -202,6 +203,7 @@ scw_status build_graph(scw_batch b, const std::vector<int>& idx, int lanes, int 
             scw::sv::Carver c{b->lane_arena[l], 0};
             scw::sv::SolveWs ws{};
             scw::sv::carve_ws(it.sp, c, ws);
+            ws.gemm.err = b->lane_ctx[l]->tc_err;
             SepBufs sb;
             carve_sep(it.sp, c, sb);
             char* scratch = c.take<char>(it.ep.scratch_bytes);

@@ -154,6 +154,7 @@ scw_status scw_ctx_destroy(scw_ctx c) {
     c->desc.release();
     c->planes_out.release();
     c->sep_scratch.release();
+    c->dense_ws.release();
     c->host_desc.release();
     if (c->tc_err) cudaFree(c->tc_err);
     for (auto& t : c->timings) {

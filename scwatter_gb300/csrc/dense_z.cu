@@ -8,8 +8,8 @@
 // A[i * ld + j]; complex numbers are double2 (re, im); "batched" kernels take a batch stride in
 // elements and run one matrix per blockIdx.z (GEMM) or per CTA (factorisations).
 //
-// The GB300 FP64 rate is low (about 8 GFLOP/s per SM), so the O(n^3) parts are spread over all
-// SMs where the algorithm allows it (GEMM, the trailing updates of LU); the inherently
+// The GB300 FP64 rate is low (about 8 GFLOP/s per SM), so the O(n^3) parts are products where the
+// algorithm allows it (the trailing updates of LU), and those run on the tensor cores; the inherently
 // sequential ones (Hessenberg reduction, QR sweeps) run one CTA per matrix and are batched over
 // the slices of a sample.
 #include <algorithm>
@@ -26,8 +26,10 @@ namespace scw {
 namespace z {
 
 // ------------------------------------------------------------------------------------
-// GEMM: C = alpha * op(A) * B + beta * C, op = identity.  64 x 64 tiles, 256 threads, each
-// thread a 4 x 4 complex block; K staged 16 at a time through shared memory.
+// GEMM on the FP32 / FP64 pipes: C = alpha * op(A) * B + beta * C, op = identity.  64 x 64 tiles,
+// 256 threads, each thread a 4 x 4 complex block; K staged 16 at a time through shared memory.
+// FP32 products run here.  FP64 products run on the tensor cores (gemm_tc.cu, 20 to 35 times faster)
+// and come here only without a workspace: scw_zgemm while its stream is being captured.
 // ------------------------------------------------------------------------------------
 constexpr int kGT = 64, kGK = 16;
 
@@ -1013,8 +1015,20 @@ scw_status gemm(cudaStream_t st, int M, int N, int K, C alpha, const C* A, int l
     return SCW_OK;
 }
 
+// The products inside the factorisations: FP64 on the tensor cores (gemm_tc.cu), FP32 by gemm_kernel
 template <typename C>
-scw_status getrf(cudaStream_t st, C* A, int n, long long sA, int* piv, long long sP, int* info, int batch) {
+static scw_status mm(cudaStream_t st, int M, int N, int K, C alpha, const C* A, int lda, long long sA, const C* B, int ldb,
+                     long long sB, C beta, C* Cm, int ldc, long long sC, int batch, const GemmWs& ws,
+                     const int* skip = nullptr) {
+    if constexpr (sizeof(C) == sizeof(double2))
+        return zgemm(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, Cm, ldc, sC, batch, ws, skip);
+    else
+        return gemm<C>(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, Cm, ldc, sC, batch, skip);
+}
+
+template <typename C>
+scw_status getrf(cudaStream_t st, C* A, int n, long long sA, int* piv, long long sP, int* info, int batch,
+                 const GemmWs& ws) {
     if (n <= 0 || batch <= 0) return SCW_OK;
     SCW_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(int) * batch, st));
     const C one = {1, 0}, minus = {-1, 0};
@@ -1028,9 +1042,9 @@ scw_status getrf(cudaStream_t st, C* A, int n, long long sA, int* piv, long long
         const int rem = n - k0 - nb;
         if (rem > 0) {
             // A22 -= L21 U12
-            scw_status s = gemm<C>(st, rem, rem, nb, minus, A + (long long)(k0 + nb) * n + k0, n, sA,
-                                   A + (long long)k0 * n + k0 + nb, n, sA, one, A + (long long)(k0 + nb) * n + k0 + nb,
-                                   n, sA, batch);
+            scw_status s = mm<C>(st, rem, rem, nb, minus, A + (long long)(k0 + nb) * n + k0, n, sA,
+                                 A + (long long)k0 * n + k0 + nb, n, sA, one, A + (long long)(k0 + nb) * n + k0 + nb,
+                                 n, sA, batch, ws);
             if (s != SCW_OK) return s;
         }
     }
@@ -1039,7 +1053,7 @@ scw_status getrf(cudaStream_t st, C* A, int n, long long sA, int* piv, long long
 
 template <typename C>
 scw_status getrs(cudaStream_t st, const C* LU, int n, long long sA, const int* piv, long long sP, C* B, int nrhs,
-                 long long sB, int batch) {
+                 long long sB, int batch, const GemmWs& ws) {
     // blocked: per diagonal block a small triangular solve, the rest of the rows updated by GEMM
     if (n <= 0 || nrhs <= 0 || batch <= 0) return SCW_OK;
     constexpr int kTB = 64;
@@ -1053,9 +1067,9 @@ scw_status getrs(cudaStream_t st, const C* LU, int n, long long sA, const int* p
         SCW_CUDA_TRY(cudaGetLastError());
         const int rem = n - k0 - nb;
         if (rem > 0) {
-            scw_status s = gemm<C>(st, rem, nrhs, nb, minus, LU + (long long)(k0 + nb) * n + k0, n, sA,
-                                   B + (long long)k0 * nrhs, nrhs, sB, one, B + (long long)(k0 + nb) * nrhs, nrhs, sB,
-                                   batch);
+            scw_status s = mm<C>(st, rem, nrhs, nb, minus, LU + (long long)(k0 + nb) * n + k0, n, sA,
+                                 B + (long long)k0 * nrhs, nrhs, sB, one, B + (long long)(k0 + nb) * nrhs, nrhs, sB,
+                                 batch, ws);
             if (s != SCW_OK) return s;
         }
     }
@@ -1064,8 +1078,8 @@ scw_status getrs(cudaStream_t st, const C* LU, int n, long long sA, const int* p
         z::trsm_block_kernel<C><<<g, 256, 0, st>>>(LU, n, sA, k0, nb, B, nrhs, sB, nrhs, 1);
         SCW_CUDA_TRY(cudaGetLastError());
         if (k0 > 0) {
-            scw_status s = gemm<C>(st, k0, nrhs, nb, minus, LU + k0, n, sA, B + (long long)k0 * nrhs, nrhs, sB, one, B,
-                                   nrhs, sB, batch);
+            scw_status s = mm<C>(st, k0, nrhs, nb, minus, LU + k0, n, sA, B + (long long)k0 * nrhs, nrhs, sB, one, B,
+                                 nrhs, sB, batch, ws);
             if (s != SCW_OK) return s;
         }
     }
@@ -1153,7 +1167,7 @@ static scw_status hqr_launch(cudaStream_t st, C* A, C* Q, int n, long long nn, C
 
 template <typename C>
 scw_status geev(cudaStream_t st, C* A, C* W, C* V, int n, int batch, C* work, int* status, const int* skip,
-                bool wide) {
+                bool wide, const GemmWs& ws) {
     // A (overwritten): n x n per batch entry; W: n eigenvalues; V: n x n right eigenvectors (columns)
     // work: >= batch * (n*n + 3 n) elements
     if (n <= 0 || batch <= 0) return SCW_OK;
@@ -1191,7 +1205,7 @@ scw_status geev(cudaStream_t st, C* A, C* W, C* V, int n, int batch, C* work, in
     z::trevc_kernel<C><<<gt, 256, 0, st>>>(A, V, n, nn, skip);
     SCW_CUDA_TRY(cudaGetLastError());
     const C one = {1, 0}, zero = {0, 0};
-    scw_status s = gemm<C>(st, n, n, n, one, Q, n, nn, V, n, nn, zero, A, n, nn, batch, skip);
+    scw_status s = mm<C>(st, n, n, n, one, Q, n, nn, V, n, nn, zero, A, n, nn, batch, ws, skip);
     if (s != SCW_OK) return s;
     z::copy_kernel<C><<<dim3((unsigned)std::min<long long>((nn + 255) / 256, 4096), batch), 256, 0, st>>>(A, V, nn, skip);
     SCW_CUDA_TRY(cudaGetLastError());
@@ -1201,10 +1215,10 @@ scw_status geev(cudaStream_t st, C* A, C* W, C* V, int n, int batch, C* work, in
 #define SCW_DENSE_INSTANTIATE(C)                                                                                    \
     template scw_status gemm<C>(cudaStream_t, int, int, int, C, const C*, int, long long, const C*, int, long long, \
                                 C, C*, int, long long, int, const int*);                                           \
-    template scw_status getrf<C>(cudaStream_t, C*, int, long long, int*, long long, int*, int);                    \
+    template scw_status getrf<C>(cudaStream_t, C*, int, long long, int*, long long, int*, int, const GemmWs&);     \
     template scw_status getrs<C>(cudaStream_t, const C*, int, long long, const int*, long long, C*, int, long long, \
-                                 int);                                                                             \
-    template scw_status geev<C>(cudaStream_t, C*, C*, C*, int, int, C*, int*, const int*, bool);
+                                 int, const GemmWs&);                                                              \
+    template scw_status geev<C>(cudaStream_t, C*, C*, C*, int, int, C*, int*, const int*, bool, const GemmWs&);
 SCW_DENSE_INSTANTIATE(double2)
 SCW_DENSE_INSTANTIATE(float2)
 #undef SCW_DENSE_INSTANTIATE
@@ -1224,10 +1238,16 @@ scw_status scw_zgemm(scw_ctx ctx, int M, int N, int K, const double* alpha, cons
     if (!ctx || !A || !B || !C || !alpha || !beta || M < 0 || N < 0 || K < 0 || batch < 1)
         return fail(SCW_ERR_ARG, "scw_zgemm: bad arguments");
     SCW_ON_DEVICE(ctx->device);
-    ctx->launches++;
+    // the workspace and the launches that use it go together: calls of several threads on one context
+    // must not interleave
+    std::lock_guard<std::mutex> lock(ctx->dense_mu);
+    ctx->launches += 3;
+    scw::GemmWs ws;
+    scw_status st = scw::ctx_gemm_ws(ctx, scw::zgemm_ws_bytes(M, N, K, 1), scw::zgemm_ws_bytes(M, N, K, batch), ws);
+    if (st != SCW_OK) return st;
     return scw::zgemm(ctx->stream, M, N, K, make_double2(alpha[0], alpha[1]), (const double2*)A, K, (long long)M * K,
                       (const double2*)B, N, (long long)K * N, make_double2(beta[0], beta[1]), (double2*)C, N,
-                      (long long)M * N, batch);
+                      (long long)M * N, batch, ws);
 }
 
 scw_status scw_zgesv(scw_ctx ctx, int n, int nrhs, void* A, void* B, int batch, int* info_host) {
@@ -1241,15 +1261,22 @@ scw_status scw_zgesv(scw_ctx ctx, int n, int nrhs, void* A, void* B, int batch, 
         return fail(SCW_ERR_NOMEM, "scw_zgesv: pivots");
     }
     const long long nn = (long long)n * n;
-    scw_status st = scw::zgetrf(ctx->stream, (double2*)A, n, nn, dpiv, n, dinfo, batch, nullptr);
+    scw::DevBuf wbuf;
+    scw::GemmWs ws;
+    const size_t need = std::max(scw::zgemm_ws_bytes(n, n, 32, 1), scw::zgemm_ws_bytes(n, nrhs, 64, 1));
+    scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, scw::kGemmWsCap)));
+    if (st == SCW_OK) st = scw::ctx_tc_flag(ctx);
+    ws = scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err};
+    if (st == SCW_OK) st = scw::zgetrf(ctx->stream, (double2*)A, n, nn, dpiv, n, dinfo, batch, ws);
     if (st == SCW_OK)
-        st = scw::zgetrs(ctx->stream, (const double2*)A, n, nn, dpiv, n, (double2*)B, nrhs, (long long)n * nrhs, batch);
+        st = scw::zgetrs(ctx->stream, (const double2*)A, n, nn, dpiv, n, (double2*)B, nrhs, (long long)n * nrhs, batch,
+                         ws);
     ctx->launches += 3;
     std::vector<int> info(batch, 0);
     if (st == SCW_OK) {
         cudaError_t e = cudaMemcpyAsync(info.data(), dinfo, sizeof(int) * batch, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) st = fail(SCW_ERR_CUDA, cudaGetErrorString(e));
+        else st = scw_ctx_synchronize(ctx);
     }
     cudaFree(dpiv);
     cudaFree(dinfo);
@@ -1272,13 +1299,19 @@ scw_status scw_zgeev(scw_ctx ctx, int n, void* A, void* W, void* V, int batch, i
         cudaFree(work);
         return fail(SCW_ERR_NOMEM, "scw_zgeev: workspace");
     }
-    scw_status st = scw::zgeev(ctx->stream, (double2*)A, (double2*)W, (double2*)V, n, batch, work, dst, true);
+    scw::DevBuf wbuf;
+    const size_t need = scw::zgemm_ws_bytes(n, n, n, 1);
+    scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, scw::kGemmWsCap)));
+    if (st == SCW_OK) st = scw::ctx_tc_flag(ctx);
+    if (st == SCW_OK)
+        st = scw::zgeev(ctx->stream, (double2*)A, (double2*)W, (double2*)V, n, batch, work, dst, true,
+                        scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err});
     ctx->launches += 4;
     std::vector<int> status(batch, 0);
     if (st == SCW_OK) {
         cudaError_t e = cudaMemcpyAsync(status.data(), dst, sizeof(int) * batch, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) st = fail(SCW_ERR_CUDA, cudaGetErrorString(e));
+        else st = scw_ctx_synchronize(ctx);
     }
     cudaFree(work);
     cudaFree(dst);
@@ -1303,7 +1336,7 @@ scw_status scw_cgeev(scw_ctx ctx, int n, void* A, void* W, void* V, int batch, i
         return fail(SCW_ERR_NOMEM, "scw_cgeev: workspace");
     }
     scw_status st = scw::geev<float2>(ctx->stream, (float2*)A, (float2*)W, (float2*)V, n, batch, work, dst, nullptr,
-                                      true);
+                                      true, scw::GemmWs{});
     ctx->launches += 5;
     std::vector<int> status(batch, 0);
     if (st == SCW_OK) {

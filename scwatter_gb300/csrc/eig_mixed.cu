@@ -609,7 +609,7 @@ static scw_status set_smem(const void* fn, size_t bytes) {
 }
 
 scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int n, int Z, const EigMixWs& w,
-                      double2* fb_work, int* status, const EigMixParams& prm, long long* launches) {
+                      double2* fb_work, int* status, const EigMixParams& prm, const GemmWs& ws, long long* launches) {
     if (n <= 0 || Z <= 0) return SCW_OK;
     if (n > kMaxN) return fail(SCW_ERR_ARG, "geev_mixed: matrix order above the mixed path's limit");
     const long long nn = (long long)n * n;
@@ -630,7 +630,7 @@ scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int
     to_f32_kernel<<<nblk(nn * Z), 256, 0, st>>>(A, w.S0, nn * Z);
     MX_LAUNCHED(2);
     // FP32 Householder + QR + triangular eigenvectors: eigenvectors into S2, eigenvalues lam32
-    MX_TRY(geev<float2>(st, w.S0, w.lam32, w.S2, n, Z, w.S1, w.qr, nullptr, prm.wide));
+    MX_TRY(geev<float2>(st, w.S0, w.lam32, w.S2, n, Z, w.S1, w.qr, nullptr, prm.wide, GemmWs{}));
     if (launches) *launches += 5;
     init_kernel<<<dim3(gZ, Z), 256, 0, st>>>(w.lam32, w.S2, lam, V, n, w.qr, w.state, w.steps, w.res);
     cluster_kernel<<<Z, 1024, cl_smem, st>>>(lam, n, w.anorm, prm.tau_rel, w.label, w.member, w.cstart, w.ncl, w.state);
@@ -638,7 +638,7 @@ scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int
     const int last = n >= EigMixParams::kLargeN ? std::max(prm.steps, prm.steps_large) : prm.steps;
     for (int s = 0; s <= last; s++) {
         // residual check (and right-hand side of the correction)
-        MX_TRY(gemm<double2>(st, n, n, n, d1, A, n, nn, V, n, nn, d0, AX, n, nn, Z, w.state));
+        MX_TRY(zgemm(st, n, n, n, d1, A, n, nn, V, n, nn, d0, AX, n, nn, Z, ws, w.state));
         resid_kernel<<<dim3((n + 31) / 32, Z), 256, 0, st>>>(AX, V, lam, n, w.S3, w.rn, w.xn, w.state);
         gate_kernel<<<Z, 256, 0, st>>>(n, w.rn, w.xn, w.anorm, s >= prm.steps ? prm.tol_accept : prm.tol, s, w.state,
                                        w.steps, w.res);
@@ -647,8 +647,8 @@ scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int
         // E = X^-1 R in FP32
         to32_kernel<<<dim3(gZ, Z), 256, 0, st>>>(V, w.S0, w.S2, n, w.state);
         MX_LAUNCHED(1);
-        MX_TRY(getrf<float2>(st, w.S0, n, nn, w.piv, n, w.info, Z));
-        MX_TRY(getrs<float2>(st, w.S0, n, nn, w.piv, n, w.S3, n, nn, Z));
+        MX_TRY(getrf<float2>(st, w.S0, n, nn, w.piv, n, w.info, Z, GemmWs{}));
+        MX_TRY(getrs<float2>(st, w.S0, n, nn, w.piv, n, w.S3, n, nn, Z, GemmWs{}));
         if (launches) *launches += 3 * ((n + 31) / 32) + 1 + 4 * ((n + 63) / 64);
         lu_check_kernel<<<nblk(Z), 256, 0, st>>>(w.info, Z, w.state);
         singleton_kernel<<<dim3(nblk(n), Z), 256, 0, st>>>(w.S3, w.label, lam, n, w.state);
@@ -665,7 +665,7 @@ scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int
     // slices without convergence: the FP64 Householder + QR solver (qr[] reused as the skip mask)
     final_kernel<<<nblk(Z), 256, 0, st>>>(w.state, w.qr, Z);
     MX_LAUNCHED(1);
-    MX_TRY(geev<double2>(st, A, lam, V, n, Z, fb_work, status, w.qr, prm.wide));
+    MX_TRY(geev<double2>(st, A, lam, V, n, Z, fb_work, status, w.qr, prm.wide, ws));
     if (launches) *launches += 5;
     return SCW_OK;
 }
@@ -709,8 +709,14 @@ extern "C" scw_status scw_zgeev_mixed(scw_ctx ctx, int n, void* A, void* W, void
     long long L = 0;
     mx::EigMixParams prm;
     prm.wide = true;
-    scw_status st = mx::geev_mixed(ctx->stream, (double2*)A, (double2*)W, (double2*)V, n, batch, w,
-                                   reinterpret_cast<double2*>(blk), dst, prm, &L);
+    DevBuf wbuf;
+    const size_t need = zgemm_ws_bytes(n, n, n, 1);
+    scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, kGemmWsCap)));
+    if (st == SCW_OK) st = ctx_tc_flag(ctx);
+    if (st == SCW_OK)
+        st = mx::geev_mixed(ctx->stream, (double2*)A, (double2*)W, (double2*)V, n, batch, w,
+                            reinterpret_cast<double2*>(blk), dst, prm, GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err},
+                            &L);
     ctx->launches += L;
     std::vector<int> status(batch, 0), state(batch, 0), steps(batch, 0);
     std::vector<double> res(batch, 0.0);
@@ -722,8 +728,8 @@ extern "C" scw_status scw_zgeev_mixed(scw_ctx ctx, int n, void* A, void* W, void
             e = cudaMemcpyAsync(steps.data(), w.steps, sizeof(int) * batch, cudaMemcpyDeviceToHost, ctx->stream);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(res.data(), w.res, sizeof(double) * batch, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) st = fail(SCW_ERR_CUDA, cudaGetErrorString(e));
+        else st = scw_ctx_synchronize(ctx);
     }
     cudaFree(blk);
     cudaFree(dst);

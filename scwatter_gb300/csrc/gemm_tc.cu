@@ -1,0 +1,570 @@
+// FP64 complex GEMM on the tensor cores (tcgen05, sm_103a): C = alpha A B + beta C, batched.
+//
+// GB300 issues about 1.7 FP64 FMA per SM and clock, against 4096 bf16 multiply-adds on the tensor
+// core, so an FP64 product is far cheaper as a sum of exact integer products (the error-free
+// splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59 (2012)):
+//   * the inner index is rescaled by powers of two, A'(i,k) = A(i,k) 2^f_k and B'(k,j) = B(k,j)
+//     2^-f_k with 2^f_k above row k of B, so that graded operands (the cascade's E^-1 rows) lose
+//     nothing against a plain sum; then row i of A' gets the exponent e_i, column j of B' g_j;
+//   * every value becomes a 62-bit integer in units of 2^(e_i - 62) (2^(g_j - 62)), cut into kS = 8
+//     balanced base-256 digits, each in [-128, 128] and therefore exact in bf16;
+//   * digit products of equal weight are summed on the tensor core in FP32.  A sum over K = 128
+//     of the d + 1 <= 8 products of diagonal d, for both products of a complex part, is an integer
+//     below 2^24 for d <= 3 (exact); the later diagonals weigh 2^-32 and less and could round only if
+//     every digit were extreme at once.  After 128 terms the diagonals are drained into 64-bit
+//     integers, and the final sum is rounded to FP64 once.
+// Diagonals d >= 8 are dropped: at most 2^-57 of the largest product per term.  Measured against
+// extended precision at n = 18 .. 1200 (random, constant, log-normal, diagonally dominant matrices,
+// eigenvectors): relative error 2e-17 .. 6.8e-16, where
+// a sequential FP64 sum has 9e-17 .. 1.7e-15.  With 7 digits (55 bits) the diagonally dominant and
+// eigenvector products came out 20 times less exact than an FP64 sum, so 8 it is (36 digit products
+// instead of 28).
+//
+// Work per 128 x 32 tile and 16 inner indices: digit i of A (real or imaginary part, 128 x 16)
+// multiplies digits 0 .. 7 - i of B side by side (N = 32 (8 - i) columns) and lands at column 32 i
+// of the accumulator, so that digit i of A and j of B meet in diagonal i + j.  32 MMAs of N = 32 ..
+// 256 use all 512 TMEM columns (real and imaginary diagonals).
+//
+// Measured (38.6 at n = 3200 and 26 TFLOP/s for 20 matrices of n = 648, counted as FP64 operations;
+// the FP64 pipes give 1.05-1.25): 1.66 ms instead of 38 ms for the latter, of which 0.3 ms prepare
+// the operands.  Bound by the tensor core's operand reads and the drains between chunks.
+//
+// Two launches prepare the operands (oz_inner_kernel: f_k; oz_split_kernel: e_i, g_j and the digits in
+// the order the MMA reads them, so that a pipeline stage is two contiguous bulk copies), one runs
+// the product: persistent CTAs, one thread copying, one issuing MMAs, 8 warps draining.
+// Non-finite values: a row of A or a column of B with one gives NaN in its whole row / column.
+#include <algorithm>
+#include <cstdint>
+
+#include "scw_complex.cuh"
+#include "scw_dense.h"
+#include "scw_tc.cuh"
+
+namespace scw {
+namespace oz {
+
+constexpr int kS = 8;                        // base-256 digits per value
+constexpr int kBits = 62;                    // integer bits before the cut
+constexpr int kTM = 128, kTN = 32, kTK = 16; // tile rows, columns, inner indices per stage
+constexpr int kABlk = 2 * kS * kTM * kTK * 2;   // bytes of A per stage: re, im x digits x 128 x 16 bf16
+constexpr int kBBlk = 2 * kS * kTN * kTK * 2;
+constexpr int kStages = 2;
+constexpr int kChunk = 8;                    // stages per drain (K = 128)
+constexpr int kDrainWarps = 8;
+constexpr int kThreads = (kDrainWarps + 2) * 32;
+constexpr int kSpecial = 1 << 20;            // exponent of a row or column with a non-finite value
+constexpr int kNone = -100000;               // exponent of a zero row or column
+
+// e with |v| < 2^e for the larger of the two parts; kNone for zero, kSpecial if not finite
+__device__ __forceinline__ int cexpo(double2 v) {
+    const unsigned a = (unsigned)__double2hiint(v.x) & 0x7fffffffu, b = (unsigned)__double2hiint(v.y) & 0x7fffffffu;
+    const unsigned m = max(a, b) >> 20;
+    if (m == 0x7ff) return kSpecial;
+    if (m == 0 && v.x == 0.0 && v.y == 0.0) return kNone;
+    return (int)max(m, 1u) - 1022;
+}
+
+// round(v 2^s) for |v 2^s| < 2^62 (ties away from zero)
+__device__ __forceinline__ long long fixed_point(double v, int s) {
+    const long long bits = __double_as_longlong(v);
+    const int ex = (int)((bits >> 52) & 0x7ff);
+    long long m = bits & 0xfffffffffffffll;
+    if (ex) m |= 1ll << 52;
+    const int sh = (ex ? ex : 1) - 1075 + s;
+    if (sh >= 0) m <<= min(sh, 10);
+    else m = sh < -55 ? 0 : (m + (1ll << (-sh - 1))) >> -sh;
+    return bits < 0 ? -m : m;
+}
+
+// f[b][k] with |B(k, :)| < 2^f: a warp per row of B
+__global__ void __launch_bounds__(256)
+oz_inner_kernel(const double2* __restrict__ B, int ldb, long long sB, int K, int N, int* __restrict__ f,
+                const int* __restrict__ skip) {
+    if (z::skipped(skip, blockIdx.y)) return;
+    const int k = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (k >= K) return;
+    const double2* row = B + sB * blockIdx.y + (long long)k * ldb;
+    int e = kNone;
+#pragma unroll 4
+    for (int j = lane; j < N; j += 32) {
+        const int x = cexpo(row[j]);
+        if (x != kSpecial) e = max(e, x);
+    }
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (lane == 0) f[(long long)blockIdx.y * K + k] = e;
+}
+
+// the digits of 8 consecutive inner indices of one row (or column), real or imaginary part: one
+// 16-byte store per digit, dst + digit * stride
+__device__ __forceinline__ void store_digits(const long long (&q)[8], unsigned char* dst, int stride) {
+    unsigned lo[8], hi[8];
+#pragma unroll
+    for (int t = 0; t < 8; t++) {       // + 128 in every digit below the top: bytes are digit + 128
+        const long long b = q[t] + 0x80808080808080ll;
+        lo[t] = (unsigned)b;
+        hi[t] = (unsigned)((unsigned long long)b >> 32);
+    }
+#pragma unroll
+    for (int s = 0; s < kS; s++) {
+        float v[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+            // integer to float through the low mantissa bits of 2^23
+            if (s == 0) {
+                v[t] = __uint_as_float(0x4b000000u + 256u + (unsigned)((int)hi[t] >> 24)) - (8388608.0f + 256.0f);
+            } else {
+                const int sh = 8 * (kS - 1 - s);
+                const unsigned byte = ((sh >= 32 ? hi[t] >> (sh - 32) : lo[t] >> sh) & 0xffu);
+                v[t] = __uint_as_float(0x4b000000u | byte) - (8388608.0f + 128.0f);
+            }
+        }
+        uint4 w;
+        w.x = __byte_perm(__float_as_uint(v[0]), __float_as_uint(v[1]), 0x7632);
+        w.y = __byte_perm(__float_as_uint(v[2]), __float_as_uint(v[3]), 0x7632);
+        w.z = __byte_perm(__float_as_uint(v[4]), __float_as_uint(v[5]), 0x7632);
+        w.w = __byte_perm(__float_as_uint(v[6]), __float_as_uint(v[7]), 0x7632);
+        *reinterpret_cast<uint4*>(dst + s * stride) = w;
+    }
+}
+
+struct SplitArgs {
+    const double2 *A, *B;
+    int lda, ldb;
+    long long sA, sB;
+    int M, N, K, nk, mt, nt;           // nk stages, mt x nt tiles
+    int gA, gB, nA;                    // 16-row groups of A, 16-column groups of B per matrix; A blocks in all
+    const int* f;
+    int *eA, *gN;                      // e_i [b][16 gA], g_j [b][16 gB]
+    unsigned char *dA, *dB;
+    int fstep;                         // f stride per A matrix: 0 when all matrices share one B
+};
+
+// Exponents and digits.  A block takes 16 rows of A or 16 columns of B: first the largest exponent
+// of each over the inner index, then the digits, a warp per stage of 16 inner indices (lane = 8
+// rows x 2 halves of the stage x 2 row groups, so a warp stores 512 contiguous bytes per digit).
+__global__ void __launch_bounds__(256)
+oz_split_kernel(SplitArgs p, const int* __restrict__ skip) {
+    __shared__ int se[16][17];
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const bool isA = (int)blockIdx.x < p.nA;
+    const int blk = isA ? blockIdx.x : blockIdx.x - p.nA;
+    const int per = isA ? p.gA : p.gB;
+    const int b = blk / per, g = blk - b * per;
+    if (z::skipped(skip, b)) return;
+    const int r0 = g * 16, R = isA ? p.M : p.N;
+    const double2* src = isA ? p.A + p.sA * b : p.B + p.sB * b;
+    const long long rs = isA ? p.lda : 1, ks = isA ? 1 : p.ldb;      // element (row, k) at row rs + k ks
+    const int* f = p.f + (long long)(isA ? b * p.fstep : b) * p.K;
+    {
+        // 16 x 16 threads: along k for the rows of A, along the columns of B (both contiguous)
+        const int r = isA ? t >> 4 : t & 15, kr = isA ? t & 15 : t >> 4;
+        int e = kNone;
+        if (r0 + r < R) {
+#pragma unroll 4
+            for (int k = kr; k < p.K; k += 16) {
+                const int x = cexpo(src[(r0 + r) * rs + k * ks]);
+                if (x == kSpecial) e = kSpecial;
+                else if (x != kNone) e = max(e, isA ? x + f[k] : x - f[k]);
+            }
+        }
+        se[r][kr] = e;
+    }
+    __syncthreads();
+    if (t < 16) {
+        int e = kNone;
+        for (int q = 0; q < 16; q++) e = max(e, se[t][q]);
+        se[t][16] = e;
+        (isA ? p.eA : p.gN)[(long long)b * per * 16 + r0 + t] = e;
+    }
+    __syncthreads();
+    const int rl = (lane & 7) + 8 * (lane >> 4), kh = (lane >> 3) & 1;
+    const int r = r0 + rl, e = se[rl][16];
+    const bool live = r < R && e > kNone / 2 && e < kSpecial;
+    const int T = isA ? kTM : kTN, blkb = isA ? kABlk : kBBlk, dig = T * kTK * 2;
+    unsigned char* dst = (isA ? p.dA + (long long)b * p.mt * p.nk * kABlk : p.dB + (long long)b * p.nt * p.nk * kBBlk) +
+                         (long long)(r0 / T) * p.nk * blkb + (r0 % T) * 32 + (lane >> 4) * 256 + kh * 128 + (lane & 7) * 16;
+    for (int st = warp; st < p.nk; st += 8) {
+        const int k0 = st * kTK + kh * 8;
+        long long qr[8], qi[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            qr[j] = qi[j] = 0;
+            const int k = k0 + j;
+            if (live && k < p.K) {
+                const double2 v = src[r * rs + k * ks];
+                const int s = (isA ? f[k] : -f[k]) - e + kBits;
+                qr[j] = fixed_point(v.x, s);
+                qi[j] = fixed_point(v.y, s);
+            }
+        }
+        unsigned char* o = dst + (long long)st * blkb;
+        store_digits(qr, o, dig);
+        store_digits(qi, o + kS * dig, dig);
+    }
+}
+
+// (hi 2^32 + lo) 2^e rounded once to FP64, with integer operations (FP64 ones cost 60 times more)
+__device__ __forceinline__ double fx_to_double(long long hi, long long lo, int e) {
+    hi += lo >> 32;
+    unsigned L = (unsigned)lo;
+    const bool neg = hi < 0;
+    unsigned long long H = (unsigned long long)hi;
+    if (neg) {
+        L = 0u - L;
+        H = ~H + (L == 0u ? 1ull : 0ull);
+    }
+    if (H == 0ull) {
+        H = L;
+        L = 0u;
+        e -= 32;
+        if (H == 0ull) return 0.0;
+    }
+    const int lz = __clzll((long long)H);            // >= 1: |hi| < 2^62
+    const unsigned long long L64 = (unsigned long long)L << 32;
+    const unsigned long long m = (H << lz) | (L64 >> (64 - lz));
+    const bool sticky = (L64 << lz) != 0ull;
+    unsigned long long r = m >> 11;
+    const unsigned rem = (unsigned)m & 0x7ffu;
+    r += (rem > 0x400u || (rem == 0x400u && (sticky || (r & 1ull)))) ? 1ull : 0ull;
+    const int ex = 63 + 32 + e - lz + 1023;          // biased exponent of the value
+    const unsigned long long sign = neg ? 1ull << 63 : 0ull;
+    if (ex >= 1 && ex <= 2046) return __longlong_as_double((long long)(sign + ((unsigned long long)(ex - 1) << 52) + r));
+    return scalbn(__longlong_as_double((long long)(sign + (1022ull << 52) + r)), max(-5000, min(5000, ex - 1023)));
+}
+
+struct GemmArgs {
+    const unsigned char *dA, *dB;
+    const int *eA, *gN;
+    int M, N, nk, mt, nt, gA, gB;
+    int a_shared, b_shared;            // all matrices use the digits of matrix 0
+    double2 alpha, beta;
+    double2* C;
+    int ldc;
+    long long sC;
+    int tiles;
+    int* err;
+};
+
+__global__ void __launch_bounds__(kThreads, 1)
+oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
+    using namespace tc;
+    extern __shared__ __align__(1024) unsigned char smem[];
+    unsigned char* sA = smem;
+    unsigned char* sB = smem + kStages * kABlk;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sB + kStages * kBBlk);
+    uint64_t* full = bar;                         // [kStages] copies -> MMA
+    uint64_t* empty = bar + kStages;              // [kStages] MMA -> copies
+    uint64_t* acc_full = bar + 2 * kStages;       // MMA -> drain
+    uint64_t* acc_empty = acc_full + 1;           // drain -> MMA
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(acc_full + 3);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int i = 0; i < kStages; i++) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 1);
+        }
+        mbar_init(acc_full, 1);
+        mbar_init(acc_empty, kDrainWarps * 32);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        tmem_alloc(tmem_slot, kTmemCols);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    const int per = p.mt * p.nt;
+
+    if (warp == kDrainWarps) {
+        // ---------------- copies ----------------
+        if (lane == 0) {
+            int it = 0;
+            bool ok = true;
+            for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
+                const int b = tile / per, q = tile - b * per, m = q / p.nt, n = q - m * p.nt;
+                if (z::skipped(skip, b)) continue;
+                const unsigned char* ga = p.dA + ((long long)(p.a_shared ? 0 : b) * p.mt + m) * p.nk * kABlk;
+                const unsigned char* gb = p.dB + ((long long)(p.b_shared ? 0 : b) * p.nt + n) * p.nk * kBBlk;
+                for (int k = 0; k < p.nk; k++, it++) {
+                    const int s = it % kStages;
+                    if (*abort_flag || (it >= kStages && !mbar_wait(&empty[s], (uint32_t)((it / kStages - 1) & 1)))) {
+                        *abort_flag = 1;
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(&full[s], kABlk + kBBlk);
+                    bulk_load(sA + s * kABlk, ga + (long long)k * kABlk, kABlk, &full[s]);
+                    bulk_load(sB + s * kBBlk, gb + (long long)k * kBBlk, kBBlk, &full[s]);
+                }
+            }
+            // no copy into shared memory outlives the kernel (after an abort the MMA thread may not
+            // have waited for the last ones)
+            for (int i = max(0, it - kStages); i < it; i++) mbar_wait(&full[i % kStages], (uint32_t)((i / kStages) & 1));
+        }
+        __syncwarp();
+    } else if (warp == kDrainWarps + 1) {
+        // ---------------- MMA issue ----------------
+        if (lane == 0) {
+            constexpr uint32_t base = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTM >> 4) << 24);
+            constexpr uint32_t negA = 1u << 13;
+            constexpr uint32_t im = kS * kTN;       // first column of the imaginary diagonals
+            int it = 0, chunk = 0;
+            bool ok = true;
+            for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
+                if (z::skipped(skip, tile / per)) continue;
+                for (int k = 0; k < p.nk; k++, it++) {
+                    const int s = it % kStages;
+                    const bool first = k % kChunk == 0;
+                    if (first && chunk > 0 && !mbar_wait(acc_empty, (uint32_t)((chunk - 1) & 1))) ok = false;
+                    if (!ok || *abort_flag || !mbar_wait(&full[s], (uint32_t)((it / kStages) & 1))) {
+                        *abort_flag = 1;
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t a = smem_u32(sA + s * kABlk), bb = smem_u32(sB + s * kBBlk);
+                    const uint64_t dbr = make_desc(bb, 128, 256), dbi = make_desc(bb + kS * kTN * kTK * 2, 128, 256);
+#pragma unroll
+                    for (int i = 0; i < kS; i++) {
+                        const uint32_t id = base | ((uint32_t)((kS - i) * kTN >> 3) << 17);
+                        const uint64_t dar = make_desc(a + i * kTM * kTK * 2, 128, 256);
+                        const uint64_t dai = make_desc(a + (kS + i) * kTM * kTK * 2, 128, 256);
+                        const uint32_t col = tmem + (uint32_t)(i * kTN);
+                        const uint32_t acc = !(first && i == 0);
+                        umma<1>(col, dar, dbr, id, acc);
+                        umma<1>(col + im, dar, dbi, id, acc);
+                        umma<1>(col, dai, dbi, id | negA, 1);
+                        umma<1>(col + im, dai, dbr, id, 1);
+                    }
+                    umma_commit(&empty[s]);
+                    if (k % kChunk == kChunk - 1 || k == p.nk - 1) {
+                        umma_commit(acc_full);
+                        chunk++;
+                    }
+                }
+            }
+            // the accumulators must be idle before TMEM is freed
+            for (int i = max(0, it - kStages); i < it; i++) mbar_wait(&empty[i % kStages], (uint32_t)((i / kStages) & 1));
+        }
+        __syncwarp();
+    } else {
+        // -------- drain: warp w reads TMEM lanes 32 (w % 4) .., columns 16 (w / 4) .. of each diagonal --------
+        const int quarter = warp & 3, half = warp >> 2;
+        const uint32_t tb = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 16);
+        int chunk = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
+            const int b = tile / per, q = tile - b * per, m = q / p.nt, n = q - m * p.nt;
+            if (z::skipped(skip, b)) continue;
+            // diagonals 0 .. 3 and 4 .. 7 (weights 2^24, 2^16, 2^8, 1) per part and column
+            long long hi[2][16], lo[2][16];
+#pragma unroll
+            for (int c = 0; c < 16; c++) hi[0][c] = hi[1][c] = lo[0][c] = lo[1][c] = 0;
+            for (int k = 0; k < p.nk; k += kChunk, chunk++) {
+                int stop = *abort_flag;
+                if (!stop && !mbar_wait(acc_full, (uint32_t)(chunk & 1))) stop = 1;
+                if (__any_sync(0xffffffffu, stop)) {
+                    *abort_flag = 1;
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+#pragma unroll
+                for (int part = 0; part < 2; part++)
+#pragma unroll
+                    for (int d = 0; d < kS; d++) {
+                        uint32_t v[16];
+                        tmem_ld16(tb + (uint32_t)(part * kS * kTN + d * kTN), v);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int c = 0; c < 16; c++) {
+                            const long long x = __float2int_rn(__uint_as_float(v[c]));
+                            if (d <= 3) hi[part][c] += x * (1 << (8 * (3 - d)));
+                            else lo[part][c] += x * (1 << (8 * (kS - 1 - d)));
+                        }
+                    }
+                tc_fence_before();
+                mbar_arrive(acc_empty);
+            }
+            if (!ok) break;
+            const int row = m * kTM + quarter * 32 + lane, col0 = n * kTN + half * 16;
+            if (row < p.M) {
+                const int eA = p.eA[(long long)(p.a_shared ? 0 : b) * p.gA * 16 + row];
+                const int* gN = p.gN + (long long)(p.b_shared ? 0 : b) * p.gB * 16 + col0;
+                double2* out = p.C + p.sC * b + (long long)row * p.ldc + col0;
+                const bool unit = p.alpha.y == 0.0 && (p.alpha.x == 1.0 || p.alpha.x == -1.0);
+                const bool add = p.beta.x != 0.0 || p.beta.y != 0.0;
+                const bool add1 = p.beta.x == 1.0 && p.beta.y == 0.0;
+#pragma unroll
+                for (int c = 0; c < 16; c++) {
+                    if (col0 + c < p.N) {
+                        const int g = gN[c];
+                        // the last diagonal weighs 2^(8 (kS - 1)); units 2^(eA - kBits) 2^(g - kBits)
+                        const int e = eA + g + 8 * (kS - 1) - 2 * kBits;
+                        double2 v;
+                        if (eA >= kSpecial || g >= kSpecial) {
+                            v = make_double2(__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll));
+                        } else {
+                            v.x = fx_to_double(hi[0][c], lo[0][c], e);
+                            v.y = fx_to_double(hi[1][c], lo[1][c], e);
+                        }
+                        if (unit) {
+                            if (p.alpha.x < 0.0) v = make_double2(-v.x, -v.y);
+                        } else {
+                            v = z::cmul(p.alpha, v);
+                        }
+                        if (add1) {
+                            const double2 o = out[c];
+                            v = make_double2(v.x + o.x, v.y + o.y);
+                        } else if (add) {
+                            v = z::cfma(p.beta, out[c], v);
+                        }
+                        out[c] = v;
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (tid == 0 && *abort_flag) atomicExch(p.err, 1);
+    if (warp == 0) {
+        tc_fence_after();
+        tmem_dealloc(tmem, kTmemCols);
+    }
+}
+
+// y = alpha A x + beta y, a warp per row (the one-column products of the beta recursion)
+__global__ void __launch_bounds__(256)
+zgemv_kernel(int M, int K, double2 alpha, const double2* __restrict__ A, int lda, long long sA,
+             const double2* __restrict__ x, int ldx, long long sX, double2 beta, double2* __restrict__ y, int ldy,
+             long long sY, const int* __restrict__ skip) {
+    if (z::skipped(skip, blockIdx.y)) return;
+    const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (i >= M) return;
+    const double2* row = A + sA * blockIdx.y + (long long)i * lda;
+    x += sX * blockIdx.y;
+    double2 s = make_double2(0.0, 0.0);
+#pragma unroll 4
+    for (int k = lane; k < K; k += 32) s = z::cfma(row[k], x[(long long)k * ldx], s);
+    for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    if (lane == 0) {
+        double2* o = y + sY * blockIdx.y + (long long)i * ldy;
+        double2 v = z::cmul(alpha, s);
+        if (beta.x != 0.0 || beta.y != 0.0) v = z::cfma(beta, *o, v);
+        *o = v;
+    }
+}
+
+static size_t al256(size_t x) { return (x + 255) / 256 * 256; }
+
+struct Shape {
+    int nk, mt, nt, gA, gB;
+    size_t a, b, small_a, small_b;     // bytes per matrix: digits of A, of B, exponents
+    Shape(int M, int N, int K) {
+        nk = (K + kTK - 1) / kTK;
+        mt = (M + kTM - 1) / kTM;
+        nt = (N + kTN - 1) / kTN;
+        gA = (M + 15) / 16;
+        gB = (N + 15) / 16;
+        a = (size_t)mt * nk * kABlk;
+        b = (size_t)nt * nk * kBBlk;
+        small_a = (size_t)gA * 16 * sizeof(int);
+        small_b = ((size_t)gB * 16 + K) * sizeof(int);
+    }
+    size_t bytes(int na, int nb) const { return al256(na * small_a) + al256(nb * small_b) + na * a + nb * b; }
+};
+
+}  // namespace oz
+
+scw_status ctx_tc_flag(scw_ctx ctx) {
+    if (!ctx->tc_err && cudaMalloc(&ctx->tc_err, sizeof(int)) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(SCW_ERR_NOMEM, "cudaMalloc error flag");
+    }
+    // cleared once per synchronisation: a flag raised by an earlier launch stays raised
+    if (!ctx->tc_pending_check) SCW_CUDA_TRY(cudaMemsetAsync(ctx->tc_err, 0, sizeof(int), ctx->stream));
+    ctx->tc_pending_check = true;
+    return SCW_OK;
+}
+
+scw_status ctx_gemm_ws(scw_ctx ctx, size_t one, size_t all, GemmWs& ws) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    SCW_CUDA_TRY(cudaStreamIsCapturing(ctx->stream, &cap));
+    ws = GemmWs{};
+    if (cap != cudaStreamCaptureStatusNone) return SCW_OK;
+    scw_status st = ctx->dense_ws.reserve(std::max(one, std::min(all, kGemmWsCap)));
+    if (st == SCW_OK) st = ctx_tc_flag(ctx);
+    ws = GemmWs{(char*)ctx->dense_ws.ptr, ctx->dense_ws.bytes, ctx->tc_err};
+    return st;
+}
+
+size_t zgemm_ws_bytes(int M, int N, int K, int batch) { return oz::Shape(M, N, K).bytes(batch, batch); }
+
+scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const double2* A, int lda, long long sA,
+                 const double2* B, int ldb, long long sB, double2 beta, double2* C, int ldc, long long sC, int batch,
+                 const GemmWs& ws, const int* skip) {
+    if (M <= 0 || N <= 0 || batch <= 0) return SCW_OK;
+    if (N == 1) {
+        oz::zgemv_kernel<<<dim3((M + 7) / 8, batch), 256, 0, st>>>(M, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC,
+                                                                  skip);
+        SCW_CUDA_TRY(cudaGetLastError());
+        return SCW_OK;
+    }
+    if (!ws.base) return gemm<double2>(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, skip);
+    int sms = 0, dev = 0;
+    SCW_CUDA_TRY(cudaGetDevice(&dev));
+    SCW_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    constexpr size_t smem = oz::kStages * (oz::kABlk + oz::kBBlk) + (2 * oz::kStages + 4) * sizeof(uint64_t);
+    SCW_CUDA_TRY(cudaFuncSetAttribute(oz::oz_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const oz::Shape sh(M, N, K);
+    const bool a1 = sA == 0 && !skip, b1 = sB == 0 && !skip;     // one operand for the whole batch
+    // as many matrices at a time as the workspace holds
+    int step = batch;
+    while (step > 1 && sh.bytes(a1 ? 1 : step, b1 ? 1 : step) > ws.bytes) step = (step + 1) / 2;
+    if (sh.bytes(1, 1) > ws.bytes) return fail(SCW_ERR_NOMEM, "zgemm: workspace too small");
+    for (int b0 = 0; b0 < batch; b0 += step) {
+        const int nb = std::min(step, batch - b0);
+        const int na_ = a1 ? 1 : nb, nb_ = b1 ? 1 : nb;
+        char* cur = ws.base;
+        int* eA = reinterpret_cast<int*>(cur);
+        cur += oz::al256(na_ * sh.small_a);
+        int* gN = reinterpret_cast<int*>(cur);
+        int* f = gN + (size_t)nb_ * sh.gB * 16;
+        cur += oz::al256(nb_ * sh.small_b);
+        unsigned char* dA = reinterpret_cast<unsigned char*>(cur);
+        unsigned char* dB = dA + na_ * sh.a;
+        const double2* Ab = A + sA * b0;
+        const double2* Bb = B + sB * b0;
+        const int* sk = skip ? skip + b0 : nullptr;
+        // with one A for several B the inner scaling would differ per matrix: none then
+        const bool scale = !(a1 && !b1);
+        if (K > 0) {
+            if (scale) {
+                oz::oz_inner_kernel<<<dim3((K + 7) / 8, nb_), 256, 0, st>>>(Bb, ldb, sB, K, N, f, sk);
+                SCW_CUDA_TRY(cudaGetLastError());
+            } else {
+                SCW_CUDA_TRY(cudaMemsetAsync(f, 0, sizeof(int) * (size_t)K * nb_, st));
+            }
+        }
+        oz::SplitArgs sp{Ab, Bb, lda, ldb, sA, sB, M, N, K, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB, na_ * sh.gA, f, eA, gN,
+                         dA, dB, b1 ? 0 : 1};
+        oz::oz_split_kernel<<<na_ * sh.gA + nb_ * sh.gB, 256, 0, st>>>(sp, sk);
+        SCW_CUDA_TRY(cudaGetLastError());
+        const long long tiles = (long long)sh.mt * sh.nt * nb;
+        if (tiles > (1ll << 30)) return fail(SCW_ERR_ARG, "zgemm: too many tiles");
+        oz::GemmArgs g{dA, dB, eA, gN, M, N, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB, a1, b1, alpha, beta, C + sC * b0, ldc, sC,
+                       (int)tiles, ws.err};
+        oz::oz_gemm_kernel<<<(unsigned)std::min<long long>(tiles, sms), oz::kThreads, smem, st>>>(g, sk);
+        SCW_CUDA_TRY(cudaGetLastError());
+    }
+    return SCW_OK;
+}
+
+}  // namespace scw

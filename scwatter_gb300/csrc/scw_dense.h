@@ -29,17 +29,41 @@ __device__ __forceinline__ float2 zsqrt(float2 a) {
 // precision) or float2 (FP32, the first stage of the mixed-precision eigen-solver).  A
 // non-null skip[b] != 0 makes every kernel leave batch entry b untouched.
 
+// Device workspace of the FP64 GEMM (gemm_tc.cu): any size that holds one matrix's operands; err is
+// a device flag raised when a bounded wait gave up.
+struct GemmWs {
+    char* base = nullptr;
+    size_t bytes = 0;
+    int* err = nullptr;
+};
+// cap on a workspace sized for a whole batch; larger batches go through it in parts
+constexpr size_t kGemmWsCap = 512ull << 20;
+// the context's tensor-core error flag (allocated, cleared unless a check is pending) is in use from
+// here on: the next scw_ctx_synchronize reads it
+scw_status ctx_tc_flag(scw_ctx ctx);
+// a context's own GEMM workspace of at least `one` bytes, `all` if that is below the cap; none (the
+// products then run without one) while the context's stream is being captured
+scw_status ctx_gemm_ws(scw_ctx ctx, size_t one, size_t all, GemmWs& ws);
+// workspace that takes the whole batch in one pass
+size_t zgemm_ws_bytes(int M, int N, int K, int batch);
+// C = alpha A B + beta C (row-major, batched by strides in elements), FP64 on the tensor cores; without
+// a workspace by gemm<double2>
+scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const double2* A, int lda, long long sA,
+                 const double2* B, int ldb, long long sB, double2 beta, double2* C, int ldc, long long sC, int batch,
+                 const GemmWs& ws, const int* skip = nullptr);
+
 // C = alpha A B + beta C (row-major, batched by strides in elements)
 template <typename C>
 scw_status gemm(cudaStream_t st, int M, int N, int K, C alpha, const C* A, int lda, long long sA, const C* B, int ldb,
                 long long sB, C beta, C* Cm, int ldc, long long sC, int batch, const int* skip = nullptr);
 // in-place LU with partial pivoting of n x n matrices (leading dimension n); info[b] = first zero pivot + 1
 template <typename C>
-scw_status getrf(cudaStream_t st, C* A, int n, long long sA, int* piv, long long sP, int* info, int batch);
+scw_status getrf(cudaStream_t st, C* A, int n, long long sA, int* piv, long long sP, int* info, int batch,
+                 const GemmWs& ws);
 // B := A^-1 B using getrf's factors (B: n x nrhs, leading dimension nrhs)
 template <typename C>
 scw_status getrs(cudaStream_t st, const C* LU, int n, long long sA, const int* piv, long long sP, C* B, int nrhs,
-                 long long sB, int batch);
+                 long long sB, int batch, const GemmWs& ws);
 // eigenvalues W and right eigenvectors V (columns) of A (overwritten); work >= batch (n^2 + 3 n);
 // status[b] = 1 when the QR iteration did not converge.  wide: the Hessenberg reduction of
 // matrices with n >= kWideMinN is spread over the whole GPU (3 launches per column) instead of one
@@ -47,25 +71,20 @@ scw_status getrs(cudaStream_t st, const C* LU, int n, long long sA, const int* p
 // items keeps the one-CTA form (fewer nodes).
 constexpr int kWideMinN = 128;
 template <typename C>
-scw_status geev(cudaStream_t st, C* A, C* W, C* V, int n, int batch, C* work, int* status, const int* skip = nullptr,
-                bool wide = false);
+scw_status geev(cudaStream_t st, C* A, C* W, C* V, int n, int batch, C* work, int* status, const int* skip, bool wide,
+                const GemmWs& ws);
 
-inline scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const double2* A, int lda, long long sA,
-                        const double2* B, int ldb, long long sB, double2 beta, double2* C, int ldc, long long sC,
-                        int batch) {
-    return gemm<double2>(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
-}
 inline scw_status zgetrf(cudaStream_t st, double2* A, int n, long long sA, int* piv, long long sP, int* info,
-                         int batch, double2* /*unused*/) {
-    return getrf<double2>(st, A, n, sA, piv, sP, info, batch);
+                         int batch, const GemmWs& ws) {
+    return getrf<double2>(st, A, n, sA, piv, sP, info, batch, ws);
 }
 inline scw_status zgetrs(cudaStream_t st, const double2* LU, int n, long long sA, const int* piv, long long sP,
-                         double2* B, int nrhs, long long sB, int batch) {
-    return getrs<double2>(st, LU, n, sA, piv, sP, B, nrhs, sB, batch);
+                         double2* B, int nrhs, long long sB, int batch, const GemmWs& ws) {
+    return getrs<double2>(st, LU, n, sA, piv, sP, B, nrhs, sB, batch, ws);
 }
 inline scw_status zgeev(cudaStream_t st, double2* A, double2* W, double2* V, int n, int batch, double2* work,
-                        int* status, bool wide = false) {
-    return geev<double2>(st, A, W, V, n, batch, work, status, nullptr, wide);
+                        int* status, bool wide, const GemmWs& ws) {
+    return geev<double2>(st, A, W, V, n, batch, work, status, nullptr, wide, ws);
 }
 // Hessenberg form of A (in place, n x n per batch entry) and the unitary Q (A = Q H Q^H);
 // work >= batch * 3 n

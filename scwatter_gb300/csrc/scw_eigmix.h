@@ -18,7 +18,7 @@
 
 #include <cuda_runtime.h>
 
-#include "scw_internal.h"
+#include "scw_dense.h"
 
 namespace scw {
 namespace mx {
@@ -61,7 +61,7 @@ struct EigMixParams {
 // double2, and it may alias S0..S3 / hw.  status[b] = 1 if even the FP64 fallback failed.
 // Launches only (graph-capturable); *launches is incremented by the kernels issued.
 scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int n, int Z, const EigMixWs& w,
-                      double2* fb_work, int* status, const EigMixParams& prm, long long* launches);
+                      double2* fb_work, int* status, const EigMixParams& prm, const GemmWs& ws, long long* launches);
 
 }  // namespace mx
 }  // namespace scw

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -97,6 +98,8 @@ struct scw_ctx_s {
     scw::DevBuf desc;           // per-call work descriptors
     scw::DevBuf planes_out;     // device staging of gpu_cw_evaluate's three planes
     scw::DevBuf sep_scratch;    // separable evaluator: phases, coefficients C, row products T, tables
+    scw::DevBuf dense_ws;       // operands of scw_zgemm's tensor-core product
+    std::mutex dense_mu;        // one caller of dense_ws at a time
     scw::PinnedBuf host_desc;   // pinned staging of the descriptors
     cudaEvent_t desc_done = nullptr;  // the last descriptor upload has been consumed
     void* static_scratch = nullptr;   // device address of the allocation-free entry point's array

@@ -552,6 +552,11 @@ void carve_ws(const SolvePlan& p, Carver& c, SolveWs& ws) {
         ws.mix.S2 = Wf;
         ws.mix.S3 = Wf + Z * nn;
     }
+    // operands of the FP64 products: the largest of them for one matrix, a whole batch up to the cap
+    const size_t one = std::max({zgemm_ws_bytes((int)n, (int)M3, (int)n, 1), zgemm_ws_bytes((int)M6, (int)M6, 64, 1),
+                                 zgemm_ws_bytes(p.X, p.M1, p.Y, 1), zgemm_ws_bytes(p.M0, p.M1, p.X, 1)});
+    ws.gemm.bytes = std::max(one, std::min(one * Z, kGemmWsCap));
+    ws.gemm.base = c.take<char>(ws.gemm.bytes);
     // temporary region, three overlays
     const size_t t0 = (c.off + 255) / 256 * 256;
     Carver ca{c.base, t0};
@@ -640,30 +645,30 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
     // tw2^T (M0 x X) . (F^T (X x Y) . tw1^T (Y x M1)), the M1 x M0 crop stored column-major
     n2_kernel<<<nblk(Zs * YX), 256, 0, st>>>(in.data, YX, Zs, ws.F);
     SCW_CUDA_TRY(cudaGetLastError());
-    SCW_TRY(zgemm(st, X, M1, Y, kOne, ws.F, Y, YX, in.tw1, M1, 0, kZero, ws.T, M1, (long long)X * M1, 2 * Zs));
+    SCW_TRY(zgemm(st, X, M1, Y, kOne, ws.F, Y, YX, in.tw1, M1, 0, kZero, ws.T, M1, (long long)X * M1, 2 * Zs, ws.gemm));
     SCW_TRY(zgemm(st, M0, M1, X, make_double2(1.0 / (double)YX, 0.0), in.tw2, X, 0, ws.T, M1, (long long)X * M1, kZero,
-                  ws.coef, M1, MF, 2 * Zs));
+                  ws.coef, M1, MF, 2 * Zs, ws.gemm));
     // P, Q and the reduced eigenproblem
     build_pq_kernel<<<dim3(nblk(n), n, Zs), 256, 0, st>>>(ws.coef, in.up, in.wq, in.qs, in.ps, M0, M1, k, ws.P, ws.Q);
     SCW_CUDA_TRY(cudaGetLastError());
-    SCW_TRY(zgemm(st, n, n, n, kOne, ws.P, n, nn, ws.Q, n, nn, kZero, ws.PQ, n, nn, Zs));
+    SCW_TRY(zgemm(st, n, n, n, kOne, ws.P, n, nn, ws.Q, n, nn, kZero, ws.PQ, n, nn, Zs, ws.gemm));
     if (p.eig_mixed) {
         mx::EigMixParams prm;
         prm.wide = p.wide_hess;
-        SCW_TRY(mx::geev_mixed(st, ws.PQ, ws.lam, ws.U, n, Zs, ws.mix, ws.P, out.status, prm, &L));
+        SCW_TRY(mx::geev_mixed(st, ws.PQ, ws.lam, ws.U, n, Zs, ws.mix, ws.P, out.status, prm, ws.gemm, &L));
         if (out.eig) {
             SCW_CUDA_TRY(cudaMemcpyAsync(out.eig, ws.mix.state, sizeof(int) * Zs, cudaMemcpyDeviceToDevice, st));
             SCW_CUDA_TRY(cudaMemcpyAsync(out.eig + Zs, ws.mix.steps, sizeof(int) * Zs, cudaMemcpyDeviceToDevice, st));
             SCW_CUDA_TRY(cudaMemcpyAsync(out.eig_res, ws.mix.res, sizeof(double) * Zs, cudaMemcpyDeviceToDevice, st));
         }
     } else {
-        SCW_TRY(zgeev(st, ws.PQ, ws.lam, ws.U, n, Zs, ws.P, out.status, p.wide_hess));
+        SCW_TRY(zgeev(st, ws.PQ, ws.lam, ws.U, n, Zs, ws.P, out.status, p.wide_hess, ws.gemm));
         L += 5;
     }
     roots_kernel<<<nblk((long long)n * Zs), 256, 0, st>>>(ws.lam, n, Zs, in.dz, k, out.gam, ws.E);
     SCW_CUDA_TRY(cudaGetLastError());
     // W = Q U Gamma^-1
-    SCW_TRY(zgemm(st, n, n, n, kOne, ws.Q, n, nn, ws.U, n, nn, kZero, ws.W, n, nn, Zs));
+    SCW_TRY(zgemm(st, n, n, n, kOne, ws.Q, n, nn, ws.U, n, nn, kZero, ws.W, n, nn, Zs, ws.gemm));
     coldiv_kernel<<<nblk(nn * Zs), 256, 0, st>>>(ws.W, n, out.gam, Zs);
     SCW_CUDA_TRY(cudaGetLastError());
     L += 8;
@@ -676,8 +681,8 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
         SCW_CUDA_TRY(cudaGetLastError());
         SCW_CUDA_TRY(cudaMemcpyAsync(ws.Q, which == 0 ? ws.U : ws.W, sizeof(double2) * nn * Zs,
                                      cudaMemcpyDeviceToDevice, st));
-        SCW_TRY(zgetrf(st, ws.Q, n, nn, ws.piv, n, out.status + (1 + which) * Zs, Zs, nullptr));
-        SCW_TRY(zgetrs(st, ws.Q, n, nn, ws.piv, n, inv, n, nn, Zs));
+        SCW_TRY(zgetrf(st, ws.Q, n, nn, ws.piv, n, out.status + (1 + which) * Zs, Zs, ws.gemm));
+        SCW_TRY(zgetrs(st, ws.Q, n, nn, ws.piv, n, inv, n, nn, Zs, ws.gemm));
         L += 2 + 3 * ((n + 31) / 32);
     }
     // T3 = Gd_0 Gc_static^-1 f3 = prod_l V_l diag(E_l^-1, E_l) V_l^-1 f3
@@ -685,12 +690,12 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
     SCW_CUDA_TRY(cudaGetLastError());
     for (int l = Zs - 1; l >= 0; l--) {
         const long long o = (long long)l * nn;
-        SCW_TRY(zgemm(st, n, M3, n, kOne, Uinv + o, n, 0, ws.X, M3, 0, kZero, ws.A1, M3, 0, 1));
-        SCW_TRY(zgemm(st, n, M3, n, kOne, Winv + o, n, 0, ws.X + (size_t)n * M3, M3, 0, kZero, ws.A2, M3, 0, 1));
+        SCW_TRY(zgemm(st, n, M3, n, kOne, Uinv + o, n, 0, ws.X, M3, 0, kZero, ws.A1, M3, 0, 1, ws.gemm));
+        SCW_TRY(zgemm(st, n, M3, n, kOne, Winv + o, n, 0, ws.X + (size_t)n * M3, M3, 0, kZero, ws.A2, M3, 0, 1, ws.gemm));
         mix_kernel<<<nblk((long long)n * M3), 256, 0, st>>>(ws.A1, ws.A2, ws.E + (size_t)l * n, n, M3, 0);
         SCW_CUDA_TRY(cudaGetLastError());
-        SCW_TRY(zgemm(st, n, M3, n, kOne, ws.U + o, n, 0, ws.A1, M3, 0, kZero, ws.X, M3, 0, 1));
-        SCW_TRY(zgemm(st, n, M3, n, kOne, ws.W + o, n, 0, ws.A2, M3, 0, kZero, ws.X + (size_t)n * M3, M3, 0, 1));
+        SCW_TRY(zgemm(st, n, M3, n, kOne, ws.U + o, n, 0, ws.A1, M3, 0, kZero, ws.X, M3, 0, 1, ws.gemm));
+        SCW_TRY(zgemm(st, n, M3, n, kOne, ws.W + o, n, 0, ws.A2, M3, 0, kZero, ws.X + (size_t)n * M3, M3, 0, 1, ws.gemm));
         L += 5;
     }
     // boundary system and its solve (sCWatter.cpp:393-461, 722)
@@ -698,8 +703,8 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
     SCW_CUDA_TRY(cudaGetLastError());
     bc_rhs_kernel<<<nblk(M6), 256, 0, st>>>(in.f1EF, MF, ws.b);
     SCW_CUDA_TRY(cudaGetLastError());
-    SCW_TRY(zgetrf(st, ws.A, M6, 0, ws.piv, 0, out.status + 3 * Zs, 1, nullptr));
-    SCW_TRY(zgetrs(st, ws.A, M6, 0, ws.piv, 0, ws.b, 1, 0, 1));
+    SCW_TRY(zgetrf(st, ws.A, M6, 0, ws.piv, 0, out.status + 3 * Zs, 1, ws.gemm));
+    SCW_TRY(zgetrs(st, ws.A, M6, 0, ws.piv, 0, ws.b, 1, 0, 1, ws.gemm));
     SCW_CUDA_TRY(cudaMemcpyAsync(out.x, ws.b, sizeof(double2) * M6, cudaMemcpyDeviceToDevice, st));
     L += 4 + 3 * ((M6 + 31) / 32);
     if (out.sepExt) {
@@ -723,12 +728,12 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
             SCW_CUDA_TRY(cudaMemcpyAsync(ws.A2, bp + n, sizeof(double2) * n, cudaMemcpyDeviceToDevice, st));
             mix_kernel<<<nblk(n), 256, 0, st>>>(ws.A1, ws.A2, ws.E + (size_t)(l - 1) * n, n, 1, 2);
             SCW_CUDA_TRY(cudaGetLastError());
-            SCW_TRY(zgemm(st, n, 1, n, kOne, ws.U + o - nn, n, 0, ws.A1, 1, 0, kZero, ws.v, 1, 0, 1));
-            SCW_TRY(zgemm(st, n, 1, n, kOne, ws.W + o - nn, n, 0, ws.A2, 1, 0, kZero, ws.v + n, 1, 0, 1));
+            SCW_TRY(zgemm(st, n, 1, n, kOne, ws.U + o - nn, n, 0, ws.A1, 1, 0, kZero, ws.v, 1, 0, 1, ws.gemm));
+            SCW_TRY(zgemm(st, n, 1, n, kOne, ws.W + o - nn, n, 0, ws.A2, 1, 0, kZero, ws.v + n, 1, 0, 1, ws.gemm));
             L += 3;
         }
-        SCW_TRY(zgemm(st, n, 1, n, kOne, Uinv + o, n, 0, ws.v, 1, 0, kZero, bl, 1, 0, 1));
-        SCW_TRY(zgemm(st, n, 1, n, kOne, Winv + o, n, 0, ws.v + n, 1, 0, kZero, bl + n, 1, 0, 1));
+        SCW_TRY(zgemm(st, n, 1, n, kOne, Uinv + o, n, 0, ws.v, 1, 0, kZero, bl, 1, 0, 1, ws.gemm));
+        SCW_TRY(zgemm(st, n, 1, n, kOne, Winv + o, n, 0, ws.v + n, 1, 0, kZero, bl + n, 1, 0, 1, ws.gemm));
         mix_kernel<<<nblk(n), 256, 0, st>>>(bl, bl + n, ws.E + (size_t)l * n, n, 1, 1);
         SCW_CUDA_TRY(cudaGetLastError());
         L += 3;
@@ -749,7 +754,7 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
                                                    p.pz ? ws.Hm : nullptr);
             SCW_CUDA_TRY(cudaGetLastError());
             if (p.pz) {
-                SCW_TRY(zgemm(st, MF, n, MF, kOne, ws.Kn, MF, 0, ws.Hm, n, 0, kZero, Qo + (size_t)n * n, n, 0, 1));
+                SCW_TRY(zgemm(st, MF, n, MF, kOne, ws.Kn, MF, 0, ws.Hm, n, 0, kZero, Qo + (size_t)n * n, n, 0, 1, ws.gemm));
             } else {
                 SCW_CUDA_TRY(cudaMemsetAsync(Qo + (size_t)n * n, 0, sizeof(double2) * MF * n, st));
             }
@@ -766,7 +771,7 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
                                                    p.pz ? ws.Hm : nullptr);
             SCW_CUDA_TRY(cudaGetLastError());
             if (p.pz) {
-                SCW_TRY(zgemm(st, MF, n, MF, kOne, ws.Kn, MF, 0, ws.Hm, n, 0, kZero, ws.Qtmp + (size_t)n * n, n, 0, 1));
+                SCW_TRY(zgemm(st, MF, n, MF, kOne, ws.Kn, MF, 0, ws.Hm, n, 0, kZero, ws.Qtmp + (size_t)n * n, n, 0, 1, ws.gemm));
             } else {
                 SCW_CUDA_TRY(cudaMemsetAsync(ws.Qtmp + (size_t)n * n, 0, sizeof(double2) * MF * n, st));
             }
@@ -875,6 +880,8 @@ scw_status scw_solve(scw_ctx ctx, const double* sample, int Zs, int Y, int X, co
         o.sepBeta = sol->dBeta;
     }
     cudaStream_t s = ctx->stream;
+    if ((st = scw::ctx_tc_flag(ctx)) != SCW_OK) return st;
+    ws.gemm.err = ctx->tc_err;
     if ((st = upload_inputs(p, sample, in, s)) != SCW_OK) return st;
     long long launches = 0;
     if ((st = record_solve(p, in, ws, o, s, &launches)) != SCW_OK) return st;
@@ -892,7 +899,7 @@ scw_status scw_solve(scw_ctx ctx, const double* sample, int Zs, int Y, int X, co
         SCW_CUDA_TRY(cudaMemcpyAsync(sol->eig_steps.data(), o.eig + Zs, sizeof(int) * Zs, cudaMemcpyDeviceToHost, s));
         SCW_CUDA_TRY(cudaMemcpyAsync(sol->eig_res.data(), o.eig_res, sizeof(double) * Zs, cudaMemcpyDeviceToHost, s));
     }
-    SCW_CUDA_TRY(cudaStreamSynchronize(s));
+    if ((st = scw_ctx_synchronize(ctx)) != SCW_OK) return st;
     ctx->launches += launches;
     const std::string msg = solve_status_message(status, Zs);
     if (!msg.empty()) return fail(SCW_ERR_NUMERIC, msg);
@@ -931,26 +938,28 @@ scw_status scw_layer_problem(scw_ctx ctx, const double* sample, int Zs, int Y, i
     carve_in(p, c, in);
     carve_ws(p, c, ws);
     cudaStream_t s = ctx->stream;
+    if ((st = scw::ctx_tc_flag(ctx)) != SCW_OK) return st;
+    ws.gemm.err = ctx->tc_err;
     if ((st = upload_inputs(p, sample, in, s)) != SCW_OK) return st;
     const int MF = p.MF, n = p.n;
     const long long nn = (long long)n * n, YX = (long long)Y * X;
     n2_kernel<<<nblk(Zs * YX), 256, 0, s>>>(in.data, YX, Zs, ws.F);
     SCW_CUDA_TRY(cudaGetLastError());
-    if ((st = scw::zgemm(s, X, p.M1, Y, kOne, ws.F, Y, YX, in.tw1, p.M1, 0, kZero, ws.T, p.M1, (long long)X * p.M1, 2 * Zs)) !=
+    if ((st = scw::zgemm(s, X, p.M1, Y, kOne, ws.F, Y, YX, in.tw1, p.M1, 0, kZero, ws.T, p.M1, (long long)X * p.M1, 2 * Zs, ws.gemm)) !=
         SCW_OK)
         return st;
     if ((st = scw::zgemm(s, p.M0, p.M1, X, make_double2(1.0 / (double)YX, 0.0), in.tw2, X, 0, ws.T, p.M1, (long long)X * p.M1,
-                    kZero, ws.coef, p.M1, MF, 2 * Zs)) != SCW_OK)
+                    kZero, ws.coef, p.M1, MF, 2 * Zs, ws.gemm)) != SCW_OK)
         return st;
     if (PQ) {
         build_pq_kernel<<<dim3(nblk(n), n, Zs), 256, 0, s>>>(ws.coef, in.up, in.wq, in.qs, in.ps, p.M0, p.M1, p.k, ws.P,
                                                               ws.Q);
         SCW_CUDA_TRY(cudaGetLastError());
-        if ((st = scw::zgemm(s, n, n, n, kOne, ws.P, n, nn, ws.Q, n, nn, kZero, (double2*)PQ, n, nn, Zs)) != SCW_OK) return st;
+        if ((st = scw::zgemm(s, n, n, n, kOne, ws.P, n, nn, ws.Q, n, nn, kZero, (double2*)PQ, n, nn, Zs, ws.gemm)) != SCW_OK) return st;
     }
     if (coef)
         SCW_CUDA_TRY(cudaMemcpyAsync(coef, ws.coef, sizeof(double2) * (size_t)Zs * 2 * MF, cudaMemcpyDeviceToDevice, s));
-    SCW_CUDA_TRY(cudaStreamSynchronize(s));
+    if ((st = scw_ctx_synchronize(ctx)) != SCW_OK) return st;
     ctx->launches += PQ ? 5 : 3;
     return SCW_OK;
 }

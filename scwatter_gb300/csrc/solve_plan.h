@@ -64,6 +64,7 @@ struct SolveWs {                            // scratch, reusable once the solve 
     double2 *F, *T, *X, *A1, *A2, *A, *b, *Kn, *Hm, *Qtmp;
     // mixed-precision eigen-solver: FP32 slots overlay P and W (free during the eigen-solve)
     mx::EigMixWs mix;
+    GemmWs gemm;                            // FP64 product operands; err: set by the caller
 };
 
 struct SolveOut {                           // results

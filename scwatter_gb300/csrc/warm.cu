@@ -353,6 +353,12 @@ scw_status scw_eig_warm(scw_ctx ctx, int n, const void* A_, int batch, const voi
     int* dup_of = (int*)take(sizeof(int) * (size_t)n * batch);
     long long* rep_ids = (long long*)take(sizeof(long long) * (size_t)n * batch);
     int* rep_excl = (int*)take(sizeof(int) * kMaxExcl * (size_t)n * batch);
+    // workspace of the FP64 products
+    scw::DevBuf gbuf;
+    const size_t gneed = scw::zgemm_ws_bytes(n, n, n, 1);
+    if ((s = gbuf.reserve(std::max(gneed, std::min(gneed * batch, scw::kGemmWsCap)))) != SCW_OK) return s;
+    if ((s = scw::ctx_tc_flag(ctx)) != SCW_OK) return s;
+    const scw::GemmWs gws{(char*)gbuf.ptr, gbuf.bytes, ctx->tc_err};
     // Hessenberg form and its norm
     SCW_CUDA_TRY(cudaMemcpyAsync(Hm, A, sizeof(double2) * nn * batch, cudaMemcpyDeviceToDevice, st));
     s = scw::zgehrd(st, Hm, Qm, n, batch, hw);
@@ -390,9 +396,9 @@ scw_status scw_eig_warm(scw_ctx ctx, int n, const void* A_, int batch, const voi
     int repairs = 0;
     for (int round = 0;; round++) {
         // back-transform V = Q X, residual against A, mode-count check
-        s = scw::zgemm(st, n, n, n, make_double2(1, 0), Qm, n, nn, Xm, n, nn, make_double2(0, 0), V, n, nn, batch);
+        s = scw::zgemm(st, n, n, n, make_double2(1, 0), Qm, n, nn, Xm, n, nn, make_double2(0, 0), V, n, nn, batch, gws);
         if (s != SCW_OK) return s;
-        s = scw::zgemm(st, n, n, n, make_double2(1, 0), A, n, nn, V, n, nn, make_double2(0, 0), AV, n, nn, batch);
+        s = scw::zgemm(st, n, n, n, make_double2(1, 0), A, n, nn, V, n, nn, make_double2(0, 0), AV, n, nn, batch, gws);
         if (s != SCW_OK) return s;
         SCW_CUDA_TRY(cudaMemsetAsync(worst, 0, sizeof(unsigned long long) * batch, st));
         SCW_CUDA_TRY(cudaMemsetAsync(dup, 0, sizeof(int) * batch, st));
@@ -457,7 +463,7 @@ scw_status scw_eig_warm(scw_ctx ctx, int n, const void* A_, int batch, const voi
         for (int i = 0; i < nr; i++)
             SCW_CUDA_TRY(cudaMemcpyAsync(FA + nn * i, A + nn * reject[i], sizeof(double2) * nn,
                                          cudaMemcpyDeviceToDevice, st));
-        if ((s = scw::zgeev(st, FA, FW, FV, n, nr, FWk, fst)) != SCW_OK) return s;
+        if ((s = scw::zgeev(st, FA, FW, FV, n, nr, FWk, fst, false, gws)) != SCW_OK) return s;
         for (int i = 0; i < nr; i++) {
             SCW_CUDA_TRY(cudaMemcpyAsync(V + nn * reject[i], FV + nn * i, sizeof(double2) * nn, cudaMemcpyDeviceToDevice, st));
             SCW_CUDA_TRY(cudaMemcpyAsync(W + (long long)n * reject[i], FW + (long long)n * i, sizeof(double2) * n,
@@ -470,6 +476,7 @@ scw_status scw_eig_warm(scw_ctx ctx, int n, const void* A_, int batch, const voi
         for (int v : hst)
             if (v) return fail(SCW_ERR_NUMERIC, "scw_eig_warm: the fallback eigen-solver did not converge");
     }
+    if ((s = scw_ctx_synchronize(ctx)) != SCW_OK) return s;
     ctx->launches += launches;
     if (stats_host) {
         double sum = 0;
