@@ -28,8 +28,8 @@ namespace z {
 // ------------------------------------------------------------------------------------
 // GEMM on the FP32 / FP64 pipes: C = alpha * op(A) * B + beta * C, op = identity.  64 x 64 tiles,
 // 256 threads, each thread a 4 x 4 complex block; K staged 16 at a time through shared memory.
-// FP32 products run here.  FP64 products run on the tensor cores (gemm_tc.cu, 20 to 35 times faster)
-// and come here only without a workspace: scw_zgemm while its stream is being captured.
+// FP64 products run on the tensor cores (gemm_tc.cu, 20 to 35 times faster) and come here only
+// without a workspace: scw_zgemm while its stream is being captured.
 // ------------------------------------------------------------------------------------
 constexpr int kGT = 64, kGK = 16;
 
@@ -93,114 +93,231 @@ gemm_kernel(int M, int N, int K, C alpha, const C* __restrict__ A, int lda, long
 }
 
 // ------------------------------------------------------------------------------------
-// LU with partial pivoting, blocked (panel width kNB), batched: one CTA per matrix for the
-// panel factorisation and the row-swap / triangular-solve kernels, batched GEMM for the
-// trailing update.  piv[k] = row swapped with row k at step k (LAPACK convention, 0-based).
-// info[b] = first zero pivot + 1 (0: nonsingular).
+// FP64 LU with partial pivoting, blocked, batched.  piv[k] = row swapped with row k at step k
+// (LAPACK convention, 0-based).  info[b] = first zero pivot + 1 (0: nonsingular).
+//
+// The panel is what is serial: per column a pivot search, a swap and a rank-1 update.  A
+// thread-block cluster of 8 CTAs holds the panel in shared memory, a slice of its rows in each.
+// Per column every CTA sends its best candidate with that row's values (and the owner of row k
+// that row) to all eight, so one cluster barrier per column decides the pivot and brings
+// everything the update needs; the candidate buffers alternate, so the next column's sends
+// cannot reach a CTA that still reads.  On one CTA with the panel in global memory a panel of 32
+// columns and 648 rows took 1.05 ms.  FP64 FMA (1.7 per SM and clock) bound the update, the barrier and
+// the search the rest.
 // ------------------------------------------------------------------------------------
 constexpr int kNB = 32;
+constexpr int kLuCtas = 8, kLuThreads = 256;
 
-template <typename C>
-__global__ void __launch_bounds__(512)
-lu_panel_kernel(C* __restrict__ A, int n, int lda, long long sA, int k0, int nb, int* __restrict__ piv, long long sP,
-                int* __restrict__ info) {
-    using R = typename CT<C>::R;
-    A += sA * blockIdx.x;
-    piv += sP * blockIdx.x;
-    __shared__ R red_v[16];
-    __shared__ int red_i[16];
-    __shared__ C pivrow[kNB];
-    for (int k = k0; k < k0 + nb; k++) {
-        // pivot search over rows k..n-1 of column k
-        R best = -1;
-        int bi = k;
-        for (int i = k + threadIdx.x; i < n; i += blockDim.x) {
-            const R v = cabs1(A[(long long)i * lda + k]);
-            if (v > best) {
-                best = v;
-                bi = i;
-            }
+struct LuSlot {
+    double val;
+    int row, pad;
+    double2 v[kNB];
+};
+
+__global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuThreads)
+lu_panel_kernel(double2* __restrict__ A, int n, int lda, long long sA, int k0, int nb, int rows, int* __restrict__ piv,
+                long long sP, int* __restrict__ info, const int* __restrict__ skip) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank(), b = blockIdx.x / kLuCtas;
+    if (skipped(skip, b)) return;                        // the whole cluster, before any barrier
+    A += sA * b;
+    piv += sP * b;
+    extern __shared__ __align__(16) unsigned char lu_smem[];
+    LuSlot* slot = reinterpret_cast<LuSlot*>(lu_smem);   // [2][kLuCtas]: candidates of column parity
+    LuSlot* krow = slot + 2 * kLuCtas;                   // [2]: row k
+    double2* P = reinterpret_cast<double2*>(krow + 2);   // [rows][nb + 1]
+    const int ld = nb + 1;
+    __shared__ double red_v[kLuThreads / 32];
+    __shared__ int red_i[kLuThreads / 32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int g0 = k0 + rank * rows;                     // this CTA's rows g0 .. g0 + nr - 1
+    const int nr = max(0, min(rows, n - g0));
+    for (int e = tid; e < nr * nb; e += kLuThreads) {
+        const int r = e / nb, c = e - r * nb;
+        P[r * ld + c] = A[(long long)(g0 + r) * lda + k0 + c];
+    }
+    __syncthreads();
+    const int sub = tid & 1;                             // two threads per row
+    double best = -1.0;
+    int bi = 0x7fffffff;
+    for (int r = tid >> 1; r < nr; r += kLuThreads / 2) {
+        const double v = cabs1(P[r * ld]);
+        if (sub == 0 && v > best) {
+            best = v;
+            bi = g0 + r;
         }
-        // arg-max (largest |a|, then smallest row): butterfly within each warp, then over the
-        // warps' winners
+    }
+    cluster.sync();                                      // every CTA runs before the first remote write
+    for (int j = 0; j < nb; j++) {
+        const int k = k0 + j, par = j & 1;
+        // this CTA's candidate: largest |a|, then smallest row
         for (int o = 16; o > 0; o >>= 1) {
-            const R ov = __shfl_xor_sync(0xffffffffu, best, o);
+            const double ov = __shfl_xor_sync(0xffffffffu, best, o);
             const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
             if (ov > best || (ov == best && oi < bi)) {
                 best = ov;
                 bi = oi;
             }
         }
-        if ((threadIdx.x & 31) == 0) {
-            red_v[threadIdx.x >> 5] = best;
-            red_i[threadIdx.x >> 5] = bi;
+        if (lane == 0) {
+            red_v[warp] = best;
+            red_i[warp] = bi;
         }
         __syncthreads();
-        R pv = red_v[0];
-        int p = red_i[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++)
-            if (red_v[w] > pv || (red_v[w] == pv && red_i[w] < p)) {
-                pv = red_v[w];
-                p = red_i[w];
+        best = red_v[0];
+        bi = red_i[0];
+#pragma unroll
+        for (int w = 1; w < kLuThreads / 32; w++)
+            if (red_v[w] > best || (red_v[w] == best && red_i[w] < bi)) {
+                best = red_v[w];
+                bi = red_i[w];
             }
-        const bool zero = pv == 0;
-        if (threadIdx.x == 0) {
+        // warp w sends to CTA w: the candidate with its row, and row k from its owner
+        {
+            LuSlot* dst = cluster.map_shared_rank(slot, warp) + par * kLuCtas + rank;
+            const bool own = bi >= g0 && bi < g0 + nr;
+            if (own && lane < nb) dst->v[lane] = P[(bi - g0) * ld + lane];
+            if (lane == 0) {
+                dst->val = own ? best : -1.0;
+                dst->row = own ? bi : 0x7fffffff;
+            }
+            if (k >= g0 && k < g0 + nr) {
+                LuSlot* dk = cluster.map_shared_rank(krow, warp) + par;
+                if (lane < nb) dk->v[lane] = P[(k - g0) * ld + lane];
+            }
+        }
+        cluster.sync();
+        const LuSlot* cand = slot + par * kLuCtas;
+        double pv = cand[0].val;
+        int p = cand[0].row, pr = 0;
+#pragma unroll
+        for (int w = 1; w < kLuCtas; w++)
+            if (cand[w].val > pv || (cand[w].val == pv && cand[w].row < p)) {
+                pv = cand[w].val;
+                p = cand[w].row;
+                pr = w;
+            }
+        const bool none = pv < 0.0;                      // no comparable value (all NaN): row k stays
+        if (none) p = k;
+        const double2* prow = none ? krow[par].v : cand[pr].v;
+        const bool zero = pv == 0.0;
+        if (rank == 0 && tid == 0) {
             piv[k] = p;
-            if (zero && info[blockIdx.x] == 0) info[blockIdx.x] = k + 1;
+            if (zero && info[b] == 0) info[b] = k + 1;
         }
-        // swap rows k and p inside the panel columns k0 .. k0+nb-1
-        if (p != k) {
-            for (int j = k0 + threadIdx.x; j < k0 + nb; j += blockDim.x) {
-                const C t = A[(long long)k * lda + j];
-                A[(long long)k * lda + j] = A[(long long)p * lda + j];
-                A[(long long)p * lda + j] = t;
+        if (warp == 0 && p != k) {
+            if (p >= g0 && p < g0 + nr && lane < nb) P[(p - g0) * ld + lane] = krow[par].v[lane];
+            if (k >= g0 && k < g0 + nr && lane < nb) P[(k - g0) * ld + lane] = prow[lane];
+        }
+        __syncthreads();
+        // scale the column below the pivot, update the remaining panel columns, search the next one
+        const double2 inv = zero ? make_double2(0.0, 0.0) : cdiv(make_double2(1.0, 0.0), prow[j]);
+        best = -1.0;
+        bi = 0x7fffffff;
+        for (int rb = max(0, k + 1 - g0); rb < nr; rb += kLuThreads / 2) {
+            const int r = rb + (tid >> 1);
+            const bool live = r < nr;
+            double2* row = P + (live ? r : 0) * ld;
+            const double2 l = live ? cmul(row[j], inv) : make_double2(0.0, 0.0);
+            for (int c = j + 1 + sub; live && c < nb; c += 2) {
+                const double2 v = csub(row[c], cmul(l, prow[c]));
+                row[c] = v;
+                if (c == j + 1) {
+                    const double a = cabs1(v);
+                    if (a > best) {
+                        best = a;
+                        bi = g0 + r;
+                    }
+                }
             }
+            __syncwarp();                                // both threads of the row have read row[j]
+            if (live && sub == 0) row[j] = l;
         }
         __syncthreads();
-        const C d = A[(long long)k * lda + k];
-        for (int j = k + 1 + threadIdx.x; j < k0 + nb; j += blockDim.x) pivrow[j - k0] = A[(long long)k * lda + j];
-        __syncthreads();
-        // scale the column below the pivot and update the remaining panel columns
-        const C inv = zero ? CT<C>::mk(0, 0) : cdiv(CT<C>::mk(1, 0), d);
-        for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x) {
-            C* row = A + (long long)i * lda;
-            const C l = cmul(row[k], inv);
-            row[k] = l;
-            for (int j = k + 1; j < k0 + nb; j++) row[j] = csub(row[j], cmul(l, pivrow[j - k0]));
-        }
-        __syncthreads();
+    }
+    for (int e = tid; e < nr * nb; e += kLuThreads) {
+        const int r = e / nb, c = e - r * nb;
+        A[(long long)(g0 + r) * lda + k0 + c] = P[r * ld + c];
     }
 }
 
-// apply the panel's swaps to the columns outside the panel, then solve L11 U12 = A12
-template <typename C>
+// The panel's row interchanges on the columns outside it, then L11 U12 = A12 on the columns right of
+// it, 32 columns per CTA.  The interchanges touch at most 64 rows: warp 0 follows them to the rows'
+// sources (lane i: the source of row k0 + i, and a row below the panel that was exchanged with
+// one of the panel), so that all rows are read at once and then written.
 __global__ void __launch_bounds__(256)
-lu_swap_trsm_kernel(C* __restrict__ A, int n, int lda, long long sA, int k0, int nb, const int* __restrict__ piv,
-                    long long sP) {
+lu_apply_kernel(double2* __restrict__ A, int ncols, int lda, long long sA, int k0, int nb, const int* __restrict__ piv,
+                long long sP, const int* __restrict__ skip) {
+    if (skipped(skip, blockIdx.y)) return;
     A += sA * blockIdx.y;
     piv += sP * blockIdx.y;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;    // one column per thread
-    if (j >= n || (j >= k0 && j < k0 + nb)) return;
-    for (int k = k0; k < k0 + nb; k++) {
-        const int p = piv[k];
-        if (p != k) {
-            const C t = A[(long long)k * lda + j];
-            A[(long long)k * lda + j] = A[(long long)p * lda + j];
-            A[(long long)p * lda + j] = t;
+    __shared__ double2 X[kNB][33], L[kNB][33];
+    __shared__ int s_top[kNB], s_row[kNB], s_src[kNB];
+    const int tid = threadIdx.x, lane = tid & 31, c = lane, j = blockIdx.x * 32 + c;
+    if (tid < 32) {
+        int top = k0 + lane, orow = -1, osrc = -1;
+        const int mine = lane < nb ? piv[k0 + lane] : 0;
+        for (int i = 0; i < nb; i++) {
+            const int p = __shfl_sync(0xffffffffu, mine, i), a = __shfl_sync(0xffffffffu, top, i);
+            const unsigned hit = __ballot_sync(0xffffffffu, orow == p);
+            const int t = p < k0 + nb ? p - k0 : 0, bt = __shfl_sync(0xffffffffu, top, t);
+            const int q = hit ? __ffs(hit) - 1 : i, cur = __shfl_sync(0xffffffffu, osrc, q);
+            if (p < k0 + nb) {
+                if (lane == i) top = bt;
+                else if (lane == t) top = a;
+            } else {
+                if (lane == i) top = hit ? cur : p;
+                if (lane == q) {
+                    orow = p;
+                    osrc = a;
+                }
+            }
         }
+        s_top[lane] = top;
+        s_row[lane] = orow;
+        s_src[lane] = osrc;
     }
-    if (j < k0 + nb) return;                                // columns left of the panel: swaps only
-    for (int k = k0; k < k0 + nb; k++) {                    // unit lower triangular solve
-        C v = A[(long long)k * lda + j];
-        for (int m = k0; m < k; m++) v = csub(v, cmul(A[(long long)k * lda + m], A[(long long)m * lda + j]));
-        A[(long long)k * lda + j] = v;
+    const bool live = j < ncols && !(j >= k0 && j < k0 + nb), right = live && j >= k0 + nb;
+    __syncthreads();
+    double2 o[kNB / 8];
+#pragma unroll
+    for (int q = 0; q < kNB / 8; q++) {
+        const int r = (tid >> 5) + 8 * q;
+        o[q] = make_double2(0.0, 0.0);
+        if (live && r < nb) {
+            X[r][c] = A[(long long)s_top[r] * lda + j];
+            if (s_row[r] >= 0) o[q] = A[(long long)s_src[r] * lda + j];
+        }
+        if (r < nb && c < nb) L[r][c] = A[(long long)(k0 + r) * lda + k0 + c];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kNB / 8; q++) {
+        const int r = (tid >> 5) + 8 * q;
+        if (live && r < nb && s_row[r] >= 0) A[(long long)s_row[r] * lda + j] = o[q];
+    }
+    const int steps = blockIdx.x * 32 + 31 >= k0 + nb ? nb - 1 : 0;      // left of the panel: interchanges only
+    for (int m = 0; m < steps; m++) {
+#pragma unroll
+        for (int q = 0; q < kNB / 8; q++) {
+            const int r = (tid >> 5) + 8 * q;
+            if (right && r > m && r < nb) X[r][c] = csub(X[r][c], cmul(L[r][m], X[m][c]));
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int q = 0; q < kNB / 8; q++) {
+        const int r = (tid >> 5) + 8 * q;
+        if (live && r < nb) A[(long long)(k0 + r) * lda + j] = X[r][c];
     }
 }
 
 // Row interchanges of B from getrf's pivots (LAPACK laswp order), one thread per column.
-template <typename C>
 __global__ void __launch_bounds__(256)
-laswp_kernel(const int* __restrict__ piv, long long sP, C* __restrict__ B, int ldb, long long sB, int n, int nrhs) {
+laswp_kernel(const int* __restrict__ piv, long long sP, double2* __restrict__ B, int ldb, long long sB, int n, int nrhs,
+             const int* __restrict__ skip) {
+    if (skipped(skip, blockIdx.y)) return;
     piv += sP * blockIdx.y;
     B += sB * blockIdx.y;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -208,38 +325,49 @@ laswp_kernel(const int* __restrict__ piv, long long sP, C* __restrict__ B, int l
     for (int k = 0; k < n; k++) {
         const int p = piv[k];
         if (p != k) {
-            const C t = B[(long long)k * ldb + j];
+            const double2 t = B[(long long)k * ldb + j];
             B[(long long)k * ldb + j] = B[(long long)p * ldb + j];
             B[(long long)p * ldb + j] = t;
         }
     }
 }
 
-// Triangular solve restricted to the diagonal block rows [k0, k0 + nb) of the LU factors, one
-// thread per right-hand-side column: unit lower L (upper == 0) or U (upper == 1).  Rows
-// outside the block were already folded in by the GEMM updates of the blocked solve.
-template <typename C>
+// Triangular solve restricted to the diagonal block rows [k0, k0 + nb) of the LU factors, 32
+// right-hand-side columns per CTA in shared memory: unit lower L (upper == 0) or U (upper == 1).
+// Rows outside the block were already folded in by the GEMM updates of the blocked solve.
 __global__ void __launch_bounds__(256)
-trsm_block_kernel(const C* __restrict__ LU, int lda, long long sA, int k0, int nb, C* __restrict__ B, int ldb,
-                  long long sB, int nrhs, int upper) {
+trsm_block_kernel(const double2* __restrict__ LU, int lda, long long sA, int k0, int nb, double2* __restrict__ B, int ldb,
+                  long long sB, int nrhs, int upper, const int* __restrict__ skip) {
+    if (skipped(skip, blockIdx.y)) return;
     LU += sA * blockIdx.y;
     B += sB * blockIdx.y;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nrhs) return;
-    if (!upper) {
-        for (int i = k0; i < k0 + nb; i++) {
-            C v = B[(long long)i * ldb + j];
-            const C* row = LU + (long long)i * lda;
-            for (int m = k0; m < i; m++) v = csub(v, cmul(row[m], B[(long long)m * ldb + j]));
-            B[(long long)i * ldb + j] = v;
+    __shared__ double2 X[kNB][33], L[kNB][33];
+    const int tid = threadIdx.x, c = tid & 31, w = tid >> 5, j = blockIdx.x * 32 + c;
+    const bool live = j < nrhs;
+#pragma unroll
+    for (int q = 0; q < kNB / 8; q++) {
+        const int r = w + 8 * q;
+        if (r < nb && live) X[r][c] = B[(long long)(k0 + r) * ldb + j];
+        if (r < nb && c < nb) L[r][c] = LU[(long long)(k0 + r) * lda + k0 + c];
+    }
+    __syncthreads();
+    for (int s = 0; s < nb; s++) {
+        const int m = upper ? nb - 1 - s : s;
+        if (upper) {
+            if (w == 0 && live) X[m][c] = cdiv(X[m][c], L[m][m]);
+            __syncthreads();
         }
-    } else {
-        for (int i = k0 + nb - 1; i >= k0; i--) {
-            C v = B[(long long)i * ldb + j];
-            const C* row = LU + (long long)i * lda;
-            for (int m = i + 1; m < k0 + nb; m++) v = csub(v, cmul(row[m], B[(long long)m * ldb + j]));
-            B[(long long)i * ldb + j] = cdiv(v, row[i]);
+#pragma unroll
+        for (int q = 0; q < kNB / 8; q++) {
+            const int r = w + 8 * q;
+            if (live && r < nb && (upper ? r < m : r > m)) X[r][c] = csub(X[r][c], cmul(L[r][m], X[m][c]));
         }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int q = 0; q < kNB / 8; q++) {
+        const int r = w + 8 * q;
+        if (r < nb && live) B[(long long)(k0 + r) * ldb + j] = X[r][c];
     }
 }
 
@@ -933,9 +1061,10 @@ hqr_cluster_kernel(C* __restrict__ H, C* __restrict__ Z, int n, long long sA, C*
 }
 
 // ------------------------------------------------------------------------------------
-// Eigenvectors of the upper triangular Schur factor T (ztrevc semantics, right vectors):
-// X[:, k] solves (T - T_kk I) x = 0 with x_k = 1, x_i = 0 for i > k.  One warp per vector.
-// X is written row-major (column k = eigenvector k).
+// Eigenvectors of the upper triangular Schur factor T (ztrevc semantics, right vectors): vector k
+// solves (T - T_kk I) x = 0 with x_k = 1, x_i = 0 for i > k.  One warp per vector.
+// Vector k is written as row k of X (contiguous for the warp that builds it; the product with the
+// Schur vectors reads X transposed).
 // FP64: a denominator T_ii - T_kk below smin is replaced by smin, as ztrevc does.  FP32 (the
 // first stage of the mixed solver): where both the denominator and the coupling sum
 // sum_j T_ij x_j are within 16 ulp of max |T_jj|, the pair counts as one degenerate eigenvalue and
@@ -946,6 +1075,15 @@ hqr_cluster_kernel(C* __restrict__ H, C* __restrict__ Z, int n, long long sA, C*
 // (n = 3200 layers) could not remove.
 // ------------------------------------------------------------------------------------
 template <typename C>
+__device__ __forceinline__ C warp_sum(C s) {
+    for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    return s;
+}
+
+template <typename C>
 __global__ void __launch_bounds__(256)
 trevc_kernel(const C* __restrict__ T, C* __restrict__ X, int n, long long sA, const int* __restrict__ skip) {
     using R = typename CT<C>::R;
@@ -953,10 +1091,11 @@ trevc_kernel(const C* __restrict__ T, C* __restrict__ X, int n, long long sA, co
     if (skipped(skip, blockIdx.y)) return;
     T += sA * blockIdx.y;
     X += sA * blockIdx.y;
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    // the longest vectors first: the last warps of the grid are short
+    const int k = n - 1 - (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
-    if (warp >= n) return;
-    const int k = warp;
+    if (k < 0) return;
+    C* x = X + (long long)k * n;
     const R ulp = CT<C>::ulp;
     const C lam = T[(long long)k * n + k];
     const R smin = r_max(ulp * cabs1(lam), CT<C>::safmin * ((R)n / ulp));
@@ -967,37 +1106,50 @@ trevc_kernel(const C* __restrict__ T, C* __restrict__ X, int n, long long sA, co
         deg *= R(16) * ulp;
     }
     // x_k = 1, x_{k+1..} = 0
-    for (int i = lane; i < n; i += 32) X[(long long)i * n + k] = CT<C>::mk(i == k ? 1 : 0, 0);
+    for (int i = lane; i < n; i += 32) x[i] = CT<C>::mk(i == k ? 1 : 0, 0);
     __syncwarp();
     for (int i = k - 1; i >= 0; i--) {
         // x_i = -(sum_{j=i+1..k} T_ij x_j) / (T_ii - lam)
+        const C* row = T + (long long)i * n;
         C s = CT<C>::mk(0, 0);
-        for (int j = i + 1 + lane; j <= k; j += 32) s = cfma(T[(long long)i * n + j], X[(long long)j * n + k], s);
-        for (int o = 16; o > 0; o >>= 1) {
-            s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-            s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-        }
+#pragma unroll 4
+        for (int j = i + 1 + lane; j <= k; j += 32) s = cfma(row[j], x[j], s);
+        s = warp_sum(s);
         if (lane == 0) {
-            C d = csub(T[(long long)i * n + i], lam);
+            C d = csub(row[i], lam);
             if (kDegenerateSkip && cabs1(d) <= deg && cabs1(s) <= deg) {
-                X[(long long)i * n + k] = CT<C>::mk(0, 0);
+                x[i] = CT<C>::mk(0, 0);
             } else {
                 if (cabs1(d) < smin) d = CT<C>::mk(smin, 0);
-                X[(long long)i * n + k] = cdiv(CT<C>::mk(-s.x, -s.y), d);
+                x[i] = cdiv(CT<C>::mk(-s.x, -s.y), d);
             }
         }
         __syncwarp();
     }
 }
 
-// copy of the batch entries that are not skipped
+// Inverse Z of a unit upper triangular matrix given by its columns (column j = row j of X): row r of
+// Z X = I is z_r = 1, z_j = -sum_{i=r..j-1} z_i X_ij.  One warp per row.
 template <typename C>
-__global__ void copy_kernel(const C* __restrict__ src, C* __restrict__ dst, long long count, const int* __restrict__ skip) {
-    if (skipped(skip, blockIdx.y)) return;
-    src += count * blockIdx.y;
-    dst += count * blockIdx.y;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x)
-        dst[i] = src[i];
+__global__ void __launch_bounds__(256)
+trtri_kernel(const C* __restrict__ X, C* __restrict__ Z, int n, long long sA) {
+    X += sA * blockIdx.y;
+    Z += sA * blockIdx.y;
+    const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (r >= n) return;
+    C* z = Z + (long long)r * n;
+    for (int j = lane; j <= r; j += 32) z[j] = CT<C>::mk(j == r ? 1 : 0, 0);
+    __syncwarp();
+    for (int j = r + 1; j < n; j++) {
+        const C* col = X + (long long)j * n;
+        C s = CT<C>::mk(0, 0);
+#pragma unroll 4
+        for (int i = r + lane; i < j; i += 32) s = cfma(z[i], col[i], s);
+        s = warp_sum(s);
+        if (lane == 0) z[j] = CT<C>::mk(-s.x, -s.y);
+        __syncwarp();
+    }
 }
 
 }  // namespace z
@@ -1015,75 +1167,80 @@ scw_status gemm(cudaStream_t st, int M, int N, int K, C alpha, const C* A, int l
     return SCW_OK;
 }
 
-// The products inside the factorisations: FP64 on the tensor cores (gemm_tc.cu), FP32 by gemm_kernel
-template <typename C>
-static scw_status mm(cudaStream_t st, int M, int N, int K, C alpha, const C* A, int lda, long long sA, const C* B, int ldb,
-                     long long sB, C beta, C* Cm, int ldc, long long sC, int batch, const GemmWs& ws,
-                     const int* skip = nullptr) {
-    if constexpr (sizeof(C) == sizeof(double2))
-        return zgemm(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, Cm, ldc, sC, batch, ws, skip);
-    else
-        return gemm<C>(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, Cm, ldc, sC, batch, skip);
-}
-
-template <typename C>
-scw_status getrf(cudaStream_t st, C* A, int n, long long sA, int* piv, long long sP, int* info, int batch,
-                 const GemmWs& ws) {
+scw_status zgetrf(cudaStream_t st, double2* A, int n, int ncols, int lda, long long sA, int* piv, long long sP, int* info,
+                  int batch, const GemmWs& ws, const int* skip) {
     if (n <= 0 || batch <= 0) return SCW_OK;
     SCW_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(int) * batch, st));
-    const C one = {1, 0}, minus = {-1, 0};
-    for (int k0 = 0; k0 < n; k0 += z::kNB) {
-        const int nb = std::min(z::kNB, n - k0);
-        z::lu_panel_kernel<C><<<batch, 512, 0, st>>>(A, n, n, sA, k0, nb, piv, sP, info);
+    // panel width: as many columns as the cluster's shared memory holds of the first panel
+    constexpr size_t kLimit = 220 * 1024, kSlots = sizeof(z::LuSlot) * (2 * z::kLuCtas + 2);
+    auto smem_of = [](int rows, int nb) { return kSlots + sizeof(double2) * (size_t)rows * (nb + 1); };
+    auto rows_of = [&](int k0) { return (n - k0 + z::kLuCtas - 1) / z::kLuCtas; };
+    int width = z::kNB;
+    while (width > 1 && smem_of(rows_of(0), width) > kLimit) width /= 2;
+    if (smem_of(rows_of(0), width) > kLimit) return fail(SCW_ERR_ARG, "getrf: matrix too large");
+    SCW_CUDA_TRY(cudaFuncSetAttribute(z::lu_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLimit));
+    const double2 one = {1, 0}, minus = {-1, 0};
+    for (int k0 = 0; k0 < n; k0 += width) {
+        const int nb = std::min(width, n - k0), rows = rows_of(k0);
+        z::lu_panel_kernel<<<z::kLuCtas * batch, z::kLuThreads, smem_of(rows, nb), st>>>(A, n, lda, sA, k0, nb, rows, piv,
+                                                                                      sP, info, skip);
         SCW_CUDA_TRY(cudaGetLastError());
-        dim3 g2((n + 255) / 256, batch);
-        z::lu_swap_trsm_kernel<C><<<g2, 256, 0, st>>>(A, n, n, sA, k0, nb, piv, sP);
-        SCW_CUDA_TRY(cudaGetLastError());
+        if (ncols > nb) {
+            z::lu_apply_kernel<<<dim3((ncols + 31) / 32, batch), 256, 0, st>>>(A, ncols, lda, sA, k0, nb, piv, sP, skip);
+            SCW_CUDA_TRY(cudaGetLastError());
+        }
         const int rem = n - k0 - nb;
         if (rem > 0) {
             // A22 -= L21 U12
-            scw_status s = mm<C>(st, rem, rem, nb, minus, A + (long long)(k0 + nb) * n + k0, n, sA,
-                                 A + (long long)k0 * n + k0 + nb, n, sA, one, A + (long long)(k0 + nb) * n + k0 + nb,
-                                 n, sA, batch, ws);
+            scw_status s = zgemm(st, rem, ncols - k0 - nb, nb, minus, A + (long long)(k0 + nb) * lda + k0, lda, sA,
+                                 A + (long long)k0 * lda + k0 + nb, lda, sA, one,
+                                 A + (long long)(k0 + nb) * lda + k0 + nb, lda, sA, batch, ws, skip);
             if (s != SCW_OK) return s;
         }
     }
     return SCW_OK;
 }
 
-template <typename C>
-scw_status getrs(cudaStream_t st, const C* LU, int n, long long sA, const int* piv, long long sP, C* B, int nrhs,
-                 long long sB, int batch, const GemmWs& ws) {
+scw_status ztrsm_upper(cudaStream_t st, const double2* LU, int n, int lda, long long sA, double2* B, int nrhs, int ldb,
+                       long long sB, int batch, const GemmWs& ws, const int* skip) {
     // blocked: per diagonal block a small triangular solve, the rest of the rows updated by GEMM
     if (n <= 0 || nrhs <= 0 || batch <= 0) return SCW_OK;
-    constexpr int kTB = 64;
-    const C one = {1, 0}, minus = {-1, 0};
-    const dim3 g((nrhs + 255) / 256, batch);
-    z::laswp_kernel<C><<<g, 256, 0, st>>>(piv, sP, B, nrhs, sB, n, nrhs);
-    SCW_CUDA_TRY(cudaGetLastError());
-    for (int k0 = 0; k0 < n; k0 += kTB) {
-        const int nb = std::min(kTB, n - k0);
-        z::trsm_block_kernel<C><<<g, 256, 0, st>>>(LU, n, sA, k0, nb, B, nrhs, sB, nrhs, 0);
-        SCW_CUDA_TRY(cudaGetLastError());
-        const int rem = n - k0 - nb;
-        if (rem > 0) {
-            scw_status s = mm<C>(st, rem, nrhs, nb, minus, LU + (long long)(k0 + nb) * n + k0, n, sA,
-                                 B + (long long)k0 * nrhs, nrhs, sB, one, B + (long long)(k0 + nb) * nrhs, nrhs, sB,
-                                 batch, ws);
-            if (s != SCW_OK) return s;
-        }
-    }
+    constexpr int kTB = z::kNB;
+    const double2 one = {1, 0}, minus = {-1, 0};
+    const dim3 g((nrhs + 31) / 32, batch);
     for (int k0 = ((n - 1) / kTB) * kTB; k0 >= 0; k0 -= kTB) {
         const int nb = std::min(kTB, n - k0);
-        z::trsm_block_kernel<C><<<g, 256, 0, st>>>(LU, n, sA, k0, nb, B, nrhs, sB, nrhs, 1);
+        z::trsm_block_kernel<<<g, 256, 0, st>>>(LU, lda, sA, k0, nb, B, ldb, sB, nrhs, 1, skip);
         SCW_CUDA_TRY(cudaGetLastError());
         if (k0 > 0) {
-            scw_status s = mm<C>(st, k0, nrhs, nb, minus, LU + k0, n, sA, B + (long long)k0 * nrhs, nrhs, sB, one, B,
-                                 nrhs, sB, batch, ws);
+            scw_status s = zgemm(st, k0, nrhs, nb, minus, LU + k0, lda, sA, B + (long long)k0 * ldb, ldb, sB, one, B, ldb,
+                                 sB, batch, ws, skip);
             if (s != SCW_OK) return s;
         }
     }
     return SCW_OK;
+}
+
+scw_status zgetrs(cudaStream_t st, const double2* LU, int n, long long sA, const int* piv, long long sP, double2* B,
+                  int nrhs, long long sB, int batch, const GemmWs& ws, const int* skip) {
+    if (n <= 0 || nrhs <= 0 || batch <= 0) return SCW_OK;
+    constexpr int kTB = z::kNB;
+    const double2 one = {1, 0}, minus = {-1, 0};
+    z::laswp_kernel<<<dim3((nrhs + 255) / 256, batch), 256, 0, st>>>(piv, sP, B, nrhs, sB, n, nrhs, skip);
+    SCW_CUDA_TRY(cudaGetLastError());
+    for (int k0 = 0; k0 < n; k0 += kTB) {
+        const int nb = std::min(kTB, n - k0);
+        z::trsm_block_kernel<<<dim3((nrhs + 31) / 32, batch), 256, 0, st>>>(LU, n, sA, k0, nb, B, nrhs, sB, nrhs, 0, skip);
+        SCW_CUDA_TRY(cudaGetLastError());
+        const int rem = n - k0 - nb;
+        if (rem > 0) {
+            scw_status s = zgemm(st, rem, nrhs, nb, minus, LU + (long long)(k0 + nb) * n + k0, n, sA,
+                                 B + (long long)k0 * nrhs, nrhs, sB, one, B + (long long)(k0 + nb) * nrhs, nrhs, sB,
+                                 batch, ws, skip);
+            if (s != SCW_OK) return s;
+        }
+    }
+    return ztrsm_upper(st, LU, n, n, sA, B, nrhs, nrhs, sB, batch, ws, skip);
 }
 
 scw_status zgehrd(cudaStream_t st, double2* A, double2* Q, int n, int batch, double2* work) {
@@ -1166,14 +1323,9 @@ static scw_status hqr_launch(cudaStream_t st, C* A, C* Q, int n, long long nn, C
 }
 
 template <typename C>
-scw_status geev(cudaStream_t st, C* A, C* W, C* V, int n, int batch, C* work, int* status, const int* skip,
-                bool wide, const GemmWs& ws) {
-    // A (overwritten): n x n per batch entry; W: n eigenvalues; V: n x n right eigenvectors (columns)
-    // work: >= batch * (n*n + 3 n) elements
+scw_status schur(cudaStream_t st, C* A, C* Q, C* W, int n, int batch, C* hw, int* status, const int* skip, bool wide) {
     if (n <= 0 || batch <= 0) return SCW_OK;
     const long long nn = (long long)n * n;
-    C* Q = work;                             // batch * n * n: Schur vectors
-    C* hw = work + nn * batch;               // batch * 3n
     SCW_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int) * batch, st));
     // single solves outside a stream capture count the matrices the skip mask leaves (and do
     // nothing when it leaves none)
@@ -1196,32 +1348,49 @@ scw_status geev(cudaStream_t st, C* A, C* W, C* V, int n, int batch, C* work, in
         z::hessenberg_kernel<C><<<batch, 1024, 0, st>>>(A, Q, n, nn, hw, skip);
         SCW_CUDA_TRY(cudaGetLastError());
     }
-    {
-        scw_status s = hqr_launch<C>(st, A, Q, n, nn, W, status, skip, batch, active, wide);
-        if (s != SCW_OK) return s;
-    }
-    // X (triangular eigenvectors) into V, then A := Q X, copied to V
-    dim3 gt((n * 32 + 255) / 256, batch);
-    z::trevc_kernel<C><<<gt, 256, 0, st>>>(A, V, n, nn, skip);
-    SCW_CUDA_TRY(cudaGetLastError());
-    const C one = {1, 0}, zero = {0, 0};
-    scw_status s = mm<C>(st, n, n, n, one, Q, n, nn, V, n, nn, zero, A, n, nn, batch, ws, skip);
-    if (s != SCW_OK) return s;
-    z::copy_kernel<C><<<dim3((unsigned)std::min<long long>((nn + 255) / 256, 4096), batch), 256, 0, st>>>(A, V, nn, skip);
+    return hqr_launch<C>(st, A, Q, n, nn, W, status, skip, batch, active, wide);
+}
+
+template <typename C>
+scw_status trevc(cudaStream_t st, const C* T, C* X, int n, int batch, const int* skip) {
+    z::trevc_kernel<C><<<dim3((n * 32 + 255) / 256, batch), 256, 0, st>>>(T, X, n, (long long)n * n, skip);
     SCW_CUDA_TRY(cudaGetLastError());
     return SCW_OK;
 }
 
-#define SCW_DENSE_INSTANTIATE(C)                                                                                    \
-    template scw_status gemm<C>(cudaStream_t, int, int, int, C, const C*, int, long long, const C*, int, long long, \
-                                C, C*, int, long long, int, const int*);                                           \
-    template scw_status getrf<C>(cudaStream_t, C*, int, long long, int*, long long, int*, int, const GemmWs&);     \
-    template scw_status getrs<C>(cudaStream_t, const C*, int, long long, const int*, long long, C*, int, long long, \
-                                 int, const GemmWs&);                                                              \
-    template scw_status geev<C>(cudaStream_t, C*, C*, C*, int, int, C*, int*, const int*, bool, const GemmWs&);
-SCW_DENSE_INSTANTIATE(double2)
-SCW_DENSE_INSTANTIATE(float2)
-#undef SCW_DENSE_INSTANTIATE
+scw_status trtri32(cudaStream_t st, const float2* X, float2* Z, int n, int batch) {
+    z::trtri_kernel<float2><<<dim3((n * 32 + 255) / 256, batch), 256, 0, st>>>(X, Z, n, (long long)n * n);
+    SCW_CUDA_TRY(cudaGetLastError());
+    return SCW_OK;
+}
+
+template <typename C>
+scw_status geev(cudaStream_t st, C* A, C* W, C* V, int n, int batch, C* work, int* status, const int* skip,
+                bool wide, const GemmWs& ws) {
+    // A (overwritten): n x n per batch entry; W: n eigenvalues; V: n x n right eigenvectors (columns)
+    // work: >= batch * (n*n + 3 n) elements
+    if (n <= 0 || batch <= 0) return SCW_OK;
+    const long long nn = (long long)n * n;
+    C* Q = work;                             // batch * n * n: Schur vectors
+    scw_status s = schur<C>(st, A, Q, W, n, batch, work + nn * batch, status, skip, wide);
+    // triangular eigenvectors as the rows of V, then V := Q V^T
+    if (s == SCW_OK) s = trevc<C>(st, A, V, n, batch, skip);
+    if (s != SCW_OK) return s;
+    if constexpr (sizeof(C) == sizeof(double2))
+        return zgemm(st, n, n, n, make_double2(1, 0), Q, n, nn, V, n, nn, make_double2(0, 0), V, n, nn, batch, ws, skip,
+                     0.0, kOpT);
+    else
+        return gemm32(st, n, 1.0, Q, V, kOpT, 0.0, 0.0, V, batch, ws, skip);
+}
+
+template scw_status gemm<double2>(cudaStream_t, int, int, int, double2, const double2*, int, long long, const double2*, int,
+                                  long long, double2, double2*, int, long long, int, const int*);
+template scw_status schur<float2>(cudaStream_t, float2*, float2*, float2*, int, int, float2*, int*, const int*, bool);
+template scw_status trevc<float2>(cudaStream_t, const float2*, float2*, int, int, const int*);
+template scw_status geev<double2>(cudaStream_t, double2*, double2*, double2*, int, int, double2*, int*, const int*, bool,
+                                  const GemmWs&);
+template scw_status geev<float2>(cudaStream_t, float2*, float2*, float2*, int, int, float2*, int*, const int*, bool,
+                                 const GemmWs&);
 
 }  // namespace scw
 
@@ -1263,14 +1432,14 @@ scw_status scw_zgesv(scw_ctx ctx, int n, int nrhs, void* A, void* B, int batch, 
     const long long nn = (long long)n * n;
     scw::DevBuf wbuf;
     scw::GemmWs ws;
-    const size_t need = std::max(scw::zgemm_ws_bytes(n, n, 32, 1), scw::zgemm_ws_bytes(n, nrhs, 64, 1));
+    const size_t need = std::max(scw::zgemm_ws_bytes(n, n, 32, 1), scw::zgemm_ws_bytes(n, nrhs, 32, 1));
     scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, scw::kGemmWsCap)));
     if (st == SCW_OK) st = scw::ctx_tc_flag(ctx);
     ws = scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err};
-    if (st == SCW_OK) st = scw::zgetrf(ctx->stream, (double2*)A, n, nn, dpiv, n, dinfo, batch, ws);
+    if (st == SCW_OK) st = scw::zgetrf(ctx->stream, (double2*)A, n, n, n, nn, dpiv, n, dinfo, batch, ws, nullptr);
     if (st == SCW_OK)
         st = scw::zgetrs(ctx->stream, (const double2*)A, n, nn, dpiv, n, (double2*)B, nrhs, (long long)n * nrhs, batch,
-                         ws);
+                         ws, nullptr);
     ctx->launches += 3;
     std::vector<int> info(batch, 0);
     if (st == SCW_OK) {
@@ -1304,8 +1473,8 @@ scw_status scw_zgeev(scw_ctx ctx, int n, void* A, void* W, void* V, int batch, i
     scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, scw::kGemmWsCap)));
     if (st == SCW_OK) st = scw::ctx_tc_flag(ctx);
     if (st == SCW_OK)
-        st = scw::zgeev(ctx->stream, (double2*)A, (double2*)W, (double2*)V, n, batch, work, dst, true,
-                        scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err});
+        st = scw::geev<double2>(ctx->stream, (double2*)A, (double2*)W, (double2*)V, n, batch, work, dst, nullptr, true,
+                                scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err});
     ctx->launches += 4;
     std::vector<int> status(batch, 0);
     if (st == SCW_OK) {
@@ -1335,14 +1504,19 @@ scw_status scw_cgeev(scw_ctx ctx, int n, void* A, void* W, void* V, int batch, i
         cudaFree(work);
         return fail(SCW_ERR_NOMEM, "scw_cgeev: workspace");
     }
-    scw_status st = scw::geev<float2>(ctx->stream, (float2*)A, (float2*)W, (float2*)V, n, batch, work, dst, nullptr,
-                                      true, scw::GemmWs{});
+    scw::DevBuf wbuf;
+    const size_t need = scw::zgemm_ws_bytes(n, n, n, 1);
+    scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, scw::kGemmWsCap)));
+    if (st == SCW_OK) st = scw::ctx_tc_flag(ctx);
+    if (st == SCW_OK)
+        st = scw::geev<float2>(ctx->stream, (float2*)A, (float2*)W, (float2*)V, n, batch, work, dst, nullptr, true,
+                               scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err});
     ctx->launches += 5;
     std::vector<int> status(batch, 0);
     if (st == SCW_OK) {
         cudaError_t e = cudaMemcpyAsync(status.data(), dst, sizeof(int) * batch, cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) st = fail(SCW_ERR_CUDA, cudaGetErrorString(e));
+        else st = scw_ctx_synchronize(ctx);
     }
     cudaFree(work);
     cudaFree(dst);

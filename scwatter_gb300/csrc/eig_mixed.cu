@@ -7,6 +7,7 @@
 // The algorithm is in scw_eigmix.h.
 #include <algorithm>
 #include <cmath>
+#include <vector>
 
 #include "scw_complex.cuh"
 #include "scw_dense.h"
@@ -55,12 +56,11 @@ void eigmix_carve_small(EigMixWs& w, char* base, int n, int Z) {
     w.member = (int*)take(sizeof(int) * zn);
     w.cstart = (int*)take(sizeof(int) * (size_t)Z * (n + 1));
     w.ncl = (int*)take(sizeof(int) * Z);
-    w.piv = (int*)take(sizeof(int) * zn);
-    w.info = (int*)take(sizeof(int) * Z);
     w.qr = (int*)take(sizeof(int) * Z);
     w.state = (int*)take(sizeof(int) * Z);
     w.steps = (int*)take(sizeof(int) * Z);
     w.Y = (double2*)take(sizeof(double2) * zn * kMaxCluster);
+    w.Yi = (float2*)take(sizeof(float2) * zn * kMaxCluster);
     w.rn = (double*)take(sizeof(double) * zn);
     w.xn = (double*)take(sizeof(double) * zn);
     w.anorm = (double*)take(sizeof(double) * Z);
@@ -73,31 +73,34 @@ enum : int {
     kConverged = 1,
     kQrFailed = 2,          // FP32 QR iteration did not converge
     kClusterTooLarge = 3,   // a cluster above kMaxCluster eigenvalues (or label propagation did not settle)
-    kSingularX = 4,         // zero pivot in the FP32 LU of the eigenvector matrix
+    kSingularX = 4,         // the FP32 inverse of the eigenvector matrix is not finite
     kClusterFailed = 5,     // the small FP64 Schur solve of a cluster did not converge
     kNotConverged = 6       // residual above tol_accept after the last step
 };
 
-// ||A||_1 (largest column sum of |a_ij|) per matrix
+// ||A||_1 (largest column sum of |a_ij|) per matrix; anorm starts at zero.  32 columns x 8 row lanes
+// per block (one block per matrix took 2.1 ms for 20 matrices of n = 648).
 __global__ void __launch_bounds__(256) norm1_kernel(const double2* __restrict__ A, int n, double* __restrict__ anorm) {
-    A += (long long)n * n * blockIdx.x;
-    __shared__ double red[256];
-    double best = 0.0;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        double s = 0.0;
-        for (int i = 0; i < n; i++) {
+    A += (long long)n * n * blockIdx.y;
+    __shared__ double red[8][32];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, j = blockIdx.x * 32 + tx;
+    double s = 0.0;
+    if (j < n)
+        for (int i = ty; i < n; i += 8) {
             const double2 a = A[(long long)i * n + j];
             s += hypot(a.x, a.y);
         }
-        best = fmax(best, s);
-    }
-    red[threadIdx.x] = best;
+    red[ty][tx] = s;
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + s]);
-        __syncthreads();
+    if (ty == 0) {
+        for (int t = 1; t < 8; t++) s += red[t][tx];
+        for (int o = 16; o > 0; o >>= 1) {
+            const double v = __shfl_xor_sync(0xffffffffu, s, o);
+            s = v > s || v != v ? v : s;
+        }
+        // non-negative doubles order as integers (and NaN above all of them)
+        if (tx == 0) atomicMax(reinterpret_cast<unsigned long long*>(anorm + blockIdx.y), (unsigned long long)__double_as_longlong(s));
     }
-    if (threadIdx.x == 0) anorm[blockIdx.x] = red[0];
 }
 
 __global__ void to_f32_kernel(const double2* __restrict__ A, float2* __restrict__ B, long long count) {
@@ -105,21 +108,15 @@ __global__ void to_f32_kernel(const double2* __restrict__ A, float2* __restrict_
         B[i] = make_float2((float)A[i].x, (float)A[i].y);
 }
 
-// FP32 eigenpairs -> FP64 starting point; state from the FP32 QR status
-__global__ void init_kernel(const float2* __restrict__ lam32, const float2* __restrict__ X32, double2* __restrict__ lam,
-                            double2* __restrict__ X, int n, const int* __restrict__ qr, int* __restrict__ state,
-                            int* __restrict__ steps, double* __restrict__ res) {
-    const int b = blockIdx.y;
-    const long long nn = (long long)n * n;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nn; i += (long long)gridDim.x * blockDim.x) {
-        const float2 v = X32[nn * b + i];
-        X[nn * b + i] = make_double2(v.x, v.y);
-        if (i < n) {
-            const float2 l = lam32[(long long)n * b + i];
-            lam[(long long)n * b + i] = make_double2(l.x, l.y);
-        }
+// FP32 eigenvalues -> FP64 starting point; state from the FP32 QR status
+__global__ void init_kernel(const float2* __restrict__ lam32, double2* __restrict__ lam, int n, const int* __restrict__ qr,
+                            int* __restrict__ state, int* __restrict__ steps, double* __restrict__ res) {
+    const int b = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        const float2 l = lam32[(long long)n * b + i];
+        lam[(long long)n * b + i] = make_double2(l.x, l.y);
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (i == 0) {
         state[b] = qr[b] ? kQrFailed : kRefining;
         steps[b] = -1;
         res[b] = INFINITY;
@@ -289,33 +286,18 @@ gate_kernel(int n, const double* __restrict__ rn, const double* __restrict__ xn,
     }
 }
 
-// X (FP64) rounded to FP32 twice: the LU input and the GEMM operand
-__global__ void to32_kernel(const double2* __restrict__ X, float2* __restrict__ L, float2* __restrict__ X32, int n,
-                            const int* __restrict__ state) {
-    const int b = blockIdx.y;
-    if (state[b] != kRefining) return;
-    const long long nn = (long long)n * n;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nn; i += (long long)gridDim.x * blockDim.x) {
-        const double2 v = X[nn * b + i];
-        const float2 f = make_float2((float)v.x, (float)v.y);
-        L[nn * b + i] = f;
-        X32[nn * b + i] = f;
-    }
-}
-
-__global__ void lu_check_kernel(const int* __restrict__ info, int Z, int* __restrict__ state) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b < Z && state[b] == kRefining && info[b] != 0) state[b] = kSingularX;
-}
-
 // lambda_i += E_ii for eigenvalues outside every cluster
 __global__ void singleton_kernel(const float2* __restrict__ E, const int* __restrict__ label, double2* __restrict__ lam,
-                                 int n, const int* __restrict__ state) {
+                                 int n, int* __restrict__ state) {
     const int b = blockIdx.y;
     if (state[b] != kRefining) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || label[(long long)n * b + i] >= 0) return;
     const float2 e = E[(long long)n * n * b + (long long)i * n + i];
+    if (!isfinite(e.x) || !isfinite(e.y)) {
+        state[b] = kSingularX;
+        return;
+    }
     double2& l = lam[(long long)n * b + i];
     l = make_double2(l.x + (double)e.x, l.y + (double)e.y);
 }
@@ -324,11 +306,12 @@ __global__ void singleton_kernel(const float2* __restrict__ E, const int* __rest
 // M = diag(lambda_S) + E_SS in FP64 -> Householder Hessenberg form -> single-shift complex QR
 // (Schur form T, unitary U) -> eigenvectors of T with pairs closer than deg_rel ||A||_1 left
 // uncoupled (a degenerate eigenvalue keeps the unitary Schur basis) -> Y = U Yt.
-// Y goes to Yout (k x k, row-major, at the cluster's slot), the eigenvalues to lambda.
+// Y goes to Yout and Y^-1 = Yt^-1 U^H to Yinv (k x k, row-major, at the cluster's slot), the eigenvalues
+// to lambda.
 __global__ void __launch_bounds__(kMaxCluster)
 cluster_eig_kernel(const float2* __restrict__ E, const int* __restrict__ member, const int* __restrict__ cstart,
                    const int* __restrict__ ncl, double2* __restrict__ lam, int n, const double* __restrict__ anorm,
-                   double deg_rel, double2* __restrict__ Yout, int* __restrict__ state) {
+                   double deg_rel, double2* __restrict__ Yout, float2* __restrict__ Yinv, int* __restrict__ state) {
     const int b = blockIdx.y, c = blockIdx.x;
     if (state[b] != kRefining || c >= ncl[b]) return;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -530,6 +513,25 @@ cluster_eig_kernel(const float2* __restrict__ E, const int* __restrict__ member,
         }
         lam[mem[t]] = T[t * k + t];
     }
+    __syncthreads();
+    if (t < k) {                            // T := Yt^-1 (unit upper triangular), column t
+        for (int i = t + 1; i < k; i++) T[i * k + t] = make_double2(0.0, 0.0);
+        T[t * k + t] = make_double2(1.0, 0.0);
+        for (int i = t - 1; i >= 0; i--) {
+            double2 s = make_double2(0.0, 0.0);
+            for (int m = i + 1; m <= t; m++) s = cfma(Yt[i * k + m], T[m * k + t], s);
+            T[i * k + t] = make_double2(-s.x, -s.y);
+        }
+    }
+    __syncthreads();
+    if (t < k) {
+        float2* Yc = Yinv + ((long long)n * b + s0) * kMaxCluster;
+        for (int i = 0; i < k; i++) {
+            double2 s = make_double2(0.0, 0.0);
+            for (int m = i; m < k; m++) s = cfma(T[i * k + m], make_double2(U[t * k + m].x, -U[t * k + m].y), s);
+            Yc[i * k + t] = make_float2((float)s.x, (float)s.y);
+        }
+    }
 }
 
 // F_ij = E_ij / (lambda_j - lambda_i) between different clusters / singletons, 0 within one
@@ -554,17 +556,6 @@ __global__ void f_kernel(const float2* __restrict__ E, const double2* __restrict
             }
         }
         F[e] = f;
-    }
-}
-
-__global__ void xupdate_kernel(const float2* __restrict__ P, double2* __restrict__ X, int n, const int* __restrict__ state) {
-    const int b = blockIdx.y;
-    if (state[b] != kRefining) return;
-    const long long nn = (long long)n * n;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nn; i += (long long)gridDim.x * blockDim.x) {
-        const float2 p = P[nn * b + i];
-        double2& x = X[nn * b + i];
-        x = make_double2(x.x + (double)p.x, x.y + (double)p.y);
     }
 }
 
@@ -596,6 +587,33 @@ rotate_kernel(double2* __restrict__ X, const int* __restrict__ member, const int
     }
 }
 
+// Yx[S, :] := Y_S^-1 Yx[S, :] for every cluster S, Yx the FP32 inverse of X (one CTA of kMaxCluster
+// threads per cluster; each thread stages its column's k entries in shared memory)
+__global__ void __launch_bounds__(kMaxCluster)
+rotate_rows_kernel(float2* __restrict__ Yx, const int* __restrict__ member, const int* __restrict__ cstart,
+                   const int* __restrict__ ncl, const float2* __restrict__ Yinv, int n, const int* __restrict__ state) {
+    const int b = blockIdx.y, c = blockIdx.x;
+    if (state[b] != kRefining || c >= ncl[b]) return;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int* cs = cstart + (long long)(n + 1) * b;
+    const int s0 = cs[c], k = cs[c + 1] - s0;
+    const int* mem = member + (long long)n * b + s0;
+    float2* Ys = reinterpret_cast<float2*>(smem);
+    float2* xs = Ys + k * k + threadIdx.x * k;
+    const float2* Yc = Yinv + ((long long)n * b + s0) * kMaxCluster;
+    for (int e = threadIdx.x; e < k * k; e += blockDim.x) Ys[e] = Yc[e];
+    __syncthreads();
+    Yx += (long long)n * n * b;
+    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+        for (int l = 0; l < k; l++) xs[l] = Yx[(long long)mem[l] * n + j];
+        for (int i = 0; i < k; i++) {
+            float2 s = make_float2(0.f, 0.f);
+            for (int l = 0; l < k; l++) s = cfma(Ys[i * k + l], xs[l], s);
+            Yx[(long long)mem[i] * n + j] = s;
+        }
+    }
+}
+
 __global__ void final_kernel(int* __restrict__ state, int* __restrict__ accepted, int Z) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= Z) return;
@@ -621,18 +639,29 @@ scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int
     MX_TRY(set_smem((const void*)cluster_kernel, cl_smem));
     MX_TRY(set_smem((const void*)cluster_eig_kernel, eig_smem));
     MX_TRY(set_smem((const void*)rotate_kernel, rot_smem));
+    MX_TRY(set_smem((const void*)rotate_rows_kernel, rot_smem / 2));
     const int maxcl = std::max(1, n / 2);
-    const float2 f1 = {1.f, 0.f}, f0 = {0.f, 0.f};
     const double2 d1 = {1.0, 0.0}, d0 = {0.0, 0.0};
     double2* AX = reinterpret_cast<double2*>(w.S0);      // S0 and S1 together: one FP64 slot
+    float2* Yx = w.S2;                                   // X^-1 in FP32, kept through the refinement
+    // a call that is not being captured may look at the states between steps and stop early
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    SCW_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+    std::vector<int> hstate(Z);
 
-    norm1_kernel<<<Z, 256, 0, st>>>(A, n, w.anorm);
-    to_f32_kernel<<<nblk(nn * Z), 256, 0, st>>>(A, w.S0, nn * Z);
+    SCW_CUDA_TRY(cudaMemsetAsync(w.anorm, 0, sizeof(double) * Z, st));
+    norm1_kernel<<<dim3((n + 31) / 32, Z), 256, 0, st>>>(A, n, w.anorm);
+    to_f32_kernel<<<nblk(n * Z), 256, 0, st>>>(A, w.S0, nn * Z);
     MX_LAUNCHED(2);
-    // FP32 Householder + QR + triangular eigenvectors: eigenvectors into S2, eigenvalues lam32
-    MX_TRY(geev<float2>(st, w.S0, w.lam32, w.S2, n, Z, w.S1, w.qr, nullptr, prm.wide, GemmWs{}));
-    if (launches) *launches += 5;
-    init_kernel<<<dim3(gZ, Z), 256, 0, st>>>(w.lam32, w.S2, lam, V, n, w.qr, w.state, w.steps, w.res);
+    // FP32 Householder + QR: T in S0, Schur vectors Q in S1, eigenvalues lam32.  Triangular
+    // eigenvectors Xt (rows of S2) and their inverse (S3): X = Q Xt, X^-1 = Xt^-1 Q^H
+    MX_TRY(schur<float2>(st, w.S0, w.S1, w.lam32, n, Z, w.hw, w.qr, nullptr, prm.wide));
+    MX_TRY(trevc<float2>(st, w.S0, w.S2, n, Z, nullptr));
+    MX_TRY(trtri32(st, w.S2, w.S3, n, Z));
+    MX_TRY(gemm32(st, n, 1.0, w.S1, w.S2, kOpT, 0.0, 0.0, V, Z, ws, nullptr));
+    MX_TRY(gemm32(st, n, 1.0, w.S3, w.S1, kOpC, 0.0, 0.0, Yx, Z, ws, nullptr));
+    if (launches) *launches += 10;
+    init_kernel<<<dim3(nblk(n), Z), 256, 0, st>>>(w.lam32, lam, n, w.qr, w.state, w.steps, w.res);
     cluster_kernel<<<Z, 1024, cl_smem, st>>>(lam, n, w.anorm, prm.tau_rel, w.label, w.member, w.cstart, w.ncl, w.state);
     MX_LAUNCHED(2);
     const int last = n >= EigMixParams::kLargeN ? std::max(prm.steps, prm.steps_large) : prm.steps;
@@ -642,25 +671,29 @@ scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int
         resid_kernel<<<dim3((n + 31) / 32, Z), 256, 0, st>>>(AX, V, lam, n, w.S3, w.rn, w.xn, w.state);
         gate_kernel<<<Z, 256, 0, st>>>(n, w.rn, w.xn, w.anorm, s >= prm.steps ? prm.tol_accept : prm.tol, s, w.state,
                                        w.steps, w.res);
-        MX_LAUNCHED(3);
+        MX_LAUNCHED(5);
         if (s == last) break;
-        // E = X^-1 R in FP32
-        to32_kernel<<<dim3(gZ, Z), 256, 0, st>>>(V, w.S0, w.S2, n, w.state);
-        MX_LAUNCHED(1);
-        MX_TRY(getrf<float2>(st, w.S0, n, nn, w.piv, n, w.info, Z, GemmWs{}));
-        MX_TRY(getrs<float2>(st, w.S0, n, nn, w.piv, n, w.S3, n, nn, Z, GemmWs{}));
-        if (launches) *launches += 3 * ((n + 31) / 32) + 1 + 4 * ((n + 63) / 64);
-        lu_check_kernel<<<nblk(Z), 256, 0, st>>>(w.info, Z, w.state);
-        singleton_kernel<<<dim3(nblk(n), Z), 256, 0, st>>>(w.S3, w.label, lam, n, w.state);
-        cluster_eig_kernel<<<dim3(maxcl, Z), kMaxCluster, eig_smem, st>>>(w.S3, w.member, w.cstart, w.ncl, lam, n,
-                                                                         w.anorm, prm.deg_rel, w.Y, w.state);
-        f_kernel<<<dim3(gZ, Z), 256, 0, st>>>(w.S3, lam, w.label, n, w.S1, w.state);
-        MX_LAUNCHED(4);
-        // X += X F (FP32 product, FP64 sum), then the cluster rotations
-        MX_TRY(gemm<float2>(st, n, n, n, f1, w.S2, n, nn, w.S1, n, nn, f0, w.S0, n, nn, Z, w.state));
-        xupdate_kernel<<<dim3(gZ, Z), 256, 0, st>>>(w.S0, V, n, w.state);
+        if (s >= 2 && cap == cudaStreamCaptureStatusNone) {
+            SCW_CUDA_TRY(cudaMemcpyAsync(hstate.data(), w.state, sizeof(int) * Z, cudaMemcpyDeviceToHost, st));
+            SCW_CUDA_TRY(cudaStreamSynchronize(st));
+            if (std::count(hstate.begin(), hstate.end(), (int)kRefining) == 0) break;
+        }
+        // E = X^-1 R
+        MX_TRY(gemm32(st, n, 1.0, Yx, w.S3, kOpN, 0.0, 0.0, w.S0, Z, ws, w.state));
+        singleton_kernel<<<dim3(nblk(n), Z), 256, 0, st>>>(w.S0, w.label, lam, n, w.state);
+        cluster_eig_kernel<<<dim3(maxcl, Z), kMaxCluster, eig_smem, st>>>(w.S0, w.member, w.cstart, w.ncl, lam, n,
+                                                                         w.anorm, prm.deg_rel, w.Y, w.Yi, w.state);
+        f_kernel<<<dim3(gZ, Z), 256, 0, st>>>(w.S0, lam, w.label, n, w.S1, w.state);
+        MX_LAUNCHED(6);
+        // X += X F, then the cluster rotations; X^-1 follows by the inverse rotations and a Newton
+        // step, Yx += Yx (I - X Yx), which squares the error F left in it
+        MX_TRY(gemm32(st, n, 1.0, V, w.S1, kOpN, 1.0, 0.0, V, Z, ws, w.state));
         rotate_kernel<<<dim3(maxcl, Z), kMaxCluster, rot_smem, st>>>(V, w.member, w.cstart, w.ncl, w.Y, n, w.state);
-        MX_LAUNCHED(3);
+        rotate_rows_kernel<<<dim3(maxcl, Z), kMaxCluster, rot_smem / 2, st>>>(Yx, w.member, w.cstart, w.ncl, w.Yi, n,
+                                                                             w.state);
+        MX_TRY(gemm32(st, n, -1.0, V, Yx, kOpN, 0.0, 1.0, w.S0, Z, ws, w.state));
+        MX_TRY(gemm32(st, n, 1.0, Yx, w.S0, kOpN, 1.0, 0.0, Yx, Z, ws, w.state));
+        MX_LAUNCHED(11);
     }
     // slices without convergence: the FP64 Householder + QR solver (qr[] reused as the skip mask)
     final_kernel<<<nblk(Z), 256, 0, st>>>(w.state, w.qr, Z);

@@ -29,6 +29,9 @@
 // the FP64 pipes give 1.05-1.25): 1.66 ms instead of 38 ms for the latter, of which 0.3 ms prepare
 // the operands.  Bound by the tensor core's operand reads and the drains between chunks.
 //
+// The same kernel with 4 digits (30 bits) and 64 columns per tile serves the corrections of the
+// eigen-solver and of the inverses, which need FP32 accuracy: 10 digit products instead of 36.
+//
 // Two launches prepare the operands (oz_inner_kernel: f_k; oz_split_kernel: e_i, g_j and the digits in
 // the order the MMA reads them, so that a pipeline stage is two contiguous bulk copies), one runs
 // the product: persistent CTAs, one thread copying, one issuing MMAs, 8 warps draining.
@@ -43,12 +46,16 @@
 namespace scw {
 namespace oz {
 
-constexpr int kS = 8;                        // base-256 digits per value
-constexpr int kBits = 62;                    // integer bits before the cut
-constexpr int kTM = 128, kTN = 32, kTK = 16; // tile rows, columns, inner indices per stage
-constexpr int kABlk = 2 * kS * kTM * kTK * 2;   // bytes of A per stage: re, im x digits x 128 x 16 bf16
-constexpr int kBBlk = 2 * kS * kTN * kTK * 2;
-constexpr int kStages = 2;
+constexpr int kTM = 128, kTK = 16;           // tile rows, inner indices per stage
+template <int S>                             // S base-256 digits per value
+struct Cfg {
+    static constexpr int kBits = 8 * S - 2;      // integer bits before the cut
+    static constexpr int kTN = 256 / S;          // tile columns: S diagonals x 2 parts fill the TMEM
+    static constexpr int kABlk = 2 * S * kTM * kTK * 2;   // bytes of A per stage: re, im x digits x 128 x 16 bf16
+    static constexpr int kBBlk = 2 * S * kTN * kTK * 2;
+    static constexpr int kStages = S == 8 ? 2 : 4;
+    static constexpr size_t kSmem = (size_t)kStages * (kABlk + kBBlk) + (2 * kStages + 4) * sizeof(uint64_t);
+};
 constexpr int kChunk = 8;                    // stages per drain (K = 128)
 constexpr int kDrainWarps = 8;
 constexpr int kThreads = (kDrainWarps + 2) * 32;
@@ -63,57 +70,93 @@ __device__ __forceinline__ int cexpo(double2 v) {
     if (m == 0 && v.x == 0.0 && v.y == 0.0) return kNone;
     return (int)max(m, 1u) - 1022;
 }
+__device__ __forceinline__ int cexpo(float2 v) {
+    const unsigned m = max(__float_as_uint(v.x) & 0x7fffffffu, __float_as_uint(v.y) & 0x7fffffffu);
+    if (m >= 0x7f800000u) return kSpecial;
+    if (m == 0u) return kNone;
+    return (int)max(m >> 23, 1u) - 126;
+}
 
-// round(v 2^s) for |v 2^s| < 2^62 (ties away from zero)
+// round(v 2^s) for |v 2^s| < 2^62 (ties away from zero); v = +-m 2^(ex - 1075)
+__device__ __forceinline__ long long fixed_point(bool neg, int ex, long long m, int s) {
+    const int sh = ex - 1075 + s;
+    if (sh >= 0) m <<= min(sh, 10);
+    else m = sh < -55 ? 0 : (m + (1ll << (-sh - 1))) >> -sh;
+    return neg ? -m : m;
+}
 __device__ __forceinline__ long long fixed_point(double v, int s) {
     const long long bits = __double_as_longlong(v);
     const int ex = (int)((bits >> 52) & 0x7ff);
-    long long m = bits & 0xfffffffffffffll;
-    if (ex) m |= 1ll << 52;
-    const int sh = (ex ? ex : 1) - 1075 + s;
-    if (sh >= 0) m <<= min(sh, 10);
-    else m = sh < -55 ? 0 : (m + (1ll << (-sh - 1))) >> -sh;
-    return bits < 0 ? -m : m;
+    return fixed_point(bits < 0, max(ex, 1), (bits & 0xfffffffffffffll) | (ex ? 1ll << 52 : 0ll), s);
+}
+__device__ __forceinline__ long long fixed_point(float v, int s) {
+    const unsigned bits = __float_as_uint(v);
+    const int ex = (int)((bits >> 23) & 0xff);
+    return fixed_point((int)bits < 0, max(ex, 1) - 127 + 1023, (long long)((bits & 0x7fffffu) | (ex ? 1u << 23 : 0u)) << 29, s);
 }
 
-// f[b][k] with |B(k, :)| < 2^f: a warp per row of B
+// f[b][k] with |B(k, :)| < 2^f: a warp per inner index k; element (k, j) of B at k ks + j js
+template <typename T>
 __global__ void __launch_bounds__(256)
-oz_inner_kernel(const double2* __restrict__ B, int ldb, long long sB, int K, int N, int* __restrict__ f,
+oz_inner_kernel(const T* __restrict__ B, long long ks, long long js, long long sB, int K, int N, int* __restrict__ f,
                 const int* __restrict__ skip) {
     if (z::skipped(skip, blockIdx.y)) return;
-    const int k = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (k >= K) return;
-    const double2* row = B + sB * blockIdx.y + (long long)k * ldb;
-    int e = kNone;
+    B += sB * blockIdx.y;
+    f += (long long)blockIdx.y * K;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (js == 1) {
+        const int k = blockIdx.x * 8 + warp;
+        if (k >= K) return;
+        const T* row = B + k * ks;
+        int e = kNone;
 #pragma unroll 4
-    for (int j = lane; j < N; j += 32) {
-        const int x = cexpo(row[j]);
-        if (x != kSpecial) e = max(e, x);
+        for (int j = lane; j < N; j += 32) {
+            const int x = cexpo(row[j]);
+            if (x != kSpecial) e = max(e, x);
+        }
+        e = __reduce_max_sync(0xffffffffu, e);
+        if (lane == 0) f[k] = e;
+    } else {
+        // inner index contiguous: 8 of them per block, threads 8 (k) x 32 (j)
+        __shared__ int se[8][33];
+        const int k = blockIdx.x * 8 + (threadIdx.x & 7), j0 = threadIdx.x >> 3;
+        int e = kNone;
+        if (k < K) {
+#pragma unroll 4
+            for (int j = j0; j < N; j += 32) {
+                const int x = cexpo(B[k * ks + j * js]);
+                if (x != kSpecial) e = max(e, x);
+            }
+        }
+        se[threadIdx.x & 7][j0] = e;
+        __syncthreads();
+        const int r = __reduce_max_sync(0xffffffffu, se[warp][lane]);
+        if (lane == 0 && blockIdx.x * 8 + warp < K) f[blockIdx.x * 8 + warp] = r;
     }
-    e = __reduce_max_sync(0xffffffffu, e);
-    if (lane == 0) f[(long long)blockIdx.y * K + k] = e;
 }
 
 // the digits of 8 consecutive inner indices of one row (or column), real or imaginary part: one
 // 16-byte store per digit, dst + digit * stride
+template <int S>
 __device__ __forceinline__ void store_digits(const long long (&q)[8], unsigned char* dst, int stride) {
     unsigned lo[8], hi[8];
 #pragma unroll
     for (int t = 0; t < 8; t++) {       // + 128 in every digit below the top: bytes are digit + 128
-        const long long b = q[t] + 0x80808080808080ll;
+        const unsigned long long b = (unsigned long long)(q[t] + (S == 8 ? 0x80808080808080ll : 0x808080ll));
         lo[t] = (unsigned)b;
-        hi[t] = (unsigned)((unsigned long long)b >> 32);
+        hi[t] = (unsigned)(b >> 32);
     }
 #pragma unroll
-    for (int s = 0; s < kS; s++) {
+    for (int s = 0; s < S; s++) {
         float v[8];
 #pragma unroll
         for (int t = 0; t < 8; t++) {
             // integer to float through the low mantissa bits of 2^23
             if (s == 0) {
-                v[t] = __uint_as_float(0x4b000000u + 256u + (unsigned)((int)hi[t] >> 24)) - (8388608.0f + 256.0f);
+                v[t] = __uint_as_float(0x4b000000u + 256u + (unsigned)((int)(S == 8 ? hi[t] : lo[t]) >> 24)) -
+                       (8388608.0f + 256.0f);
             } else {
-                const int sh = 8 * (kS - 1 - s);
+                const int sh = 8 * (S - 1 - s);
                 const unsigned byte = ((sh >= 32 ? hi[t] >> (sh - 32) : lo[t] >> sh) & 0xffu);
                 v[t] = __uint_as_float(0x4b000000u | byte) - (8388608.0f + 128.0f);
             }
@@ -128,9 +171,10 @@ __device__ __forceinline__ void store_digits(const long long (&q)[8], unsigned c
 }
 
 struct SplitArgs {
-    const double2 *A, *B;
-    int lda, ldb;
+    const void *A, *B;
+    long long rsA, ksA, rsB, ksB;      // element (row of A or column of B, inner index k) at row rs + k ks
     long long sA, sB;
+    int conjB;                         // 1: the conjugate of B
     int M, N, K, nk, mt, nt;           // nk stages, mt x nt tiles
     int gA, gB, nA;                    // 16-row groups of A, 16-column groups of B per matrix; A blocks in all
     const int* f;
@@ -139,32 +183,28 @@ struct SplitArgs {
     int fstep;                         // f stride per A matrix: 0 when all matrices share one B
 };
 
-// Exponents and digits.  A block takes 16 rows of A or 16 columns of B: first the largest exponent
-// of each over the inner index, then the digits, a warp per stage of 16 inner indices (lane = 8
-// rows x 2 halves of the stage x 2 row groups, so a warp stores 512 contiguous bytes per digit).
-__global__ void __launch_bounds__(256)
-oz_split_kernel(SplitArgs p, const int* __restrict__ skip) {
-    __shared__ int se[16][17];
+// Exponents and digits of 16 rows of A or 16 columns of B: first the largest exponent of each over
+// the inner index, then the digits, a warp per stage of 16 inner indices (lane = 8 rows x 2 halves of
+// the stage x 2 row groups, so a warp stores 512 contiguous bytes per digit).
+template <int S, bool kA, typename T>
+__device__ __forceinline__ void split_group(const SplitArgs& p, int b, int g, int (*se)[17]) {
+    using C = Cfg<S>;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const bool isA = (int)blockIdx.x < p.nA;
-    const int blk = isA ? blockIdx.x : blockIdx.x - p.nA;
-    const int per = isA ? p.gA : p.gB;
-    const int b = blk / per, g = blk - b * per;
-    if (z::skipped(skip, b)) return;
-    const int r0 = g * 16, R = isA ? p.M : p.N;
-    const double2* src = isA ? p.A + p.sA * b : p.B + p.sB * b;
-    const long long rs = isA ? p.lda : 1, ks = isA ? 1 : p.ldb;      // element (row, k) at row rs + k ks
-    const int* f = p.f + (long long)(isA ? b * p.fstep : b) * p.K;
+    const int per = kA ? p.gA : p.gB, r0 = g * 16, R = kA ? p.M : p.N;
+    const T* src = (kA ? (const T*)p.A + p.sA * b : (const T*)p.B + p.sB * b);
+    const long long rs = kA ? p.rsA : p.rsB, ks = kA ? p.ksA : p.ksB;
+    const int* f = p.f + (long long)(kA ? b * p.fstep : b) * p.K;
     {
-        // 16 x 16 threads: along k for the rows of A, along the columns of B (both contiguous)
-        const int r = isA ? t >> 4 : t & 15, kr = isA ? t & 15 : t >> 4;
+        // 16 x 16 threads, the faster ones along the contiguous index
+        const bool kfast = ks == 1;
+        const int r = kfast ? t >> 4 : t & 15, kr = kfast ? t & 15 : t >> 4;
         int e = kNone;
         if (r0 + r < R) {
 #pragma unroll 4
             for (int k = kr; k < p.K; k += 16) {
                 const int x = cexpo(src[(r0 + r) * rs + k * ks]);
                 if (x == kSpecial) e = kSpecial;
-                else if (x != kNone) e = max(e, isA ? x + f[k] : x - f[k]);
+                else if (x != kNone) e = max(e, kA ? x + f[k] : x - f[k]);
             }
         }
         se[r][kr] = e;
@@ -174,15 +214,15 @@ oz_split_kernel(SplitArgs p, const int* __restrict__ skip) {
         int e = kNone;
         for (int q = 0; q < 16; q++) e = max(e, se[t][q]);
         se[t][16] = e;
-        (isA ? p.eA : p.gN)[(long long)b * per * 16 + r0 + t] = e;
+        (kA ? p.eA : p.gN)[(long long)b * per * 16 + r0 + t] = e;
     }
     __syncthreads();
     const int rl = (lane & 7) + 8 * (lane >> 4), kh = (lane >> 3) & 1;
     const int r = r0 + rl, e = se[rl][16];
     const bool live = r < R && e > kNone / 2 && e < kSpecial;
-    const int T = isA ? kTM : kTN, blkb = isA ? kABlk : kBBlk, dig = T * kTK * 2;
-    unsigned char* dst = (isA ? p.dA + (long long)b * p.mt * p.nk * kABlk : p.dB + (long long)b * p.nt * p.nk * kBBlk) +
-                         (long long)(r0 / T) * p.nk * blkb + (r0 % T) * 32 + (lane >> 4) * 256 + kh * 128 + (lane & 7) * 16;
+    constexpr int TR = kA ? kTM : C::kTN, blkb = kA ? C::kABlk : C::kBBlk, dig = TR * kTK * 2;
+    unsigned char* dst = (kA ? p.dA + (long long)b * p.mt * p.nk * C::kABlk : p.dB + (long long)b * p.nt * p.nk * C::kBBlk) +
+                         (long long)(r0 / TR) * p.nk * blkb + (r0 % TR) * 32 + (lane >> 4) * 256 + kh * 128 + (lane & 7) * 16;
     for (int st = warp; st < p.nk; st += 8) {
         const int k0 = st * kTK + kh * 8;
         long long qr[8], qi[8];
@@ -191,16 +231,29 @@ oz_split_kernel(SplitArgs p, const int* __restrict__ skip) {
             qr[j] = qi[j] = 0;
             const int k = k0 + j;
             if (live && k < p.K) {
-                const double2 v = src[r * rs + k * ks];
-                const int s = (isA ? f[k] : -f[k]) - e + kBits;
+                const T v = src[r * rs + k * ks];
+                const int s = (kA ? f[k] : -f[k]) - e + C::kBits;
                 qr[j] = fixed_point(v.x, s);
                 qi[j] = fixed_point(v.y, s);
+                if (!kA && p.conjB) qi[j] = -qi[j];
             }
         }
         unsigned char* o = dst + (long long)st * blkb;
-        store_digits(qr, o, dig);
-        store_digits(qi, o + kS * dig, dig);
+        store_digits<S>(qr, o, dig);
+        store_digits<S>(qi, o + S * dig, dig);
     }
+}
+
+template <int S, typename TA, typename TB>
+__global__ void __launch_bounds__(256) oz_split_kernel(SplitArgs p, const int* __restrict__ skip) {
+    __shared__ int se[16][17];
+    const bool isA = (int)blockIdx.x < p.nA;
+    const int blk = isA ? blockIdx.x : blockIdx.x - p.nA;
+    const int per = isA ? p.gA : p.gB;
+    const int b = blk / per, g = blk - b * per;
+    if (z::skipped(skip, b)) return;
+    if (isA) split_group<S, true, TA>(p, b, g, se);
+    else split_group<S, false, TB>(p, b, g, se);
 }
 
 // (hi 2^32 + lo) 2^e rounded once to FP64, with integer operations (FP64 ones cost 60 times more)
@@ -238,16 +291,25 @@ struct GemmArgs {
     int M, N, nk, mt, nt, gA, gB;
     int a_shared, b_shared;            // all matrices use the digits of matrix 0
     double2 alpha, beta;
-    double2* C;
+    double diag;                       // added on the diagonal of alpha A B
+    void* C;
     int ldc;
     long long sC;
     int tiles;
     int* err;
 };
 
+__device__ __forceinline__ double2 to_d(double2 v) { return v; }
+__device__ __forceinline__ double2 to_d(float2 v) { return make_double2(v.x, v.y); }
+__device__ __forceinline__ void put(double2* p, double2 v) { *p = v; }
+__device__ __forceinline__ void put(float2* p, double2 v) { *p = make_float2((float)v.x, (float)v.y); }
+
+template <int S, typename TC>
 __global__ void __launch_bounds__(kThreads, 1)
 oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
     using namespace tc;
+    constexpr int kS = S, kTN = Cfg<S>::kTN, kABlk = Cfg<S>::kABlk, kBBlk = Cfg<S>::kBBlk, kStages = Cfg<S>::kStages;
+    constexpr int kCols = kTN / 2;               // columns of a drain warp
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* sA = smem;
     unsigned char* sB = smem + kStages * kABlk;
@@ -352,18 +414,20 @@ oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
         }
         __syncwarp();
     } else {
-        // -------- drain: warp w reads TMEM lanes 32 (w % 4) .., columns 16 (w / 4) .. of each diagonal --------
+        // -------- drain: warp w reads TMEM lanes 32 (w % 4) .., half w / 4 of each diagonal's columns --------
         const int quarter = warp & 3, half = warp >> 2;
-        const uint32_t tb = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 16);
+        const uint32_t tb = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * kCols);
+        constexpr int kW = S == 8 ? 2 : 1;       // 64-bit words per value: diagonals 0 .. 3 (and 4 .. 7)
         int chunk = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < p.tiles && ok; tile += gridDim.x) {
             const int b = tile / per, q = tile - b * per, m = q / p.nt, n = q - m * p.nt;
             if (z::skipped(skip, b)) continue;
-            // diagonals 0 .. 3 and 4 .. 7 (weights 2^24, 2^16, 2^8, 1) per part and column
-            long long hi[2][16], lo[2][16];
+            long long w[kW][2][kCols];
 #pragma unroll
-            for (int c = 0; c < 16; c++) hi[0][c] = hi[1][c] = lo[0][c] = lo[1][c] = 0;
+            for (int c = 0; c < kCols; c++)
+#pragma unroll
+                for (int h = 0; h < kW; h++) w[h][0][c] = w[h][1][c] = 0;
             for (int k = 0; k < p.nk; k += kChunk, chunk++) {
                 int stop = *abort_flag;
                 if (!stop && !mbar_wait(acc_full, (uint32_t)(chunk & 1))) stop = 1;
@@ -377,53 +441,58 @@ oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
                 for (int part = 0; part < 2; part++)
 #pragma unroll
                     for (int d = 0; d < kS; d++) {
-                        uint32_t v[16];
-                        tmem_ld16(tb + (uint32_t)(part * kS * kTN + d * kTN), v);
-                        tmem_ld_wait();
 #pragma unroll
-                        for (int c = 0; c < 16; c++) {
-                            const long long x = __float2int_rn(__uint_as_float(v[c]));
-                            if (d <= 3) hi[part][c] += x * (1 << (8 * (3 - d)));
-                            else lo[part][c] += x * (1 << (8 * (kS - 1 - d)));
+                        for (int c16 = 0; c16 < kCols; c16 += 16) {
+                            uint32_t v[16];
+                            tmem_ld16(tb + (uint32_t)(part * kS * kTN + d * kTN + c16), v);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int c = 0; c < 16; c++)
+                                w[d >> 2][part][c16 + c] +=
+                                    (long long)__float2int_rn(__uint_as_float(v[c])) * (1 << (8 * (3 - (d & 3))));
                         }
                     }
                 tc_fence_before();
                 mbar_arrive(acc_empty);
             }
             if (!ok) break;
-            const int row = m * kTM + quarter * 32 + lane, col0 = n * kTN + half * 16;
+            const int row = m * kTM + quarter * 32 + lane, col0 = n * kTN + half * kCols;
             if (row < p.M) {
                 const int eA = p.eA[(long long)(p.a_shared ? 0 : b) * p.gA * 16 + row];
                 const int* gN = p.gN + (long long)(p.b_shared ? 0 : b) * p.gB * 16 + col0;
-                double2* out = p.C + p.sC * b + (long long)row * p.ldc + col0;
+                TC* out = (TC*)p.C + p.sC * b + (long long)row * p.ldc + col0;
                 const bool unit = p.alpha.y == 0.0 && (p.alpha.x == 1.0 || p.alpha.x == -1.0);
                 const bool add = p.beta.x != 0.0 || p.beta.y != 0.0;
                 const bool add1 = p.beta.x == 1.0 && p.beta.y == 0.0;
 #pragma unroll
-                for (int c = 0; c < 16; c++) {
+                for (int c = 0; c < kCols; c++) {
                     if (col0 + c < p.N) {
                         const int g = gN[c];
-                        // the last diagonal weighs 2^(8 (kS - 1)); units 2^(eA - kBits) 2^(g - kBits)
-                        const int e = eA + g + 8 * (kS - 1) - 2 * kBits;
+                        // the last diagonal weighs 2^(8 (S - 1)); units 2^(eA - kBits) 2^(g - kBits)
+                        const int e = eA + g + 8 * (kS - 1) - 2 * Cfg<S>::kBits;
                         double2 v;
                         if (eA >= kSpecial || g >= kSpecial) {
-                            v = make_double2(__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll));
+                            v.x = v.y = __longlong_as_double(0x7ff8000000000000ll);
+                        } else if (kW == 2) {
+                            v.x = fx_to_double(w[0][0][c], w[kW - 1][0][c], e);
+                            v.y = fx_to_double(w[0][1][c], w[kW - 1][1][c], e);
                         } else {
-                            v.x = fx_to_double(hi[0][c], lo[0][c], e);
-                            v.y = fx_to_double(hi[1][c], lo[1][c], e);
+                            v.x = fx_to_double(0, w[0][0][c], e);
+                            v.y = fx_to_double(0, w[0][1][c], e);
                         }
                         if (unit) {
                             if (p.alpha.x < 0.0) v = make_double2(-v.x, -v.y);
                         } else {
                             v = z::cmul(p.alpha, v);
                         }
+                        if (p.diag != 0.0 && row == col0 + c) v.x += p.diag;
                         if (add1) {
-                            const double2 o = out[c];
+                            const double2 o = to_d(out[c]);
                             v = make_double2(v.x + o.x, v.y + o.y);
                         } else if (add) {
-                            v = z::cfma(p.beta, out[c], v);
+                            v = z::cfma(p.beta, to_d(out[c]), v);
                         }
-                        out[c] = v;
+                        put(out + c, v);
                     }
                 }
             }
@@ -467,19 +536,77 @@ static size_t al256(size_t x) { return (x + 255) / 256 * 256; }
 struct Shape {
     int nk, mt, nt, gA, gB;
     size_t a, b, small_a, small_b;     // bytes per matrix: digits of A, of B, exponents
-    Shape(int M, int N, int K) {
+    Shape(int S, int M, int N, int K) {
+        const int tn = 256 / S;
         nk = (K + kTK - 1) / kTK;
         mt = (M + kTM - 1) / kTM;
-        nt = (N + kTN - 1) / kTN;
+        nt = (N + tn - 1) / tn;
         gA = (M + 15) / 16;
         gB = (N + 15) / 16;
-        a = (size_t)mt * nk * kABlk;
-        b = (size_t)nt * nk * kBBlk;
+        a = (size_t)mt * nk * (2 * S * kTM * kTK * 2);
+        b = (size_t)nt * nk * (2 * S * tn * kTK * 2);
         small_a = (size_t)gA * 16 * sizeof(int);
         small_b = ((size_t)gB * 16 + K) * sizeof(int);
     }
     size_t bytes(int na, int nb) const { return al256(na * small_a) + al256(nb * small_b) + na * a + nb * b; }
 };
+
+// One product with S digits; element types double2 or float2 by operand.
+template <int S, typename TA, typename TB, typename TC>
+static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const TA* A, int lda, long long sA, const TB* B,
+                      int ldb, long long sB, int opB, double2 beta, double diag, TC* C, int ldc, long long sC, int batch,
+                      const GemmWs& ws, const int* skip) {
+    if (M <= 0 || N <= 0 || batch <= 0) return SCW_OK;
+    int sms = 0, dev = 0;
+    SCW_CUDA_TRY(cudaGetDevice(&dev));
+    SCW_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    constexpr size_t smem = Cfg<S>::kSmem;
+    SCW_CUDA_TRY(cudaFuncSetAttribute(oz_gemm_kernel<S, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const Shape sh(S, M, N, K);
+    const bool a1 = sA == 0 && !skip, b1 = sB == 0 && !skip;     // one operand for the whole batch
+    // element (k, j) of op(B) at k ksB + j rsB
+    const long long ksB = opB == kOpN ? ldb : 1, rsB = opB == kOpN ? 1 : ldb;
+    // as many matrices at a time as the workspace holds
+    int step = batch;
+    while (step > 1 && sh.bytes(a1 ? 1 : step, b1 ? 1 : step) > ws.bytes) step = (step + 1) / 2;
+    if (sh.bytes(1, 1) > ws.bytes) return fail(SCW_ERR_NOMEM, "zgemm: workspace too small");
+    for (int b0 = 0; b0 < batch; b0 += step) {
+        const int nb = std::min(step, batch - b0);
+        const int na_ = a1 ? 1 : nb, nb_ = b1 ? 1 : nb;
+        char* cur = ws.base;
+        int* eA = reinterpret_cast<int*>(cur);
+        cur += al256(na_ * sh.small_a);
+        int* gN = reinterpret_cast<int*>(cur);
+        int* f = gN + (size_t)nb_ * sh.gB * 16;
+        cur += al256(nb_ * sh.small_b);
+        unsigned char* dA = reinterpret_cast<unsigned char*>(cur);
+        unsigned char* dB = dA + na_ * sh.a;
+        const TA* Ab = A + sA * b0;
+        const TB* Bb = B + sB * b0;
+        const int* sk = skip ? skip + b0 : nullptr;
+        // with one A for several B the inner scaling would differ per matrix: none then
+        const bool scale = !(a1 && !b1);
+        if (K > 0) {
+            if (scale) {
+                oz_inner_kernel<TB><<<dim3((K + 7) / 8, nb_), 256, 0, st>>>(Bb, ksB, rsB, sB, K, N, f, sk);
+                SCW_CUDA_TRY(cudaGetLastError());
+            } else {
+                SCW_CUDA_TRY(cudaMemsetAsync(f, 0, sizeof(int) * (size_t)K * nb_, st));
+            }
+        }
+        SplitArgs sp{Ab, Bb, lda, 1, rsB, ksB, sA, sB, opB == kOpC, M, N, K, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB,
+                     na_ * sh.gA, f, eA, gN, dA, dB, b1 ? 0 : 1};
+        oz_split_kernel<S, TA, TB><<<na_ * sh.gA + nb_ * sh.gB, 256, 0, st>>>(sp, sk);
+        SCW_CUDA_TRY(cudaGetLastError());
+        const long long tiles = (long long)sh.mt * sh.nt * nb;
+        if (tiles > (1ll << 30)) return fail(SCW_ERR_ARG, "zgemm: too many tiles");
+        GemmArgs g{dA, dB, eA, gN, M, N, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB, a1, b1, alpha, beta, diag,
+                   (void*)(C + sC * b0), ldc, sC, (int)tiles, ws.err};
+        oz_gemm_kernel<S, TC><<<(unsigned)std::min<long long>(tiles, sms), kThreads, smem, st>>>(g, sk);
+        SCW_CUDA_TRY(cudaGetLastError());
+    }
+    return SCW_OK;
+}
 
 }  // namespace oz
 
@@ -505,66 +632,38 @@ scw_status ctx_gemm_ws(scw_ctx ctx, size_t one, size_t all, GemmWs& ws) {
     return st;
 }
 
-size_t zgemm_ws_bytes(int M, int N, int K, int batch) { return oz::Shape(M, N, K).bytes(batch, batch); }
+size_t zgemm_ws_bytes(int M, int N, int K, int batch) { return oz::Shape(8, M, N, K).bytes(batch, batch); }
 
 scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const double2* A, int lda, long long sA,
                  const double2* B, int ldb, long long sB, double2 beta, double2* C, int ldc, long long sC, int batch,
-                 const GemmWs& ws, const int* skip) {
+                 const GemmWs& ws, const int* skip, double diag, int opB) {
     if (M <= 0 || N <= 0 || batch <= 0) return SCW_OK;
-    if (N == 1) {
+    if (N == 1 && diag == 0.0 && opB == kOpN) {
         oz::zgemv_kernel<<<dim3((M + 7) / 8, batch), 256, 0, st>>>(M, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC,
                                                                   skip);
         SCW_CUDA_TRY(cudaGetLastError());
         return SCW_OK;
     }
+    if (!ws.base && (diag != 0.0 || opB != kOpN)) return fail(SCW_ERR_ARG, "zgemm: this product needs a workspace");
     if (!ws.base) return gemm<double2>(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, skip);
-    int sms = 0, dev = 0;
-    SCW_CUDA_TRY(cudaGetDevice(&dev));
-    SCW_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    constexpr size_t smem = oz::kStages * (oz::kABlk + oz::kBBlk) + (2 * oz::kStages + 4) * sizeof(uint64_t);
-    SCW_CUDA_TRY(cudaFuncSetAttribute(oz::oz_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const oz::Shape sh(M, N, K);
-    const bool a1 = sA == 0 && !skip, b1 = sB == 0 && !skip;     // one operand for the whole batch
-    // as many matrices at a time as the workspace holds
-    int step = batch;
-    while (step > 1 && sh.bytes(a1 ? 1 : step, b1 ? 1 : step) > ws.bytes) step = (step + 1) / 2;
-    if (sh.bytes(1, 1) > ws.bytes) return fail(SCW_ERR_NOMEM, "zgemm: workspace too small");
-    for (int b0 = 0; b0 < batch; b0 += step) {
-        const int nb = std::min(step, batch - b0);
-        const int na_ = a1 ? 1 : nb, nb_ = b1 ? 1 : nb;
-        char* cur = ws.base;
-        int* eA = reinterpret_cast<int*>(cur);
-        cur += oz::al256(na_ * sh.small_a);
-        int* gN = reinterpret_cast<int*>(cur);
-        int* f = gN + (size_t)nb_ * sh.gB * 16;
-        cur += oz::al256(nb_ * sh.small_b);
-        unsigned char* dA = reinterpret_cast<unsigned char*>(cur);
-        unsigned char* dB = dA + na_ * sh.a;
-        const double2* Ab = A + sA * b0;
-        const double2* Bb = B + sB * b0;
-        const int* sk = skip ? skip + b0 : nullptr;
-        // with one A for several B the inner scaling would differ per matrix: none then
-        const bool scale = !(a1 && !b1);
-        if (K > 0) {
-            if (scale) {
-                oz::oz_inner_kernel<<<dim3((K + 7) / 8, nb_), 256, 0, st>>>(Bb, ldb, sB, K, N, f, sk);
-                SCW_CUDA_TRY(cudaGetLastError());
-            } else {
-                SCW_CUDA_TRY(cudaMemsetAsync(f, 0, sizeof(int) * (size_t)K * nb_, st));
-            }
-        }
-        oz::SplitArgs sp{Ab, Bb, lda, ldb, sA, sB, M, N, K, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB, na_ * sh.gA, f, eA, gN,
-                         dA, dB, b1 ? 0 : 1};
-        oz::oz_split_kernel<<<na_ * sh.gA + nb_ * sh.gB, 256, 0, st>>>(sp, sk);
-        SCW_CUDA_TRY(cudaGetLastError());
-        const long long tiles = (long long)sh.mt * sh.nt * nb;
-        if (tiles > (1ll << 30)) return fail(SCW_ERR_ARG, "zgemm: too many tiles");
-        oz::GemmArgs g{dA, dB, eA, gN, M, N, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB, a1, b1, alpha, beta, C + sC * b0, ldc, sC,
-                       (int)tiles, ws.err};
-        oz::oz_gemm_kernel<<<(unsigned)std::min<long long>(tiles, sms), oz::kThreads, smem, st>>>(g, sk);
-        SCW_CUDA_TRY(cudaGetLastError());
-    }
-    return SCW_OK;
+    return oz::run<8>(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, opB, beta, diag, C, ldc, sC, batch, ws, skip);
 }
+
+template <typename TA, typename TB, typename TC>
+scw_status gemm32(cudaStream_t st, int n, double alpha, const TA* A, const TB* B, int opB, double beta, double diag, TC* C,
+                  int batch, const GemmWs& ws, const int* skip) {
+    const long long nn = (long long)n * n;
+    return oz::run<4>(st, n, n, n, make_double2(alpha, 0.0), A, n, nn, B, n, nn, opB, make_double2(beta, 0.0), diag, C, n,
+                      nn, batch, ws, skip);
+}
+#define SCW_GEMM32(TA, TB, TC)                                                                                        \
+    template scw_status gemm32<TA, TB, TC>(cudaStream_t, int, double, const TA*, const TB*, int, double, double, TC*, \
+                                           int, const GemmWs&, const int*);
+SCW_GEMM32(float2, float2, float2)
+SCW_GEMM32(float2, float2, double2)
+SCW_GEMM32(double2, float2, double2)
+SCW_GEMM32(double2, float2, float2)
+SCW_GEMM32(double2, double2, double2)
+#undef SCW_GEMM32
 
 }  // namespace scw

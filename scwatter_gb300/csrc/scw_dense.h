@@ -46,24 +46,41 @@ scw_status ctx_tc_flag(scw_ctx ctx);
 scw_status ctx_gemm_ws(scw_ctx ctx, size_t one, size_t all, GemmWs& ws);
 // workspace that takes the whole batch in one pass
 size_t zgemm_ws_bytes(int M, int N, int K, int batch);
-// C = alpha A B + beta C (row-major, batched by strides in elements), FP64 on the tensor cores; without
-// a workspace by gemm<double2>
+// C = alpha A op(B) + beta C + diag I (row-major, batched by strides in elements), FP64 on the tensor
+// cores; op = identity, transpose or conjugate transpose.  C may be A or B.  Without a workspace
+// by gemm<double2> (plain products only).
+enum : int { kOpN = 0, kOpT = 1, kOpC = 2 };
 scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const double2* A, int lda, long long sA,
                  const double2* B, int ldb, long long sB, double2 beta, double2* C, int ldc, long long sC, int batch,
-                 const GemmWs& ws, const int* skip = nullptr);
+                 const GemmWs& ws, const int* skip = nullptr, double diag = 0.0, int opB = kOpN);
+// The same kernel with 30-bit operands, for corrections that need FP32 accuracy: n x n matrices back
+// to back, C = alpha A op(B) + beta C + diag I.
+template <typename TA, typename TB, typename TC>
+scw_status gemm32(cudaStream_t st, int n, double alpha, const TA* A, const TB* B, int opB, double beta, double diag, TC* C,
+                  int batch, const GemmWs& ws, const int* skip);
 
 // C = alpha A B + beta C (row-major, batched by strides in elements)
 template <typename C>
 scw_status gemm(cudaStream_t st, int M, int N, int K, C alpha, const C* A, int lda, long long sA, const C* B, int ldb,
                 long long sB, C beta, C* Cm, int ldc, long long sC, int batch, const int* skip = nullptr);
-// in-place LU with partial pivoting of n x n matrices (leading dimension n); info[b] = first zero pivot + 1
+// in-place LU with partial pivoting of the first n columns of n x ncols matrices (leading dimension lda;
+// further columns are carried along as right-hand sides); info[b] = first zero pivot + 1
+scw_status zgetrf(cudaStream_t st, double2* A, int n, int ncols, int lda, long long sA, int* piv, long long sP, int* info,
+                  int batch, const GemmWs& ws, const int* skip);
+// B := U^-1 B with the upper factor of getrf
+scw_status ztrsm_upper(cudaStream_t st, const double2* LU, int n, int lda, long long sA, double2* B, int nrhs, int ldb,
+                       long long sB, int batch, const GemmWs& ws, const int* skip);
+// B := A^-1 B using getrf's factors (leading dimension n; B: n x nrhs, leading dimension nrhs)
+scw_status zgetrs(cudaStream_t st, const double2* LU, int n, long long sA, const int* piv, long long sP, double2* B,
+                  int nrhs, long long sB, int batch, const GemmWs& ws, const int* skip);
+// Schur form A = Q T Q^H (T over A, eigenvalues W); hw: 3 n per matrix
 template <typename C>
-scw_status getrf(cudaStream_t st, C* A, int n, long long sA, int* piv, long long sP, int* info, int batch,
-                 const GemmWs& ws);
-// B := A^-1 B using getrf's factors (B: n x nrhs, leading dimension nrhs)
+scw_status schur(cudaStream_t st, C* A, C* Q, C* W, int n, int batch, C* hw, int* status, const int* skip, bool wide);
+// eigenvectors of the triangular T as the rows of X (unit diagonal), and the inverse Z of the unit
+// triangular matrix whose columns those are
 template <typename C>
-scw_status getrs(cudaStream_t st, const C* LU, int n, long long sA, const int* piv, long long sP, C* B, int nrhs,
-                 long long sB, int batch, const GemmWs& ws);
+scw_status trevc(cudaStream_t st, const C* T, C* X, int n, int batch, const int* skip);
+scw_status trtri32(cudaStream_t st, const float2* X, float2* Z, int n, int batch);
 // eigenvalues W and right eigenvectors V (columns) of A (overwritten); work >= batch (n^2 + 3 n);
 // status[b] = 1 when the QR iteration did not converge.  wide: the Hessenberg reduction of
 // matrices with n >= kWideMinN is spread over the whole GPU (3 launches per column) instead of one
@@ -74,18 +91,6 @@ template <typename C>
 scw_status geev(cudaStream_t st, C* A, C* W, C* V, int n, int batch, C* work, int* status, const int* skip, bool wide,
                 const GemmWs& ws);
 
-inline scw_status zgetrf(cudaStream_t st, double2* A, int n, long long sA, int* piv, long long sP, int* info,
-                         int batch, const GemmWs& ws) {
-    return getrf<double2>(st, A, n, sA, piv, sP, info, batch, ws);
-}
-inline scw_status zgetrs(cudaStream_t st, const double2* LU, int n, long long sA, const int* piv, long long sP,
-                         double2* B, int nrhs, long long sB, int batch, const GemmWs& ws) {
-    return getrs<double2>(st, LU, n, sA, piv, sP, B, nrhs, sB, batch, ws);
-}
-inline scw_status zgeev(cudaStream_t st, double2* A, double2* W, double2* V, int n, int batch, double2* work,
-                        int* status, bool wide, const GemmWs& ws) {
-    return geev<double2>(st, A, W, V, n, batch, work, status, nullptr, wide, ws);
-}
 // Hessenberg form of A (in place, n x n per batch entry) and the unitary Q (A = Q H Q^H);
 // work >= batch * 3 n
 scw_status zgehrd(cudaStream_t st, double2* A, double2* Q, int n, int batch, double2* work);

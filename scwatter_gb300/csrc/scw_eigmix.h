@@ -5,11 +5,15 @@
 // and FP64 accuracy comes back through Newton refinement of all eigenpairs at once, which
 // costs one FP64 GEMM per step spread over every SM:
 //   R = A X - X diag(lambda)          (FP64 GEMM)
-//   E = X^-1 R                        (FP32 LU of X)
-//   lambda_i += E_ii, X += X F,  F_ij = E_ij / (lambda_j - lambda_i)   (FP32 GEMM, FP64 sum)
+//   E = X^-1 R                        (FP32 inverse, kept)
+//   lambda_i += E_ii, X += X F,  F_ij = E_ij / (lambda_j - lambda_i)   (30-bit product, FP64 sum)
+//   X^-1 += X^-1 (I - X X^-1)         (30-bit products; Newton-Schulz)
+// The first X^-1 is that of the FP32 eigenvectors, X = Q Xt: Xt^-1 Q^H with Xt triangular.  Every
+// product runs on the tensor cores; an FP32 LU of X per step, as before, spent 9 of 10 parts of a
+// step's time in its panels and triangular solves.
 // Eigenvalues closer than tau_rel * ||A||_1 form clusters.  Within a cluster the k x k block
 // diag(lambda) + E is solved in FP64 by a small Schur decomposition.  Its eigenvectors then
-// rotate the cluster's columns.  A slice stops refining when every column's relative residual
+// rotate the cluster's columns (and their inverse its rows of X^-1).  A slice stops refining when every column's relative residual
 // ||A x - lambda x|| / (||A||_1 ||x||) is at most tol, and after the last step it is accepted
 // when that residual is at most tol_accept.  Otherwise (FP32 QR not converged, a cluster above
 // kMaxCluster, a singular X, no convergence within the step limit) that slice goes through the
@@ -28,11 +32,13 @@ constexpr int kMaxN = 4096;         // largest matrix taken by the mixed path
 
 struct EigMixWs {
     // four FP32 n x n slots per matrix (S0 and S1 adjacent: together one FP64 n x n slot)
+    // (after a solve S2 holds the FP32 inverse of every accepted eigenvector matrix)
     float2 *S0, *S1, *S2, *S3;
     float2 *hw;                     // 3 n per matrix, directly after S1 (FP32 QR work)
     float2 *lam32;                  // n per matrix
-    int *label, *member, *cstart, *ncl, *piv, *info, *qr, *state, *steps;
+    int *label, *member, *cstart, *ncl, *qr, *state, *steps;
     double2* Y;                     // kMaxCluster * n per matrix: cluster eigenvector blocks
+    float2* Yi;                     // and their inverses
     double *rn, *xn, *anorm, *res;  // column residual / norm sums, ||A||_1, max residual
 };
 

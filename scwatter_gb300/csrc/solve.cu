@@ -148,21 +148,59 @@ __global__ void roots_kernel(const double2* __restrict__ lam, int n, int Z, cons
     E[e] = make_double2(m * c, m * s);
 }
 
-// X[b][:, j] /= f[b][j]
-__global__ void coldiv_kernel(double2* __restrict__ X, int n, const double2* __restrict__ f, int batch) {
+// X[b][:, j] /= f[b][j] (columns), or X[b][i, :] /= f[b][i] (rows)
+__global__ void scale_inv_kernel(double2* __restrict__ X, int n, const double2* __restrict__ f, int batch, int rows) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long per = (long long)n * n;
     if (e >= per * batch) return;
-    const int b = (int)(e / per), j = (int)(e % n);
+    const int b = (int)(e / per), j = rows ? (int)((e % per) / n) : (int)(e % n);
     X[e] = cmul(X[e], cinv(f[(long long)b * n + j]));
 }
 
-__global__ void identity_kernel(double2* __restrict__ X, int n, int batch) {
+// identity matrices (skip[b] != 0: matrix b stays)
+__global__ void identity_kernel(double2* __restrict__ X, int n, int batch, const int* __restrict__ skip) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long per = (long long)n * n;
-    if (e >= per * batch) return;
+    if (e >= per * batch || (skip && skip[e / per])) return;
     const long long r = e % per;
     X[e] = make_double2((r / n) == (r % n) ? 1.0 : 0.0, 0.0);
+}
+
+__global__ void copy_matrices_kernel(const double2* __restrict__ src, double2* __restrict__ dst, long long per, int batch,
+                                     const int* __restrict__ skip) {
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < per * batch && !skip[e / per]) dst[e] = src[e];
+}
+
+__global__ void widen_kernel(const float2* __restrict__ a, double2* __restrict__ b, long long n) {
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < n) b[e] = make_double2(a[e].x, a[e].y);
+}
+
+// worst[b] = largest part of any entry of G[b] (NaN above all); worst starts at zero
+__global__ void __launch_bounds__(256) max_part_kernel(const double2* __restrict__ G, long long per, double* __restrict__ worst) {
+    G += per * blockIdx.y;
+    double m = 0.0;
+    for (long long e = blockIdx.x * 256ll + threadIdx.x; e < per; e += gridDim.x * 256ll) {
+        const double2 g = G[e];
+        const double a = fabs(g.x), c = fabs(g.y);
+        m = a > m || a != a ? a : m;
+        m = c > m || c != c ? c : m;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const double v = __shfl_xor_sync(0xffffffffu, m, o);
+        m = v > m || v != v ? v : m;
+    }
+    // non-negative doubles order as integers, NaN above them
+    if ((threadIdx.x & 31) == 0)
+        atomicMax(reinterpret_cast<unsigned long long*>(worst + blockIdx.y), (unsigned long long)__double_as_longlong(m));
+}
+
+// good[b] = the last Newton step of inverse b started close enough: n max |I - M M^-1| <= 1e-7, so
+// that its result is within 1e-14
+__global__ void newton_gate_kernel(const double* __restrict__ worst, int n, int batch, int* __restrict__ good) {
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < batch) good[b] = (double)n * worst[b] <= 1e-7;
 }
 
 // [Yt; Yb] from A1 = U^-1 Xt, A2 = W^-1 Xb (rows i scaled by E_i):
@@ -209,6 +247,74 @@ __global__ void f3_kernel(const double* __restrict__ Sx, const double* __restric
     F[e] = v;
 }
 
+// f3 with the z columns eliminated by the divergence rows, Tz = -(Sx Tx + Sy Ty) / Sz1 (4MF x 2MF)
+__global__ void f3_reduced_kernel(const double* __restrict__ Sx, const double* __restrict__ Sy,
+                                  const double2* __restrict__ Sz1, int MF, double2* __restrict__ F) {
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = 2 * MF;
+    if (e >= 4LL * MF * n) return;
+    const int r = (int)(e / n), c = (int)(e % n);
+    const int blk = r / MF, m = r % MF;
+    double2 v = make_double2(0, 0);
+    if (c % MF == m) {
+        const double2 i1 = cinv(Sz1[m]);
+        const double sx = Sx[m], sy = Sy[m];
+        const bool y = c >= MF;
+        if (blk == 0 && !y) v = make_double2(-1, 0);
+        else if (blk == 1 && y) v = make_double2(-1, 0);
+        else if (blk == 2 && !y) v = make_double2(sx * sy * i1.x, sx * sy * i1.y);
+        else if (blk == 2) v = make_double2(Sz1[m].x + sy * sy * i1.x, Sz1[m].y + sy * sy * i1.y);
+        else if (blk == 3 && !y) v = make_double2(-Sz1[m].x - sx * sx * i1.x, -Sz1[m].y - sx * sx * i1.y);
+        else if (blk == 3) v = make_double2(-sx * sy * i1.x, -sx * sy * i1.y);
+    }
+    F[e] = v;
+}
+
+// The boundary system with Rz (divergence rows), Rx and Ry (first 2MF matching rows) eliminated: the
+// 2MF x 2MF matrix for (Tx, Ty) and its right-hand side as column 2MF.  T3: 4MF x 2MF, f: f1 EF.
+//   Rx = -f0 - t0 T, Ry = -f1 - t1 T, Rz = (Sx Rx + Sy Ry) / Sz0,
+//   row m: (t2 - a t0 - b t1) T = -f2 + a f0 + b f1,  a = Sx Sy / Sz0,  b = Sz0 + Sy^2 / Sz0
+//   row MF + m: (t3 - c t0 - d t1) T = -f3 + c f0 + d f1,  c = -Sz0 - Sx^2 / Sz0,  d = -a
+__global__ void bc_reduced_kernel(const double* __restrict__ Sx, const double* __restrict__ Sy,
+                                  const double2* __restrict__ Sz0, const double2* __restrict__ T3,
+                                  const double2* __restrict__ f, int MF, double2* __restrict__ A) {
+    const int n = 2 * MF, ld = n + 1;
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (long long)MF * ld) return;
+    const int m = (int)(e / ld), j = (int)(e % ld);
+    const double2 s0 = Sz0[m], i0 = cinv(s0);
+    const double sx = Sx[m], sy = Sy[m];
+    const double2 a = make_double2(sx * sy * i0.x, sx * sy * i0.y);
+    const double2 b = make_double2(s0.x + sy * sy * i0.x, s0.y + sy * sy * i0.y);
+    const double2 c = make_double2(-s0.x - sx * sx * i0.x, -s0.y - sx * sx * i0.y);
+    double2 t[4];
+    for (int q = 0; q < 4; q++) {
+        t[q] = j < n ? T3[((long long)q * MF + m) * n + j] : f[q * MF + m];
+        if (j == n) t[q] = make_double2(-t[q].x, -t[q].y);
+    }
+    A[(long long)m * ld + j] = csub(csub(t[2], cmul(a, t[0])), cmul(b, t[1]));
+    A[(long long)(MF + m) * ld + j] = cadd(csub(t[3], cmul(c, t[0])), cmul(a, t[1]));
+}
+
+// x (6MF) from (Tx, Ty) = column 2MF of A and r = [t0; t1] T
+__global__ void bc_expand_kernel(const double* __restrict__ Sx, const double* __restrict__ Sy,
+                                 const double2* __restrict__ Sz0, const double2* __restrict__ Sz1,
+                                 const double2* __restrict__ f, const double2* __restrict__ A,
+                                 const double2* __restrict__ r, int MF, double2* __restrict__ x) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x, n = 2 * MF, ld = n + 1;
+    if (m >= MF) return;
+    const double2 tx = A[(long long)m * ld + n], ty = A[(long long)(MF + m) * ld + n];
+    const double2 rx = make_double2(-f[m].x - r[m].x, -f[m].y - r[m].y);
+    const double2 ry = make_double2(-f[MF + m].x - r[MF + m].x, -f[MF + m].y - r[MF + m].y);
+    const double sx = Sx[m], sy = Sy[m];
+    x[m] = rx;
+    x[MF + m] = ry;
+    x[2 * MF + m] = cmul(make_double2(sx * rx.x + sy * ry.x, sx * rx.y + sy * ry.y), cinv(Sz0[m]));
+    x[3 * MF + m] = tx;
+    x[4 * MF + m] = ty;
+    x[5 * MF + m] = cmul(make_double2(-sx * tx.x - sy * ty.x, -sx * tx.y - sy * ty.y), cinv(Sz1[m]));
+}
+
 // the 6MF x 6MF boundary matrix (sCWatter.cpp:143-146, 393-461): divergence constraints,
 // then [f2 | T3] with T3 = Gd_0 Gc_static^-1 f3 (4MF x 3MF)
 __global__ void bc_matrix_kernel(const double* __restrict__ Sx, const double* __restrict__ Sy,
@@ -246,35 +352,61 @@ __global__ void bc_matrix_kernel(const double* __restrict__ Sx, const double* __
     A[e] = v;
 }
 
-// Kn[m_i][m_j] = scale * NIf[lin] with lin the wrapped difference index read column-major
-// (sCWatter.cpp:839-871 reads NIf(lin) on a column-major Eigen matrix)
-__global__ void kn_kernel(const double2* __restrict__ NiF, int M0, int M1, double scale, double2* __restrict__ Kn) {
+// Kn[l][m_i][m_j] = scale * NIf[lin] with lin the wrapped difference index read column-major
+// (sCWatter.cpp:839-871 reads NIf(lin) on a column-major Eigen matrix); coef as in build_pq_kernel
+__global__ void kn_kernel(const double2* __restrict__ coef, int M0, int M1, int Z, double scale, double2* __restrict__ Kn) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int MF = M0 * M1;
-    if (e >= (long long)MF * MF) return;
-    const int mi = (int)(e / MF), mj = (int)(e % MF);
+    const long long per = (long long)MF * MF;
+    if (e >= per * Z) return;
+    const int l = (int)(e / per), mi = (int)(e % per / MF), mj = (int)(e % MF);
     const int qi = mi / M0, pi_ = mi % M0, qj = mj / M0, pj = mj % M0;
     const int lin = (((qi - qj + M1) % M1 + M1 / 2) % M1) * M0 + ((pi_ - pj + M0) % M0 + M0 / 2) % M0;
-    const double2 v = NiF[lin];
+    const double2 v = coef[((long long)2 * l + 1) * MF + lin];
     Kn[e] = make_double2(v.x * scale, v.y * scale);
 }
 
-// rows Ex, Ey of Q_check / Q_hat: U diag(beta);  Hm = sign (up_m Hy - wq_m Hx) for the Ez step,
-// with Hx, Hy = rows of W diag(beta) (sign -1 for the upward modes, whose H rows are -W).
-// beta == null: unit amplitudes (the paired set's block V = [U; Kn (up W_y - wq W_x)])
-__global__ void q_rows_kernel(const double2* __restrict__ U, const double2* __restrict__ Wm,
-                              const double2* __restrict__ beta, int MF, double sign, const double* __restrict__ up_pz,
-                              const double* __restrict__ wq_pz, double2* __restrict__ Qout, double2* __restrict__ Hm) {
+// Hm[l] = up Hy - wq Hx with Hx, Hy the rows of W (unit amplitudes): the right factor of the Ez step.
+// The upward modes' H rows are -W and every amplitude is a column factor, so one product Kn Hm per
+// slice serves Q_check, Q_hat and the paired set.
+__global__ void hm_kernel(const double2* __restrict__ Wm, int MF, int Z, const double* __restrict__ up_pz,
+                          const double* __restrict__ wq_pz, double2* __restrict__ Hm) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int n = 2 * MF;
-    if (e >= (long long)n * n) return;
-    const int r = (int)(e / n), j = (int)(e % n);
-    const double2 b = beta ? beta[j] : make_double2(1.0, 0.0);
-    Qout[e] = cmul(U[e], b);
-    if (Hm && r < MF) {
-        const double2 hx = cmul(Wm[e], b);
-        const double2 hy = cmul(Wm[(long long)(MF + r) * n + j], b);
-        Hm[e] = make_double2(sign * (up_pz[r] * hy.x - wq_pz[r] * hx.x), sign * (up_pz[r] * hy.y - wq_pz[r] * hx.y));
+    const long long per = (long long)MF * n;
+    if (e >= per * Z) return;
+    const int l = (int)(e / per), r = (int)(e % per / n), j = (int)(e % n);
+    const double2 hx = Wm[((long long)l * n + r) * n + j], hy = Wm[((long long)l * n + MF + r) * n + j];
+    Hm[e] = make_double2(up_pz[r] * hy.x - wq_pz[r] * hx.x, up_pz[r] * hy.y - wq_pz[r] * hx.y);
+}
+
+// Mode amplitudes of every slice from the rows [U; Ez] (Ez null: zero): Q_check = [U; Ez] beta_dn,
+// Q_hat = [U; -Ez] beta_up (sCWatter.cpp:781-871) in FP64 and / or complex64, and the paired set's
+// block V = [U; Ez].  Any output may be null.
+__global__ void modes_kernel(const double2* __restrict__ U, const double2* __restrict__ Ez,
+                             const double2* __restrict__ beta, int MF, int Z, double2* __restrict__ Q64,
+                             float2* __restrict__ Qsep, float2* __restrict__ Vsep) {
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = 2 * MF, M3 = 3 * MF;
+    const long long per = (long long)M3 * n;
+    if (e >= per * Z) return;
+    const int l = (int)(e / per), r = (int)(e % per / n), j = (int)(e % n);
+    double2 v = make_double2(0.0, 0.0);
+    if (r < n) v = U[((long long)l * n + r) * n + j];
+    else if (Ez) v = Ez[((long long)l * MF + r - n) * n + j];
+    if (Vsep) Vsep[e] = make_float2((float)v.x, (float)v.y);
+    const double2 bd = beta[(long long)l * 2 * n + j], bu = beta[(long long)l * 2 * n + n + j];
+    const double2 qd = cmul(v, bd);
+    double2 qu = cmul(v, bu);
+    if (r >= n) qu = make_double2(-qu.x, -qu.y);
+    const long long od = ((long long)2 * l * M3 + r) * n + j, ou = od + per;
+    if (Q64) {
+        Q64[od] = qd;
+        Q64[ou] = qu;
+    }
+    if (Qsep) {
+        Qsep[od] = make_float2((float)qd.x, (float)qd.y);
+        Qsep[ou] = make_float2((float)qu.x, (float)qu.y);
     }
 }
 
@@ -466,6 +598,10 @@ scw_status plan_solve(const scw_solve_params* prm, int Zs, int Y, int X, SolvePl
         p.Sz0[f] = std::sqrt(ni0 * ni0 - cd(sx * sx) - cd(sy * sy));
         p.Sz1[f] = std::sqrt(ni1 * ni1 - cd(sx * sx) - cd(sy * sy));
     }
+    // no harmonic grazes an outer medium: the boundary system can divide by every Sz
+    p.reduced_bc = true;
+    for (int f = 0; f < MF; f++)
+        p.reduced_bc = p.reduced_bc && std::abs(p.Sz0[f]) >= 0.02 && std::abs(p.Sz1[f]) >= 0.02;
     // the DFT rows / columns that land in the centred crop after the shift
     std::vector<int> ix, iy;
     fft_shift_index(Y, X, ix, iy);
@@ -528,9 +664,9 @@ void carve_in(const SolvePlan& p, Carver& c, SolveIn& in) {
 void carve_ws(const SolvePlan& p, Carver& c, SolveWs& ws) {
     const size_t Z = p.Z, MF = p.MF, n = p.n, nn = n * n, N4 = 4 * MF, M3 = 3 * MF, M6 = 6 * MF;
     ws.coef = c.take<double2>(Z * 2 * MF);
-    ws.P = c.take<double2>(Z * (nn + 3 * n));     // P, then eigen-solver work, then U^-1
-    ws.Q = c.take<double2>(Z * nn);               // Q, then LU factors
-    ws.PQ = c.take<double2>(Z * nn);              // PQ, then W^-1
+    ws.P = c.take<double2>(Z * (nn + 3 * n));     // P, then eigen-solver work, then the inverses' scratch
+    ws.Q = c.take<double2>(Z * nn);               // Q, then W^-1
+    ws.PQ = c.take<double2>(Z * nn);              // PQ, then U^-1
     ws.U = c.take<double2>(Z * nn);
     ws.W = c.take<double2>(Z * nn);
     ws.lam = c.take<double2>(Z * n);
@@ -538,6 +674,8 @@ void carve_ws(const SolvePlan& p, Carver& c, SolveWs& ws) {
     ws.beta = c.take<double2>(Z * N4);
     ws.v = c.take<double2>(N4);
     ws.piv = c.take<int>(std::max(Z * n, M6));
+    ws.worst = c.take<double>(2 * Z);
+    ws.good = c.take<int>(2 * Z);
     // mixed eigen-solver: small buffers of its own; S0, S1 (adjacent), its QR work and the FP32
     // eigenvalues inside P (Z (n^2 + 3 n) double2 >= 2 Z n^2 + 4 Z n float2), S2, S3 inside W
     if (p.eig_mixed) {
@@ -553,27 +691,23 @@ void carve_ws(const SolvePlan& p, Carver& c, SolveWs& ws) {
         ws.mix.S3 = Wf + Z * nn;
     }
     // operands of the FP64 products: the largest of them for one matrix, a whole batch up to the cap
-    const size_t one = std::max({zgemm_ws_bytes((int)n, (int)M3, (int)n, 1), zgemm_ws_bytes((int)M6, (int)M6, 64, 1),
+    const size_t one = std::max({zgemm_ws_bytes((int)n, (int)M3, (int)n, 1), zgemm_ws_bytes((int)M6, (int)M6, 32, 1),
                                  zgemm_ws_bytes(p.X, p.M1, p.Y, 1), zgemm_ws_bytes(p.M0, p.M1, p.X, 1)});
     ws.gemm.bytes = std::max(one, std::min(one * Z, kGemmWsCap));
     ws.gemm.base = c.take<char>(ws.gemm.bytes);
-    // temporary region, three overlays
+    // temporary region, two overlays
     const size_t t0 = (c.off + 255) / 256 * 256;
     Carver ca{c.base, t0};
     ws.F = ca.take<double2>(2 * Z * (size_t)p.Y * p.X);
     ws.T = ca.take<double2>(2 * Z * (size_t)p.X * p.M1);
     Carver cc{c.base, t0};
-    ws.X = cc.take<double2>(N4 * M3);
-    ws.A1 = cc.take<double2>(n * M3);
-    ws.A2 = cc.take<double2>(n * M3);
-    const size_t tA = (cc.off + 255) / 256 * 256;
-    ws.A = cc.take<double2>(M6 * M6);
-    ws.b = cc.take<double2>(M6);
-    Carver cm{c.base, tA};
-    ws.Kn = cm.take<double2>(MF * MF);
-    ws.Hm = cm.take<double2>(MF * n);
-    ws.Qtmp = cm.take<double2>(M3 * n);
-    c.off = std::max(ca.off, std::max(cc.off, cm.off));
+    // columns of the cascade: (Tx, Ty), or all three components where a harmonic grazes
+    const size_t nc = p.reduced_bc ? n : M3, nb = p.reduced_bc ? n : M6;
+    ws.X = cc.take<double2>(N4 * nc);
+    ws.A1 = cc.take<double2>(2 * n * nc);
+    ws.A = cc.take<double2>(nb * (nb + 1));
+    ws.b = cc.take<double2>(nb);
+    c.off = std::max(ca.off, cc.off);
 }
 
 void carve_out(const SolvePlan& p, Carver& c, SolveOut& out, bool q64, bool sep) {
@@ -633,6 +767,85 @@ scw_status upload_inputs(const SolvePlan& p, const double* sample, const SolveIn
 // ---------------------------------------------------------------------------------------
 // Recording (launches only): sCWatter.cpp:248-871 restated on the reduced problem
 // ---------------------------------------------------------------------------------------
+// W = Q U Gamma^-1 and the inverses of U and W.  The eigen-solver leaves U^-1 in FP32; two Newton steps
+// Y += Y (I - U Y) make it an FP64 inverse (the residuals in FP64, the corrections need 30 bits).
+// P W = P Q U Gamma^-1 = U Gamma gives W^-1 = Gamma^-1 U^-1 P, and one Newton step removes the
+// eigenpairs' residual from it.  All of it is products.  A slice whose last step started too far off
+// (the FP64 solver took its eigenpairs, or U is ill-conditioned) is inverted by LU, as every slice
+// is when the FP64 solver ran throughout.  On entry U holds the modes and mix.S2 (in the W block) the
+// FP32 inverse; PQ and P are free.
+static scw_status record_inverses(const SolvePlan& p, const SolveIn& in, const SolveWs& ws, const SolveOut& out,
+                                  double2* Uinv, double2* Winv, cudaStream_t st, long long* L) {
+    const int Zs = p.Z, n = p.n;
+    const long long nn = (long long)n * n;
+    const double2 minus = {-1.0, 0.0};
+    double2* G = ws.P;
+    int *goodU = ws.good, *goodW = ws.good + Zs;
+    auto residual = [&](const double2* M, const double2* Y, double* worst) -> scw_status {     // G = I - M Y
+        SCW_TRY(zgemm(st, n, n, n, minus, M, n, nn, Y, n, nn, kZero, G, n, nn, Zs, ws.gemm, nullptr, 1.0));
+        if (worst) {
+            max_part_kernel<<<dim3((unsigned)std::min<long long>(nblk(nn), 256), Zs), 256, 0, st>>>(G, nn, worst);
+            SCW_CUDA_TRY(cudaGetLastError());
+        }
+        *L += 4;
+        return SCW_OK;
+    };
+    auto correct = [&](double2* Y) { *L += 3; return scw::gemm32(st, n, 1.0, Y, G, kOpN, 1.0, 0.0, Y, Zs, ws.gemm, nullptr); };
+    if (p.eig_mixed) {
+        SCW_CUDA_TRY(cudaMemsetAsync(ws.worst, 0, sizeof(double) * 2 * Zs, st));
+        widen_kernel<<<nblk(nn * Zs), 256, 0, st>>>(ws.mix.S2, Uinv, nn * Zs);
+        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_TRY(residual(ws.U, Uinv, nullptr));
+        SCW_TRY(correct(Uinv));
+        SCW_TRY(residual(ws.U, Uinv, ws.worst));
+        SCW_TRY(correct(Uinv));
+    }
+    // W = Q U Gamma^-1
+    SCW_TRY(zgemm(st, n, n, n, kOne, ws.Q, n, nn, ws.U, n, nn, kZero, ws.W, n, nn, Zs, ws.gemm));
+    scale_inv_kernel<<<nblk(nn * Zs), 256, 0, st>>>(ws.W, n, out.gam, Zs, 0);
+    SCW_CUDA_TRY(cudaGetLastError());
+    *L += 4;
+    if (p.eig_mixed) {
+        // P again (the eigen-solver worked in its block; Q gets the values it has)
+        build_pq_kernel<<<dim3(nblk(n), n, Zs), 256, 0, st>>>(ws.coef, in.up, in.wq, in.qs, in.ps, p.M0, p.M1, p.k, ws.P,
+                                                              ws.Q);
+        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_TRY(zgemm(st, n, n, n, kOne, Uinv, n, nn, ws.P, n, nn, kZero, Winv, n, nn, Zs, ws.gemm));
+        scale_inv_kernel<<<nblk(nn * Zs), 256, 0, st>>>(Winv, n, out.gam, Zs, 1);
+        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_TRY(residual(ws.W, Winv, ws.worst + Zs));
+        SCW_TRY(correct(Winv));
+        newton_gate_kernel<<<nblk(2 * Zs), 256, 0, st>>>(ws.worst, n, 2 * Zs, ws.good);
+        SCW_CUDA_TRY(cudaGetLastError());
+        *L += 7;
+        // outside a capture the host looks whether any slice is left for the LU
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        SCW_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+        if (cap == cudaStreamCaptureStatusNone) {
+            std::vector<int> good(2 * Zs);
+            SCW_CUDA_TRY(cudaMemcpyAsync(good.data(), ws.good, sizeof(int) * 2 * Zs, cudaMemcpyDeviceToHost, st));
+            SCW_CUDA_TRY(cudaStreamSynchronize(st));
+            if (std::count(good.begin(), good.end(), 0) == 0) {
+                SCW_CUDA_TRY(cudaMemsetAsync(out.status + Zs, 0, sizeof(int) * 2 * Zs, st));
+                return SCW_OK;
+            }
+        }
+    } else {
+        SCW_CUDA_TRY(cudaMemsetAsync(ws.good, 0, sizeof(int) * 2 * Zs, st));
+    }
+    for (int which = 0; which < 2; which++) {
+        double2* inv = which == 0 ? Uinv : Winv;
+        const int* good = which == 0 ? goodU : goodW;
+        copy_matrices_kernel<<<nblk(nn * Zs), 256, 0, st>>>(which == 0 ? ws.U : ws.W, ws.P, nn, Zs, good);
+        identity_kernel<<<nblk(nn * Zs), 256, 0, st>>>(inv, n, Zs, good);
+        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_TRY(zgetrf(st, ws.P, n, n, n, nn, ws.piv, n, out.status + (1 + which) * Zs, Zs, ws.gemm, good));
+        SCW_TRY(zgetrs(st, ws.P, n, nn, ws.piv, n, inv, n, nn, Zs, ws.gemm, good));
+        *L += 3 + 13 * ((n + 31) / 32);
+    }
+    return SCW_OK;
+}
+
 scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws, const SolveOut& out,
                         cudaStream_t st, long long* launches) {
     const int Zs = p.Z, Y = p.Y, X = p.X, M0 = p.M0, M1 = p.M1, MF = p.MF, n = p.n;
@@ -662,51 +875,52 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
             SCW_CUDA_TRY(cudaMemcpyAsync(out.eig_res, ws.mix.res, sizeof(double) * Zs, cudaMemcpyDeviceToDevice, st));
         }
     } else {
-        SCW_TRY(zgeev(st, ws.PQ, ws.lam, ws.U, n, Zs, ws.P, out.status, p.wide_hess, ws.gemm));
+        SCW_TRY(scw::geev<double2>(st, ws.PQ, ws.lam, ws.U, n, Zs, ws.P, out.status, nullptr, p.wide_hess, ws.gemm));
         L += 5;
     }
     roots_kernel<<<nblk((long long)n * Zs), 256, 0, st>>>(ws.lam, n, Zs, in.dz, k, out.gam, ws.E);
     SCW_CUDA_TRY(cudaGetLastError());
-    // W = Q U Gamma^-1
-    SCW_TRY(zgemm(st, n, n, n, kOne, ws.Q, n, nn, ws.U, n, nn, kZero, ws.W, n, nn, Zs, ws.gemm));
-    coldiv_kernel<<<nblk(nn * Zs), 256, 0, st>>>(ws.W, n, out.gam, Zs);
-    SCW_CUDA_TRY(cudaGetLastError());
-    L += 8;
-    // U^-1 into P, W^-1 into PQ (LU factors in Q)
-    double2* Uinv = ws.P;
-    double2* Winv = ws.PQ;
-    for (int which = 0; which < 2; which++) {
-        double2* inv = which == 0 ? Uinv : Winv;
-        identity_kernel<<<nblk(nn * Zs), 256, 0, st>>>(inv, n, Zs);
-        SCW_CUDA_TRY(cudaGetLastError());
-        SCW_CUDA_TRY(cudaMemcpyAsync(ws.Q, which == 0 ? ws.U : ws.W, sizeof(double2) * nn * Zs,
-                                     cudaMemcpyDeviceToDevice, st));
-        SCW_TRY(zgetrf(st, ws.Q, n, nn, ws.piv, n, out.status + (1 + which) * Zs, Zs, ws.gemm));
-        SCW_TRY(zgetrs(st, ws.Q, n, nn, ws.piv, n, inv, n, nn, Zs, ws.gemm));
-        L += 2 + 3 * ((n + 31) / 32);
-    }
+    // U^-1 (into PQ) and W = Q U Gamma^-1, W^-1 (into Q)
+    double2* Uinv = ws.PQ;
+    double2* Winv = ws.Q;
+    SCW_TRY(record_inverses(p, in, ws, out, Uinv, Winv, st, &L));
     // T3 = Gd_0 Gc_static^-1 f3 = prod_l V_l diag(E_l^-1, E_l) V_l^-1 f3
-    f3_kernel<<<nblk((long long)N4 * M3), 256, 0, st>>>(in.Sx, in.Sy, in.Sz1, MF, ws.X);
+    const int nc = p.reduced_bc ? n : M3;
+    if (p.reduced_bc)
+        f3_reduced_kernel<<<nblk((long long)N4 * nc), 256, 0, st>>>(in.Sx, in.Sy, in.Sz1, MF, ws.X);
+    else
+        f3_kernel<<<nblk((long long)N4 * nc), 256, 0, st>>>(in.Sx, in.Sy, in.Sz1, MF, ws.X);
     SCW_CUDA_TRY(cudaGetLastError());
+    // the two products of each half-step (U^-1 and W^-1, then U and W) run as one batch of two
+    double2* A2 = ws.A1 + (size_t)n * nc;
     for (int l = Zs - 1; l >= 0; l--) {
-        const long long o = (long long)l * nn;
-        SCW_TRY(zgemm(st, n, M3, n, kOne, Uinv + o, n, 0, ws.X, M3, 0, kZero, ws.A1, M3, 0, 1, ws.gemm));
-        SCW_TRY(zgemm(st, n, M3, n, kOne, Winv + o, n, 0, ws.X + (size_t)n * M3, M3, 0, kZero, ws.A2, M3, 0, 1, ws.gemm));
-        mix_kernel<<<nblk((long long)n * M3), 256, 0, st>>>(ws.A1, ws.A2, ws.E + (size_t)l * n, n, M3, 0);
+        const long long o = (long long)l * nn, half = (long long)n * nc;
+        SCW_TRY(zgemm(st, n, nc, n, kOne, Uinv + o, n, Winv - Uinv, ws.X, nc, half, kZero, ws.A1, nc, half, 2, ws.gemm));
+        mix_kernel<<<nblk(half), 256, 0, st>>>(ws.A1, A2, ws.E + (size_t)l * n, n, nc, 0);
         SCW_CUDA_TRY(cudaGetLastError());
-        SCW_TRY(zgemm(st, n, M3, n, kOne, ws.U + o, n, 0, ws.A1, M3, 0, kZero, ws.X, M3, 0, 1, ws.gemm));
-        SCW_TRY(zgemm(st, n, M3, n, kOne, ws.W + o, n, 0, ws.A2, M3, 0, kZero, ws.X + (size_t)n * M3, M3, 0, 1, ws.gemm));
-        L += 5;
+        SCW_TRY(zgemm(st, n, nc, n, kOne, ws.U + o, n, ws.W - ws.U, ws.A1, nc, half, kZero, ws.X, nc, half, 2, ws.gemm));
+        L += 7;
     }
     // boundary system and its solve (sCWatter.cpp:393-461, 722)
-    bc_matrix_kernel<<<nblk((long long)M6 * M6), 256, 0, st>>>(in.Sx, in.Sy, in.Sz0, in.Sz1, ws.X, MF, ws.A);
-    SCW_CUDA_TRY(cudaGetLastError());
-    bc_rhs_kernel<<<nblk(M6), 256, 0, st>>>(in.f1EF, MF, ws.b);
-    SCW_CUDA_TRY(cudaGetLastError());
-    SCW_TRY(zgetrf(st, ws.A, M6, 0, ws.piv, 0, out.status + 3 * Zs, 1, ws.gemm));
-    SCW_TRY(zgetrs(st, ws.A, M6, 0, ws.piv, 0, ws.b, 1, 0, 1, ws.gemm));
-    SCW_CUDA_TRY(cudaMemcpyAsync(out.x, ws.b, sizeof(double2) * M6, cudaMemcpyDeviceToDevice, st));
-    L += 4 + 3 * ((M6 + 31) / 32);
+    if (p.reduced_bc) {
+        bc_reduced_kernel<<<nblk((long long)MF * (n + 1)), 256, 0, st>>>(in.Sx, in.Sy, in.Sz0, ws.X, in.f1EF, MF, ws.A);
+        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_TRY(zgetrf(st, ws.A, n, n + 1, n + 1, 0, ws.piv, 0, out.status + 3 * Zs, 1, ws.gemm, nullptr));
+        SCW_TRY(ztrsm_upper(st, ws.A, n, n + 1, 0, ws.A + n, 1, n + 1, 0, 1, ws.gemm, nullptr));
+        SCW_TRY(zgemm(st, n, 1, n, kOne, ws.X, n, 0, ws.A + n, n + 1, 0, kZero, ws.b, 1, 0, 1, ws.gemm));
+        bc_expand_kernel<<<nblk(MF), 256, 0, st>>>(in.Sx, in.Sy, in.Sz0, in.Sz1, in.f1EF, ws.A, ws.b, MF, out.x);
+        SCW_CUDA_TRY(cudaGetLastError());
+        L += 4 + 7 * ((n + 31) / 32);
+    } else {
+        bc_matrix_kernel<<<nblk((long long)M6 * M6), 256, 0, st>>>(in.Sx, in.Sy, in.Sz0, in.Sz1, ws.X, MF, ws.A);
+        SCW_CUDA_TRY(cudaGetLastError());
+        bc_rhs_kernel<<<nblk(M6), 256, 0, st>>>(in.f1EF, MF, ws.b);
+        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_TRY(zgetrf(st, ws.A, M6, M6, M6, 0, ws.piv, 0, out.status + 3 * Zs, 1, ws.gemm, nullptr));
+        SCW_TRY(zgetrs(st, ws.A, M6, 0, ws.piv, 0, ws.b, 1, 0, 1, ws.gemm, nullptr));
+        SCW_CUDA_TRY(cudaMemcpyAsync(out.x, ws.b, sizeof(double2) * M6, cudaMemcpyDeviceToDevice, st));
+        L += 4 + 9 * ((M6 + 31) / 32);
+    }
     if (out.sepExt) {
         sep_ext_kernel<<<nblk(M3), 256, 0, st>>>(in.EF, out.x, in.Sz0, in.Sz1, MF, k, p.n0, p.n1, out.sepExt);
         SCW_CUDA_TRY(cudaGetLastError());
@@ -725,11 +939,11 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
         if (l > 0) {   // v = Gc_{l-1} beta_{l-1} = [U (E bt + bb); W (E bt - bb)]
             const double2* bp = ws.beta + (size_t)(l - 1) * N4;
             SCW_CUDA_TRY(cudaMemcpyAsync(ws.A1, bp, sizeof(double2) * n, cudaMemcpyDeviceToDevice, st));
-            SCW_CUDA_TRY(cudaMemcpyAsync(ws.A2, bp + n, sizeof(double2) * n, cudaMemcpyDeviceToDevice, st));
-            mix_kernel<<<nblk(n), 256, 0, st>>>(ws.A1, ws.A2, ws.E + (size_t)(l - 1) * n, n, 1, 2);
+            SCW_CUDA_TRY(cudaMemcpyAsync(A2, bp + n, sizeof(double2) * n, cudaMemcpyDeviceToDevice, st));
+            mix_kernel<<<nblk(n), 256, 0, st>>>(ws.A1, A2, ws.E + (size_t)(l - 1) * n, n, 1, 2);
             SCW_CUDA_TRY(cudaGetLastError());
             SCW_TRY(zgemm(st, n, 1, n, kOne, ws.U + o - nn, n, 0, ws.A1, 1, 0, kZero, ws.v, 1, 0, 1, ws.gemm));
-            SCW_TRY(zgemm(st, n, 1, n, kOne, ws.W + o - nn, n, 0, ws.A2, 1, 0, kZero, ws.v + n, 1, 0, 1, ws.gemm));
+            SCW_TRY(zgemm(st, n, 1, n, kOne, ws.W + o - nn, n, 0, A2, 1, 0, kZero, ws.v + n, 1, 0, 1, ws.gemm));
             L += 3;
         }
         SCW_TRY(zgemm(st, n, 1, n, kOne, Uinv + o, n, 0, ws.v, 1, 0, kZero, bl, 1, 0, 1, ws.gemm));
@@ -738,51 +952,23 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
         SCW_CUDA_TRY(cudaGetLastError());
         L += 3;
     }
-    // Q_check / Q_hat with Ez from the magnetic field (sCWatter.cpp:781-871)
-    for (int l = 0; l < Zs; l++) {
-        const long long o = (long long)l * nn;
-        if (p.pz) {
-            kn_kernel<<<nblk((long long)MF * MF), 256, 0, st>>>(ws.coef + (size_t)l * 2 * MF + MF, M0, M1, -1.0 / k,
-                                                                ws.Kn);
-            SCW_CUDA_TRY(cudaGetLastError());
-            L++;
-        }
-        for (int h = 0; h < 2; h++) {
-            double2* Qo = out.Q64 ? out.Q64 + ((size_t)l * 2 + h) * M3 * n : ws.Qtmp;
-            const double2* beta = ws.beta + (size_t)l * N4 + (h ? n : 0);
-            q_rows_kernel<<<nblk(nn), 256, 0, st>>>(ws.U + o, ws.W + o, beta, MF, h ? -1.0 : 1.0, in.uppz, in.wqpz, Qo,
-                                                   p.pz ? ws.Hm : nullptr);
-            SCW_CUDA_TRY(cudaGetLastError());
-            if (p.pz) {
-                SCW_TRY(zgemm(st, MF, n, MF, kOne, ws.Kn, MF, 0, ws.Hm, n, 0, kZero, Qo + (size_t)n * n, n, 0, 1, ws.gemm));
-            } else {
-                SCW_CUDA_TRY(cudaMemsetAsync(Qo + (size_t)n * n, 0, sizeof(double2) * MF * n, st));
-            }
-            if (out.Qsep) {
-                const long long cnt = (long long)M3 * n;
-                to_c64_kernel<<<nblk(cnt), 256, 0, st>>>(Qo, out.Qsep + ((size_t)l * 2 + h) * M3 * n, cnt);
-                SCW_CUDA_TRY(cudaGetLastError());
-                L++;
-            }
-            L += 2;
-        }
-        if (out.Vsep) {      // the paired set: V = [U; Kn (up W_y - wq W_x)] and beta_dn, beta_up
-            q_rows_kernel<<<nblk(nn), 256, 0, st>>>(ws.U + o, ws.W + o, nullptr, MF, 1.0, in.uppz, in.wqpz, ws.Qtmp,
-                                                   p.pz ? ws.Hm : nullptr);
-            SCW_CUDA_TRY(cudaGetLastError());
-            if (p.pz) {
-                SCW_TRY(zgemm(st, MF, n, MF, kOne, ws.Kn, MF, 0, ws.Hm, n, 0, kZero, ws.Qtmp + (size_t)n * n, n, 0, 1, ws.gemm));
-            } else {
-                SCW_CUDA_TRY(cudaMemsetAsync(ws.Qtmp + (size_t)n * n, 0, sizeof(double2) * MF * n, st));
-            }
-            const long long cnt = (long long)M3 * n;
-            to_c64_kernel<<<nblk(cnt), 256, 0, st>>>(ws.Qtmp, out.Vsep + (size_t)l * M3 * n, cnt);
-            SCW_CUDA_TRY(cudaGetLastError());
-            SCW_CUDA_TRY(cudaMemcpyAsync(out.sepBeta + (size_t)l * 2 * n, ws.beta + (size_t)l * N4,
-                                         sizeof(double2) * 2 * n, cudaMemcpyDeviceToDevice, st));
-            L += 3;
-        }
+    // Q_check / Q_hat with Ez from the magnetic field (sCWatter.cpp:781-871): Hm in P, Kn over U^-1, Ez
+    // over W^-1
+    double2* Ez = nullptr;
+    if (p.pz) {
+        Ez = Winv;
+        kn_kernel<<<nblk((long long)Zs * MF * MF), 256, 0, st>>>(ws.coef, M0, M1, Zs, -1.0 / k, Uinv);
+        hm_kernel<<<nblk((long long)Zs * MF * n), 256, 0, st>>>(ws.W, MF, Zs, in.uppz, in.wqpz, ws.P);
+        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_TRY(zgemm(st, MF, n, MF, kOne, Uinv, MF, (long long)MF * MF, ws.P, n, (long long)MF * n, kZero, Ez, n,
+                      (long long)MF * n, Zs, ws.gemm));
+        L += 5;
     }
+    modes_kernel<<<nblk((long long)Zs * M3 * n), 256, 0, st>>>(ws.U, Ez, ws.beta, MF, Zs, out.Q64, out.Qsep, out.Vsep);
+    SCW_CUDA_TRY(cudaGetLastError());
+    L++;
+    if (out.Vsep)      // beta_dn, beta_up of the paired set
+        SCW_CUDA_TRY(cudaMemcpyAsync(out.sepBeta, ws.beta, sizeof(double2) * Zs * N4, cudaMemcpyDeviceToDevice, st));
     if (out.sepKz) {
         sep_kz_kernel<<<nblk((long long)Zs * n), 256, 0, st>>>(out.gam, Zs, n, k, out.sepKz);
         SCW_CUDA_TRY(cudaGetLastError());

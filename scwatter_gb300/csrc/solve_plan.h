@@ -28,6 +28,7 @@ struct SolvePlan {
     double k = 0, n0 = 1, n1 = 1;
     bool external = false, pz = true;
     bool eig_mixed = true;                  // FP32 QR + FP64 refinement (else FP64 QR throughout)
+    bool reduced_bc = true;                 // boundary system of order 2MF (no |Sz| near zero), else 6MF
     bool wide_hess = false;                 // Hessenberg reductions over the whole GPU (single solves)
     std::vector<double> zb, dz;             // Z + 1 boundaries, Z thicknesses
     std::vector<int> ps, qs;                // integer harmonic series
@@ -60,8 +61,10 @@ struct SolveIn {                            // uploaded once
 struct SolveWs {                            // scratch, reusable once the solve has finished
     double2 *coef, *P, *Q, *PQ, *U, *W, *lam, *E, *beta, *v;
     int* piv;
-    // temporary region: DFT stage (data planes, T) / cascade + boundary (X, A1, A2, A, b) / modes (Kn, Hm, Qtmp)
-    double2 *F, *T, *X, *A1, *A2, *A, *b, *Kn, *Hm, *Qtmp;
+    double* worst;                          // [2 Z] residuals of the Newton inverses of U and W
+    int* good;                              // [2 Z] 1: that inverse is done, 0: by LU
+    // temporary region: DFT stage (data planes, T) / cascade + boundary (X, A1 and A2, A, b)
+    double2 *F, *T, *X, *A1, *A, *b;
     // mixed-precision eigen-solver: FP32 slots overlay P and W (free during the eigen-solve)
     mx::EigMixWs mix;
     GemmWs gemm;                            // FP64 product operands; err: set by the caller
