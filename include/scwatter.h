@@ -261,7 +261,7 @@ SCW_API scw_status scw_zgesv(scw_ctx ctx, int n, int nrhs, void* A, void* B, int
  * overwritten); SCW_ERR_NUMERIC if the QR iteration does not converge. */
 SCW_API scw_status scw_zgeev(scw_ctx ctx, int n, void* A, void* W, void* V, int batch, int* status_host);
 /* Same contract as scw_zgeev (n <= 4096), computed by the mixed-precision solver: FP32
- * Householder + QR + triangular eigenvectors, then Newton refinement of all eigenpairs with FP64
+ * Householder + multishift QR + triangular eigenvectors, then Newton refinement of all eigenpairs with FP64
  * residuals (clusters of close eigenvalues solved as small FP64 Schur problems).  Refinement stops
  * once max_i ||A x_i - lambda_i x_i|| / (||A||_1 ||x_i||) <= 1e-14; a matrix at or below 1e-12 from
  * step 10 on is accepted, and one still above 1e-12 after 10 steps (16 for n >= 1600) is solved by
@@ -273,11 +273,12 @@ SCW_API scw_status scw_zgeev(scw_ctx ctx, int n, void* A, void* W, void* V, int 
 /* FP32 counterpart of scw_zgeev (complex64 A, W, V; LAPACK cgeev semantics), the first stage of
  * scw_zgeev_mixed.  No reference counterpart. */
 SCW_API scw_status scw_cgeev(scw_ctx ctx, int n, void* A, void* W, void* V, int batch, int* status_host);
-/* CTAs per matrix of the QR sweeps in scw_zgeev, scw_cgeev, scw_zgeev_mixed and scw_solve, for the
- * whole process: 0 (default) chooses per call (a thread-block cluster of up to 8 CTAs per matrix
- * where all matrices' clusters fit on the GPU at once, else one CTA), 1 one CTA per matrix, 2..8
- * a cluster of that size where it fits.  Results agree to rounding in every setting.
- * Batches (scw_batch_*) always use one CTA per matrix.  No reference counterpart. */
+/* CTAs per matrix of the QR iterations in scw_zgeev, scw_cgeev, scw_zgeev_mixed, scw_solve and the
+ * batches' FP32 stage, for the whole process: 0 (default) chooses per call (a thread-block cluster
+ * of up to 8 CTAs per matrix where all matrices' clusters fit on the GPU at once, else fewer or one),
+ * 1 one CTA per matrix, 2..8 a cluster of that size where it fits.  Results agree to rounding in
+ * every setting.  The FP64 fallback inside batches always uses one CTA per matrix.  No reference
+ * counterpart. */
 SCW_API scw_status scw_set_qr_cluster(int ctas);
 SCW_API scw_status scw_zgeev_mixed(scw_ctx ctx, int n, void* A, void* W, void* V, int batch, int* accepted_host,
                                    int* steps_host, double* residual_host);

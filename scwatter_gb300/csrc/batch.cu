@@ -200,6 +200,7 @@ scw_status build_graph(scw_batch b, const std::vector<int>& idx, int lanes, int 
     for (int l = 0; l < lanes && rec == SCW_OK; l++) {
         for (int i : per_lane[l]) {
             Item& it = b->items[i];
+            it.sp.share = lanes;
             scw::sv::Carver c{b->lane_arena[l], 0};
             scw::sv::SolveWs ws{};
             scw::sv::carve_ws(it.sp, c, ws);

@@ -375,27 +375,25 @@ trsm_block_kernel(const double2* __restrict__ LU, int lda, long long sA, int k0,
 // Hessenberg reduction A -> Q^H A Q (zgehd2 semantics: H(k) = I - tau v v^H, v(k+1) = 1),
 // one CTA per matrix, with the explicit unitary Q accumulated (Q := Q H(k)).
 // ------------------------------------------------------------------------------------
-template <typename R>
-__device__ R block_sum(R v, R* sh) {
+__device__ double block_sum(double v, double* sh) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     __syncthreads();
     if (lane == 0) sh[w] = v;
     __syncthreads();
-    R s = 0;
+    double s = 0;
     for (int i = 0; i < (int)(blockDim.x >> 5); i++) s += sh[i];
     return s;
 }
 
 // y[i] = tau * sum_{j >= j0} M[i][j] v[j] for every row i: a warp per row, lanes along the row
 // (coalesced), then a butterfly sum
-template <typename C>
-__device__ __forceinline__ void row_products(const C* __restrict__ M, const C* __restrict__ v, C* __restrict__ y, int n,
-                                             int j0, C tau) {
+__device__ __forceinline__ void row_products(const double2* __restrict__ M, const double2* __restrict__ v, double2* __restrict__ y, int n,
+                                             int j0, double2 tau) {
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (int i = threadIdx.x >> 5; i < n; i += nw) {
-        const C* row = M + (long long)i * n;
-        C s = CT<C>::mk(0, 0);
+        const double2* row = M + (long long)i * n;
+        double2 s = CT<double2>::mk(0, 0);
 #pragma unroll 4
         for (int j = j0 + lane; j < n; j += 32) s = cfma(row[j], v[j], s);
         for (int o = 16; o > 0; o >>= 1) {
@@ -409,12 +407,11 @@ __device__ __forceinline__ void row_products(const C* __restrict__ M, const C* _
 // col[i * ld] += u[i] * alpha for i in [i0, i1): kStripe rows at a time, loads before the
 // updates, so that a thread has kStripe independent loads in flight instead of one
 // load-update-store chain per row
-template <typename C>
-__device__ __forceinline__ void column_axpy(C* __restrict__ col, long long ld, int i0, int i1, const C* __restrict__ u,
-                                            C alpha) {
-    constexpr int kStripe = sizeof(typename CT<C>::R) == sizeof(float) ? 8 : 4;
+__device__ __forceinline__ void column_axpy(double2* __restrict__ col, long long ld, int i0, int i1, const double2* __restrict__ u,
+                                            double2 alpha) {
+    constexpr int kStripe = 4;
     for (int b = i0; b < i1; b += kStripe) {
-        C a[kStripe];
+        double2 a[kStripe];
 #pragma unroll
         for (int q = 0; q < kStripe; q++)
             if (b + q < i1) a[q] = col[(long long)(b + q) * ld];
@@ -424,64 +421,44 @@ __device__ __forceinline__ void column_axpy(C* __restrict__ col, long long ld, i
     }
 }
 
-template <typename C>
 __global__ void __launch_bounds__(1024)
-hessenberg_kernel(C* __restrict__ A, C* __restrict__ Q, int n, long long sA, C* __restrict__ work,
+hessenberg_kernel(double2* __restrict__ A, double2* __restrict__ Q, int n, long long sA, double2* __restrict__ work,
                   const int* __restrict__ skip) {
-    using R = typename CT<C>::R;
     if (skipped(skip, blockIdx.x)) return;
     A += sA * blockIdx.x;
     Q += sA * blockIdx.x;
-    C* v = work + (long long)blockIdx.x * 3 * n;      // Householder vector (rows k+1..n-1)
-    C* y = v + 2 * n;                                   // tau A v / tau Q v (the work keeps 3 n per matrix)
-    __shared__ R sh[32];
-    __shared__ C s_tau, s_beta;
-    // FP32 (first stage of the mixed solver): a column whose part below the diagonal is under
-    // ulp ||A||_F / sqrt(n) (ulp times the root-mean-square row norm) is set to zero instead of
-    // reflected.  That is a backward error of rounding size, and it keeps a (nearly) diagonal
-    // matrix, e.g. the reduced matrix of a homogeneous layer whose off-diagonal entries are DFT
-    // rounding, from being scrambled by reflectors built from noise.  (ulp ||A||_F itself grows as
-    // sqrt(n) and at n = 3200 dropped real couplings.)  FP64 keeps zgehd2's behaviour.
-    constexpr bool kDropNegligible = sizeof(R) == sizeof(float);
-    constexpr int kStripe = sizeof(R) == sizeof(float) ? 8 : 4;
-    R neg2 = 0;
-    if (kDropNegligible) {
-        R a2 = 0;
-        for (long long i = threadIdx.x; i < (long long)n * n; i += blockDim.x) a2 += cabs2(A[i]);
-        neg2 = block_sum(a2, sh) * CT<C>::ulp * CT<C>::ulp / (R)n;
-    }
-    for (int i = threadIdx.x; i < n * n; i += blockDim.x) Q[i] = CT<C>::mk((i / n) == (i % n) ? 1 : 0, 0);
+    double2* v = work + (long long)blockIdx.x * 3 * n;      // Householder vector (rows k+1..n-1)
+    double2* y = v + 2 * n;                                   // tau A v / tau Q v (the work keeps 3 n per matrix)
+    __shared__ double sh[32];
+    __shared__ double2 s_tau, s_beta;
+    constexpr int kStripe = 4;
+    for (int i = threadIdx.x; i < n * n; i += blockDim.x) Q[i] = CT<double2>::mk((i / n) == (i % n) ? 1 : 0, 0);
     __syncthreads();
     for (int k = 0; k + 2 < n; k++) {
         // Householder for x = A[k+1:n, k] (zlarfg)
-        R xn2 = 0;
+        double xn2 = 0;
         for (int i = k + 2 + threadIdx.x; i < n; i += blockDim.x) xn2 += cabs2(A[(long long)i * n + k]);
         xn2 = block_sum(xn2, sh);
-        const C alpha = A[(long long)(k + 1) * n + k];
-        if (kDropNegligible && xn2 + cabs2(alpha) <= neg2) {
-            for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x) A[(long long)i * n + k] = CT<C>::mk(0, 0);
-            __syncthreads();
-            continue;
-        }
+        const double2 alpha = A[(long long)(k + 1) * n + k];
         if (threadIdx.x == 0) {
             if (xn2 == 0 && alpha.y == 0) {
-                s_tau = CT<C>::mk(0, 0);
+                s_tau = CT<double2>::mk(0, 0);
                 s_beta = alpha;
             } else {
-                const R beta = -r_copysign(r_sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn2), alpha.x);
-                s_tau = CT<C>::mk((beta - alpha.x) / beta, -alpha.y / beta);
-                s_beta = CT<C>::mk(beta, 0);
+                const double beta = -r_copysign(r_sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn2), alpha.x);
+                s_tau = CT<double2>::mk((beta - alpha.x) / beta, -alpha.y / beta);
+                s_beta = CT<double2>::mk(beta, 0);
             }
         }
         __syncthreads();
-        const C tau = s_tau;
+        const double2 tau = s_tau;
         if (tau.x == 0 && tau.y == 0) {
             __syncthreads();
             continue;
         }
-        const C scal = cdiv(CT<C>::mk(1, 0), csub(alpha, s_beta));
+        const double2 scal = cdiv(CT<double2>::mk(1, 0), csub(alpha, s_beta));
         for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x)
-            v[i] = (i == k + 1) ? CT<C>::mk(1, 0) : cmul(A[(long long)i * n + k], scal);
+            v[i] = (i == k + 1) ? CT<double2>::mk(1, 0) : cmul(A[(long long)i * n + k], scal);
         __syncthreads();
         // right: A[:, k+1:] -= tau (A[:, k+1:] v) v^H   (all rows; a warp per row for the products)
         row_products(A, v, y, n, k + 1, tau);
@@ -490,12 +467,12 @@ hessenberg_kernel(C* __restrict__ A, C* __restrict__ Q, int n, long long sA, C* 
         // at a time, so each thread owns its columns: right update (all rows) while summing
         // v^H of the updated column, then the left update of that column.
         for (int j = k + 1 + threadIdx.x; j < n; j += blockDim.x) {
-            const C vc = CT<C>::mk(v[j].x, -v[j].y);
-            C s = CT<C>::mk(0, 0);
-            C* col = A + j;
+            const double2 vc = CT<double2>::mk(v[j].x, -v[j].y);
+            double2 s = CT<double2>::mk(0, 0);
+            double2* col = A + j;
             // kStripe rows at a time: loads first, then the updates (see column_axpy)
             for (int i0 = 0; i0 < n; i0 += kStripe) {
-                C a[kStripe];
+                double2 a[kStripe];
 #pragma unroll
                 for (int q = 0; q < kStripe; q++)
                     if (i0 + q < n) a[q] = col[(long long)(i0 + q) * n];
@@ -505,22 +482,22 @@ hessenberg_kernel(C* __restrict__ A, C* __restrict__ Q, int n, long long sA, C* 
                     if (i < n) {
                         a[q] = csub(a[q], cmul(y[i], vc));
                         col[(long long)i * n] = a[q];
-                        if (i > k) s = cfma(CT<C>::mk(v[i].x, -v[i].y), a[q], s);
+                        if (i > k) s = cfma(CT<double2>::mk(v[i].x, -v[i].y), a[q], s);
                     }
                 }
             }
-            const C wj = cmul(CT<C>::mk(tau.x, -tau.y), s);
-            column_axpy(col, n, k + 1, n, v, CT<C>::mk(-wj.x, -wj.y));
+            const double2 wj = cmul(CT<double2>::mk(tau.x, -tau.y), s);
+            column_axpy(col, n, k + 1, n, v, CT<double2>::mk(-wj.x, -wj.y));
         }
         // column k below the subdiagonal
         for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x)
-            A[(long long)i * n + k] = (i == k + 1) ? s_beta : CT<C>::mk(0, 0);
+            A[(long long)i * n + k] = (i == k + 1) ? s_beta : CT<double2>::mk(0, 0);
         // Q[:, k+1:] -= (Q[:, k+1:] v) tau v^H
         __syncthreads();
         row_products(Q, v, y, n, k + 1, tau);
         __syncthreads();
         for (int j = k + 1 + threadIdx.x; j < n; j += blockDim.x)
-            column_axpy(Q + j, n, 0, n, y, CT<C>::mk(-v[j].x, v[j].y));
+            column_axpy(Q + j, n, 0, n, y, CT<double2>::mk(-v[j].x, v[j].y));
         __syncthreads();
     }
 }
@@ -532,95 +509,64 @@ hessenberg_kernel(C* __restrict__ A, C* __restrict__ Q, int n, long long sA, C* 
 // the columns k+1.. of A (right then left, one thread per column) and of Q.  Every element sees
 // the operations of hessenberg_kernel in the same order; the kernel boundaries replace its
 // block barriers, so the O(n^2) work of a column runs on every SM instead of one per matrix.
-// Per matrix the 3n work entries hold v (slot 0: tau), y and z; ||A||_F^2 for the FP32 drop
-// threshold ulp^2 ||A||_F^2 / n (||A||_F is invariant under the reduction) is kept in Q[n-1][0],
-// which the reflectors never touch, and cleared at the end.
+// Per matrix the 3n work entries hold v (slot 0: tau), y and z.
 // ------------------------------------------------------------------------------------
 constexpr int kHwRows = 8;        // rows (warps) per CTA of the product kernel
 constexpr int kHwCols = 128;      // columns (threads) per CTA of the update kernel
 
-template <typename C>
-__global__ void __launch_bounds__(256) hw_init_kernel(C* __restrict__ Q, int n, long long sA, const int* __restrict__ skip) {
+__global__ void __launch_bounds__(256) hw_init_kernel(double2* __restrict__ Q, int n, long long sA, const int* __restrict__ skip) {
     if (skipped(skip, blockIdx.y)) return;
     Q += sA * blockIdx.y;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)n * n;
          i += (long long)gridDim.x * blockDim.x)
-        Q[i] = CT<C>::mk((i / n) == (i % n) ? 1 : 0, 0);
+        Q[i] = CT<double2>::mk((i / n) == (i % n) ? 1 : 0, 0);
 }
 
-// ||A||_F^2 into Q[n-1][0].x (after hw_init_kernel)
-template <typename C>
-__global__ void __launch_bounds__(256) hw_fro_kernel(const C* __restrict__ A, C* __restrict__ Q, int n, long long sA,
+__global__ void __launch_bounds__(256) hw_vec_kernel(double2* __restrict__ A, int n, long long sA, double2* __restrict__ work, int k,
                                                      const int* __restrict__ skip) {
-    using R = typename CT<C>::R;
-    if (skipped(skip, blockIdx.y)) return;
-    A += sA * blockIdx.y;
-    __shared__ R sh[32];
-    R a2 = 0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)n * n;
-         i += (long long)gridDim.x * blockDim.x)
-        a2 += cabs2(A[i]);
-    a2 = block_sum(a2, sh);
-    if (threadIdx.x == 0) atomicAdd(&Q[sA * blockIdx.y + (long long)(n - 1) * n].x, a2);
-}
-
-template <typename C>
-__global__ void __launch_bounds__(256) hw_vec_kernel(C* __restrict__ A, const C* __restrict__ Q, int n, long long sA,
-                                                     C* __restrict__ work, int k, const int* __restrict__ skip) {
-    using R = typename CT<C>::R;
     if (skipped(skip, blockIdx.x)) return;
     A += sA * blockIdx.x;
-    C* v = work + (long long)blockIdx.x * 3 * n;
-    __shared__ R sh[32];
-    __shared__ C s_beta;
+    double2* v = work + (long long)blockIdx.x * 3 * n;
+    __shared__ double sh[32];
+    __shared__ double2 s_beta;
     __shared__ int s_skip;
-    constexpr bool kDropNegligible = sizeof(R) == sizeof(float);
-    R xn2 = 0;
+    double xn2 = 0;
     for (int i = k + 2 + threadIdx.x; i < n; i += blockDim.x) xn2 += cabs2(A[(long long)i * n + k]);
     xn2 = block_sum(xn2, sh);
-    const C alpha = A[(long long)(k + 1) * n + k];
+    const double2 alpha = A[(long long)(k + 1) * n + k];
     if (threadIdx.x == 0) {
         s_skip = 0;
-        const R neg2 =
-            kDropNegligible ? Q[sA * blockIdx.x + (long long)(n - 1) * n].x * CT<C>::ulp * CT<C>::ulp / (R)n : R(0);
-        if (kDropNegligible && xn2 + cabs2(alpha) <= neg2) {
-            s_skip = 2;                       // drop: zero the column below the diagonal
-        } else if (xn2 == 0 && alpha.y == 0) {
+        if (xn2 == 0 && alpha.y == 0) {
             s_skip = 1;                       // already reduced
         } else {
-            const R beta = -r_copysign(r_sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn2), alpha.x);
-            v[0] = CT<C>::mk((beta - alpha.x) / beta, -alpha.y / beta);      // tau
-            s_beta = CT<C>::mk(beta, 0);
+            const double beta = -r_copysign(r_sqrt(alpha.x * alpha.x + alpha.y * alpha.y + xn2), alpha.x);
+            v[0] = CT<double2>::mk((beta - alpha.x) / beta, -alpha.y / beta);      // tau
+            s_beta = CT<double2>::mk(beta, 0);
         }
-        if (s_skip) v[0] = CT<C>::mk(0, 0);
+        if (s_skip) v[0] = CT<double2>::mk(0, 0);
     }
     __syncthreads();
-    if (s_skip == 1) return;
-    if (s_skip == 2) {
-        for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x) A[(long long)i * n + k] = CT<C>::mk(0, 0);
-        return;
-    }
-    const C scal = cdiv(CT<C>::mk(1, 0), csub(alpha, s_beta));
+    if (s_skip) return;
+    const double2 scal = cdiv(CT<double2>::mk(1, 0), csub(alpha, s_beta));
     for (int i = k + 1 + threadIdx.x; i < n; i += blockDim.x) {
-        v[i] = (i == k + 1) ? CT<C>::mk(1, 0) : cmul(A[(long long)i * n + k], scal);
-        A[(long long)i * n + k] = (i == k + 1) ? s_beta : CT<C>::mk(0, 0);
+        v[i] = (i == k + 1) ? CT<double2>::mk(1, 0) : cmul(A[(long long)i * n + k], scal);
+        A[(long long)i * n + k] = (i == k + 1) ? s_beta : CT<double2>::mk(0, 0);
     }
 }
 
 // rows 0..n-1: y[i] = tau sum_{j > k} A[i][j] v[j]; rows n..2n-1: z[i] = tau sum_{j > k} Q[i][j] v[j]
-template <typename C>
-__global__ void __launch_bounds__(kHwRows * 32) hw_prod_kernel(const C* __restrict__ A, const C* __restrict__ Q, int n,
-                                                               long long sA, C* __restrict__ work, int k,
+__global__ void __launch_bounds__(kHwRows * 32) hw_prod_kernel(const double2* __restrict__ A, const double2* __restrict__ Q, int n,
+                                                               long long sA, double2* __restrict__ work, int k,
                                                                const int* __restrict__ skip) {
     if (skipped(skip, blockIdx.y)) return;
-    C* v = work + (long long)blockIdx.y * 3 * n;
-    const C tau = v[0];
+    double2* v = work + (long long)blockIdx.y * 3 * n;
+    const double2 tau = v[0];
     if (tau.x == 0 && tau.y == 0) return;
     const int lane = threadIdx.x & 31;
     const int r = blockIdx.x * kHwRows + (threadIdx.x >> 5);
     if (r >= 2 * n) return;
-    const C* row = (r < n ? A + (long long)r * n : Q + (long long)(r - n) * n) + sA * blockIdx.y;
-    C acc = CT<C>::mk(0, 0);
+    const double2* row = (r < n ? A + (long long)r * n : Q + (long long)(r - n) * n) + sA * blockIdx.y;
+    double2 acc = CT<double2>::mk(0, 0);
 #pragma unroll 4
     for (int j = k + 1 + lane; j < n; j += 32) acc = cfma(row[j], v[j], acc);
     for (int o = 16; o > 0; o >>= 1) {
@@ -632,25 +578,24 @@ __global__ void __launch_bounds__(kHwRows * 32) hw_prod_kernel(const C* __restri
 
 // columns j > k of A: right update (all rows) while summing v^H of the updated column, then the
 // left update; columns j > k of Q (blocks past the A blocks): Q[:, j] -= z conj(v_j)
-template <typename C>
-__global__ void __launch_bounds__(kHwCols) hw_update_kernel(C* __restrict__ A, C* __restrict__ Q, int n, long long sA,
-                                                            const C* __restrict__ work, int k, int nblk_a,
+__global__ void __launch_bounds__(kHwCols) hw_update_kernel(double2* __restrict__ A, double2* __restrict__ Q, int n, long long sA,
+                                                            const double2* __restrict__ work, int k, int nblk_a,
                                                             const int* __restrict__ skip) {
     if (skipped(skip, blockIdx.y)) return;
-    const C* v = work + (long long)blockIdx.y * 3 * n;
-    const C tau = v[0];
+    const double2* v = work + (long long)blockIdx.y * 3 * n;
+    const double2 tau = v[0];
     if (tau.x == 0 && tau.y == 0) return;
-    constexpr int kStripe = sizeof(typename CT<C>::R) == sizeof(float) ? 8 : 4;
+    constexpr int kStripe = 4;
     const bool isA = (int)blockIdx.x < nblk_a;
     const int j = k + 1 + (isA ? (int)blockIdx.x : (int)blockIdx.x - nblk_a) * kHwCols + threadIdx.x;
     if (j >= n) return;
     if (isA) {
-        const C* y = v + n;
-        const C vc = CT<C>::mk(v[j].x, -v[j].y);
-        C* col = A + sA * blockIdx.y + j;
-        C s = CT<C>::mk(0, 0);
+        const double2* y = v + n;
+        const double2 vc = CT<double2>::mk(v[j].x, -v[j].y);
+        double2* col = A + sA * blockIdx.y + j;
+        double2 s = CT<double2>::mk(0, 0);
         for (int i0 = 0; i0 < n; i0 += kStripe) {
-            C a[kStripe];
+            double2 a[kStripe];
 #pragma unroll
             for (int q = 0; q < kStripe; q++)
                 if (i0 + q < n) a[q] = col[(long long)(i0 + q) * n];
@@ -660,21 +605,15 @@ __global__ void __launch_bounds__(kHwCols) hw_update_kernel(C* __restrict__ A, C
                 if (i < n) {
                     a[q] = csub(a[q], cmul(y[i], vc));
                     col[(long long)i * n] = a[q];
-                    if (i > k) s = cfma(CT<C>::mk(v[i].x, -v[i].y), a[q], s);
+                    if (i > k) s = cfma(CT<double2>::mk(v[i].x, -v[i].y), a[q], s);
                 }
             }
         }
-        const C wj = cmul(CT<C>::mk(tau.x, -tau.y), s);
-        column_axpy(col, n, k + 1, n, v, CT<C>::mk(-wj.x, -wj.y));
+        const double2 wj = cmul(CT<double2>::mk(tau.x, -tau.y), s);
+        column_axpy(col, n, k + 1, n, v, CT<double2>::mk(-wj.x, -wj.y));
     } else {
-        column_axpy(Q + sA * blockIdx.y + j, n, 0, n, v + 2 * n, CT<C>::mk(-v[j].x, v[j].y));
+        column_axpy(Q + sA * blockIdx.y + j, n, 0, n, v + 2 * n, CT<double2>::mk(-v[j].x, v[j].y));
     }
-}
-
-template <typename C>
-__global__ void hw_finish_kernel(C* __restrict__ Q, int n, long long sA, int batch, const int* __restrict__ skip) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b < batch && !skipped(skip, b)) Q[sA * b + (long long)(n - 1) * n] = CT<C>::mk(0, 0);
 }
 
 // ------------------------------------------------------------------------------------
@@ -683,17 +622,15 @@ __global__ void hw_finish_kernel(C* __restrict__ Q, int n, long long sA, int bat
 // 1 no convergence within 30 n iterations.
 // ------------------------------------------------------------------------------------
 // G [x; y] (rows) and [x, y] G^H (columns) for G = [c, s; -conj(s), c]
-template <typename C>
-__device__ __forceinline__ void rot_rows(typename CT<C>::R c, C s, C& x, C& y) {
-    const C nx = CT<C>::mk(c * x.x + (s.x * y.x - s.y * y.y), c * x.y + (s.x * y.y + s.y * y.x));
-    const C ny = CT<C>::mk(c * y.x - (s.x * x.x + s.y * x.y), c * y.y - (s.x * x.y - s.y * x.x));
+__device__ __forceinline__ void rot_rows(double c, double2 s, double2& x, double2& y) {
+    const double2 nx = CT<double2>::mk(c * x.x + (s.x * y.x - s.y * y.y), c * x.y + (s.x * y.y + s.y * y.x));
+    const double2 ny = CT<double2>::mk(c * y.x - (s.x * x.x + s.y * x.y), c * y.y - (s.x * x.y - s.y * x.x));
     x = nx;
     y = ny;
 }
-template <typename C>
-__device__ __forceinline__ void rot_cols(typename CT<C>::R c, C s, C& x, C& y) {
-    const C nx = CT<C>::mk(c * x.x + (y.x * s.x + y.y * s.y), c * x.y + (y.y * s.x - y.x * s.y));
-    const C ny = CT<C>::mk(c * y.x - (x.x * s.x - x.y * s.y), c * y.y - (x.x * s.y + x.y * s.x));
+__device__ __forceinline__ void rot_cols(double c, double2 s, double2& x, double2& y) {
+    const double2 nx = CT<double2>::mk(c * x.x + (y.x * s.x + y.y * s.y), c * x.y + (y.y * s.x - y.x * s.y));
+    const double2 ny = CT<double2>::mk(c * y.x - (x.x * s.x - x.y * s.y), c * y.y - (x.x * s.y + x.y * s.x));
     x = nx;
     y = ny;
 }
@@ -711,45 +648,37 @@ constexpr int kHqrW = 64;
 // s = conj(g) f / (|f| d), r = f d / |f| with d = sqrt(|f|^2 + |g|^2)), which keeps the rotation
 // unitary to a few ulp.  In FP64 this replaces zlartg's two square roots and five divisions:
 // the chase is one warp working through each rotation's dependent chain, and GB300 issues FP64
-// at about 2 operations per clock per SM, so that chain sets the FP64 sweep's time.  (In FP32,
-// one Newton-Raphson step on each reciprocal square root, unitary to about 1 ulp, was measured on
-// two n = 3200 layers: eigenpair residuals 1.6-2.5x larger and fewer layers accepted by the
-// refinement, so the plain form stays.)
-__device__ __forceinline__ float r_rsqrt(float x) { return rsqrtf(x); }
-__device__ __forceinline__ double r_rsqrt(double x) { return rsqrt(x); }
+// at about 2 operations per clock per SM, so that chain sets the FP64 sweep's time.
 
-template <typename C>
-__device__ __forceinline__ void givens_chase(C f, C g, typename CT<C>::R& c, C& s, C& r) {
-    using R = typename CT<C>::R;
-    const R gf = cabs2(g), ff = cabs2(f);
-    if (gf == R(0)) {
-        c = R(1);
-        s = CT<C>::mk(R(0), R(0));
+__device__ __forceinline__ void givens_chase(double2 f, double2 g, double& c, double2& s, double2& r) {
+    const double gf = cabs2(g), ff = cabs2(f);
+    if (gf == 0.0) {
+        c = 1.0;
+        s = CT<double2>::mk(0.0, 0.0);
         r = f;
         return;
     }
-    if (ff == R(0)) {
-        const R ig = r_rsqrt(gf);
-        c = R(0);
-        s = CT<C>::mk(g.x * ig, -g.y * ig);
-        r = CT<C>::mk(gf * ig, R(0));
+    if (ff == 0.0) {
+        const double ig = rsqrt(gf);
+        c = 0.0;
+        s = CT<double2>::mk(g.x * ig, -g.y * ig);
+        r = CT<double2>::mk(gf * ig, 0.0);
         return;
     }
-    const R iaf = r_rsqrt(ff), id = r_rsqrt(ff + gf);
+    const double iaf = rsqrt(ff), id = rsqrt(ff + gf);
     c = ff * iaf * id;
-    const C fs = CT<C>::mk(f.x * iaf, f.y * iaf);
-    const C t = cmulc(g, fs);
-    s = CT<C>::mk(t.x * id, t.y * id);
-    const R d = (ff + gf) * id;
-    r = CT<C>::mk(fs.x * d, fs.y * d);
+    const double2 fs = CT<double2>::mk(f.x * iaf, f.y * iaf);
+    const double2 t = cmulc(g, fs);
+    s = CT<double2>::mk(t.x * id, t.y * id);
+    const double d = (ff + gf) * id;
+    r = CT<double2>::mk(fs.x * d, fs.y * d);
 }
 
 // The chase of rotations k0 .. k1-1 inside the shared-memory window (loaded from H, a block
 // barrier, the chase by warp 0, a block barrier, stored back), the rotations recorded in hc / hs.
-template <typename C, bool kCg>
-__device__ void hqr_chase(C* __restrict__ H, int n, int l, int ihi, int k0, int k1, C shift, C* hw,
-                          typename CT<C>::R* hc, C* hs) {
-    using R = typename CT<C>::R;
+template <bool kCg>
+__device__ void hqr_chase(double2* __restrict__ H, int n, int l, int ihi, int k0, int k1, double2 shift, double2* hw,
+                          double* hc, double2* hs) {
     constexpr int ldw = kHqrW + 2;
     const int r1 = min(k1 + 1, ihi);
     const int c0 = (k0 > l) ? k0 - 1 : k0;
@@ -764,8 +693,8 @@ __device__ void hqr_chase(C* __restrict__ H, int n, int l, int ihi, int k0, int 
         const int lane = threadIdx.x;
         for (int k = k0; k < k1; k++) {
             // every lane generates the rotation (no broadcast needed); lane 0 records it
-            C f, g, r, s;
-            R c;
+            double2 f, g, r, s;
+            double c;
             if (k == l) {
                 f = csub(HW(l, l), shift);
                 g = HW(l + 1, l);
@@ -778,7 +707,7 @@ __device__ void hqr_chase(C* __restrict__ H, int n, int l, int ihi, int k0, int 
             if (lane == 0) {
                 if (k > l) {
                     HW(k, k - 1) = r;
-                    HW(k + 1, k - 1) = CT<C>::mk(0, 0);
+                    HW(k + 1, k - 1) = CT<double2>::mk(0, 0);
                 }
                 hc[k - k0] = c;
                 hs[k - k0] = s;
@@ -804,15 +733,14 @@ __device__ void hqr_chase(C* __restrict__ H, int n, int l, int ihi, int k0, int 
 // registers before the rotations run through them: a load-rotate-store chain per element would
 // wait a full memory latency per element (the compiler cannot move a load of the stripe above the
 // store to the element before it).
-template <typename C, bool kCg>
-__device__ void hqr_apply(C* __restrict__ H, C* __restrict__ Z, int n, int k0, int k1, const typename CT<C>::R* hc,
-                          const C* hs, int t0, int dt) {
-    using R = typename CT<C>::R;
-    constexpr int kStripe = sizeof(R) == sizeof(float) ? 16 : 4;
+template <bool kCg>
+__device__ void hqr_apply(double2* __restrict__ H, double2* __restrict__ Z, int n, int k0, int k1, const double* hc,
+                          const double2* hs, int t0, int dt) {
+    constexpr int kStripe = 4;
     const int nright = n - 1 - k1, nabove = k0;
     for (int t = t0; t < nright + nabove + n; t += dt) {
         const bool right = t < nright;              // column j (rows k0..k1), else a row (columns k0..k1)
-        C* base;
+        double2* base;
         long long step;
         if (right) {
             base = H + k1 + 1 + t;
@@ -821,10 +749,10 @@ __device__ void hqr_apply(C* __restrict__ H, C* __restrict__ Z, int n, int k0, i
             base = (t < nright + nabove) ? H + (long long)(t - nright) * n : Z + (long long)(t - nright - nabove) * n;
             step = 1;
         }
-        C x = hld<kCg>(base + (long long)k0 * step);
+        double2 x = hld<kCg>(base + (long long)k0 * step);
         for (int kb = k0; kb < k1; kb += kStripe) {
             const int m = min(kStripe, k1 - kb);
-            C y[kStripe];
+            double2 y[kStripe];
 #pragma unroll
             for (int q = 0; q < kStripe; q++)
                 if (q < m) y[q] = hld<kCg>(base + (long long)(kb + q + 1) * step);
@@ -844,59 +772,54 @@ __device__ void hqr_apply(C* __restrict__ H, C* __restrict__ Z, int n, int k0, i
     }
 }
 
-template <typename C>
-__device__ void hqr_chunk(C* __restrict__ H, C* __restrict__ Z, int n, int l, int ihi, int k0, int k1, C shift,
-                          C* hw, typename CT<C>::R* hc, C* hs) {
-    hqr_chase<C, false>(H, n, l, ihi, k0, k1, shift, hw, hc, hs);
-    hqr_apply<C, false>(H, Z, n, k0, k1, hc, hs, threadIdx.x, blockDim.x);
+__device__ void hqr_chunk(double2* __restrict__ H, double2* __restrict__ Z, int n, int l, int ihi, int k0, int k1, double2 shift,
+                          double2* hw, double* hc, double2* hs) {
+    hqr_chase<false>(H, n, l, ihi, k0, k1, shift, hw, hc, hs);
+    hqr_apply<false>(H, Z, n, k0, k1, hc, hs, threadIdx.x, blockDim.x);
     __syncthreads();
 }
 
 // Shift of the next sweep over [l, ihi]: Wilkinson's from the trailing 2 x 2 block, and
 // exceptional shifts every 10 iterations without a deflation (zlahqr's KEXSH rule).
-template <typename C, bool kCg>
-__device__ C hqr_shift(const C* __restrict__ H, int n, int l, int ihi, int its) {
-    using R = typename CT<C>::R;
-    const C hii = hld<kCg>(H + (long long)ihi * n + ihi);
-    if (its % 20 == 0) return CT<C>::mk(R(0.75) * r_abs(hld<kCg>(H + (long long)ihi * n + ihi - 1).x) + hii.x, hii.y);
+template <bool kCg>
+__device__ double2 hqr_shift(const double2* __restrict__ H, int n, int l, int ihi, int its) {
+    const double2 hii = hld<kCg>(H + (long long)ihi * n + ihi);
+    if (its % 20 == 0) return CT<double2>::mk(0.75 * r_abs(hld<kCg>(H + (long long)ihi * n + ihi - 1).x) + hii.x, hii.y);
     if (its % 10 == 0) {
-        const C hll = hld<kCg>(H + (long long)l * n + l);
-        return CT<C>::mk(R(0.75) * r_abs(hld<kCg>(H + (long long)(l + 1) * n + l).x) + hll.x, hll.y);
+        const double2 hll = hld<kCg>(H + (long long)l * n + l);
+        return CT<double2>::mk(0.75 * r_abs(hld<kCg>(H + (long long)(l + 1) * n + l).x) + hll.x, hll.y);
     }
-    const C a = hld<kCg>(H + (long long)(ihi - 1) * n + ihi - 1);
-    const C b = hld<kCg>(H + (long long)(ihi - 1) * n + ihi);
-    const C c = hld<kCg>(H + (long long)ihi * n + ihi - 1);
-    const C d = hii;
-    const C half = CT<C>::mk(R(0.5) * (a.x - d.x), R(0.5) * (a.y - d.y));
-    const C bc = cmul(b, c);
-    const C disc = cfma(half, half, bc);
-    const C sq = zsqrt(disc);
+    const double2 a = hld<kCg>(H + (long long)(ihi - 1) * n + ihi - 1);
+    const double2 b = hld<kCg>(H + (long long)(ihi - 1) * n + ihi);
+    const double2 c = hld<kCg>(H + (long long)ihi * n + ihi - 1);
+    const double2 d = hii;
+    const double2 half = CT<double2>::mk(0.5 * (a.x - d.x), 0.5 * (a.y - d.y));
+    const double2 bc = cmul(b, c);
+    const double2 disc = cfma(half, half, bc);
+    const double2 sq = zsqrt(disc);
     // choose the root that makes the shift closer to d
-    C e1 = cadd(half, sq), e2 = csub(half, sq);
-    const C den = cabs2(e1) >= cabs2(e2) ? e1 : e2;
+    double2 e1 = cadd(half, sq), e2 = csub(half, sq);
+    const double2 den = cabs2(e1) >= cabs2(e2) ? e1 : e2;
     return (cabs2(den) == 0) ? d : csub(d, cdiv(bc, den));
 }
 
-template <typename C>
 constexpr size_t hqr_smem_bytes() {
-    return sizeof(C) * ((kHqrW + 2) * (kHqrW + 2) + kHqrW) + sizeof(typename CT<C>::R) * kHqrW;
+    return sizeof(double2) * ((kHqrW + 2) * (kHqrW + 2) + kHqrW) + sizeof(double) * kHqrW;
 }
 
-template <typename C>
 __global__ void __launch_bounds__(1024)
-hqr_kernel(C* __restrict__ H, C* __restrict__ Z, int n, long long sA, C* __restrict__ eig, int* __restrict__ status,
+hqr_kernel(double2* __restrict__ H, double2* __restrict__ Z, int n, long long sA, double2* __restrict__ eig, int* __restrict__ status,
            const int* __restrict__ skip) {
-    using R = typename CT<C>::R;
     if (skipped(skip, blockIdx.x)) return;
     H += sA * blockIdx.x;
     Z += sA * blockIdx.x;
     eig += (long long)n * blockIdx.x;
-    __shared__ C s_s;
+    __shared__ double2 s_s;
     __shared__ int s_red[32];
     extern __shared__ __align__(16) unsigned char hqr_smem[];
-    C* hw = reinterpret_cast<C*>(hqr_smem);                         // (kHqrW + 2)^2 window
-    C* hs = hw + (kHqrW + 2) * (kHqrW + 2);                         // kHqrW rotation sines
-    R* hc = reinterpret_cast<R*>(hs + kHqrW);                       // kHqrW rotation cosines
+    double2* hw = reinterpret_cast<double2*>(hqr_smem);                         // (kHqrW + 2)^2 window
+    double2* hs = hw + (kHqrW + 2) * (kHqrW + 2);                         // kHqrW rotation sines
+    double* hc = reinterpret_cast<double*>(hs + kHqrW);                       // kHqrW rotation cosines
     int ihi = n - 1;
     int its = 0;
     const int itmax = 30 * max(10, n);
@@ -917,7 +840,7 @@ hqr_kernel(C* __restrict__ H, C* __restrict__ Z, int n, long long sA, C* __restr
         for (int w = 0; w < (int)(blockDim.x >> 5); w++) l = max(l, s_red[w]);
         __syncthreads();
         if (l > 0) {
-            if (threadIdx.x == 0) H[(long long)l * n + l - 1] = CT<C>::mk(0, 0);
+            if (threadIdx.x == 0) H[(long long)l * n + l - 1] = CT<double2>::mk(0, 0);
         }
         if (l >= ihi) {                                   // 1x1 block: eigenvalue converged
             if (threadIdx.x == 0) eig[ihi] = H[(long long)ihi * n + ihi];
@@ -933,9 +856,9 @@ hqr_kernel(C* __restrict__ H, C* __restrict__ Z, int n, long long sA, C* __restr
         its++;
         total++;
         // shift; exceptional shifts every 10 iterations without a deflation (zlahqr's KEXSH rule)
-        if (threadIdx.x == 0) s_s = hqr_shift<C, false>(H, n, l, ihi, its);
+        if (threadIdx.x == 0) s_s = hqr_shift<false>(H, n, l, ihi, its);
         __syncthreads();
-        const C shift = s_s;
+        const double2 shift = s_s;
         __syncthreads();
         // implicit single-shift QR sweep over the active block [l, ihi], kHqrW rotations at a time
         for (int k0 = l; k0 < ihi; k0 += kHqrW) {
@@ -959,11 +882,9 @@ hqr_kernel(C* __restrict__ H, C* __restrict__ Z, int n, long long sA, C* __restr
 // update).  The deferred updates, 72-80 % of a sweep on one CTA (and nearly all of it in FP64,
 // whose rate per SM is low), are spread over K SMs.
 // ------------------------------------------------------------------------------------
-template <typename C>
 __global__ void __launch_bounds__(1024)
-hqr_cluster_kernel(C* __restrict__ H, C* __restrict__ Z, int n, long long sA, C* __restrict__ eig,
+hqr_cluster_kernel(double2* __restrict__ H, double2* __restrict__ Z, int n, long long sA, double2* __restrict__ eig,
                    int* __restrict__ status, const int* __restrict__ skip) {
-    using R = typename CT<C>::R;
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int K = (int)cluster.num_blocks();
@@ -973,16 +894,16 @@ hqr_cluster_kernel(C* __restrict__ H, C* __restrict__ Z, int n, long long sA, C*
     H += sA * b;
     Z += sA * b;
     eig += (long long)n * b;
-    __shared__ C s_shift;
+    __shared__ double2 s_shift;
     __shared__ int s_red[32];
     __shared__ int s_cmd[3];                            // rank 0: operation (0 sweep, 1 end), l, ihi
     extern __shared__ __align__(16) unsigned char hqr_smem[];
-    C* hw = reinterpret_cast<C*>(hqr_smem);
-    C* hs = hw + (kHqrW + 2) * (kHqrW + 2);
-    R* hc = reinterpret_cast<R*>(hs + kHqrW);
+    double2* hw = reinterpret_cast<double2*>(hqr_smem);
+    double2* hs = hw + (kHqrW + 2) * (kHqrW + 2);
+    double* hc = reinterpret_cast<double*>(hs + kHqrW);
     const int* cmd0 = cluster.map_shared_rank(s_cmd, 0);
-    const C* hs0 = cluster.map_shared_rank(hs, 0);
-    const R* hc0 = cluster.map_shared_rank(hc, 0);
+    const double2* hs0 = cluster.map_shared_rank(hs, 0);
+    const double* hc0 = cluster.map_shared_rank(hc, 0);
     int ihi = n - 1;                                    // rank 0's state
     int its = 0;
     const int itmax = 30 * max(10, n);
@@ -998,7 +919,7 @@ hqr_cluster_kernel(C* __restrict__ H, C* __restrict__ Z, int n, long long sA, C*
                 }
                 int lk = 0;
                 for (int k = ihi - (int)threadIdx.x; k > 0; k -= blockDim.x)
-                    if (hqr_deflates<C, true>(H, n, k, ihi)) {
+                    if (hqr_deflates<double2, true>(H, n, k, ihi)) {
                         lk = k;
                         break;
                     }
@@ -1008,7 +929,7 @@ hqr_cluster_kernel(C* __restrict__ H, C* __restrict__ Z, int n, long long sA, C*
                 l = 0;
                 for (int w = 0; w < (int)(blockDim.x >> 5); w++) l = max(l, s_red[w]);
                 __syncthreads();
-                if (l > 0 && threadIdx.x == 0) H[(long long)l * n + l - 1] = CT<C>::mk(0, 0);
+                if (l > 0 && threadIdx.x == 0) H[(long long)l * n + l - 1] = CT<double2>::mk(0, 0);
                 if (l >= ihi) {                           // 1x1 block: eigenvalue converged
                     if (threadIdx.x == 0) eig[ihi] = hld<true>(H + (long long)ihi * n + ihi);
                     __syncthreads();
@@ -1023,7 +944,7 @@ hqr_cluster_kernel(C* __restrict__ H, C* __restrict__ Z, int n, long long sA, C*
                 }
                 its++;
                 total++;
-                if (threadIdx.x == 0) s_shift = hqr_shift<C, true>(H, n, l, ihi, its);
+                if (threadIdx.x == 0) s_shift = hqr_shift<true>(H, n, l, ihi, its);
                 break;
             }
             if (threadIdx.x == 0) {
@@ -1042,7 +963,7 @@ hqr_cluster_kernel(C* __restrict__ H, C* __restrict__ Z, int n, long long sA, C*
         // implicit single-shift QR sweep over [l, hi], kHqrW rotations at a time (l < hi)
         for (int k0 = l; k0 < hi; k0 += kHqrW) {
             const int k1 = min(k0 + kHqrW, hi);
-            if (rank == 0) hqr_chase<C, true>(H, n, l, hi, k0, k1, s_shift, hw, hc, hs);
+            if (rank == 0) hqr_chase<true>(H, n, l, hi, k0, k1, s_shift, hw, hc, hs);
             __threadfence();
             cluster.sync();
             if (rank != 0) {
@@ -1052,7 +973,7 @@ hqr_cluster_kernel(C* __restrict__ H, C* __restrict__ Z, int n, long long sA, C*
                 }
                 __syncthreads();
             }
-            hqr_apply<C, true>(H, Z, n, k0, k1, hc, hs, rank * (int)blockDim.x + (int)threadIdx.x,
+            hqr_apply<true>(H, Z, n, k0, k1, hc, hs, rank * (int)blockDim.x + (int)threadIdx.x,
                                K * (int)blockDim.x);
             __threadfence();
             cluster.sync();
@@ -1245,27 +1166,24 @@ scw_status zgetrs(cudaStream_t st, const double2* LU, int n, long long sA, const
 
 scw_status zgehrd(cudaStream_t st, double2* A, double2* Q, int n, int batch, double2* work) {
     if (n <= 0 || batch <= 0) return SCW_OK;
-    z::hessenberg_kernel<double2><<<batch, 1024, 0, st>>>(A, Q, n, (long long)n * n, work, nullptr);
+    z::hessenberg_kernel<<<batch, 1024, 0, st>>>(A, Q, n, (long long)n * n, work, nullptr);
     SCW_CUDA_TRY(cudaGetLastError());
     return SCW_OK;
 }
 
 // Hessenberg reduction with Schur-vector accumulation, spread over the GPU (3 launches per column)
-template <typename C>
-static scw_status gehrd_wide(cudaStream_t st, C* A, C* Q, int n, int batch, C* hw, const int* skip) {
+static scw_status gehrd_wide(cudaStream_t st, double2* A, double2* Q, int n, int batch, double2* hw, const int* skip) {
     const long long nn = (long long)n * n;
     const unsigned gi = (unsigned)std::min<long long>((nn + 255) / 256, 1024);
-    z::hw_init_kernel<C><<<dim3(gi, batch), 256, 0, st>>>(Q, n, nn, skip);
-    z::hw_fro_kernel<C><<<dim3(gi, batch), 256, 0, st>>>(A, Q, n, nn, skip);
+    z::hw_init_kernel<<<dim3(gi, batch), 256, 0, st>>>(Q, n, nn, skip);
     SCW_CUDA_TRY(cudaGetLastError());
     for (int k = 0; k + 2 < n; k++) {
-        z::hw_vec_kernel<C><<<batch, 256, 0, st>>>(A, Q, n, nn, hw, k, skip);
-        z::hw_prod_kernel<C><<<dim3((2 * n + z::kHwRows - 1) / z::kHwRows, batch), z::kHwRows * 32, 0, st>>>(
+        z::hw_vec_kernel<<<batch, 256, 0, st>>>(A, n, nn, hw, k, skip);
+        z::hw_prod_kernel<<<dim3((2 * n + z::kHwRows - 1) / z::kHwRows, batch), z::kHwRows * 32, 0, st>>>(
             A, Q, n, nn, hw, k, skip);
         const int nblk = (n - k - 1 + z::kHwCols - 1) / z::kHwCols;
-        z::hw_update_kernel<C><<<dim3(2 * nblk, batch), z::kHwCols, 0, st>>>(A, Q, n, nn, hw, k, nblk, skip);
+        z::hw_update_kernel<<<dim3(2 * nblk, batch), z::kHwCols, 0, st>>>(A, Q, n, nn, hw, k, nblk, skip);
     }
-    z::hw_finish_kernel<C><<<(batch + 255) / 256, 256, 0, st>>>(Q, n, nn, batch, skip);
     SCW_CUDA_TRY(cudaGetLastError());
     return SCW_OK;
 }
@@ -1276,22 +1194,19 @@ static std::atomic<int> g_qr_cluster{0};
 
 // The QR sweeps of `batch` matrices, `active` of them not skipped.  Single solves (wide) put each
 // matrix on a cluster of K CTAs: the largest K <= 8 for which all active matrices' clusters are
-// resident at once (cudaOccupancyMaxActiveClusters) and, in FP32, no larger than the stripes of a
-// window fill (2n tasks for K x 1024 threads; FP64 updates are bound by the FP64 rate of each SM
-// and gain from more SMs down to fewer tasks per CTA).  Otherwise one CTA per matrix.
-template <typename C>
-static scw_status hqr_launch(cudaStream_t st, C* A, C* Q, int n, long long nn, C* W, int* status, const int* skip,
+// resident at once (cudaOccupancyMaxActiveClusters; the updates are bound by the FP64 rate of each
+// SM and gain from more SMs down to few tasks per CTA).  Otherwise one CTA per matrix.
+static scw_status hqr_launch(cudaStream_t st, double2* A, double2* Q, int n, long long nn, double2* W, int* status, const int* skip,
                              int batch, int active, bool wide) {
-    const size_t smem = z::hqr_smem_bytes<C>();
+    const size_t smem = z::hqr_smem_bytes();
     const int force = g_qr_cluster.load();
     if (wide && force != 1 && active > 0) {
         int dev = 0, sms = 0;
         SCW_CUDA_TRY(cudaGetDevice(&dev));
         SCW_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        SCW_CUDA_TRY(cudaFuncSetAttribute(z::hqr_cluster_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        SCW_CUDA_TRY(cudaFuncSetAttribute(z::hqr_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)smem));
         int kmax = force > 1 ? std::min(force, 8) : std::min(8, sms / active);
-        if (force <= 1 && sizeof(C) == sizeof(float2)) kmax = std::min(kmax, (2 * n + 1023) / 1024);
         for (int k = kmax; k >= 2; k--) {
             cudaLaunchConfig_t cfg = {};
             cudaLaunchAttribute at[1];
@@ -1306,26 +1221,41 @@ static scw_status hqr_launch(cudaStream_t st, C* A, C* Q, int n, long long nn, C
             cfg.attrs = at;
             cfg.numAttrs = 1;
             int resident = 0;
-            if (cudaOccupancyMaxActiveClusters(&resident, z::hqr_cluster_kernel<C>, &cfg) != cudaSuccess) {
+            if (cudaOccupancyMaxActiveClusters(&resident, z::hqr_cluster_kernel, &cfg) != cudaSuccess) {
                 cudaGetLastError();
                 continue;
             }
             if (resident >= (force > 1 ? 1 : active)) {
-                SCW_CUDA_TRY(cudaLaunchKernelEx(&cfg, z::hqr_cluster_kernel<C>, A, Q, n, nn, W, status, skip));
+                SCW_CUDA_TRY(cudaLaunchKernelEx(&cfg, z::hqr_cluster_kernel, A, Q, n, nn, W, status, skip));
                 return SCW_OK;
             }
         }
     }
-    SCW_CUDA_TRY(cudaFuncSetAttribute(z::hqr_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    z::hqr_kernel<C><<<batch, 1024, smem, st>>>(A, Q, n, nn, W, status, skip);
+    SCW_CUDA_TRY(cudaFuncSetAttribute(z::hqr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    z::hqr_kernel<<<batch, 1024, smem, st>>>(A, Q, n, nn, W, status, skip);
     SCW_CUDA_TRY(cudaGetLastError());
     return SCW_OK;
 }
 
 template <typename C>
-scw_status schur(cudaStream_t st, C* A, C* Q, C* W, int n, int batch, C* hw, int* status, const int* skip, bool wide) {
+scw_status trevc(cudaStream_t st, const C* T, C* X, int n, int batch, const int* skip) {
+    z::trevc_kernel<C><<<dim3((n * 32 + 255) / 256, batch), 256, 0, st>>>(T, X, n, (long long)n * n, skip);
+    SCW_CUDA_TRY(cudaGetLastError());
+    return SCW_OK;
+}
+
+scw_status trtri32(cudaStream_t st, const float2* X, float2* Z, int n, int batch) {
+    z::trtri_kernel<float2><<<dim3((n * 32 + 255) / 256, batch), 256, 0, st>>>(X, Z, n, (long long)n * n);
+    SCW_CUDA_TRY(cudaGetLastError());
+    return SCW_OK;
+}
+
+scw_status zgeev(cudaStream_t st, double2* A, double2* W, double2* V, int n, int batch, double2* work, int* status,
+                 const int* skip, bool wide, const GemmWs& ws) {
     if (n <= 0 || batch <= 0) return SCW_OK;
     const long long nn = (long long)n * n;
+    double2* Q = work;                       // batch * n * n: Schur vectors
+    double2* hw = work + nn * batch;         // batch * 3n
     SCW_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int) * batch, st));
     // single solves outside a stream capture count the matrices the skip mask leaves (and do
     // nothing when it leaves none)
@@ -1342,55 +1272,39 @@ scw_status schur(cudaStream_t st, C* A, C* Q, C* W, int n, int batch, C* hw, int
         }
     }
     if (wide && n >= kWideMinN) {
-        scw_status s = gehrd_wide<C>(st, A, Q, n, batch, hw, skip);
+        scw_status s = gehrd_wide(st, A, Q, n, batch, hw, skip);
         if (s != SCW_OK) return s;
     } else {
-        z::hessenberg_kernel<C><<<batch, 1024, 0, st>>>(A, Q, n, nn, hw, skip);
+        z::hessenberg_kernel<<<batch, 1024, 0, st>>>(A, Q, n, nn, hw, skip);
         SCW_CUDA_TRY(cudaGetLastError());
     }
-    return hqr_launch<C>(st, A, Q, n, nn, W, status, skip, batch, active, wide);
-}
-
-template <typename C>
-scw_status trevc(cudaStream_t st, const C* T, C* X, int n, int batch, const int* skip) {
-    z::trevc_kernel<C><<<dim3((n * 32 + 255) / 256, batch), 256, 0, st>>>(T, X, n, (long long)n * n, skip);
-    SCW_CUDA_TRY(cudaGetLastError());
-    return SCW_OK;
-}
-
-scw_status trtri32(cudaStream_t st, const float2* X, float2* Z, int n, int batch) {
-    z::trtri_kernel<float2><<<dim3((n * 32 + 255) / 256, batch), 256, 0, st>>>(X, Z, n, (long long)n * n);
-    SCW_CUDA_TRY(cudaGetLastError());
-    return SCW_OK;
-}
-
-template <typename C>
-scw_status geev(cudaStream_t st, C* A, C* W, C* V, int n, int batch, C* work, int* status, const int* skip,
-                bool wide, const GemmWs& ws) {
-    // A (overwritten): n x n per batch entry; W: n eigenvalues; V: n x n right eigenvectors (columns)
-    // work: >= batch * (n*n + 3 n) elements
-    if (n <= 0 || batch <= 0) return SCW_OK;
-    const long long nn = (long long)n * n;
-    C* Q = work;                             // batch * n * n: Schur vectors
-    scw_status s = schur<C>(st, A, Q, W, n, batch, work + nn * batch, status, skip, wide);
+    scw_status s = hqr_launch(st, A, Q, n, nn, W, status, skip, batch, active, wide);
     // triangular eigenvectors as the rows of V, then V := Q V^T
-    if (s == SCW_OK) s = trevc<C>(st, A, V, n, batch, skip);
+    if (s == SCW_OK) s = trevc<double2>(st, A, V, n, batch, skip);
     if (s != SCW_OK) return s;
-    if constexpr (sizeof(C) == sizeof(double2))
-        return zgemm(st, n, n, n, make_double2(1, 0), Q, n, nn, V, n, nn, make_double2(0, 0), V, n, nn, batch, ws, skip,
-                     0.0, kOpT);
-    else
-        return gemm32(st, n, 1.0, Q, V, kOpT, 0.0, 0.0, V, batch, ws, skip);
+    return zgemm(st, n, n, n, make_double2(1, 0), Q, n, nn, V, n, nn, make_double2(0, 0), V, n, nn, batch, ws, skip, 0.0,
+                 kOpT);
+}
+
+scw_status schur32(cudaStream_t st, float2* A, float2* Q, float2* W, int n, int batch, float2* work, int* status,
+                   const GemmWs& ws, int share) {
+    scw_status s = hess32(st, A, Q, n, batch, work, ws, share);
+    if (s == SCW_OK) s = hqr32(st, A, Q, n, W, status, batch, g_qr_cluster.load(), share);
+    return s;
+}
+
+scw_status cgeev(cudaStream_t st, float2* A, float2* W, float2* V, int n, int batch, float2* work, int* status,
+                 const GemmWs& ws, int share) {
+    float2* Q = work;                        // batch * n * n: Schur vectors
+    scw_status s = schur32(st, A, Q, W, n, batch, work + (long long)n * n * batch, status, ws, share);
+    if (s == SCW_OK) s = trevc<float2>(st, A, V, n, batch, nullptr);
+    if (s != SCW_OK) return s;
+    return gemm32(st, n, 1.0, Q, V, kOpT, 0.0, 0.0, V, batch, ws, nullptr);
 }
 
 template scw_status gemm<double2>(cudaStream_t, int, int, int, double2, const double2*, int, long long, const double2*, int,
                                   long long, double2, double2*, int, long long, int, const int*);
-template scw_status schur<float2>(cudaStream_t, float2*, float2*, float2*, int, int, float2*, int*, const int*, bool);
 template scw_status trevc<float2>(cudaStream_t, const float2*, float2*, int, int, const int*);
-template scw_status geev<double2>(cudaStream_t, double2*, double2*, double2*, int, int, double2*, int*, const int*, bool,
-                                  const GemmWs&);
-template scw_status geev<float2>(cudaStream_t, float2*, float2*, float2*, int, int, float2*, int*, const int*, bool,
-                                 const GemmWs&);
 
 }  // namespace scw
 
@@ -1473,8 +1387,8 @@ scw_status scw_zgeev(scw_ctx ctx, int n, void* A, void* W, void* V, int batch, i
     scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, scw::kGemmWsCap)));
     if (st == SCW_OK) st = scw::ctx_tc_flag(ctx);
     if (st == SCW_OK)
-        st = scw::geev<double2>(ctx->stream, (double2*)A, (double2*)W, (double2*)V, n, batch, work, dst, nullptr, true,
-                                scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err});
+        st = scw::zgeev(ctx->stream, (double2*)A, (double2*)W, (double2*)V, n, batch, work, dst, nullptr, true,
+                        scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err});
     ctx->launches += 4;
     std::vector<int> status(batch, 0);
     if (st == SCW_OK) {
@@ -1498,7 +1412,7 @@ scw_status scw_cgeev(scw_ctx ctx, int n, void* A, void* W, void* V, int batch, i
     SCW_ON_DEVICE(ctx->device);
     float2* work = nullptr;
     int* dst = nullptr;
-    const size_t wbytes = sizeof(float2) * ((size_t)n * n + 3 * (size_t)n) * batch;
+    const size_t wbytes = sizeof(float2) * ((size_t)n * n + scw::hess32_ws_elems(n)) * batch;
     if (cudaMalloc(&work, wbytes) != cudaSuccess || cudaMalloc(&dst, sizeof(int) * batch) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(work);
@@ -1509,8 +1423,8 @@ scw_status scw_cgeev(scw_ctx ctx, int n, void* A, void* W, void* V, int batch, i
     scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, scw::kGemmWsCap)));
     if (st == SCW_OK) st = scw::ctx_tc_flag(ctx);
     if (st == SCW_OK)
-        st = scw::geev<float2>(ctx->stream, (float2*)A, (float2*)W, (float2*)V, n, batch, work, dst, nullptr, true,
-                               scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err});
+        st = scw::cgeev(ctx->stream, (float2*)A, (float2*)W, (float2*)V, n, batch, work, dst,
+                        scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err}, 1);
     ctx->launches += 5;
     std::vector<int> status(batch, 0);
     if (st == SCW_OK) {

@@ -61,6 +61,8 @@ void eigmix_carve_small(EigMixWs& w, char* base, int n, int Z) {
     w.steps = (int*)take(sizeof(int) * Z);
     w.Y = (double2*)take(sizeof(double2) * zn * kMaxCluster);
     w.Yi = (float2*)take(sizeof(float2) * zn * kMaxCluster);
+    w.hp = (float2*)take(sizeof(float2) * Z * hess32_ws_elems(n));
+    w.lam32 = (float2*)take(sizeof(float2) * zn);
     w.rn = (double*)take(sizeof(double) * zn);
     w.xn = (double*)take(sizeof(double) * zn);
     w.anorm = (double*)take(sizeof(double) * Z);
@@ -631,7 +633,6 @@ scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int
     if (n <= 0 || Z <= 0) return SCW_OK;
     if (n > kMaxN) return fail(SCW_ERR_ARG, "geev_mixed: matrix order above the mixed path's limit");
     const long long nn = (long long)n * n;
-    if (w.hw != w.S1 + nn * Z) return fail(SCW_ERR_ARG, "geev_mixed: the FP32 QR work must follow slot S1");
     const unsigned gZ = std::min<long long>(nblk(nn), 2048);
     const size_t cl_smem = (size_t)n * (sizeof(double2) + 4 * sizeof(int));
     const size_t eig_smem = 3 * sizeof(double2) * kMaxCluster * kMaxCluster;
@@ -655,7 +656,7 @@ scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int
     MX_LAUNCHED(2);
     // FP32 Householder + QR: T in S0, Schur vectors Q in S1, eigenvalues lam32.  Triangular
     // eigenvectors Xt (rows of S2) and their inverse (S3): X = Q Xt, X^-1 = Xt^-1 Q^H
-    MX_TRY(schur<float2>(st, w.S0, w.S1, w.lam32, n, Z, w.hw, w.qr, nullptr, prm.wide));
+    MX_TRY(schur32(st, w.S0, w.S1, w.lam32, n, Z, w.hp, w.qr, ws, prm.share));
     MX_TRY(trevc<float2>(st, w.S0, w.S2, n, Z, nullptr));
     MX_TRY(trtri32(st, w.S2, w.S3, n, Z));
     MX_TRY(gemm32(st, n, 1.0, w.S1, w.S2, kOpT, 0.0, 0.0, V, Z, ws, nullptr));
@@ -698,7 +699,7 @@ scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int
     // slices without convergence: the FP64 Householder + QR solver (qr[] reused as the skip mask)
     final_kernel<<<nblk(Z), 256, 0, st>>>(w.state, w.qr, Z);
     MX_LAUNCHED(1);
-    MX_TRY(geev<double2>(st, A, lam, V, n, Z, fb_work, status, w.qr, prm.wide, ws));
+    MX_TRY(zgeev(st, A, lam, V, n, Z, fb_work, status, w.qr, prm.wide, ws));
     if (launches) *launches += 5;
     return SCW_OK;
 }
@@ -717,7 +718,7 @@ extern "C" scw_status scw_zgeev_mixed(scw_ctx ctx, int n, void* A, void* W, void
     if (n > mx::kMaxN) return fail(SCW_ERR_ARG, "scw_zgeev_mixed: n above 4096");
     SCW_ON_DEVICE(ctx->device);
     const size_t nn = (size_t)n * n;
-    // FP64 fallback work (>= 2 Z n^2 + 4 Z n float2 for S0, S1, hw, lam32), W region (S2, S3), small buffers
+    // FP64 fallback work (>= 2 Z n^2 float2 for S0, S1), W region (S2, S3), small buffers
     const size_t pbytes = sizeof(double2) * (nn + 3 * (size_t)n) * batch;
     const size_t wbytes = sizeof(double2) * nn * batch;
     const size_t sbytes = mx::eigmix_small_bytes(n, batch);
@@ -735,8 +736,6 @@ extern "C" scw_status scw_zgeev_mixed(scw_ctx ctx, int n, void* A, void* W, void
     float2* Wf = reinterpret_cast<float2*>(blk + pal);
     w.S0 = Pf;
     w.S1 = Pf + nn * batch;
-    w.hw = Pf + 2 * nn * batch;
-    w.lam32 = w.hw + 3 * (size_t)n * batch;
     w.S2 = Wf;
     w.S3 = Wf + nn * batch;
     long long L = 0;

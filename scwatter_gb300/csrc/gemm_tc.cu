@@ -53,8 +53,10 @@ struct Cfg {
     static constexpr int kTN = 256 / S;          // tile columns: S diagonals x 2 parts fill the TMEM
     static constexpr int kABlk = 2 * S * kTM * kTK * 2;   // bytes of A per stage: re, im x digits x 128 x 16 bf16
     static constexpr int kBBlk = 2 * S * kTN * kTK * 2;
-    static constexpr int kStages = S == 8 ? 2 : 4;
-    static constexpr size_t kSmem = (size_t)kStages * (kABlk + kBBlk) + (2 * kStages + 4) * sizeof(uint64_t);
+    static constexpr int kStages = S == 8 ? 2 : 3;
+    static constexpr int kStageOff = kStages * (kABlk + kBBlk);      // output staging after the operands
+    static constexpr int kBarOff = kStageOff + 8 * 32 * 144;
+    static constexpr size_t kSmem = (size_t)kBarOff + (2 * kStages + 4) * sizeof(uint64_t);
 };
 constexpr int kChunk = 8;                    // stages per drain (K = 128)
 constexpr int kDrainWarps = 8;
@@ -174,7 +176,7 @@ struct SplitArgs {
     const void *A, *B;
     long long rsA, ksA, rsB, ksB;      // element (row of A or column of B, inner index k) at row rs + k ks
     long long sA, sB;
-    int conjB;                         // 1: the conjugate of B
+    int conjA, conjB;                  // 1: the conjugate
     int M, N, K, nk, mt, nt;           // nk stages, mt x nt tiles
     int gA, gB, nA;                    // 16-row groups of A, 16-column groups of B per matrix; A blocks in all
     const int* f;
@@ -235,7 +237,7 @@ __device__ __forceinline__ void split_group(const SplitArgs& p, int b, int g, in
                 const int s = (kA ? f[k] : -f[k]) - e + C::kBits;
                 qr[j] = fixed_point(v.x, s);
                 qi[j] = fixed_point(v.y, s);
-                if (!kA && p.conjB) qi[j] = -qi[j];
+                if (kA ? p.conjA : p.conjB) qi[j] = -qi[j];
             }
         }
         unsigned char* o = dst + (long long)st * blkb;
@@ -285,6 +287,15 @@ __device__ __forceinline__ double fx_to_double(long long hi, long long lo, int e
     return scalbn(__longlong_as_double((long long)(sign + (1022ull << 52) + r)), max(-5000, min(5000, ex - 1023)));
 }
 
+// w 2^e in FP32 for |w| < 2^56: the two 24-bit and 32-bit parts are converted exactly but for the upper
+// one's rounding
+__device__ __forceinline__ float fx_to_float(long long w, int e) {
+    const float f = fmaf((float)(int)(w >> 24), 16777216.f, (float)(int)((unsigned)w & 0xffffffu));
+    e = max(-250, min(250, e));
+    const int h = e >> 1;
+    return f * __int_as_float((h + 127) << 23) * __int_as_float((e - h + 127) << 23);
+}
+
 struct GemmArgs {
     const unsigned char *dA, *dB;
     const int *eA, *gN;
@@ -303,6 +314,8 @@ __device__ __forceinline__ double2 to_d(double2 v) { return v; }
 __device__ __forceinline__ double2 to_d(float2 v) { return make_double2(v.x, v.y); }
 __device__ __forceinline__ void put(double2* p, double2 v) { *p = v; }
 __device__ __forceinline__ void put(float2* p, double2 v) { *p = make_float2((float)v.x, (float)v.y); }
+__device__ __forceinline__ void put(double2* p, float x, float y) { *p = make_double2(x, y); }
+__device__ __forceinline__ void put(float2* p, float x, float y) { *p = make_float2(x, y); }
 
 template <int S, typename TC>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -313,7 +326,7 @@ oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* sA = smem;
     unsigned char* sB = smem + kStages * kABlk;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sB + kStages * kBBlk);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + Cfg<S>::kBarOff);
     uint64_t* full = bar;                         // [kStages] copies -> MMA
     uint64_t* empty = bar + kStages;              // [kStages] MMA -> copies
     uint64_t* acc_full = bar + 2 * kStages;       // MMA -> drain
@@ -456,44 +469,69 @@ oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
                 mbar_arrive(acc_empty);
             }
             if (!ok) break;
-            const int row = m * kTM + quarter * 32 + lane, col0 = n * kTN + half * kCols;
-            if (row < p.M) {
-                const int eA = p.eA[(long long)(p.a_shared ? 0 : b) * p.gA * 16 + row];
-                const int* gN = p.gN + (long long)(p.b_shared ? 0 : b) * p.gB * 16 + col0;
-                TC* out = (TC*)p.C + p.sC * b + (long long)row * p.ldc + col0;
-                const bool unit = p.alpha.y == 0.0 && (p.alpha.x == 1.0 || p.alpha.x == -1.0);
-                const bool add = p.beta.x != 0.0 || p.beta.y != 0.0;
-                const bool add1 = p.beta.x == 1.0 && p.beta.y == 0.0;
+            // kSeg columns at a time: every lane converts its row's values into the warp's staging rows
+            // (144 bytes apart: no bank conflicts), then the warp reads and writes C in segments of
+            // 128 contiguous bytes per row
+            constexpr int kSeg = 128 / (int)sizeof(TC);
+            unsigned char* stg = smem + Cfg<S>::kStageOff + warp * 32 * 144;
+            const int row0 = m * kTM + quarter * 32, row = row0 + lane, col0 = n * kTN + half * kCols;
+            const int eA = row < p.M ? p.eA[(long long)(p.a_shared ? 0 : b) * p.gA * 16 + row] : kNone;
+            const int* gN = p.gN + (long long)(p.b_shared ? 0 : b) * p.gB * 16 + col0;
+            TC* out = (TC*)p.C + p.sC * b + (long long)row0 * p.ldc + col0;
+            const bool unit = p.alpha.y == 0.0 && (p.alpha.x == 1.0 || p.alpha.x == -1.0);
+            const bool add = p.beta.x != 0.0 || p.beta.y != 0.0;
+            const bool add1 = p.beta.x == 1.0 && p.beta.y == 0.0;
+            // an FP32 result without a diagonal needs no FP64 on the way
+            const bool narrow = sizeof(TC) == sizeof(float2) && unit && p.diag == 0.0;
 #pragma unroll
-                for (int c = 0; c < kCols; c++) {
-                    if (col0 + c < p.N) {
-                        const int g = gN[c];
-                        // the last diagonal weighs 2^(8 (S - 1)); units 2^(eA - kBits) 2^(g - kBits)
-                        const int e = eA + g + 8 * (kS - 1) - 2 * Cfg<S>::kBits;
-                        double2 v;
-                        if (eA >= kSpecial || g >= kSpecial) {
-                            v.x = v.y = __longlong_as_double(0x7ff8000000000000ll);
-                        } else if (kW == 2) {
-                            v.x = fx_to_double(w[0][0][c], w[kW - 1][0][c], e);
-                            v.y = fx_to_double(w[0][1][c], w[kW - 1][1][c], e);
-                        } else {
-                            v.x = fx_to_double(0, w[0][0][c], e);
-                            v.y = fx_to_double(0, w[0][1][c], e);
-                        }
-                        if (unit) {
-                            if (p.alpha.x < 0.0) v = make_double2(-v.x, -v.y);
-                        } else {
-                            v = z::cmul(p.alpha, v);
-                        }
-                        if (p.diag != 0.0 && row == col0 + c) v.x += p.diag;
-                        if (add1) {
-                            const double2 o = to_d(out[c]);
-                            v = make_double2(v.x + o.x, v.y + o.y);
-                        } else if (add) {
-                            v = z::cfma(p.beta, to_d(out[c]), v);
-                        }
-                        put(out + c, v);
+            for (int c0 = 0; c0 < kCols; c0 += kSeg) {
+                if (row0 >= p.M || col0 + c0 >= p.N) break;      // uniform
+                __syncwarp();
+#pragma unroll
+                for (int cc = 0; cc < kSeg; cc++) {
+                    const int c = c0 + cc;
+                    TC* dst = reinterpret_cast<TC*>(stg + lane * 144) + cc;
+                    const int g = col0 + c < p.N ? gN[c] : kNone;
+                    // the last diagonal weighs 2^(8 (S - 1)); units 2^(eA - kBits) 2^(g - kBits)
+                    const int e = eA + g + 8 * (kS - 1) - 2 * Cfg<S>::kBits;
+                    if (narrow && eA < kSpecial && g < kSpecial) {
+                        const float sg = p.alpha.x < 0.0 ? -1.f : 1.f;
+                        put(dst, sg * fx_to_float(w[0][0][c], e), sg * fx_to_float(w[0][1][c], e));
+                        continue;
                     }
+                    double2 v;
+                    if (eA >= kSpecial || g >= kSpecial) {
+                        v.x = v.y = __longlong_as_double(0x7ff8000000000000ll);
+                    } else if (kW == 2) {
+                        v.x = fx_to_double(w[0][0][c], w[kW - 1][0][c], e);
+                        v.y = fx_to_double(w[0][1][c], w[kW - 1][1][c], e);
+                    } else {
+                        v.x = fx_to_double(0, w[0][0][c], e);
+                        v.y = fx_to_double(0, w[0][1][c], e);
+                    }
+                    if (unit) {
+                        if (p.alpha.x < 0.0) v = make_double2(-v.x, -v.y);
+                    } else {
+                        v = z::cmul(p.alpha, v);
+                    }
+                    if (p.diag != 0.0 && row == col0 + c) v.x += p.diag;
+                    put(dst, v);
+                }
+                __syncwarp();
+#pragma unroll 4
+                for (int q = lane; q < 32 * kSeg; q += 32) {
+                    const int r = q / kSeg, cc = q % kSeg;
+                    if (row0 + r >= p.M || col0 + c0 + cc >= p.N) continue;
+                    TC v = reinterpret_cast<const TC*>(stg + r * 144)[cc];
+                    TC* o = out + (long long)r * p.ldc + c0 + cc;
+                    if (add1) {
+                        const TC x = *o;
+                        v.x += x.x;
+                        v.y += x.y;
+                    } else if (add) {
+                        put(&v, z::cfma(p.beta, to_d(*o), to_d(v)));
+                    }
+                    *o = v;
                 }
             }
         }
@@ -553,8 +591,8 @@ struct Shape {
 
 // One product with S digits; element types double2 or float2 by operand.
 template <int S, typename TA, typename TB, typename TC>
-static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const TA* A, int lda, long long sA, const TB* B,
-                      int ldb, long long sB, int opB, double2 beta, double diag, TC* C, int ldc, long long sC, int batch,
+static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const TA* A, int lda, long long sA, int opA,
+                      const TB* B, int ldb, long long sB, int opB, double2 beta, double diag, TC* C, int ldc, long long sC, int batch,
                       const GemmWs& ws, const int* skip) {
     if (M <= 0 || N <= 0 || batch <= 0) return SCW_OK;
     int sms = 0, dev = 0;
@@ -564,7 +602,8 @@ static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const
     SCW_CUDA_TRY(cudaFuncSetAttribute(oz_gemm_kernel<S, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const Shape sh(S, M, N, K);
     const bool a1 = sA == 0 && !skip, b1 = sB == 0 && !skip;     // one operand for the whole batch
-    // element (k, j) of op(B) at k ksB + j rsB
+    // element (i, k) of op(A) at i rsA + k ksA, (k, j) of op(B) at k ksB + j rsB
+    const long long rsA = opA == kOpN ? lda : 1, ksA = opA == kOpN ? 1 : lda;
     const long long ksB = opB == kOpN ? ldb : 1, rsB = opB == kOpN ? 1 : ldb;
     // as many matrices at a time as the workspace holds
     int step = batch;
@@ -594,7 +633,7 @@ static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const
                 SCW_CUDA_TRY(cudaMemsetAsync(f, 0, sizeof(int) * (size_t)K * nb_, st));
             }
         }
-        SplitArgs sp{Ab, Bb, lda, 1, rsB, ksB, sA, sB, opB == kOpC, M, N, K, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB,
+        SplitArgs sp{Ab, Bb, rsA, ksA, rsB, ksB, sA, sB, opA == kOpC, opB == kOpC, M, N, K, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB,
                      na_ * sh.gA, f, eA, gN, dA, dB, b1 ? 0 : 1};
         oz_split_kernel<S, TA, TB><<<na_ * sh.gA + nb_ * sh.gB, 256, 0, st>>>(sp, sk);
         SCW_CUDA_TRY(cudaGetLastError());
@@ -646,16 +685,24 @@ scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const doub
     }
     if (!ws.base && (diag != 0.0 || opB != kOpN)) return fail(SCW_ERR_ARG, "zgemm: this product needs a workspace");
     if (!ws.base) return gemm<double2>(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, skip);
-    return oz::run<8>(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, opB, beta, diag, C, ldc, sC, batch, ws, skip);
+    return oz::run<8>(st, M, N, K, alpha, A, lda, sA, kOpN, B, ldb, sB, opB, beta, diag, C, ldc, sC, batch, ws, skip);
 }
 
 template <typename TA, typename TB, typename TC>
 scw_status gemm32(cudaStream_t st, int n, double alpha, const TA* A, const TB* B, int opB, double beta, double diag, TC* C,
                   int batch, const GemmWs& ws, const int* skip) {
     const long long nn = (long long)n * n;
-    return oz::run<4>(st, n, n, n, make_double2(alpha, 0.0), A, n, nn, B, n, nn, opB, make_double2(beta, 0.0), diag, C, n,
+    return oz::run<4>(st, n, n, n, make_double2(alpha, 0.0), A, n, nn, kOpN, B, n, nn, opB, make_double2(beta, 0.0), diag, C, n,
                       nn, batch, ws, skip);
 }
+
+scw_status gemm32x(cudaStream_t st, int M, int N, int K, double alpha, const float2* A, int lda, long long sA, int opA,
+                   const float2* B, int ldb, long long sB, int opB, double beta, float2* C, int ldc, long long sC, int batch,
+                   const GemmWs& ws) {
+    return oz::run<4>(st, M, N, K, make_double2(alpha, 0.0), A, lda, sA, opA, B, ldb, sB, opB, make_double2(beta, 0.0), 0.0,
+                      C, ldc, sC, batch, ws, nullptr);
+}
+
 #define SCW_GEMM32(TA, TB, TC)                                                                                        \
     template scw_status gemm32<TA, TB, TC>(cudaStream_t, int, double, const TA*, const TB*, int, double, double, TC*, \
                                            int, const GemmWs&, const int*);

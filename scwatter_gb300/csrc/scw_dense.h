@@ -58,6 +58,10 @@ scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const doub
 template <typename TA, typename TB, typename TC>
 scw_status gemm32(cudaStream_t st, int n, double alpha, const TA* A, const TB* B, int opB, double beta, double diag, TC* C,
                   int batch, const GemmWs& ws, const int* skip);
+// any shape in FP32, with an operation on A too
+scw_status gemm32x(cudaStream_t st, int M, int N, int K, double alpha, const float2* A, int lda, long long sA, int opA,
+                   const float2* B, int ldb, long long sB, int opB, double beta, float2* C, int ldc, long long sC, int batch,
+                   const GemmWs& ws);
 
 // C = alpha A B + beta C (row-major, batched by strides in elements)
 template <typename C>
@@ -73,24 +77,31 @@ scw_status ztrsm_upper(cudaStream_t st, const double2* LU, int n, int lda, long 
 // B := A^-1 B using getrf's factors (leading dimension n; B: n x nrhs, leading dimension nrhs)
 scw_status zgetrs(cudaStream_t st, const double2* LU, int n, long long sA, const int* piv, long long sP, double2* B,
                   int nrhs, long long sB, int batch, const GemmWs& ws, const int* skip);
-// Schur form A = Q T Q^H (T over A, eigenvalues W); hw: 3 n per matrix
-template <typename C>
-scw_status schur(cudaStream_t st, C* A, C* Q, C* W, int n, int batch, C* hw, int* status, const int* skip, bool wide);
+// Schur form A = Q T Q^H in FP32 (T over A, eigenvalues W); work: hess32_ws_elems(n) per matrix; share:
+// solves of this size that run at the same time (lanes of a batch)
+scw_status schur32(cudaStream_t st, float2* A, float2* Q, float2* W, int n, int batch, float2* work, int* status,
+                   const GemmWs& ws, int share);
+// its stages: Hessenberg form of A with Q (hess32.cu), then the QR iteration with vectors accumulated into Z
+// (hqr32.cu; ctas: CTAs per matrix, 0 = chosen by size and batch)
+size_t hess32_ws_elems(int n);
+scw_status hess32(cudaStream_t st, float2* A, float2* Q, int n, int batch, float2* work, const GemmWs& ws, int share);
+scw_status hqr32(cudaStream_t st, float2* H, float2* Z, int n, float2* W, int* status, int batch, int ctas, int share);
 // eigenvectors of the triangular T as the rows of X (unit diagonal), and the inverse Z of the unit
 // triangular matrix whose columns those are
 template <typename C>
 scw_status trevc(cudaStream_t st, const C* T, C* X, int n, int batch, const int* skip);
 scw_status trtri32(cudaStream_t st, const float2* X, float2* Z, int n, int batch);
-// eigenvalues W and right eigenvectors V (columns) of A (overwritten); work >= batch (n^2 + 3 n);
+// eigenvalues W and right eigenvectors V (columns) of A (overwritten), FP64; work >= batch (n^2 + 3 n);
 // status[b] = 1 when the QR iteration did not converge.  wide: the Hessenberg reduction of
 // matrices with n >= kWideMinN is spread over the whole GPU (3 launches per column) instead of one
 // CTA per matrix -- for batches too small to fill the SMs; a batch graph with many concurrent
 // items keeps the one-CTA form (fewer nodes).
 constexpr int kWideMinN = 128;
-template <typename C>
-scw_status geev(cudaStream_t st, C* A, C* W, C* V, int n, int batch, C* work, int* status, const int* skip, bool wide,
-                const GemmWs& ws);
-
+scw_status zgeev(cudaStream_t st, double2* A, double2* W, double2* V, int n, int batch, double2* work, int* status,
+                 const int* skip, bool wide, const GemmWs& ws);
+// the same in FP32 (the first stage of the mixed solver); work >= batch (n^2 + hess32_ws_elems(n))
+scw_status cgeev(cudaStream_t st, float2* A, float2* W, float2* V, int n, int batch, float2* work, int* status,
+                 const GemmWs& ws, int share);
 // Hessenberg form of A (in place, n x n per batch entry) and the unitary Q (A = Q H Q^H);
 // work >= batch * 3 n
 scw_status zgehrd(cudaStream_t st, double2* A, double2* Q, int n, int batch, double2* work);

@@ -34,8 +34,8 @@ struct EigMixWs {
     // four FP32 n x n slots per matrix (S0 and S1 adjacent: together one FP64 n x n slot)
     // (after a solve S2 holds the FP32 inverse of every accepted eigenvector matrix)
     float2 *S0, *S1, *S2, *S3;
-    float2 *hw;                     // 3 n per matrix, directly after S1 (FP32 QR work)
-    float2 *lam32;                  // n per matrix
+    float2 *lam32;                  // n per matrix: FP32 eigenvalues
+    float2 *hp;                     // hess32_ws_elems(n) per matrix: the reduction's panels
     int *label, *member, *cstart, *ncl, *qr, *state, *steps;
     double2* Y;                     // kMaxCluster * n per matrix: cluster eigenvector blocks
     float2* Yi;                     // and their inverses
@@ -59,12 +59,13 @@ struct EigMixParams {
     double tol = 1e-14;             // a slice stops refining once its max relative column residual is this small
     double tol_accept = 1e-12;      // from step `steps` on: accepted at or below this; after the last
                                     // step, else the FP64 solver
-    bool wide = false;              // Hessenberg reductions spread over the GPU (see geev)
+    bool wide = false;              // the FP64 fallback spread over the GPU (see zgeev)
+    int share = 1;                  // solves that run at the same time (see schur32)
 };
 
 // Eigenpairs of Z matrices A (n x n, row-major, preserved unless a matrix falls back) into
 // lam (n per matrix) and V (n x n, columns).  fb_work: the FP64 fallback's work, >= Z (n^2 + 3 n)
-// double2, and it may alias S0..S3 / hw.  status[b] = 1 if even the FP64 fallback failed.
+// double2, and it may alias S0..S3.  status[b] = 1 if even the FP64 fallback failed.
 // Launches only (graph-capturable); *launches is incremented by the kernels issued.
 scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int n, int Z, const EigMixWs& w,
                       double2* fb_work, int* status, const EigMixParams& prm, const GemmWs& ws, long long* launches);

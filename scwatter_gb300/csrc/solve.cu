@@ -676,8 +676,7 @@ void carve_ws(const SolvePlan& p, Carver& c, SolveWs& ws) {
     ws.piv = c.take<int>(std::max(Z * n, M6));
     ws.worst = c.take<double>(2 * Z);
     ws.good = c.take<int>(2 * Z);
-    // mixed eigen-solver: small buffers of its own; S0, S1 (adjacent), its QR work and the FP32
-    // eigenvalues inside P (Z (n^2 + 3 n) double2 >= 2 Z n^2 + 4 Z n float2), S2, S3 inside W
+    // mixed eigen-solver: small buffers of its own; S0, S1 (adjacent) inside P, S2, S3 inside W
     if (p.eig_mixed) {
         char* small = c.take<char>(mx::eigmix_small_bytes((int)n, (int)Z));
         mx::eigmix_carve_small(ws.mix, small, (int)n, (int)Z);
@@ -685,8 +684,6 @@ void carve_ws(const SolvePlan& p, Carver& c, SolveWs& ws) {
         float2* Wf = reinterpret_cast<float2*>(ws.W);
         ws.mix.S0 = Pf;
         ws.mix.S1 = Pf + Z * nn;
-        ws.mix.hw = Pf + 2 * Z * nn;
-        ws.mix.lam32 = ws.mix.hw + 3 * Z * n;
         ws.mix.S2 = Wf;
         ws.mix.S3 = Wf + Z * nn;
     }
@@ -868,6 +865,7 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
     if (p.eig_mixed) {
         mx::EigMixParams prm;
         prm.wide = p.wide_hess;
+        prm.share = p.share;
         SCW_TRY(mx::geev_mixed(st, ws.PQ, ws.lam, ws.U, n, Zs, ws.mix, ws.P, out.status, prm, ws.gemm, &L));
         if (out.eig) {
             SCW_CUDA_TRY(cudaMemcpyAsync(out.eig, ws.mix.state, sizeof(int) * Zs, cudaMemcpyDeviceToDevice, st));
@@ -875,7 +873,7 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
             SCW_CUDA_TRY(cudaMemcpyAsync(out.eig_res, ws.mix.res, sizeof(double) * Zs, cudaMemcpyDeviceToDevice, st));
         }
     } else {
-        SCW_TRY(scw::geev<double2>(st, ws.PQ, ws.lam, ws.U, n, Zs, ws.P, out.status, nullptr, p.wide_hess, ws.gemm));
+        SCW_TRY(scw::zgeev(st, ws.PQ, ws.lam, ws.U, n, Zs, ws.P, out.status, nullptr, p.wide_hess, ws.gemm));
         L += 5;
     }
     roots_kernel<<<nblk((long long)n * Zs), 256, 0, st>>>(ws.lam, n, Zs, in.dz, k, out.gam, ws.E);

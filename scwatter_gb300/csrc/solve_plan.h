@@ -30,6 +30,7 @@ struct SolvePlan {
     bool eig_mixed = true;                  // FP32 QR + FP64 refinement (else FP64 QR throughout)
     bool reduced_bc = true;                 // boundary system of order 2MF (no |Sz| near zero), else 6MF
     bool wide_hess = false;                 // Hessenberg reductions over the whole GPU (single solves)
+    int share = 1;                          // solves recorded to run at the same time (lanes of a batch)
     std::vector<double> zb, dz;             // Z + 1 boundaries, Z thicknesses
     std::vector<int> ps, qs;                // integer harmonic series
     std::vector<double> up, wq;             // k grids (reference PI)

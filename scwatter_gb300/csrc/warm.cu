@@ -463,7 +463,7 @@ scw_status scw_eig_warm(scw_ctx ctx, int n, const void* A_, int batch, const voi
         for (int i = 0; i < nr; i++)
             SCW_CUDA_TRY(cudaMemcpyAsync(FA + nn * i, A + nn * reject[i], sizeof(double2) * nn,
                                          cudaMemcpyDeviceToDevice, st));
-        if ((s = scw::geev<double2>(st, FA, FW, FV, n, nr, FWk, fst, nullptr, false, gws)) != SCW_OK) return s;
+        if ((s = scw::zgeev(st, FA, FW, FV, n, nr, FWk, fst, nullptr, false, gws)) != SCW_OK) return s;
         for (int i = 0; i < nr; i++) {
             SCW_CUDA_TRY(cudaMemcpyAsync(V + nn * reject[i], FV + nn * i, sizeof(double2) * nn, cudaMemcpyDeviceToDevice, st));
             SCW_CUDA_TRY(cudaMemcpyAsync(W + (long long)n * reject[i], FW + (long long)n * i, sizeof(double2) * n,
