@@ -231,8 +231,8 @@ SCW_API scw_status scw_sep_eval_slab_host(scw_sep s, const void* Q_host, float x
  * 192 MiB) and output bytes per read-back slab (whole planes, at least one; default 64 MiB; three
  * slabs are kept on the device).  0 restores a default. */
 SCW_API scw_status scw_sep_set_streaming(scw_sep s, int64_t chunk_bytes, int64_t slab_bytes);
-/* Tile shape of the coefficient contraction: 0 (default) = 8, 8, 4, 2 mode rows per warp for
- * launches of 1, 2, 4, 8 planes per group; 1 = half as many.  Results are bit-identical; the
+/* Tile shape of the coefficient contraction: 0 (default) = 8 mode rows per warp for launches of 1 or 2
+ * planes per group, 4 for 3 to 8; 1 = half as many.  Results are bit-identical; the
  * batch autotuner picks it for its items. */
 SCW_API scw_status scw_sep_set_tiles(scw_sep s, int ctr_shape);
 /* Device slabs of >= 32 planes in `chunks` chunks whose stages overlap on two streams (stage 1 of

@@ -17,6 +17,7 @@
 #include <cstring>
 #include <map>
 #include <new>
+#include <type_traits>
 
 #include "scw_internal.h"
 #include "scw_sep.h"
@@ -40,50 +41,45 @@ __device__ __forceinline__ float2 phase_fp64(double kr, double ki, double dz) {
 //   paired sets (beta != null): the mode amplitudes folded in, in FP64,
 //     h = 0 (rows Ex, Ey): beta_dn_j exp(i kz_dn_j (z - z_l)) + beta_up_j exp(i kz_up_j (z - z_{l+1}))
 //     h = 1 (rows Ez):     beta_dn_j exp(i kz_dn_j (z - z_l)) - beta_up_j exp(i kz_up_j (z - z_{l+1}))
+// One thread per mode (and half, of a two-half set) and plane, planes fastest (consecutive stores): with one
+// thread per mode looping over the planes, the chain of FP64 phases took 20 us for 200 modes.
 __global__ void sep_phase_kernel(const PGroup* __restrict__ groups, const float* __restrict__ zlist,
                                  const double2* __restrict__ kz, const double2* __restrict__ beta,
                                  const double* __restrict__ zb, int J, int nks, float2* __restrict__ Phi) {
-    const PGroup g = groups[blockIdx.y];
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    const PGroup& g = groups[blockIdx.y];
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = e / nks, kk = e - j * nks;
     const int l = g.region - 1;
+    float2* out = Phi + (long long)blockIdx.y * 2 * J * nks + e;
+    const bool live = kk < g.nk;
     if (!beta) {
-        // two-half set: one thread per (half, mode), j < 2 J
+        // two-half set: j < 2 J runs over (half, mode)
         if (j >= 2 * J) return;
-        const int half = j / J, jj = j - half * J;
-        float2* out = Phi + ((long long)blockIdx.y * 2 * J + j) * nks;
-        const double2 k = kz[((long long)l * 2 + half) * J + jj];
-        const double zref = half == 0 ? zb[l] : zb[l + 1];
-        for (int kk = 0; kk < nks; kk++) {
-            if (kk < g.nk) {
-                const double dz = (double)zlist[g.zi[kk]] - zref;
-                out[kk] = phase_fp64(k.x, k.y, dz);
-            } else {
-                out[kk] = make_float2(0.f, 0.f);
-            }
+        const int half = j >= J ? 1 : 0, jj = j - half * J;
+        float2 v = make_float2(0.f, 0.f);
+        if (live) {
+            const double2 k = kz[((long long)l * 2 + half) * J + jj];
+            v = phase_fp64(k.x, k.y, (double)zlist[g.zi[kk]] - zb[l + half]);
         }
+        *out = v;
         return;
     }
-    // paired set: one thread per mode j < J writes both halves from the same two phases
+    // paired set: one thread writes both halves from the same two phases
     if (j >= J) return;
-    const int jj = j;
-    float2* out0 = Phi + ((long long)blockIdx.y * 2 * J + jj) * nks;
-    float2* out1 = Phi + ((long long)blockIdx.y * 2 * J + J + jj) * nks;
-    const double2 kd = kz[(long long)l * 2 * J + jj], ku = kz[((long long)l * 2 + 1) * J + jj];
-    const double2 bd = beta[(long long)l * 2 * J + jj], bu = beta[((long long)l * 2 + 1) * J + jj];
-    for (int kk = 0; kk < nks; kk++) {
-        if (kk < g.nk) {
-            const double z = (double)zlist[g.zi[kk]];
-            const float2 fd = phase_fp64(kd.x, kd.y, z - zb[l]);
-            const float2 fu = phase_fp64(ku.x, ku.y, z - zb[l + 1]);
-            const double dre = bd.x * fd.x - bd.y * fd.y, dim = bd.x * fd.y + bd.y * fd.x;
-            const double ure = bu.x * fu.x - bu.y * fu.y, uim = bu.x * fu.y + bu.y * fu.x;
-            out0[kk] = make_float2((float)(dre + ure), (float)(dim + uim));
-            out1[kk] = make_float2((float)(dre - ure), (float)(dim - uim));
-        } else {
-            out0[kk] = make_float2(0.f, 0.f);
-            out1[kk] = make_float2(0.f, 0.f);
-        }
+    float2 v0 = make_float2(0.f, 0.f), v1 = v0;
+    if (live) {
+        const double z = (double)zlist[g.zi[kk]];
+        const double2 kd = kz[(long long)l * 2 * J + j], ku = kz[((long long)l * 2 + 1) * J + j];
+        const double2 bd = beta[(long long)l * 2 * J + j], bu = beta[((long long)l * 2 + 1) * J + j];
+        const float2 fd = phase_fp64(kd.x, kd.y, z - zb[l]);
+        const float2 fu = phase_fp64(ku.x, ku.y, z - zb[l + 1]);
+        const double dre = bd.x * fd.x - bd.y * fd.y, dim = bd.x * fd.y + bd.y * fd.x;
+        const double ure = bu.x * fu.x - bu.y * fu.y, uim = bu.x * fu.y + bu.y * fu.x;
+        v0 = make_float2((float)(dre + ure), (float)(dim + uim));
+        v1 = make_float2((float)(dre - ure), (float)(dim - uim));
     }
+    out[0] = v0;
+    out[(long long)J * nks] = v1;
 }
 
 // C[zi][c][p] = sum over the slice's modes of Q[l][h][c][p][j] * Phi[g][h'][j][kk]:
@@ -99,10 +95,11 @@ __global__ void sep_phase_kernel(const PGroup* __restrict__ groups, const float*
 constexpr int kCtrWarps = 8;
 constexpr int kCtrChunk = 1024;
 
-// pipeline depth of the Q stream: stages x rows per warp = 16 float4 in flight per lane
+// pipeline depth of the Q stream: stages x rows per warp = 16 float4 in flight per lane, 12 where the
+// phases of 7 or 8 planes leave no more shared memory for two CTAs per SM
 template <int RW, int NK>
 struct CtrCfg {
-    static constexpr int kStages = NK == 8 ? 4 : (16 / RW < 2 ? 2 : 16 / RW);
+    static constexpr int kStages = NK >= 7 ? 12 / RW : (16 / RW < 2 ? 2 : 16 / RW);
     static constexpr size_t kSmem = (size_t)NK * (kCtrChunk / 2) * 16 + (size_t)kCtrWarps * kStages * RW * 32 * 16;
 };
 
@@ -212,46 +209,49 @@ sep_contract_kernel(const PGroup* __restrict__ groups, const float2* __restrict_
 }
 
 // Exterior regions: region 0 = incident (referenced at the origin) + reflected (at z_0),
-// last region = transmitted (at z_Z).  One thread per (z entry, c, p), FP64.
+// last region = transmitted (at z_Z).  One thread per (z entry, p), FP64; the phases serve all three
+// components.
 __global__ void sep_exterior_kernel(const int2* __restrict__ ext, int n_ext, const float* __restrict__ zlist,
                                     const double2* __restrict__ xd, int MF, double z0, double zZ,
                                     float2* __restrict__ C) {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long)n_ext * 3 * MF) return;
-    const int e = (int)(idx / (3 * MF));
-    const int rem = (int)(idx % (3 * MF));
-    const int c = rem / MF, p = rem % MF;
+    if (idx >= (long long)n_ext * MF) return;
+    const int e = (int)(idx / MF), p = (int)(idx % MF);
     const int2 ent = ext[e];     // (zi, 0 = top exterior / 1 = bottom exterior)
     const double z = (double)zlist[ent.x];
     // xd layout: inc[3][MF], refl[3][MF], trans[3][MF], kz_inc[MF], kz_refl[MF], kz_trans[MF]
-    const double2* inc = xd;
-    const double2* refl = xd + 3 * MF;
-    const double2* trans = xd + 6 * MF;
     const double2* kzi = xd + 9 * MF;
-    const double2* kzr = xd + 10 * MF;
-    const double2* kzt = xd + 11 * MF;
-    double sr = 0.0, si = 0.0;
-    auto add = [&](double2 a, double2 k, double dz) {
-        const float2 f = phase_fp64(k.x, k.y, dz);
-        sr += a.x * (double)f.x - a.y * (double)f.y;
-        si += a.x * (double)f.y + a.y * (double)f.x;
-    };
-    if (ent.y == 0) {
-        add(inc[c * MF + p], kzi[p], z);
-        add(refl[c * MF + p], kzr[p], z - z0);
-    } else {
-        add(trans[c * MF + p], kzt[p], z - zZ);
+    const bool top = ent.y == 0;
+    const double2 ka = top ? kzi[p] : kzi[2 * MF + p], kb = kzi[MF + p];
+    const float2 fa = phase_fp64(ka.x, ka.y, top ? z : z - zZ);
+    const float2 fb = top ? phase_fp64(kb.x, kb.y, z - z0) : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        const double2 a = xd[(top ? c : 6 + c) * MF + p], b = xd[(3 + c) * MF + p];
+        double sr = a.x * (double)fa.x - a.y * (double)fa.y, si = a.x * (double)fa.y + a.y * (double)fa.x;
+        if (top) {
+            sr += b.x * (double)fb.x - b.y * (double)fb.y;
+            si += b.x * (double)fb.y + b.y * (double)fb.x;
+        }
+        C[((long long)ent.x * 3 + c) * MF + p] = make_float2((float)sr, (float)si);
     }
-    C[((long long)ent.x * 3 + c) * MF + p] = make_float2((float)sr, (float)si);
 }
 
-// tab[m][i] = exp(i k_m x_i), x_i = s + d * i in float (one rounding per operation)
-__global__ void sep_table_kernel(const double* __restrict__ k, int M, float s, float d, int N, float2* __restrict__ tab) {
+// The two phase tables of an evaluation in one launch (block row 0 or 1): tab[m][i] = exp(i k_m x_i),
+// x_i = s + d * i in float (one rounding per operation)
+struct TableArgs {
+    const double* k;
+    int M, N;
+    float s, d;
+    float2* tab;
+};
+__global__ void sep_table_kernel(TableArgs t0, TableArgs t1) {
+    const TableArgs t = blockIdx.y == 0 ? t0 : t1;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long long)M * N) return;
-    const int m = (int)(idx / N), i = (int)(idx % N);
-    const float x = __fadd_rn(s, __fmul_rn(d, (float)i));
-    tab[idx] = phase_fp64(k[m], 0.0, (double)x);
+    if (idx >= (long long)t.M * t.N) return;
+    const int m = (int)(idx / t.N), i = (int)(idx % t.N);
+    const float x = __fadd_rn(t.s, __fmul_rn(t.d, (float)i));
+    t.tab[idx] = phase_fp64(t.k[m], 0.0, (double)x);
 }
 
 // Stage 2a: T[r][c][m] = sum_n R(r, n) * C[zi(r)][c][p(m, n)]
@@ -455,10 +455,13 @@ static void stage1_plan(const scw_sep_s* s, SepEvalPlan& p) {
             for (int zi : kv.second) p.ext.push_back(make_int2(zi, r == 0 ? 0 : 1));
             continue;
         }
-        for (size_t o = 0; o < kv.second.size(); o += kMaxGroup) {
+        // as few passes as kMaxGroup planes each allow, of equal size: the widest group sets the kernel
+        const size_t np = kv.second.size(), ng = (np + kMaxGroup - 1) / kMaxGroup;
+        for (size_t gi = 0; gi < ng; gi++) {
+            const size_t o = gi * np / ng;
             PGroup g{};
             g.region = (int)r;
-            g.nk = (int)std::min<size_t>(kMaxGroup, kv.second.size() - o);
+            g.nk = (int)((gi + 1) * np / ng - o);
             for (int kk = 0; kk < g.nk; kk++) g.zi[kk] = kv.second[o + kk];
             p.max_nk = std::max(p.max_nk, g.nk);
             p.groups.push_back(g);
@@ -489,14 +492,14 @@ static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_d
     const float* dz = (const float*)(d_desc + p.off_z);
     if (!groups.empty()) {
         if (J > 0) {
-            const int nks = max_nk <= 1 ? 1 : max_nk <= 2 ? 2 : max_nk <= 4 ? 4 : 8;
+            const int nks = max_nk;            // a kernel per plane count: 5 planes cost 5, not 8
             float2* dPhi = (float2*)cursor;
             cursor += align256(groups.size() * 2 * (size_t)J * nks * sizeof(float2));
-            // one thread per (half, mode) for a two-half set, per mode for a paired set
-            dim3 gp(((s->halves == 1 ? J : 2 * J) + 255) / 256, (unsigned)groups.size());
+            // one thread per (half, mode, plane) for a two-half set, per (mode, plane) for a paired set
+            dim3 gp(((s->halves == 1 ? J : 2 * J) * nks + 127) / 128, (unsigned)groups.size());
             {
                 LaunchTimer lt(ctx, "sep_phase_kernel");
-                sep_phase_kernel<<<gp, 256, 0, ctx->stream>>>(dg, dz, s->dKz, s->halves == 1 ? s->dBeta : nullptr,
+                sep_phase_kernel<<<gp, 128, 0, ctx->stream>>>(dg, dz, s->dKz, s->halves == 1 ? s->dBeta : nullptr,
                                                               s->dzb, J, nks, dPhi);
             }
             SCW_CUDA_TRY(cudaGetLastError());
@@ -512,16 +515,21 @@ static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_d
                 return SCW_OK;
             };
             scw_status ls;
-            if (s->ctr_shape == 0) {
-                if (nks == 1) ls = launch(sep_contract_kernel<1, 8>, 8, CtrCfg<8, 1>::kSmem);
-                else if (nks == 2) ls = launch(sep_contract_kernel<2, 8>, 8, CtrCfg<8, 2>::kSmem);
-                else if (nks == 4) ls = launch(sep_contract_kernel<4, 4>, 4, CtrCfg<4, 4>::kSmem);
-                else ls = launch(sep_contract_kernel<8, 2>, 2, CtrCfg<2, 8>::kSmem);
-            } else {
-                if (nks == 1) ls = launch(sep_contract_kernel<1, 4>, 4, CtrCfg<4, 1>::kSmem);
-                else if (nks == 2) ls = launch(sep_contract_kernel<2, 4>, 4, CtrCfg<4, 2>::kSmem);
-                else if (nks == 4) ls = launch(sep_contract_kernel<4, 2>, 2, CtrCfg<2, 4>::kSmem);
-                else ls = launch(sep_contract_kernel<8, 1>, 1, CtrCfg<1, 8>::kSmem);
+            auto shapes = [&](auto nk) -> scw_status {
+                // rows per warp: 8 for one or two planes, 4 beyond; half as many in shape 1
+                constexpr int NK = decltype(nk)::value, RW = NK <= 2 ? 8 : 4;
+                if (s->ctr_shape == 0) return launch(sep_contract_kernel<NK, RW>, RW, CtrCfg<RW, NK>::kSmem);
+                return launch(sep_contract_kernel<NK, RW / 2>, RW / 2, CtrCfg<RW / 2, NK>::kSmem);
+            };
+            switch (nks) {
+                case 1: ls = shapes(std::integral_constant<int, 1>()); break;
+                case 2: ls = shapes(std::integral_constant<int, 2>()); break;
+                case 3: ls = shapes(std::integral_constant<int, 3>()); break;
+                case 4: ls = shapes(std::integral_constant<int, 4>()); break;
+                case 5: ls = shapes(std::integral_constant<int, 5>()); break;
+                case 6: ls = shapes(std::integral_constant<int, 6>()); break;
+                case 7: ls = shapes(std::integral_constant<int, 7>()); break;
+                default: ls = shapes(std::integral_constant<int, 8>()); break;
             }
             if (ls != SCW_OK) return ls;
             SCW_CUDA_TRY(cudaGetLastError());
@@ -535,7 +543,7 @@ static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_d
         }
     }
     if (!ext.empty()) {
-        const long long n = (long long)ext.size() * 3 * MF;
+        const long long n = (long long)ext.size() * MF;
         LaunchTimer lt(ctx, "sep_exterior_kernel");
         sep_exterior_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(de, (int)ext.size(), dz, s->dExt, MF,
                                                                                  s->zb[0], s->zb[s->Z], dC);
@@ -545,10 +553,10 @@ static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_d
     return SCW_OK;
 }
 
-static scw_status launch_table(scw_ctx ctx, const double* dk, int M, float st, float d, int N, float2* tab) {
-    const long long n = (long long)M * N;
+static scw_status launch_tables(scw_ctx ctx, const TableArgs& a, const TableArgs& b) {
+    const long long n = std::max((long long)a.M * a.N, (long long)b.M * b.N);
     LaunchTimer lt(ctx, "sep_table_kernel");
-    sep_table_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(dk, M, st, d, N, tab);
+    sep_table_kernel<<<dim3((unsigned)((n + 127) / 128), 2), 128, 0, ctx->stream>>>(a, b);
     SCW_CUDA_TRY(cudaGetLastError());
     ctx->launches++;
     return SCW_OK;
@@ -671,8 +679,8 @@ static scw_status stage2_record(scw_sep s, const SepEvalPlan& p, char* scratch, 
     const int nrows = p.nrows, ncols = p.ncols, Mk = p.Mk, Na = p.Na, Nb = p.Nb, Nz = p.Nz;
     if (p.kind == 0) {
         // F = Ex table [a][x]; R = Ey table [b][y]
-        if ((st = launch_table(ctx, s->dkx, M0, p.a0, p.da, Na, tabA)) != SCW_OK) return st;
-        if ((st = launch_table(ctx, s->dky, M1, p.b0, p.db, Nb, tabB)) != SCW_OK) return st;
+        if ((st = launch_tables(ctx, {s->dkx, M0, Na, p.a0, p.da, tabA}, {s->dky, M1, Nb, p.b0, p.db, tabB})) != SCW_OK)
+            return st;
         {
             const size_t smem = (size_t)(rows_phase_off(M0, M1) + kRowsBlk * M1) * sizeof(float2);
             SCW_CUDA_TRY(cudaFuncSetAttribute(sep_rows_volume_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -686,14 +694,12 @@ static scw_status stage2_record(scw_sep s, const SepEvalPlan& p, char* scratch, 
         return sep_synth(ctx, dT, tabA, nrows, ncols, Mk, dE, p.method);
     } else if (p.kind == 1) {
         // xz plane at y = c: R = Ey(c) [b]; F = Ex table [a][x]
-        if ((st = launch_table(ctx, s->dkx, M0, p.a0, p.da, Na, tabA)) != SCW_OK) return st;
-        if ((st = launch_table(ctx, s->dky, M1, p.c, 0.f, 1, tabB)) != SCW_OK) return st;
+        if ((st = launch_tables(ctx, {s->dkx, M0, Na, p.a0, p.da, tabA}, {s->dky, M1, 1, p.c, 0.f, tabB})) != SCW_OK) return st;
         if ((st = launch_rows(ctx, dC, tabB, 1, 1, 1, 0, nrows, 0, M0, M1, dT)) != SCW_OK) return st;
         return sep_synth(ctx, dT, tabA, nrows, ncols, Mk, dE, p.method);
     } else {
         // yz plane at x = c: R = Ex(c) [a]; F = Ey table [b][y]
-        if ((st = launch_table(ctx, s->dky, M1, p.a0, p.da, Na, tabA)) != SCW_OK) return st;
-        if ((st = launch_table(ctx, s->dkx, M0, p.c, 0.f, 1, tabB)) != SCW_OK) return st;
+        if ((st = launch_tables(ctx, {s->dky, M1, Na, p.a0, p.da, tabA}, {s->dkx, M0, 1, p.c, 0.f, tabB})) != SCW_OK) return st;
         if ((st = launch_rows(ctx, dC, tabB, 1, 1, 1, 0, nrows, 1, M0, M1, dT)) != SCW_OK) return st;
         return sep_synth(ctx, dT, tabA, nrows, ncols, Mk, dE, p.method);
     }
