@@ -7,6 +7,9 @@
 // AoS global memory):
 //  * Waves live on the device as SoA tables: Re k and Im k (double, 3 x n), the reference
 //    plane z_ref (double) and the amplitude at that plane (complex float, 3 x n).
+//  * Ordinary grids are summed as a matrix product on the tensor cores (eval_plain_tc.cu); the kernels here
+//    take what its operands cannot hold: waves that grow too much across a tile, coordinates so far out that
+//    their rounding matters, wave vectors that are not finite, and the capturable single plane.
 //  * A CTA evaluates a 16 x 32 tile of points (2 points per thread) against a chunk of one
 //    region's waves.  Waves are staged through shared memory 256 at a time; while staging,
 //    each thread re-bases one wave to the tile centre r_c in FP64:
@@ -27,6 +30,7 @@
 #include <cstring>
 #include <new>
 
+#include "plain_tc.h"
 #include "scw_internal.h"
 
 namespace scw {
@@ -37,14 +41,7 @@ constexpr int kThreads = 256;    // 16 x 16 threads, 2 rows each (j and j + 16)
 constexpr int kBatch = 256;      // waves staged in shared memory per step
 constexpr int kTilePts = kTI * kTJ;
 
-struct PlaneGeom {
-    float a0, b0, c;   // start along i (a) and j (b), fixed coordinate c
-    float da, db;      // spacings along i and j
-    int Ni, Nj;
-    int mode;          // 0: (a,b,c) = (x,y,z); 1: (y,z,x); 2: (x,z,y)
-    int pad;
-    float* out;        // [Nj][Ni][6] floats
-};
+using PlaneGeom = ptc::Plane;
 
 struct WorkItem {
     int plane;
@@ -385,9 +382,157 @@ static void plan_planes(const scw_waves_s* w, const std::vector<PlaneGeom>& plan
     }
 }
 
+// ------------------------------------------------------------------------------------
+// The tensor-core form (eval_plain_tc.cu): tiles of 40 columns x up to 64 rows of one region
+// ------------------------------------------------------------------------------------
+// What rounding a grid's coordinates leaves of whole steps, at most, between two of them.
+static double grid_dev(float s, float d, int n) {
+    double m = 0.0;
+    for (int i = 0; i < n; i++) m = std::max(m, std::fabs((double)host_grid_coord(s, d, i) - ((double)s + (double)d * i)));
+    return 2.0 * m;
+}
+
+// Rows of region r that a tile of plane g may have (a multiple of 8), 0 if none: along a tile's axes a wave
+// may grow by at most e^2.4 (columns) and e^4 (rows), which the scales of its fp16 operands leave room
+// for, and turns fewer than 2^21 times (the phase's two floats); the rounding of the grid's coordinates (devA,
+// devB), taken to first order, stays below 3e-4 radians.  Also 0 for wave vectors that are not finite.
+static int tc_rows(const scw_waves_s* w, const PlaneGeom& g, int64_t r, double devA = 0.0, double devB = 0.0) {
+    const int cA = g.mode == 1 ? 1 : 0, cB = g.mode == 0 ? 1 : 2;
+    const double da = std::fabs((double)g.da), db = std::fabs((double)g.db);
+    const double* m = &w->kmax[6 * (size_t)r];
+    const double kA = m[cA] + m[3 + cA], kB = m[cB] + m[3 + cB];
+    if (!(kA * da * ptc::kTileI < 2e7) || !(kB * db * ptc::kTileJ < 2e7) || !(m[3 + cA] * da * (ptc::kTileI / 2) <= 2.4) ||
+        !(kA * devA < 3e-4) || !(kB * devB < 3e-4))
+        return 0;
+    const double grow = m[3 + cB] * db * 0.5 * 1.05;      // per row; a margin for rounded coordinates
+    return grow * ptc::kTileJ <= 4.0 ? ptc::kTileJ : (int)(4.0 / grow) / 8 * 8;
+}
+
+// Whether the tensor-core form suits all planes: a tile of at least 16 rows in every region and
+// finite grids; otherwise the summation kernel.
+static bool tc_suits(const scw_waves_s* w, const std::vector<PlaneGeom>& planes) {
+    double devA = 0.0, devB = 0.0;
+    for (size_t i = 0; i < planes.size(); i++) {
+        const auto& g = planes[i];
+        const double far = std::fabs((double)g.a0) + std::fabs((double)g.da) * (g.Ni + ptc::kTileI) + std::fabs((double)g.b0) +
+                           std::fabs((double)g.db) * (g.Nj + ptc::kTileJ) + std::fabs((double)g.c);
+        if (!(far < 1e15)) return false;
+        if (i == 0 || g.a0 != planes[i - 1].a0 || g.da != planes[i - 1].da || g.Ni != planes[i - 1].Ni) devA = grid_dev(g.a0, g.da, g.Ni + ptc::kTileI);
+        if (i == 0 || g.b0 != planes[i - 1].b0 || g.db != planes[i - 1].db || g.Nj != planes[i - 1].Nj) devB = grid_dev(g.b0, g.db, g.Nj + ptc::kTileJ);
+        int64_t last = -1;
+        for (int j = 0; j < g.Nj; j++) {
+            const int64_t r = region_of(w, g.mode == 0 ? g.c : host_grid_coord(g.b0, g.db, j));
+            if (r != last && tc_rows(w, g, r, devA, devB) < 16) return false;
+            last = r;
+            if (g.mode == 0) break;
+        }
+    }
+    return true;
+}
+
+constexpr int kTcSlots = 2048;        // partial sums of one launch: 250 MB of scratch; more tiles take more launches
+
+struct TcPlan {
+    std::vector<ptc::Item> items;
+    std::vector<ptc::Tile> tiles;
+    int nslots = 0, max_rows = 1;
+};
+
+static void tc_plan(const scw_waves_s* w, const std::vector<PlaneGeom>& planes, int sm_count, std::vector<TcPlan>& plans) {
+    struct Run {
+        int plane, jr0, jr1;
+        int64_t region;
+    };
+    std::vector<Run> runs;            // rows of one region, at most kTileJ
+    double work = 0;
+    for (int pi = 0; pi < (int)planes.size(); pi++) {
+        const auto& g = planes[pi];
+        const int ti = (g.Ni + ptc::kTileI - 1) / ptc::kTileI;
+        for (int j = 0; j < g.Nj;) {
+            const int64_t r = region_of(w, g.mode == 0 ? g.c : host_grid_coord(g.b0, g.db, j));
+            int je = g.Nj;
+            if (g.mode != 0)
+                for (je = j + 1; je < g.Nj && region_of(w, host_grid_coord(g.b0, g.db, je)) == r;) je++;
+            const int h = tc_rows(w, g, r), nt = (je - j + h - 1) / h;     // tiles of equal height
+            for (int t = 0; t < nt; t++)
+                runs.push_back({pi, j + (int)((long long)(je - j) * t / nt), j + (int)((long long)(je - j) * (t + 1) / nt), r});
+            work += (double)nt * ti * (double)(w->end[r] - w->begin[r]);
+            j = je;
+        }
+    }
+    // waves per item: about 6 items per SM where there is enough, at least 128
+    long long chunk = (long long)std::ceil(work / (6.0 * sm_count));
+    chunk = (std::max<long long>(chunk, 128) + 31) / 32 * 32;
+    for (const auto& u : runs) {
+        const auto& g = planes[u.plane];
+        const long long b = w->begin[u.region], e = w->end[u.region];
+        const long long parts = std::max<long long>(1, (e - b + chunk - 1) / chunk);
+        const long long len = ((e - b + parts - 1) / parts + 31) / 32 * 32;
+        for (int i0 = 0; i0 < g.Ni; i0 += ptc::kTileI) {
+            if (plans.empty() || plans.back().nslots >= kTcSlots) plans.emplace_back();
+            TcPlan& P = plans.back();
+            P.max_rows = std::max(P.max_rows, u.jr1 - u.jr0);
+            const bool direct = e - b <= std::min<long long>(std::max<long long>(len, 1), ptc::kMaxRun);
+            ptc::Tile t{u.plane, i0, u.jr0, u.jr1, P.nslots, 0};
+            for (long long c0 = b; c0 < e || c0 == b; c0 += std::max<long long>(len, 32)) {
+                ptc::Item it{};
+                it.plane = u.plane;
+                it.i0 = i0;
+                it.jr0 = u.jr0;
+                it.jr1 = u.jr1;
+                it.slot = direct ? -1 : P.nslots++;
+                it.w0 = c0;
+                it.w1 = std::min(e, c0 + len);
+                P.items.push_back(it);
+                t.nslots++;
+            }
+            if (!direct) P.tiles.push_back(t);
+        }
+    }
+    // longest items first, so the short exterior-region items fill the tail of the grid
+    for (auto& P : plans)
+        std::stable_sort(P.items.begin(), P.items.end(),
+                     [](const ptc::Item& a, const ptc::Item& b) { return (a.w1 - a.w0) > (b.w1 - b.w0); });
+}
+
+static scw_status launch_planes_tc(scw_waves w, const std::vector<PlaneGeom>& planes, const TcPlan& P) {
+    scw_ctx ctx = w->ctx;
+    const size_t planes_bytes = planes.size() * sizeof(ptc::Plane);
+    const size_t items_off = (planes_bytes + 255) / 256 * 256, items_bytes = P.items.size() * sizeof(ptc::Item);
+    const size_t tiles_off = (items_off + items_bytes + 255) / 256 * 256, tiles_bytes = P.tiles.size() * sizeof(ptc::Tile);
+    const size_t total = tiles_off + tiles_bytes;
+    // the pinned staging buffer may still be read by the previous upload
+    SCW_CUDA_TRY(cudaEventSynchronize(ctx->desc_done));
+    scw_status st = ctx->host_desc.reserve(total);
+    if (st == SCW_OK) st = ctx->desc.reserve(total);
+    if (st == SCW_OK && P.nslots)
+        st = ctx->scratch.reserve((size_t)P.nslots * ptc::kTileJ * 3 * ptc::kTileI * sizeof(double2));
+    if (st != SCW_OK) return st;
+    char* h = (char*)ctx->host_desc.ptr;
+    std::memcpy(h, planes.data(), planes_bytes);
+    std::memcpy(h + items_off, P.items.data(), items_bytes);
+    if (tiles_bytes) std::memcpy(h + tiles_off, P.tiles.data(), tiles_bytes);
+    SCW_CUDA_TRY(cudaMemcpyAsync(ctx->desc.ptr, h, total, cudaMemcpyHostToDevice, ctx->stream));
+    SCW_CUDA_TRY(cudaEventRecord(ctx->desc_done, ctx->stream));
+    char* d = (char*)ctx->desc.ptr;
+    const ptc::Waves waves{w->kre, w->kim, w->zref, w->amp, (long long)w->n};
+    return ptc::launch(ctx, (const ptc::Plane*)d, (const ptc::Item*)(d + items_off), (int)P.items.size(),
+                       (const ptc::Tile*)(d + tiles_off), (int)P.tiles.size(), P.max_rows, waves,
+                       (double2*)ctx->scratch.ptr);
+}
+
 static scw_status launch_planes(scw_waves w, std::vector<PlaneGeom>& planes) {
     scw_ctx ctx = w->ctx;
     SCW_ON_DEVICE(ctx->device);
+    if (tc_suits(w, planes)) {
+        std::vector<TcPlan> plans;
+        tc_plan(w, planes, ctx->sm_count, plans);
+        for (const auto& T : plans) {
+            const scw_status st = launch_planes_tc(w, planes, T);
+            if (st != SCW_OK) return st;
+        }
+        return SCW_OK;
+    }
     Plan P;
     plan_planes(w, planes, ctx->sm_count, P);
     if (P.items.empty()) return SCW_OK;
@@ -445,6 +590,19 @@ scw_status waves_upload(scw_waves w, const std::vector<double>& kre, const std::
     scw_ctx ctx = w->ctx;
     SCW_ON_DEVICE(ctx->device);
     const size_t n = (size_t)w->n;
+    // largest |Re k| and |Im k| per axis and region (NaN stays: no bound holds then)
+    w->kmax.assign(6 * w->begin.size(), 0.0);
+    for (size_t r = 0; r < w->begin.size(); r++)
+        for (int c = 0; c < 3; c++) {
+            double a = 0.0, b = 0.0;
+            for (int64_t i = w->begin[r]; i < w->end[r]; i++) {
+                const double x = std::fabs(kre[c * n + (size_t)i]), y = std::fabs(kim[c * n + (size_t)i]);
+                a = x > a || x != x ? x : a;
+                b = y > b || y != y ? y : b;
+            }
+            w->kmax[6 * r + c] = a;
+            w->kmax[6 * r + 3 + c] = b;
+        }
     if (n == 0) return SCW_OK;
     if (cudaMalloc(&w->kre, 3 * n * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&w->kim, 3 * n * sizeof(double)) != cudaSuccess ||

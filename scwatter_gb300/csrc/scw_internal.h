@@ -138,6 +138,7 @@ struct scw_waves_s {
     int rule = 0;                           // 0: z >= z_l - 0.001, 1: z >= z_l
     std::vector<float> z_layers;
     std::vector<int64_t> begin, end;        // layers + 1 regions
+    std::vector<double> kmax;               // per region: largest |Re k| x, y, z, then |Im k|
     // device SoA tables (n entries each)
     double* kre = nullptr;                  // [3][n] Re k
     double* kim = nullptr;                  // [3][n] Im k
