@@ -27,14 +27,19 @@
 //
 // Measured (38.6 at n = 3200 and 26 TFLOP/s for 20 matrices of n = 648, counted as FP64 operations;
 // the FP64 pipes give 1.05-1.25): 1.66 ms instead of 38 ms for the latter, of which 0.3 ms prepare
-// the operands.  Bound by the tensor core's operand reads and the drains between chunks.
+// the operands.  Measured parts of the latter: without copies 1.64 ms, without drains 1.42; an MMA takes
+// N / 2 clocks but at least 57 (N = 32 .. 96), so a stage's 32 MMAs take 2660 clocks where the tensor core's rate alone
+// would allow 2300; the drains add 400.  The drain runs on 16 warps with the next TMEM load on its way: against 8 warps
+// and loads waited for one by one 67 instead of 79 us for 10 matrices of n = 216, 145 instead of 164 for one of
+// n = 648 (where few tiles leave nothing else to hide it).  Neither a ring of single digits nor CTA pairs with
+// multicast copies of A gained anything (1.87 and 1.76 ms): the copies are not what bounds it.
 //
 // The same kernel with 4 digits (30 bits) and 64 columns per tile serves the corrections of the
 // eigen-solver and of the inverses, which need FP32 accuracy: 10 digit products instead of 36.
 //
 // Two launches prepare the operands (oz_inner_kernel: f_k; oz_split_kernel: e_i, g_j and the digits in
 // the order the MMA reads them, so that a pipeline stage is two contiguous bulk copies), one runs
-// the product: persistent CTAs, one thread copying, one issuing MMAs, 8 warps draining.
+// the product: persistent CTAs, one thread copying, one issuing MMAs, 16 warps draining.
 // Non-finite values: a row of A or a column of B with one gives NaN in its whole row / column.
 #include <algorithm>
 #include <cstdint>
@@ -47,6 +52,9 @@ namespace scw {
 namespace oz {
 
 constexpr int kTM = 128, kTK = 16;           // tile rows, inner indices per stage
+constexpr int kDrainWarps = 16;
+constexpr int kLd = 8;                       // columns per TMEM load
+constexpr int kStageRow = 80;                // bytes of an output staging row: 64 and padding
 template <int S>                             // S base-256 digits per value
 struct Cfg {
     static constexpr int kBits = 8 * S - 2;      // integer bits before the cut
@@ -55,11 +63,10 @@ struct Cfg {
     static constexpr int kBBlk = 2 * S * kTN * kTK * 2;
     static constexpr int kStages = S == 8 ? 2 : 3;
     static constexpr int kStageOff = kStages * (kABlk + kBBlk);      // output staging after the operands
-    static constexpr int kBarOff = kStageOff + 8 * 32 * 144;
+    static constexpr int kBarOff = kStageOff + kDrainWarps * 32 * kStageRow;
     static constexpr size_t kSmem = (size_t)kBarOff + (2 * kStages + 4) * sizeof(uint64_t);
 };
 constexpr int kChunk = 8;                    // stages per drain (K = 128)
-constexpr int kDrainWarps = 8;
 constexpr int kThreads = (kDrainWarps + 2) * 32;
 constexpr int kSpecial = 1 << 20;            // exponent of a row or column with a non-finite value
 constexpr int kNone = -100000;               // exponent of a zero row or column
@@ -322,7 +329,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
     using namespace tc;
     constexpr int kS = S, kTN = Cfg<S>::kTN, kABlk = Cfg<S>::kABlk, kBBlk = Cfg<S>::kBBlk, kStages = Cfg<S>::kStages;
-    constexpr int kCols = kTN / 2;               // columns of a drain warp
+    constexpr int kCols = kTN * 4 / kDrainWarps;  // columns of a drain warp
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* sA = smem;
     unsigned char* sB = smem + kStages * kABlk;
@@ -427,9 +434,9 @@ oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
         }
         __syncwarp();
     } else {
-        // -------- drain: warp w reads TMEM lanes 32 (w % 4) .., half w / 4 of each diagonal's columns --------
-        const int quarter = warp & 3, half = warp >> 2;
-        const uint32_t tb = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * kCols);
+        // -------- drain: warp w reads TMEM lanes 32 (w % 4) .., part w / 4 of each diagonal's columns --------
+        const int quarter = warp & 3, part4 = warp >> 2;
+        const uint32_t tb = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(part4 * kCols);
         constexpr int kW = S == 8 ? 2 : 1;       // 64-bit words per value: diagonals 0 .. 3 (and 4 .. 7)
         int chunk = 0;
         bool ok = true;
@@ -450,31 +457,37 @@ oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
                     break;
                 }
                 tc_fence_after();
+                // kLd columns at a time, the next ones on their way while these are added up
+                uint32_t v[2][kLd];
+                auto fetch = [&](int q) {
+                    const int part = q / (kS * (kCols / kLd)), d = q / (kCols / kLd) % kS, c0 = q % (kCols / kLd) * kLd;
+                    tmem_ld8(tb + (uint32_t)(part * kS * kTN + d * kTN + c0), v[q & 1]);
+                };
+                constexpr int kN = 2 * kS * (kCols / kLd);
+                fetch(0);
 #pragma unroll
-                for (int part = 0; part < 2; part++)
+                for (int q = 0; q < kN; q++) {
+                    tmem_ld_wait8(v[q & 1]);
+                    if (q + 1 < kN) fetch(q + 1);
+                    const int part = q / (kS * (kCols / kLd)), d = q / (kCols / kLd) % kS, c0 = q % (kCols / kLd) * kLd;
 #pragma unroll
-                    for (int d = 0; d < kS; d++) {
-#pragma unroll
-                        for (int c16 = 0; c16 < kCols; c16 += 16) {
-                            uint32_t v[16];
-                            tmem_ld16(tb + (uint32_t)(part * kS * kTN + d * kTN + c16), v);
-                            tmem_ld_wait();
-#pragma unroll
-                            for (int c = 0; c < 16; c++)
-                                w[d >> 2][part][c16 + c] +=
-                                    (long long)__float2int_rn(__uint_as_float(v[c])) * (1 << (8 * (3 - (d & 3))));
-                        }
+                    for (int c = 0; c < kLd; c++) {
+                        long long& acc = w[d >> 2][part][c0 + c];
+                        asm("mad.wide.s32 %0, %1, %2, %0;"
+                            : "+l"(acc)
+                            : "r"(__float2int_rn(__uint_as_float(v[q & 1][c]))), "r"(1 << (8 * (3 - (d & 3)))));
                     }
+                }
                 tc_fence_before();
                 mbar_arrive(acc_empty);
             }
             if (!ok) break;
             // kSeg columns at a time: every lane converts its row's values into the warp's staging rows
-            // (144 bytes apart: no bank conflicts), then the warp reads and writes C in segments of
-            // 128 contiguous bytes per row
-            constexpr int kSeg = 128 / (int)sizeof(TC);
-            unsigned char* stg = smem + Cfg<S>::kStageOff + warp * 32 * 144;
-            const int row0 = m * kTM + quarter * 32, row = row0 + lane, col0 = n * kTN + half * kCols;
+            // (80 bytes apart: no bank conflicts), then the warp reads and writes C in segments of
+            // 64 contiguous bytes per row
+            constexpr int kSeg = 64 / (int)sizeof(TC);
+            unsigned char* stg = smem + Cfg<S>::kStageOff + warp * 32 * kStageRow;
+            const int row0 = m * kTM + quarter * 32, row = row0 + lane, col0 = n * kTN + part4 * kCols;
             const int eA = row < p.M ? p.eA[(long long)(p.a_shared ? 0 : b) * p.gA * 16 + row] : kNone;
             const int* gN = p.gN + (long long)(p.b_shared ? 0 : b) * p.gB * 16 + col0;
             TC* out = (TC*)p.C + p.sC * b + (long long)row0 * p.ldc + col0;
@@ -490,7 +503,7 @@ oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
 #pragma unroll
                 for (int cc = 0; cc < kSeg; cc++) {
                     const int c = c0 + cc;
-                    TC* dst = reinterpret_cast<TC*>(stg + lane * 144) + cc;
+                    TC* dst = reinterpret_cast<TC*>(stg + lane * kStageRow) + cc;
                     const int g = col0 + c < p.N ? gN[c] : kNone;
                     // the last diagonal weighs 2^(8 (S - 1)); units 2^(eA - kBits) 2^(g - kBits)
                     const int e = eA + g + 8 * (kS - 1) - 2 * Cfg<S>::kBits;
@@ -522,7 +535,7 @@ oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
                 for (int q = lane; q < 32 * kSeg; q += 32) {
                     const int r = q / kSeg, cc = q % kSeg;
                     if (row0 + r >= p.M || col0 + c0 + cc >= p.N) continue;
-                    TC v = reinterpret_cast<const TC*>(stg + r * 144)[cc];
+                    TC v = reinterpret_cast<const TC*>(stg + r * kStageRow)[cc];
                     TC* o = out + (long long)r * p.ldc + c0 + cc;
                     if (add1) {
                         const TC x = *o;
