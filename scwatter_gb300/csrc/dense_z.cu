@@ -98,21 +98,57 @@ gemm_kernel(int M, int N, int K, C alpha, const C* __restrict__ A, int lda, long
 //
 // The panel is what is serial: per column a pivot search, a swap and a rank-1 update.  A
 // thread-block cluster of 8 CTAs holds the panel in shared memory, a slice of its rows in each.
-// Per column every CTA sends its best candidate with that row's values (and the owner of row k
-// that row) to all eight, so one cluster barrier per column decides the pivot and brings
+// Per column every CTA sends its best candidate with that row's values and the candidate's inverse (and the
+// owner of row k that row) to all eight, so one cluster barrier per column decides the pivot and brings
 // everything the update needs; the candidate buffers alternate, so the next column's sends
-// cannot reach a CTA that still reads.  On one CTA with the panel in global memory a panel of 32
-// columns and 648 rows took 1.05 ms.  FP64 FMA (1.7 per SM and clock) bound the update, the barrier and
-// the search the rest.
+// cannot reach a CTA that still reads.  FP64 instructions are the scarce thing (75 clocks a warp): the search
+// compares integers, one lane per CTA divides, while the other warps bring the columns after the next one up to
+// date.  A panel of 32 columns: 260 us when every thread compared and divided in FP64, now 94 us with 648
+// rows and 63 with 50, where the barrier, the division and the sends are left; 1.05 ms on one CTA with the panel in
+// global memory.
 // ------------------------------------------------------------------------------------
 constexpr int kNB = 32;
 constexpr int kLuCtas = 8, kLuThreads = 256;
 
 struct LuSlot {
-    double val;
+    double2 inv;                       // of the candidate
+    int hi;                            // |a| of the candidate: the double's upper and lower half; hi < 0: none
+    unsigned lo;
     int row, pad;
     double2 v[kNB];
 };
+
+// 1 / p with one division: conj(p) / |p|^2 with p scaled by a power of two (Smith's form has two divisions in a row)
+__device__ __forceinline__ double2 lu_inverse(double2 p) {
+    const int be = max(__double2hiint(p.x) & 0x7ff00000, __double2hiint(p.y) & 0x7ff00000) >> 20;
+    if (be == 2047) return cdiv(make_double2(1.0, 0.0), p);
+    const double s = __hiloint2double((2046 - min(be, 2045)) << 20, 0);
+    const double x = p.x * s, y = p.y * s, r = s / fma(x, x, y * y);
+    return make_double2(x * r, -y * r);
+}
+
+// Pivot candidates are compared as integers (non-negative doubles order as their bits): an FP64 comparison by
+// all threads costs as much as 75 clocks a warp.  Larger value first, then the smaller row; NaN: none.
+struct LuKey {
+    int hi, row;
+    unsigned lo;
+};
+__device__ __forceinline__ LuKey lu_key(double2 v, int row) {
+    const double a = cabs1(v);
+    const long long bits = __double_as_longlong(a);
+    const int hi = (int)(bits >> 32);
+    const bool nan = (hi & 0x7fffffff) > 0x7ff00000 || ((hi & 0x7fffffff) == 0x7ff00000 && (unsigned)bits != 0u);
+    return LuKey{nan ? -1 : hi, row, (unsigned)bits};
+}
+__device__ __forceinline__ LuKey lu_best(LuKey k) {      // over a warp
+    const int hi = __reduce_max_sync(0xffffffffu, k.hi);
+    const unsigned lo = __reduce_max_sync(0xffffffffu, k.hi == hi ? k.lo : 0u);
+    const int row = __reduce_min_sync(0xffffffffu, k.hi == hi && k.lo == lo ? k.row : 0x7fffffff);
+    return LuKey{hi, row, lo};
+}
+__device__ __forceinline__ double2 lu_sub(double2 x, double2 l, double2 p) {     // x - l p
+    return make_double2(fma(-l.x, p.x, fma(l.y, p.y, x.x)), fma(-l.x, p.y, fma(-l.y, p.x, x.y)));
+}
 
 __global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuThreads)
 lu_panel_kernel(double2* __restrict__ A, int n, int lda, long long sA, int k0, int nb, int rows, int* __restrict__ piv,
@@ -128,8 +164,9 @@ lu_panel_kernel(double2* __restrict__ A, int n, int lda, long long sA, int k0, i
     LuSlot* krow = slot + 2 * kLuCtas;                   // [2]: row k
     double2* P = reinterpret_cast<double2*>(krow + 2);   // [rows][nb + 1]
     const int ld = nb + 1;
-    __shared__ double red_v[kLuThreads / 32];
-    __shared__ int red_i[kLuThreads / 32];
+    constexpr int kWarps = kLuThreads / 32;
+    __shared__ LuKey red[kWarps], mine;
+    __shared__ double2 mine_inv;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g0 = k0 + rank * rows;                     // this CTA's rows g0 .. g0 + nr - 1
     const int nr = max(0, min(rows, n - g0));
@@ -138,49 +175,58 @@ lu_panel_kernel(double2* __restrict__ A, int n, int lda, long long sA, int k0, i
         P[r * ld + c] = A[(long long)(g0 + r) * lda + k0 + c];
     }
     __syncthreads();
-    const int sub = tid & 1;                             // two threads per row
-    double best = -1.0;
-    int bi = 0x7fffffff;
-    for (int r = tid >> 1; r < nr; r += kLuThreads / 2) {
-        const double v = cabs1(P[r * ld]);
-        if (sub == 0 && v > best) {
-            best = v;
-            bi = g0 + r;
-        }
+    const LuKey nothing{-1, 0x7fffffff, 0u};
+    auto better = [](const LuKey& x, const LuKey& y) {
+        return x.hi > y.hi || (x.hi == y.hi && (x.lo > y.lo || (x.lo == y.lo && x.row < y.row)));
+    };
+    LuKey best = nothing;
+    for (int r = tid; r < nr; r += kLuThreads) {
+        const LuKey k = lu_key(P[r * ld], g0 + r);
+        if (k.hi >= 0 && better(k, best)) best = k;
     }
+    best = lu_best(best);
+    if (lane == 0) red[warp] = best;
     cluster.sync();                                      // every CTA runs before the first remote write
+    const double2* prow = nullptr;                       // the pivot row of the column before
     for (int j = 0; j < nb; j++) {
         const int k = k0 + j, par = j & 1;
-        // this CTA's candidate: largest |a|, then smallest row
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ov = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ov > best || (ov == best && oi < bi)) {
-                best = ov;
-                bi = oi;
+        if (warp == 0) {
+            // this CTA's candidate and its inverse
+            best = lu_best(lane < kWarps ? red[lane] : nothing);
+            if (lane == 0) {
+                mine = best;
+                const double2 d = best.hi >= 0 ? P[(best.row - g0) * ld + j] : make_double2(0.0, 0.0);
+                mine_inv = best.hi >= 0 && (best.hi | (int)best.lo) != 0 ? lu_inverse(d) : make_double2(0.0, 0.0);
             }
-        }
-        if (lane == 0) {
-            red_v[warp] = best;
-            red_i[warp] = bi;
+        } else if (j > 0) {
+            // meanwhile the others bring the columns from j + 1 on up to date, every lane with an entry
+            const int w = nb - 1 - j, f = max(0, k - g0), cnt = (nr - f) * w, step = kLuThreads - 32;
+            if (w > 0 && cnt > 0) {
+                int e = tid - 32, r = e / w, c = e - r * w;
+                const int dr = step / w, dc = step - dr * w;
+                for (; e < cnt; e += step) {
+                    double2* row = P + (f + r) * ld;
+                    row[j + 1 + c] = lu_sub(row[j + 1 + c], row[j - 1], prow[j + 1 + c]);
+                    r += dr;
+                    c += dc;
+                    if (c >= w) {
+                        c -= w;
+                        r++;
+                    }
+                }
+            }
         }
         __syncthreads();
-        best = red_v[0];
-        bi = red_i[0];
-#pragma unroll
-        for (int w = 1; w < kLuThreads / 32; w++)
-            if (red_v[w] > best || (red_v[w] == best && red_i[w] < bi)) {
-                best = red_v[w];
-                bi = red_i[w];
-            }
         // warp w sends to CTA w: the candidate with its row, and row k from its owner
         {
             LuSlot* dst = cluster.map_shared_rank(slot, warp) + par * kLuCtas + rank;
-            const bool own = bi >= g0 && bi < g0 + nr;
-            if (own && lane < nb) dst->v[lane] = P[(bi - g0) * ld + lane];
+            const LuKey m = mine;
+            if (m.hi >= 0 && lane < nb) dst->v[lane] = P[(m.row - g0) * ld + lane];
             if (lane == 0) {
-                dst->val = own ? best : -1.0;
-                dst->row = own ? bi : 0x7fffffff;
+                dst->hi = m.hi;
+                dst->lo = m.lo;
+                dst->row = m.row;
+                dst->inv = mine_inv;
             }
             if (k >= g0 && k < g0 + nr) {
                 LuSlot* dk = cluster.map_shared_rank(krow, warp) + par;
@@ -189,19 +235,14 @@ lu_panel_kernel(double2* __restrict__ A, int n, int lda, long long sA, int k0, i
         }
         cluster.sync();
         const LuSlot* cand = slot + par * kLuCtas;
-        double pv = cand[0].val;
-        int p = cand[0].row, pr = 0;
-#pragma unroll
-        for (int w = 1; w < kLuCtas; w++)
-            if (cand[w].val > pv || (cand[w].val == pv && cand[w].row < p)) {
-                pv = cand[w].val;
-                p = cand[w].row;
-                pr = w;
-            }
-        const bool none = pv < 0.0;                      // no comparable value (all NaN): row k stays
-        if (none) p = k;
-        const double2* prow = none ? krow[par].v : cand[pr].v;
-        const bool zero = pv == 0.0;
+        const LuKey got = lane < kLuCtas ? LuKey{cand[lane].hi, cand[lane].row, cand[lane].lo} : nothing;
+        best = lu_best(got);
+        const bool none = best.hi < 0;                   // no comparable value (all NaN): row k stays
+        const unsigned who = __ballot_sync(0xffffffffu, got.hi == best.hi && got.lo == best.lo && got.row == best.row);
+        const int pr = __ffs(who) - 1, p = none ? k : best.row;
+        prow = none ? krow[par].v : cand[pr].v;
+        const bool zero = best.hi == 0 && best.lo == 0u;
+        const double2 inv = none ? make_double2(nan(""), nan("")) : cand[pr].inv;
         if (rank == 0 && tid == 0) {
             piv[k] = p;
             if (zero && info[b] == 0) info[b] = k + 1;
@@ -211,29 +252,21 @@ lu_panel_kernel(double2* __restrict__ A, int n, int lda, long long sA, int k0, i
             if (k >= g0 && k < g0 + nr && lane < nb) P[(k - g0) * ld + lane] = prow[lane];
         }
         __syncthreads();
-        // scale the column below the pivot, update the remaining panel columns, search the next one
-        const double2 inv = zero ? make_double2(0.0, 0.0) : cdiv(make_double2(1.0, 0.0), prow[j]);
-        best = -1.0;
-        bi = 0x7fffffff;
-        for (int rb = max(0, k + 1 - g0); rb < nr; rb += kLuThreads / 2) {
-            const int r = rb + (tid >> 1);
-            const bool live = r < nr;
-            double2* row = P + (live ? r : 0) * ld;
-            const double2 l = live ? cmul(row[j], inv) : make_double2(0.0, 0.0);
-            for (int c = j + 1 + sub; live && c < nb; c += 2) {
-                const double2 v = csub(row[c], cmul(l, prow[c]));
-                row[c] = v;
-                if (c == j + 1) {
-                    const double a = cabs1(v);
-                    if (a > best) {
-                        best = a;
-                        bi = g0 + r;
-                    }
-                }
+        // scale the column below the pivot, the next column, and its candidate
+        best = nothing;
+        for (int r = max(0, k + 1 - g0) + tid; r < nr; r += kLuThreads) {
+            double2* row = P + r * ld;
+            const double2 l = cmul(row[j], inv);
+            row[j] = l;
+            if (j + 1 < nb) {
+                const double2 v = lu_sub(row[j + 1], l, prow[j + 1]);
+                row[j + 1] = v;
+                const LuKey q = lu_key(v, g0 + r);
+                if (q.hi >= 0 && better(q, best)) best = q;
             }
-            __syncwarp();                                // both threads of the row have read row[j]
-            if (live && sub == 0) row[j] = l;
         }
+        best = lu_best(best);
+        if (lane == 0) red[warp] = best;
         __syncthreads();
     }
     for (int e = tid; e < nr * nb; e += kLuThreads) {
@@ -246,15 +279,17 @@ lu_panel_kernel(double2* __restrict__ A, int n, int lda, long long sA, int k0, i
 // it, 32 columns per CTA.  The interchanges touch at most 64 rows: warp 0 follows them to the rows'
 // sources (lane i: the source of row k0 + i, and a row below the panel that was exchanged with
 // one of the panel), so that all rows are read at once and then written.
+template <int C>
 __global__ void __launch_bounds__(256)
 lu_apply_kernel(double2* __restrict__ A, int ncols, int lda, long long sA, int k0, int nb, const int* __restrict__ piv,
                 long long sP, const int* __restrict__ skip) {
     if (skipped(skip, blockIdx.y)) return;
     A += sA * blockIdx.y;
     piv += sP * blockIdx.y;
-    __shared__ double2 X[kNB][33], L[kNB][33];
+    __shared__ double2 X[kNB][C + 1], L[kNB][33];
     __shared__ int s_top[kNB], s_row[kNB], s_src[kNB];
-    const int tid = threadIdx.x, lane = tid & 31, c = lane, j = blockIdx.x * 32 + c;
+    constexpr int G = 256 / C, Q = kNB / G;             // row groups, rows per thread
+    const int tid = threadIdx.x, lane = tid & 31, c = tid % C, j = blockIdx.x * C + c;
     if (tid < 32) {
         int top = k0 + lane, orow = -1, osrc = -1;
         const int mine = lane < nb ? piv[k0 + lane] : 0;
@@ -280,35 +315,38 @@ lu_apply_kernel(double2* __restrict__ A, int ncols, int lda, long long sA, int k
     }
     const bool live = j < ncols && !(j >= k0 && j < k0 + nb), right = live && j >= k0 + nb;
     __syncthreads();
-    double2 o[kNB / 8];
+    for (int e = tid; e < nb * nb; e += 256) {
+        const int r = e / nb, q = e - r * nb;
+        L[r][q] = A[(long long)(k0 + r) * lda + k0 + q];
+    }
+    double2 o[Q];
 #pragma unroll
-    for (int q = 0; q < kNB / 8; q++) {
-        const int r = (tid >> 5) + 8 * q;
+    for (int q = 0; q < Q; q++) {
+        const int r = tid / C + G * q;
         o[q] = make_double2(0.0, 0.0);
         if (live && r < nb) {
             X[r][c] = A[(long long)s_top[r] * lda + j];
             if (s_row[r] >= 0) o[q] = A[(long long)s_src[r] * lda + j];
         }
-        if (r < nb && c < nb) L[r][c] = A[(long long)(k0 + r) * lda + k0 + c];
     }
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < kNB / 8; q++) {
-        const int r = (tid >> 5) + 8 * q;
+    for (int q = 0; q < Q; q++) {
+        const int r = tid / C + G * q;
         if (live && r < nb && s_row[r] >= 0) A[(long long)s_row[r] * lda + j] = o[q];
     }
-    const int steps = blockIdx.x * 32 + 31 >= k0 + nb ? nb - 1 : 0;      // left of the panel: interchanges only
+    const int steps = blockIdx.x * C + C - 1 >= k0 + nb ? nb - 1 : 0;      // left of the panel: interchanges only
     for (int m = 0; m < steps; m++) {
 #pragma unroll
-        for (int q = 0; q < kNB / 8; q++) {
-            const int r = (tid >> 5) + 8 * q;
-            if (right && r > m && r < nb) X[r][c] = csub(X[r][c], cmul(L[r][m], X[m][c]));
+        for (int q = 0; q < Q; q++) {
+            const int r = tid / C + G * q;
+            if (right && r > m && r < nb) X[r][c] = lu_sub(X[r][c], L[r][m], X[m][c]);
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int q = 0; q < kNB / 8; q++) {
-        const int r = (tid >> 5) + 8 * q;
+    for (int q = 0; q < Q; q++) {
+        const int r = tid / C + G * q;
         if (live && r < nb) A[(long long)(k0 + r) * lda + j] = X[r][c];
     }
 }
@@ -332,41 +370,61 @@ laswp_kernel(const int* __restrict__ piv, long long sP, double2* __restrict__ B,
     }
 }
 
+// q = x (1 / d) brought to the accuracy of a division; as it is where the correction is not finite (d
+// infinite), and a division where 1 / d is not (d zero or below the range of its inverse)
+__device__ __forceinline__ double2 z_div_fix(double2 x, double2 q, double2 d, double2 id) {
+    if (!isfinite(id.x) || !isfinite(id.y)) return cdiv(x, d);
+    const double2 r = lu_sub(x, q, d);
+    const double2 f = make_double2(fma(r.x, id.x, fma(-r.y, id.y, q.x)), fma(r.x, id.y, fma(r.y, id.x, q.y)));
+    return isfinite(f.x) && isfinite(f.y) ? f : q;
+}
+
 // Triangular solve restricted to the diagonal block rows [k0, k0 + nb) of the LU factors, 32
 // right-hand-side columns per CTA in shared memory: unit lower L (upper == 0) or U (upper == 1).
 // Rows outside the block were already folded in by the GEMM updates of the blocked solve.
+template <int C>
 __global__ void __launch_bounds__(256)
 trsm_block_kernel(const double2* __restrict__ LU, int lda, long long sA, int k0, int nb, double2* __restrict__ B, int ldb,
                   long long sB, int nrhs, int upper, const int* __restrict__ skip) {
     if (skipped(skip, blockIdx.y)) return;
     LU += sA * blockIdx.y;
     B += sB * blockIdx.y;
-    __shared__ double2 X[kNB][33], L[kNB][33];
-    const int tid = threadIdx.x, c = tid & 31, w = tid >> 5, j = blockIdx.x * 32 + c;
+    constexpr int G = 256 / C, Q = kNB / G;             // row groups, rows per thread
+    __shared__ double2 X[kNB][C + 1], L[kNB][33], D[kNB];
+    const int tid = threadIdx.x, c = tid % C, w = tid / C, j = blockIdx.x * C + c;
     const bool live = j < nrhs;
 #pragma unroll
-    for (int q = 0; q < kNB / 8; q++) {
-        const int r = w + 8 * q;
+    for (int q = 0; q < Q; q++) {
+        const int r = w + G * q;
         if (r < nb && live) X[r][c] = B[(long long)(k0 + r) * ldb + j];
-        if (r < nb && c < nb) L[r][c] = LU[(long long)(k0 + r) * lda + k0 + c];
+    }
+    for (int e = tid; e < nb * nb; e += 256) {
+        const int r = e / nb, q = e - r * nb;
+        const double2 v = LU[(long long)(k0 + r) * lda + k0 + q];
+        L[r][q] = v;
+        if (upper && r == q) D[r] = lu_inverse(v);
     }
     __syncthreads();
     for (int s = 0; s < nb; s++) {
         const int m = upper ? nb - 1 - s : s;
         if (upper) {
-            if (w == 0 && live) X[m][c] = cdiv(X[m][c], L[m][m]);
+            // x / d as x (1 / d) and one correction by the residual x - (x / d) d
+            if (w == 0 && live) {
+                const double2 x = X[m][c], q = cmul(x, D[m]);
+                X[m][c] = z_div_fix(x, q, L[m][m], D[m]);
+            }
             __syncthreads();
         }
 #pragma unroll
-        for (int q = 0; q < kNB / 8; q++) {
-            const int r = w + 8 * q;
-            if (live && r < nb && (upper ? r < m : r > m)) X[r][c] = csub(X[r][c], cmul(L[r][m], X[m][c]));
+        for (int q = 0; q < Q; q++) {
+            const int r = w + G * q;
+            if (live && r < nb && (upper ? r < m : r > m)) X[r][c] = lu_sub(X[r][c], L[r][m], X[m][c]);
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int q = 0; q < kNB / 8; q++) {
-        const int r = w + 8 * q;
+    for (int q = 0; q < Q; q++) {
+        const int r = w + G * q;
         if (r < nb && live) B[(long long)(k0 + r) * ldb + j] = X[r][c];
     }
 }
@@ -1088,6 +1146,18 @@ scw_status gemm(cudaStream_t st, int M, int N, int K, C alpha, const C* A, int l
     return SCW_OK;
 }
 
+// Columns per CTA of the triangular kernels: 32 reuse the block of L or U for more columns, but their FP64
+// work (16 000 operations per column of 32 rows) then takes 20 us on one SM; 8 where 32 would leave SMs idle.
+static bool few_columns(int cols, int batch) { return (long long)((cols + 31) / 32) * batch < 152; }
+
+static void trsm_block(cudaStream_t st, const double2* LU, int lda, long long sA, int k0, int nb, double2* B, int ldb, long long sB,
+                       int nrhs, int upper, int batch, const int* skip) {
+    if (few_columns(nrhs, batch))
+        z::trsm_block_kernel<8><<<dim3((nrhs + 7) / 8, batch), 256, 0, st>>>(LU, lda, sA, k0, nb, B, ldb, sB, nrhs, upper, skip);
+    else
+        z::trsm_block_kernel<32><<<dim3((nrhs + 31) / 32, batch), 256, 0, st>>>(LU, lda, sA, k0, nb, B, ldb, sB, nrhs, upper, skip);
+}
+
 scw_status zgetrf(cudaStream_t st, double2* A, int n, int ncols, int lda, long long sA, int* piv, long long sP, int* info,
                   int batch, const GemmWs& ws, const int* skip) {
     if (n <= 0 || batch <= 0) return SCW_OK;
@@ -1107,7 +1177,10 @@ scw_status zgetrf(cudaStream_t st, double2* A, int n, int ncols, int lda, long l
                                                                                       sP, info, skip);
         SCW_CUDA_TRY(cudaGetLastError());
         if (ncols > nb) {
-            z::lu_apply_kernel<<<dim3((ncols + 31) / 32, batch), 256, 0, st>>>(A, ncols, lda, sA, k0, nb, piv, sP, skip);
+            if (few_columns(ncols, batch))
+                z::lu_apply_kernel<8><<<dim3((ncols + 7) / 8, batch), 256, 0, st>>>(A, ncols, lda, sA, k0, nb, piv, sP, skip);
+            else
+                z::lu_apply_kernel<32><<<dim3((ncols + 31) / 32, batch), 256, 0, st>>>(A, ncols, lda, sA, k0, nb, piv, sP, skip);
             SCW_CUDA_TRY(cudaGetLastError());
         }
         const int rem = n - k0 - nb;
@@ -1128,10 +1201,9 @@ scw_status ztrsm_upper(cudaStream_t st, const double2* LU, int n, int lda, long 
     if (n <= 0 || nrhs <= 0 || batch <= 0) return SCW_OK;
     constexpr int kTB = z::kNB;
     const double2 one = {1, 0}, minus = {-1, 0};
-    const dim3 g((nrhs + 31) / 32, batch);
     for (int k0 = ((n - 1) / kTB) * kTB; k0 >= 0; k0 -= kTB) {
         const int nb = std::min(kTB, n - k0);
-        z::trsm_block_kernel<<<g, 256, 0, st>>>(LU, lda, sA, k0, nb, B, ldb, sB, nrhs, 1, skip);
+        trsm_block(st, LU, lda, sA, k0, nb, B, ldb, sB, nrhs, 1, batch, skip);
         SCW_CUDA_TRY(cudaGetLastError());
         if (k0 > 0) {
             scw_status s = zgemm(st, k0, nrhs, nb, minus, LU + k0, lda, sA, B + (long long)k0 * ldb, ldb, sB, one, B, ldb,
@@ -1151,7 +1223,7 @@ scw_status zgetrs(cudaStream_t st, const double2* LU, int n, long long sA, const
     SCW_CUDA_TRY(cudaGetLastError());
     for (int k0 = 0; k0 < n; k0 += kTB) {
         const int nb = std::min(kTB, n - k0);
-        z::trsm_block_kernel<<<dim3((nrhs + 31) / 32, batch), 256, 0, st>>>(LU, n, sA, k0, nb, B, nrhs, sB, nrhs, 0, skip);
+        trsm_block(st, LU, n, sA, k0, nb, B, nrhs, sB, nrhs, 0, batch, skip);
         SCW_CUDA_TRY(cudaGetLastError());
         const int rem = n - k0 - nb;
         if (rem > 0) {
