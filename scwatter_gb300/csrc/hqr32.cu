@@ -14,10 +14,11 @@
 //     right, rows above, Schur vectors), a thread per vector of 64 values staged in shared memory, four
 //     bulges per pass over the vector.  The leader applies them to the columns that the next
 //     window needs and goes on chasing; the other CTAs of the cluster do the rest meanwhile.
-// What bounds it: at n = 648 half of the time is the serial QR of the deflation windows (40 of them, 0.23 ms
-// each) and a third the leader's chase (280 windows of 512 rotations, 20 us each).  Measured: 18.7 ms for
-// 20 matrices of n = 648 on clusters of 7 CTAs, where a chase of one bulge at a time (800 clocks per
-// rotation, no deflation windows) took 316 ms; 4.2 instead of 23.6 ms for 10 matrices of n = 216.
+// What bounds it: at n = 648 half of the time is the serial QR of the deflation windows (44 of them, 0.18 ms
+// each) and a third the leader's chase (290 windows of 512 rotations, 18 us each).  Measured: 17.5 ms for
+// 20 matrices of n = 648 on clusters of 6 CTAs, 3.67 ms for 10 of n = 216, 0.50 ms for 4 of n = 50; with the deflation
+// window's column operations after each sweep 19.7, 4.40 and 0.64; a chase of one bulge at a time (800 clocks per
+// rotation, no deflation windows) took 316 and 23.6 ms.
 // H and Z are read through L2 (ld.global.cg): other CTAs of the cluster write them between barriers.
 #include <algorithm>
 #include <atomic>
@@ -52,9 +53,8 @@ struct QrSmem {
     QrRot rot[2][kStep][kM / 4];
     float2 vec[kVec * kLd];                   // staged vectors of the updates
     float2 shift[kNW], refl[kNW];
-    float lc[2][kNW];                         // rotations of the deflation window's sweeps (two in flight)
-    float2 ls[2][kNW];
-    int ll[2], ln[2];
+    float4 lr[2][kNW];                        // rotations c, s of the deflation window's sweeps (two in flight)
+    int ll[2], ln[2], wl, wh, wbuf;           // sweeps for warp 1, the current one for warp 2
     int cmd[8];                               // op, l, hi, shifts | op, kw, nw
     int red[kM];
     float2 spike;
@@ -96,6 +96,27 @@ __device__ __forceinline__ void givens32(float2 f, float2 g, float& c, float2& s
     r = make_float2(fs.x * d, fs.y * d);
 }
 
+// The same where no branch is needed but for values near the ends of the range.
+__device__ __forceinline__ float rsqrt_fast(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ void givens32_fast(float2 f, float2 g, float& c, float2& s, float2& r) {
+    const float gf = cabs2(g), ff = cabs2(f);
+    if (fminf(gf, ff) < 1e-36f) {
+        givens32(f, g, c, s, r);
+        return;
+    }
+    const float iaf = rsqrt_fast(ff), id = rsqrt_fast(ff + gf);
+    const float2 fs = make_float2(f.x * iaf, f.y * iaf);
+    const float2 t = cmulc(g, fs);
+    c = ff * iaf * id;
+    s = make_float2(t.x * id, t.y * id);
+    const float d = (ff + gf) * id;
+    r = make_float2(fs.x * d, fs.y * d);
+}
+
 // Wilkinson's shift of the trailing 2 x 2 block; exceptional ones every 10 iterations (zlahqr's rule).
 // Approximate square root and division: a shift need not be exact.
 __device__ __forceinline__ float2 shift32(const float2* T, int ld, int l, int ihi, int its) {
@@ -123,10 +144,20 @@ __device__ __forceinline__ float2 shift32(const float2* T, int ld, int l, int ih
     return make_float2(d.x - __fdividef(x.x, dd), d.y - __fdividef(x.y, dd));
 }
 
+// hqr_deflates of the window's entry (k, k - 1), all entries loaded at once and without exact divisions
+__device__ __forceinline__ bool window_deflates(const float2* T, int k, int ihi) {
+    const float2 a = T[k * kLdn + k - 1], d = T[k * kLdn + k], p = T[(k - 1) * kLdn + k - 1], u = T[(k - 1) * kLdn + k];
+    const float ulp = CT<float2>::ulp, small = CT<float2>::safmin * ((float)kLdn / ulp);
+    const float a1 = cabs1(a), u1 = cabs1(u), d1 = cabs1(d), dd = cabs1(csub(p, d)), tst = cabs1(p) + d1;
+    if (tst == 0.f) return hqr_deflates<float2, false>(T, kLdn, k, ihi);
+    const float ab = fmaxf(a1, u1), ba = fminf(a1, u1), aa = fmaxf(d1, dd), bb = fminf(d1, dd), is = __fdividef(1.f, aa + ab);
+    const bool far = ba * (ab * is) <= fmaxf(small, ulp * (bb * (aa * is))) || ba * ab <= (ulp * d1) * (ulp * d1);
+    return a1 <= small || (fabsf(a.x) <= ulp * tst && far);
+}
+
 // The rotations of a sweep over columns l .. l + cnt - 1, in order, on row `row` of X from column ks on: a
 // lane per row, the running value in a register, the values four columns ahead already loaded.
-__device__ __forceinline__ void sweep_columns(float2* X, int row, bool live, int ks, int l, int cnt, const float* c,
-                                              const float2* s) {
+__device__ __forceinline__ void sweep_columns(float2* X, int row, bool live, int ks, int l, int cnt, const float4* rot) {
     float2* p = X + row * kLdn;
     const int k1 = l + cnt;
     float2 x = live && ks < k1 ? p[ks] : make_float2(0.f, 0.f);
@@ -137,8 +168,9 @@ __device__ __forceinline__ void sweep_columns(float2* X, int row, bool live, int
 #pragma unroll
         for (int i = 0; i < 4; i++) {
             if (k + i < k1) {
-                const float cc = c[k + i - l];
-                const float2 ss = conjf2(s[k + i - l]);
+                const float4 g = rot[k + i - l];
+                const float cc = g.x;
+                const float2 ss = make_float2(g.y, -g.z);
                 if (live && k + i >= ks) {
                     rot32_rows(cc, ss, x, y[i]);
                     p[k + i] = x;
@@ -169,19 +201,64 @@ __device__ __forceinline__ void reflector32(float2& x, int lane, int cnt, float2
 }
 
 __device__ __forceinline__ void pair_sync() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
+// warp 0 announces, warp 2 waits; the barriers 2 .. 12 are used once per sweep each
+constexpr int kColGroup = 3, kColDone = 14;
+static_assert(2 + (kNW - 2) / kColGroup < kColDone, "named barriers");
+__device__ __forceinline__ void bar_arrive(int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void bar_wait(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
 
-// Schur form of the nw x nw Hessenberg window T with vectors V (warps 0 and 1), then deflation against the
+// Schur form of the nw x nw Hessenberg window T with vectors V (warps 0 .. 2), then deflation against the
 // spike s, the Hessenberg form of what is left (warp 0).  Sets S.ns (undeflated, at the top), S.shift (their
 // eigenvalues) and S.fail.
 //
 // A sweep is one chain of rotations, so its latency per rotation is what counts.  Lane j carries column
-// j of the row that the chase is at: row operations need no shared-memory round trip, and the next
-// rotation's two entries come from three shuffles.  The column operations on the rows above follow
-// after the sweep, a lane per row; warp 1 applies them to V meanwhile.  (With every operation going
-// through shared memory a rotation took 550 clocks.)
+// j of the row that the chase is at: row operations need no shared-memory round trip.  What the next
+// rotation is made of (columns k, k + 1 of the rows k .. k + 2) every lane computes for itself, from the
+// diagonal and subdiagonal entries, loaded ahead, and one value of row k, whose shuffle overlaps the
+// rotation's square roots.  Warp 2 applies the column operations to the rows above, a lane per row, three
+// rotations behind, and warp 1 those of the sweep before to V.  A rotation takes 305 clocks (106 the
+// rotation itself, 60 what the next is made of, 120 the rows and their stores); with those columns from shuffles in the
+// chain and the column operations after the sweep 317 + 143, through shared memory 550.
 __device__ void deflation_window(QrSmem& S, int nw) {
     const int lane = threadIdx.x & 31;
     float2 *T = S.T, *V = S.V;
+    if (threadIdx.x >= 64) {
+        while (true) {
+            bar_wait(2);
+            const int l = S.wl, hi = S.wh;
+            if (hi < 0) return;
+            const float4* rot = S.lr[S.wbuf];
+            float2 x = make_float2(0.f, 0.f);
+            float2* row = T + lane * kLdn;
+            for (int q = 0, k = l;; q++) {
+                if (q > 0) bar_wait(2 + q);
+                // rows up to k + i are complete, each takes part from its own column on
+                float2 y[kColGroup], d[kColGroup];
+                float4 g[kColGroup];
+#pragma unroll
+                for (int i = 0; i < kColGroup; i++) {
+                    const int kk = min(k + i, hi - 1);
+                    y[i] = lane <= kk ? row[kk + 1] : make_float2(0.f, 0.f);
+                    d[i] = lane <= kk ? row[kk] : make_float2(0.f, 0.f);
+                    g[i] = rot[kk - l];
+                }
+#pragma unroll
+                for (int i = 0; i < kColGroup; i++) {
+                    if (k + i < hi && lane <= k + i) {
+                        if (lane == k + i || k + i == l) x = d[i];
+                        rot32_rows(g[i].x, make_float2(g[i].y, -g[i].z), x, y[i]);
+                        row[k + i] = x;
+                        x = y[i];
+                    }
+                }
+                k += kColGroup;
+                if (k >= hi) break;
+            }
+            if (lane < hi) row[hi] = x;
+            __syncwarp();
+            bar_wait(kColDone);
+        }
+    }
     if (threadIdx.x >= 32) {
         for (int i = 0; i < nw; i++) V[i * kLdn + lane] = make_float2(i == lane ? 1.f : 0.f, 0.f);
         __syncwarp();
@@ -189,7 +266,7 @@ __device__ void deflation_window(QrSmem& S, int nw) {
             pair_sync();
             const int cnt = S.ln[q], l = S.ll[q];
             if (cnt < 0) return;
-            sweep_columns(V, lane, lane < nw, l, l, cnt, S.lc[q], S.ls[q]);
+            sweep_columns(V, lane, lane < nw, l, l, cnt, S.lr[q]);
             __syncwarp();
         }
     }
@@ -197,7 +274,7 @@ __device__ void deflation_window(QrSmem& S, int nw) {
     int ihi = nw - 1, its = 0, total = 0, buf = 0;
     bool fail = false;
     while (ihi >= 0) {
-        const bool d = lane >= 1 && lane <= ihi && hqr_deflates<float2, false>(T, kLdn, lane, ihi);
+        const bool d = lane >= 1 && lane <= ihi && window_deflates(T, lane, ihi);
         const unsigned mask = __ballot_sync(0xffffffffu, d);
         const int l = mask ? 31 - __clz(mask) : 0;
         if (l > 0 && lane == 0) T[l * kLdn + l - 1] = make_float2(0.f, 0.f);
@@ -215,52 +292,73 @@ __device__ void deflation_window(QrSmem& S, int nw) {
         total++;
         const float2 shift = shift32(T, kLdn, l, ihi, its);
         const float2 zero = make_float2(0.f, 0.f);
-        // R: row k of column `lane` with the rotations so far, N: row k + 1
-        float2 R = lane < nw ? T[l * kLdn + lane] : zero, N = lane < nw ? T[(l + 1) * kLdn + lane] : zero;
-        float2 f = make_float2(__shfl_sync(0xffffffffu, R.x, l) - shift.x, __shfl_sync(0xffffffffu, R.y, l) - shift.y);
-        float2 g = make_float2(__shfl_sync(0xffffffffu, N.x, l), __shfl_sync(0xffffffffu, N.y, l));
+        if (lane == 0) {
+            S.wl = l;
+            S.wh = ihi;
+            S.wbuf = buf;
+        }
+        // R: row k of column `lane` with the rotations so far, N, M: rows k + 1 and k + 2; (k, k), (k + 1, k) and
+        // (k + 1, k + 1), (k + 2, k + 1) in every lane, the latter two without rotations.  What is read past row
+        // ihi or column nw stays in T's storage and reaches nothing that is kept.
+        const bool live = lane < nw;
+        float2 R = T[l * kLdn + lane], N = T[(l + 1) * kLdn + lane], M = T[(l + 2) * kLdn + lane];
+        float2 Rk = T[l * kLdn + l], Nk = T[(l + 1) * kLdn + l];
+        float2 n1 = T[(l + 1) * kLdn + l + 1], m1 = T[(l + 2) * kLdn + l + 1];
+        float2 f = csub(Rk, shift), g = Nk;
         __syncwarp();
-        for (int k = l; k < ihi; k++) {
-            float2 M = zero;
-            if (k + 2 <= ihi && lane < nw) M = T[(k + 2) * kLdn + lane];
+        // rotation k on R, N; R then takes row k + 3.  true: the sweep's last
+        auto step = [&](int k, float2& R, float2& N, float2& M) {
+            const float2* next = T + (k + 2) * kLdn + k + 2;
+            const float2 r1 = make_float2(__shfl_sync(0xffffffffu, R.x, k + 1), __shfl_sync(0xffffffffu, R.y, k + 1));
+            const float2 n2 = next[0], m2 = next[kLdn];
             float2 s, r;
             float c;
-            givens32(f, g, c, s, r);
-            if (lane == 0) {
-                S.lc[buf][k - l] = c;
-                S.ls[buf][k - l] = s;
-            }
-            rot32_rows(c, s, R, N);                 // R: row k done, N: row k + 1
-            if (lane >= k && lane < nw) T[k * kLdn + lane] = R;
-            if (k > l && lane == k - 1) T[k * kLdn + lane] = r;
-            // columns k, k + 1 of row k + 1, and of row k + 2 (zero, M)
-            float2 a = make_float2(__shfl_sync(0xffffffffu, N.x, k), __shfl_sync(0xffffffffu, N.y, k));
-            float2 b = make_float2(__shfl_sync(0xffffffffu, N.x, k + 1), __shfl_sync(0xffffffffu, N.y, k + 1));
-            const float2 m = make_float2(__shfl_sync(0xffffffffu, M.x, k + 1), __shfl_sync(0xffffffffu, M.y, k + 1));
+            givens32_fast(f, g, c, s, r);
+            // columns k, k + 1 of row k + 1 with this rotation from both sides, and of row k + 2 (zero, m1)
+            float2 a = make_float2(c * Nk.x - (s.x * Rk.x + s.y * Rk.y), c * Nk.y - (s.x * Rk.y - s.y * Rk.x));
+            float2 b = make_float2(c * n1.x - (s.x * r1.x + s.y * r1.y), c * n1.y - (s.x * r1.y - s.y * r1.x));
             rot32_rows(c, conjf2(s), a, b);
             f = a;
-            g = cmulc(s, m);
+            g = cmulc(s, m1);
+            Rk = b;
+            Nk = make_float2(c * m1.x, c * m1.y);
+            n1 = n2;
+            m1 = m2;
+            rot32_rows(c, s, R, N);                 // R: row k done, N: row k + 1
+            if (live && lane >= max(k - 1, l)) T[k * kLdn + lane] = lane == k - 1 ? r : R;
+            if (lane == 0) S.lr[buf][k - l] = make_float4(c, s.x, s.y, 0.f);
+            R = T[(k + 3) * kLdn + lane];
             if (lane == k + 1) {
                 N = b;
                 M = make_float2(c * M.x, c * M.y);
             }
-            R = N;
-            N = M;
+            if (k + 1 < ihi) return false;
+            if (lane >= ihi && live) T[ihi * kLdn + lane] = N;
+            if (lane == ihi - 1) T[ihi * kLdn + lane] = f;
+            return true;
+        };
+        static_assert(kColGroup == 3, "a group is one turn of the three rows");
+        for (int k = l, group = 2;; k += 3, group++) {
+            const bool end = step(k, R, N, M) || step(k + 1, N, M, R) || step(k + 2, M, R, N);
+            __syncwarp();
+            bar_arrive(group);
+            if (end) break;
         }
-        if (lane >= ihi && lane < nw) T[ihi * kLdn + lane] = R;
-        if (lane == ihi - 1) T[ihi * kLdn + lane] = f;
         if (lane == 0) {
             S.ll[buf] = l;
             S.ln[buf] = ihi - l;
         }
         __syncwarp();
         pair_sync();
-        sweep_columns(T, lane, lane <= ihi, max(l, lane), l, ihi - l, S.lc[buf], S.ls[buf]);
-        __syncwarp();
+        bar_wait(kColDone);
         buf ^= 1;
     }
-    if (lane == 0) S.ln[buf] = -1;
+    if (lane == 0) {
+        S.ln[buf] = -1;
+        S.wh = -1;
+    }
     __syncwarp();
+    bar_arrive(2);
     pair_sync();                                    // V is complete
     // From the bottom up: an eigenvalue with a negligible spike entry is moved down past those that stay
     // and deflated there.
@@ -394,7 +492,7 @@ __device__ void chase32(QrSmem& S, float2* __restrict__ H, int n, int l, int ihi
                 f = TT(u, u - 1);
                 g = TT(u + 1, u - 1);
             }
-            givens32(f, g, c, s, r);
+            givens32_fast(f, g, c, s, r);
             __syncwarp();
             if (lane == 0 && k > l) {
                 TT(u, u - 1) = r;
@@ -558,6 +656,9 @@ hqr32_kernel(float2* __restrict__ H, float2* __restrict__ Z, int n, long long sA
     int ihi = n - 1, idle = 0, rounds = 0;              // rank 0's state
     int sweep_l = 0, sweep_hi = -1, sweep_ms = 0;       // rank 0: a sweep is due
     const int limit = 30 * max(10, n);
+    // larger windows deflate more at a time, but their QR grows with the square (measured with 16, 20, 24, 28, 32: n =
+    // 216 4.08, 3.79, 3.72, 3.95, 3.99 ms; n = 648 21.3, 19.4, 18.4, 17.7, 17.8 ms)
+    const int window = n < 400 ? 24 : kNW;
     while (true) {
         if (rank == 0) {
             int op = kOpEnd, a1 = 0, a2 = 0, a3 = 0;
@@ -588,7 +689,7 @@ hqr32_kernel(float2* __restrict__ H, float2* __restrict__ Z, int n, long long sA
                         ihi = -1;
                         break;
                     }
-                    const int size = ihi - l + 1, nw = min(kNW, size), kw = ihi - nw + 1;
+                    const int size = ihi - l + 1, nw = size <= kNW ? size : window, kw = ihi - nw + 1;
                     for (int e = tid; e < nw * nw; e += kQrThreads) {
                         const int i = e / nw, j = e - i * nw;
                         S.T[i * kLdn + j] = j + 1 < i ? make_float2(0.f, 0.f) : __ldcg(H + (long long)(kw + i) * n + kw + j);
@@ -598,7 +699,7 @@ hqr32_kernel(float2* __restrict__ H, float2* __restrict__ Z, int n, long long sA
                         if (l > 0) H[(long long)l * n + l - 1] = make_float2(0.f, 0.f);
                     }
                     __syncthreads();
-                    if (warp < 2) deflation_window(S, nw);
+                    if (warp < 3) deflation_window(S, nw);
                     __syncthreads();
                     if (S.fail) {
                         if (tid == 0) status[mat] = 1;
@@ -610,8 +711,8 @@ hqr32_kernel(float2* __restrict__ H, float2* __restrict__ Z, int n, long long sA
                     if (tid < nw && tid >= ns) eig[kw + tid] = S.T[tid * kLdn + tid];
                     ihi -= nd;
                     idle = nd ? 0 : idle + 1;
-                    // a sweep unless more than half of the window deflated (measured at 14, 34, 50 and 70 %:
-                    // 23.5, 20.6, 18.7, 19.7 ms for 20 matrices of n = 648)
+                    // a sweep unless more than half of the window deflated (measured at 25, 50 and 75 %: 20.0,
+                    // 17.5, 18.1 ms for 20 matrices of n = 648, 4.03, 3.67, 3.73 for 10 of n = 216)
                     if (ihi - l + 1 > kNW && 2 * nd <= nw) {
                         sweep_l = l;
                         sweep_hi = ihi;
