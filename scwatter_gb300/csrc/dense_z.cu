@@ -1360,7 +1360,7 @@ scw_status zgeev(cudaStream_t st, double2* A, double2* W, double2* V, int n, int
 
 scw_status schur32(cudaStream_t st, float2* A, float2* Q, float2* W, int n, int batch, float2* work, int* status,
                    const GemmWs& ws, int share) {
-    scw_status s = hess32(st, A, Q, n, batch, work, ws, share);
+    scw_status s = hess32(st, A, Q, n, batch, work, share);
     if (s == SCW_OK) s = hqr32(st, A, Q, n, W, status, batch, g_qr_cluster.load(), share);
     return s;
 }

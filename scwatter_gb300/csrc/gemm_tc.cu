@@ -183,7 +183,7 @@ struct SplitArgs {
     const void *A, *B;
     long long rsA, ksA, rsB, ksB;      // element (row of A or column of B, inner index k) at row rs + k ks
     long long sA, sB;
-    int conjA, conjB;                  // 1: the conjugate
+    int conjB;                         // 1: the conjugate
     int M, N, K, nk, mt, nt;           // nk stages, mt x nt tiles
     int gA, gB, nA;                    // 16-row groups of A, 16-column groups of B per matrix; A blocks in all
     const int* f;
@@ -244,7 +244,7 @@ __device__ __forceinline__ void split_group(const SplitArgs& p, int b, int g, in
                 const int s = (kA ? f[k] : -f[k]) - e + C::kBits;
                 qr[j] = fixed_point(v.x, s);
                 qi[j] = fixed_point(v.y, s);
-                if (kA ? p.conjA : p.conjB) qi[j] = -qi[j];
+                if (!kA && p.conjB) qi[j] = -qi[j];
             }
         }
         unsigned char* o = dst + (long long)st * blkb;
@@ -604,7 +604,7 @@ struct Shape {
 
 // One product with S digits; element types double2 or float2 by operand.
 template <int S, typename TA, typename TB, typename TC>
-static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const TA* A, int lda, long long sA, int opA,
+static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const TA* A, int lda, long long sA,
                       const TB* B, int ldb, long long sB, int opB, double2 beta, double diag, TC* C, int ldc, long long sC, int batch,
                       const GemmWs& ws, const int* skip) {
     if (M <= 0 || N <= 0 || batch <= 0) return SCW_OK;
@@ -616,7 +616,7 @@ static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const
     const Shape sh(S, M, N, K);
     const bool a1 = sA == 0 && !skip, b1 = sB == 0 && !skip;     // one operand for the whole batch
     // element (i, k) of op(A) at i rsA + k ksA, (k, j) of op(B) at k ksB + j rsB
-    const long long rsA = opA == kOpN ? lda : 1, ksA = opA == kOpN ? 1 : lda;
+    const long long rsA = lda, ksA = 1;
     const long long ksB = opB == kOpN ? ldb : 1, rsB = opB == kOpN ? 1 : ldb;
     // as many matrices at a time as the workspace holds
     int step = batch;
@@ -646,7 +646,7 @@ static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const
                 SCW_CUDA_TRY(cudaMemsetAsync(f, 0, sizeof(int) * (size_t)K * nb_, st));
             }
         }
-        SplitArgs sp{Ab, Bb, rsA, ksA, rsB, ksB, sA, sB, opA == kOpC, opB == kOpC, M, N, K, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB,
+        SplitArgs sp{Ab, Bb, rsA, ksA, rsB, ksB, sA, sB, opB == kOpC, M, N, K, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB,
                      na_ * sh.gA, f, eA, gN, dA, dB, b1 ? 0 : 1};
         oz_split_kernel<S, TA, TB><<<na_ * sh.gA + nb_ * sh.gB, 256, 0, st>>>(sp, sk);
         SCW_CUDA_TRY(cudaGetLastError());
@@ -698,22 +698,15 @@ scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const doub
     }
     if (!ws.base && (diag != 0.0 || opB != kOpN)) return fail(SCW_ERR_ARG, "zgemm: this product needs a workspace");
     if (!ws.base) return gemm<double2>(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, skip);
-    return oz::run<8>(st, M, N, K, alpha, A, lda, sA, kOpN, B, ldb, sB, opB, beta, diag, C, ldc, sC, batch, ws, skip);
+    return oz::run<8>(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, opB, beta, diag, C, ldc, sC, batch, ws, skip);
 }
 
 template <typename TA, typename TB, typename TC>
 scw_status gemm32(cudaStream_t st, int n, double alpha, const TA* A, const TB* B, int opB, double beta, double diag, TC* C,
                   int batch, const GemmWs& ws, const int* skip) {
     const long long nn = (long long)n * n;
-    return oz::run<4>(st, n, n, n, make_double2(alpha, 0.0), A, n, nn, kOpN, B, n, nn, opB, make_double2(beta, 0.0), diag, C, n,
+    return oz::run<4>(st, n, n, n, make_double2(alpha, 0.0), A, n, nn, B, n, nn, opB, make_double2(beta, 0.0), diag, C, n,
                       nn, batch, ws, skip);
-}
-
-scw_status gemm32x(cudaStream_t st, int M, int N, int K, double alpha, const float2* A, int lda, long long sA, int opA,
-                   const float2* B, int ldb, long long sB, int opB, double beta, float2* C, int ldc, long long sC, int batch,
-                   const GemmWs& ws) {
-    return oz::run<4>(st, M, N, K, make_double2(alpha, 0.0), A, lda, sA, opA, B, ldb, sB, opB, make_double2(beta, 0.0), 0.0,
-                      C, ldc, sC, batch, ws, nullptr);
 }
 
 #define SCW_GEMM32(TA, TB, TC)                                                                                        \

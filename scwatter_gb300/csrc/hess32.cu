@@ -2,7 +2,7 @@
 // restated): the first stage of the mixed-precision eigen-solver.
 //
 // A panel of nb columns is reduced by one thread-block cluster per matrix; the trailing matrix and Q
-// then get its nb reflectors at once as products on the tensor cores (gemm32x).  Per column j the
+// then get its nb reflectors at once as FP32 products (cgemm32.cu).  Per column j the
 // cluster does, on the rows below the panel's top,
 //   b = A(:, j) - Y V(j, :)^H, then b -= V T^H (V^H b)
 //   the reflector v of b below row j, and y = tau (A v - Y V^H v)
@@ -15,8 +15,8 @@
 // at 11 000 clocks a column.  The rest are short phases between barriers, about 7000 clocks.  All clusters
 // have to be resident at once: 20 clusters of 7 CTAs are not (16 fit into the GPCs), and took two turns.
 // 20 matrices of n = 648: the panels 12.6 ms with every row of A read from L2 in 7-CTA clusters, 5.1 now;
-// 10 of n = 216: 1.27 -> 0.90 ms; 4 of n = 50: 254 -> 181 us.  The products: 10.9 -> 8.1 ms at n = 648, since the
-// zero rows of V above the panel are left out.  (Reduced column by column, with three launches each, every
+// 10 of n = 216: 1.27 -> 0.90 ms; 4 of n = 50: 254 -> 181 us.  The products leave out the zero rows of V above
+// the panel.  (Reduced column by column, with three launches each, every
 // column read A three times, wrote it once, and the same for Q: 84 ms.)
 //
 // A column whose part below the diagonal is under ulp ||A||_F / sqrt(n) (ulp times the root-mean-square
@@ -341,7 +341,7 @@ size_t hess32_ws_elems(int n) {
     return (size_t)n * (5 * z::kHb) + 1 + (n > 2400 ? far : 0);
 }
 
-scw_status hess32(cudaStream_t st, float2* A, float2* Q, int n, int batch, float2* work, const GemmWs& ws, int share) {
+scw_status hess32(cudaStream_t st, float2* A, float2* Q, int n, int batch, float2* work, int share) {
     if (n <= 0 || batch <= 0) return SCW_OK;
     const long long nn = (long long)n * n;
     float* fro = reinterpret_cast<float*>(work);
@@ -401,19 +401,19 @@ scw_status hess32(cudaStream_t st, float2* A, float2* Q, int n, int batch, float
                                         far ? big : (float2*)nullptr));
         // V and its products are zero above row top: from there on only.  Y(0 .. j0, :) = A V T
         const long long o = (long long)top * nb;
-        scw_status s = gemm32x(st, top, ib, m, 1.0, A + top, n, nn, kOpN, VT + o, nb, sp, kOpN, 0.0, Y, nb, sp, batch, ws);
+        scw_status s = cgemm(st, top, ib, m, 1.f, A + top, n, nn, kOpN, VT + o, nb, sp, kOpN, false, Y, nb, sp, batch);
         if (s != SCW_OK) return s;
         if (ib > 1) {
             z::hess_above_kernel<<<dim3((top + 7) / 8, batch), 256, 0, st>>>(A, n, nn, j0, ib, nb, pan);
             SCW_CUDA_TRY(cudaGetLastError());
         }
         // A(:, c..) -= Y V(c.., :)^H, then A(:, c..) -= V T^H (V^H A(:, c..)); Q -= (Q V T) V^H
-        s = gemm32x(st, n, rem, ib, -1.0, Y, nb, sp, kOpN, V + (long long)c * nb, nb, sp, kOpC, 1.0, A + c, n, nn, batch, ws);
+        s = cgemm(st, n, rem, ib, -1.f, Y, nb, sp, kOpN, V + (long long)c * nb, nb, sp, kOpC, true, A + c, n, nn, batch);
         float2* At = A + (long long)top * n + c;
-        if (s == SCW_OK) s = gemm32x(st, ib, rem, m, 1.0, V + o, nb, sp, kOpC, At, n, nn, kOpN, 0.0, W, n, sw, batch, ws);
-        if (s == SCW_OK) s = gemm32x(st, m, rem, ib, -1.0, VTH + o, nb, sp, kOpN, W, n, sw, kOpN, 1.0, At, n, nn, batch, ws);
-        if (s == SCW_OK) s = gemm32x(st, n, ib, m, 1.0, Q + top, n, nn, kOpN, VT + o, nb, sp, kOpN, 0.0, W, nb, sw, batch, ws);
-        if (s == SCW_OK) s = gemm32x(st, n, m, ib, -1.0, W, nb, sw, kOpN, V + o, nb, sp, kOpC, 1.0, Q + top, n, nn, batch, ws);
+        if (s == SCW_OK) s = cgemm(st, ib, rem, m, 1.f, V + o, nb, sp, kOpC, At, n, nn, kOpN, false, W, n, sw, batch);
+        if (s == SCW_OK) s = cgemm(st, m, rem, ib, -1.f, VTH + o, nb, sp, kOpN, W, n, sw, kOpN, true, At, n, nn, batch);
+        if (s == SCW_OK) s = cgemm(st, n, ib, m, 1.f, Q + top, n, nn, kOpN, VT + o, nb, sp, kOpN, false, W, nb, sw, batch);
+        if (s == SCW_OK) s = cgemm(st, n, m, ib, -1.f, W, nb, sw, kOpN, V + o, nb, sp, kOpC, true, Q + top, n, nn, batch);
         if (s != SCW_OK) return s;
     }
     return SCW_OK;

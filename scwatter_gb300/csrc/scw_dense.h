@@ -37,7 +37,7 @@ struct GemmWs {
     int* err = nullptr;
 };
 // cap on a workspace sized for a whole batch; larger batches go through it in parts
-constexpr size_t kGemmWsCap = 512ull << 20;
+constexpr size_t kGemmWsCap = 1024ull << 20;
 // the context's tensor-core error flag (allocated, cleared unless a check is pending) is in use from
 // here on: the next scw_ctx_synchronize reads it
 scw_status ctx_tc_flag(scw_ctx ctx);
@@ -58,10 +58,10 @@ scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const doub
 template <typename TA, typename TB, typename TC>
 scw_status gemm32(cudaStream_t st, int n, double alpha, const TA* A, const TB* B, int opB, double beta, double diag, TC* C,
                   int batch, const GemmWs& ws, const int* skip);
-// any shape in FP32, with an operation on A too
-scw_status gemm32x(cudaStream_t st, int M, int N, int K, double alpha, const float2* A, int lda, long long sA, int opA,
-                   const float2* B, int ldb, long long sB, int opB, double beta, float2* C, int ldc, long long sC, int batch,
-                   const GemmWs& ws);
+// FP32 product with a short side on the CUDA cores (cgemm32.cu): C = alpha op(A) op(B), added to C if add;
+// op = identity or conjugate transpose, alpha = +-1
+scw_status cgemm(cudaStream_t st, int M, int N, int K, float alpha, const float2* A, int lda, long long sA, int opA,
+                 const float2* B, int ldb, long long sB, int opB, bool add, float2* C, int ldc, long long sC, int batch);
 
 // C = alpha A B + beta C (row-major, batched by strides in elements)
 template <typename C>
@@ -84,7 +84,7 @@ scw_status schur32(cudaStream_t st, float2* A, float2* Q, float2* W, int n, int 
 // its stages: Hessenberg form of A with Q (hess32.cu), then the QR iteration with vectors accumulated into Z
 // (hqr32.cu; ctas: CTAs per matrix, 0 = chosen by size and batch)
 size_t hess32_ws_elems(int n);
-scw_status hess32(cudaStream_t st, float2* A, float2* Q, int n, int batch, float2* work, const GemmWs& ws, int share);
+scw_status hess32(cudaStream_t st, float2* A, float2* Q, int n, int batch, float2* work, int share);
 scw_status hqr32(cudaStream_t st, float2* H, float2* Z, int n, float2* W, int* status, int batch, int ctas, int share);
 // eigenvectors of the triangular T as the rows of X (unit diagonal), and the inverse Z of the unit
 // triangular matrix whose columns those are
