@@ -148,10 +148,7 @@ scw_status ensure_lanes(scw_batch b, int lanes) {
         scw_ctx c = nullptr;
         scw_status st = scw_ctx_create(b->ctx->device, s, &c);
         if (st != SCW_OK) return st;
-        // the tensor-core error flag is allocated here, never inside a capture
-        if (cudaMalloc(&c->tc_err, sizeof(int)) != cudaSuccess) return fail(SCW_ERR_NOMEM, "cudaMalloc error flag");
-        SCW_CUDA_TRY(cudaMemset(c->tc_err, 0, sizeof(int)));
-        c->tc_pending_check = true;        // and never cleared by a graph: scw_batch_wait reads it
+        c->tc_pending_check = true;        // the tensor-core error flag: scw_batch_wait reads it
         b->lane_ctx.push_back(c);
         b->lane_arena.push_back(nullptr);
         b->lane_bytes.push_back(0);
@@ -460,7 +457,7 @@ scw_status scw_batch_create(scw_ctx ctx, const scw_batch_item* items, int count,
     scw_status st = build_graph(b.get(), all, b->lanes, b->method, b->ctr_shape, b->g);
     if (st != SCW_OK) return st;
     // lane error flags start clear
-    for (auto c : b->lane_ctx) SCW_CUDA_TRY(cudaMemset(c->tc_err, 0, sizeof(int)));
+    for (auto c : b->lane_ctx) *(volatile int*)c->tc_host = 0;
     *out = b.release();
     return SCW_OK;
 }
@@ -481,8 +478,7 @@ scw_status scw_batch_wait(scw_batch b, int* item_status) {
     SCW_ON_DEVICE(b->ctx->device);
     SCW_CUDA_TRY(cudaStreamSynchronize(b->ctx->stream));
     std::vector<int> lane_err(b->lane_ctx.size(), 0);
-    for (size_t l = 0; l < b->lane_ctx.size(); l++)
-        SCW_CUDA_TRY(cudaMemcpy(&lane_err[l], b->lane_ctx[l]->tc_err, sizeof(int), cudaMemcpyDeviceToHost));
+    for (size_t l = 0; l < b->lane_ctx.size(); l++) lane_err[l] = *(volatile int*)b->lane_ctx[l]->tc_host;
     int bad = 0;
     for (size_t i = 0; i < b->items.size(); i++) {
         const Item& it = b->items[i];

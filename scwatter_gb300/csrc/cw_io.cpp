@@ -142,6 +142,16 @@ scw_status scw_ctx_create(int device, void* stream, scw_ctx* out) {
         delete c;
         return fail(SCW_ERR_CUDA, cudaGetErrorString(e));
     }
+    if (cudaHostAlloc((void**)&c->tc_host, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void**)&c->tc_err, c->tc_host, 0) != cudaSuccess) {
+        const cudaError_t err = cudaGetLastError();
+        if (c->tc_host) cudaFreeHost(c->tc_host);
+        cudaEventDestroy(c->desc_done);
+        if (c->own_stream) cudaStreamDestroy(c->stream);
+        delete c;
+        return fail(SCW_ERR_NOMEM, cudaGetErrorString(err));
+    }
+    *c->tc_host = 0;
     *out = c;
     return SCW_OK;
 }
@@ -156,7 +166,7 @@ scw_status scw_ctx_destroy(scw_ctx c) {
     c->sep_scratch.release();
     c->dense_ws.release();
     c->host_desc.release();
-    if (c->tc_err) cudaFree(c->tc_err);
+    if (c->tc_host) cudaFreeHost(c->tc_host);
     for (auto& t : c->timings) {
         cudaEventDestroy(t.start);
         cudaEventDestroy(t.stop);
@@ -171,11 +181,9 @@ scw_status scw_ctx_destroy(scw_ctx c) {
 scw_status scw_ctx_synchronize(scw_ctx c) {
     if (!c) return fail(SCW_ERR_ARG, "null context");
     SCW_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    if (c->tc_pending_check && c->tc_err) {
-        int flag = 0;
-        SCW_CUDA_TRY(cudaMemcpy(&flag, c->tc_err, sizeof(int), cudaMemcpyDeviceToHost));
+    if (c->tc_pending_check) {
         c->tc_pending_check = false;
-        if (flag) return fail(SCW_ERR_TIMEOUT, "a tensor-core kernel's bounded mbarrier wait gave up");
+        if (*(volatile int*)c->tc_host) return fail(SCW_ERR_TIMEOUT, "a tensor-core kernel's bounded mbarrier wait gave up");
     }
     return SCW_OK;
 }

@@ -802,8 +802,7 @@ scw_status scw_gpu_cw_evaluate(scw_waves w, float* E_xy, float* E_xz, float* E_y
     SCW_CUDA_TRY(cudaMemcpyAsync(E_xy, dxy, plane_floats * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     SCW_CUDA_TRY(cudaMemcpyAsync(E_xz, dxz, plane_floats * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     SCW_CUDA_TRY(cudaMemcpyAsync(E_yz, dyz, plane_floats * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-    SCW_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    return SCW_OK;
+    return scw_ctx_synchronize(ctx);
 }
 
 }  // extern "C"

@@ -663,12 +663,9 @@ static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const
 }  // namespace oz
 
 scw_status ctx_tc_flag(scw_ctx ctx) {
-    if (!ctx->tc_err && cudaMalloc(&ctx->tc_err, sizeof(int)) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(SCW_ERR_NOMEM, "cudaMalloc error flag");
-    }
-    // cleared once per synchronisation: a flag raised by an earlier launch stays raised
-    if (!ctx->tc_pending_check) SCW_CUDA_TRY(cudaMemsetAsync(ctx->tc_err, 0, sizeof(int), ctx->stream));
+    // cleared once per synchronisation, when no kernel that may raise it is under way: a flag raised by an
+    // earlier launch stays raised
+    if (!ctx->tc_pending_check) *(volatile int*)ctx->tc_host = 0;
     ctx->tc_pending_check = true;
     return SCW_OK;
 }

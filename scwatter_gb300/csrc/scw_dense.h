@@ -38,8 +38,7 @@ struct GemmWs {
 };
 // cap on a workspace sized for a whole batch; larger batches go through it in parts
 constexpr size_t kGemmWsCap = 1024ull << 20;
-// the context's tensor-core error flag (allocated, cleared unless a check is pending) is in use from
-// here on: the next scw_ctx_synchronize reads it
+// the context's tensor-core error flag (cleared unless a check is pending) is in use from here on: the next scw_ctx_synchronize reads it
 scw_status ctx_tc_flag(scw_ctx ctx);
 // a context's own GEMM workspace of at least `one` bytes, `all` if that is below the cap; none (the
 // products then run without one) while the context's stream is being captured

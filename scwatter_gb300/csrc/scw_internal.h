@@ -103,7 +103,8 @@ struct scw_ctx_s {
     scw::PinnedBuf host_desc;   // pinned staging of the descriptors
     cudaEvent_t desc_done = nullptr;  // the last descriptor upload has been consumed
     void* static_scratch = nullptr;   // device address of the allocation-free entry point's array
-    int* tc_err = nullptr;            // device flag: a tensor-core kernel's bounded wait gave up
+    int* tc_err = nullptr;            // flag: a tensor-core kernel's bounded wait gave up (device address)
+    int* tc_host = nullptr;           // its host address: mapped host memory, so that reading it takes no copy
     bool tc_pending_check = false;    // a tensor-core kernel ran since the flag was last read
     bool timing = false;
     std::vector<KernelTiming> timings;

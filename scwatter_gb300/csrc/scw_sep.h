@@ -78,6 +78,9 @@ struct scw_sep_s {
     // pipelined device volumes: stage 2 of one chunk of planes on hi_stream (high priority) while
     // stage 1 of the next runs on the context stream
     cudaStream_t hi_stream = nullptr;
+    // the viewer's second and third plane run beside the first (scw_sep_gpu_cw_evaluate)
+    cudaStream_t plane_stream[2] = {nullptr, nullptr};
+    cudaEvent_t plane_event[3] = {nullptr, nullptr, nullptr};
     std::vector<cudaEvent_t> pevents;
     int pipe_chunks = 0;                   // chunks of a pipelined slab (0 or 1: one pass)
     int pipe_synth_div = 2;                // the pipelined output GEMM runs on sm_count / pipe_synth_div SMs
