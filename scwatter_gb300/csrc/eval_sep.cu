@@ -44,10 +44,10 @@ __device__ __forceinline__ float2 phase_fp64(double kr, double ki, double dz) {
 //     h = 1 (rows Ez):     beta_dn_j exp(i kz_dn_j (z - z_l)) - beta_up_j exp(i kz_up_j (z - z_{l+1}))
 // One thread per mode (and half, of a two-half set) and plane, planes fastest (consecutive stores): with one
 // thread per mode looping over the planes, the chain of FP64 phases took 20 us for 200 modes.
-__global__ void sep_phase_kernel(const PGroup* __restrict__ groups, const float* __restrict__ zlist,
-                                 const double2* __restrict__ kz, const double2* __restrict__ beta,
+__global__ void sep_phase_kernel(const __grid_constant__ SepDesc desc, int off_z, const double2* __restrict__ kz, const double2* __restrict__ beta,
                                  const double* __restrict__ zb, int J, int nks, float2* __restrict__ Phi) {
-    const PGroup& g = groups[blockIdx.y];
+    const PGroup& g = reinterpret_cast<const PGroup*>(desc.base())[blockIdx.y];
+    const float* zlist = reinterpret_cast<const float*>(desc.base() + off_z);
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = e / nks, kk = e - j * nks;
     const int l = g.region - 1;
@@ -114,13 +114,13 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 template <int NK, int RW>
 __global__ void __launch_bounds__(kCtrWarps * 32, 2)
-sep_contract_kernel(const PGroup* __restrict__ groups, const float2* __restrict__ Phi,
+sep_contract_kernel(const __grid_constant__ SepDesc desc, const float2* __restrict__ Phi,
                     const float2* __restrict__ Q, int MF, int J, int H, float2* __restrict__ C) {
     constexpr int S = CtrCfg<RW, NK>::kStages;
     extern __shared__ float4 smem4[];
     // (phi[j][kk], phi[j+1][kk]) pairs per plane; then per lane S x RW private Q slots
     float4 (*ph)[kCtrChunk / 2] = reinterpret_cast<float4 (*)[kCtrChunk / 2]>(smem4);
-    const PGroup g = groups[blockIdx.y];
+    const PGroup g = reinterpret_cast<const PGroup*>(desc.base())[blockIdx.y];
     const int l = g.region - 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float4* qs = smem4 + NK * (kCtrChunk / 2) + (size_t)warp * S * RW * 32 + lane;   // slot (s, r): qs[(s*RW + r)*32]
@@ -212,13 +212,14 @@ sep_contract_kernel(const PGroup* __restrict__ groups, const float2* __restrict_
 // Exterior regions: region 0 = incident (referenced at the origin) + reflected (at z_0),
 // last region = transmitted (at z_Z).  One thread per (z entry, p), FP64; the phases serve all three
 // components.
-__global__ void sep_exterior_kernel(const int2* __restrict__ ext, int n_ext, const float* __restrict__ zlist,
+__global__ void sep_exterior_kernel(const __grid_constant__ SepDesc desc, int off_e, int n_ext, int off_z,
                                     const double2* __restrict__ xd, int MF, double z0, double zZ,
                                     float2* __restrict__ C) {
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)n_ext * MF) return;
     const int e = (int)(idx / MF), p = (int)(idx % MF);
-    const int2 ent = ext[e];     // (zi, 0 = top exterior / 1 = bottom exterior)
+    const float* zlist = reinterpret_cast<const float*>(desc.base() + off_z);
+    const int2 ent = reinterpret_cast<const int2*>(desc.base() + off_e)[e];     // (zi, 0 = top exterior / 1 = bottom exterior)
     const double z = (double)zlist[ent.x];
     // xd layout: inc[3][MF], refl[3][MF], trans[3][MF], kz_inc[MF], kz_refl[MF], kz_trans[MF]
     const double2* kzi = xd + 9 * MF;
@@ -481,16 +482,18 @@ void sep_eval_desc(const SepEvalPlan& p, char* h) {
     std::memcpy(h + p.off_z, p.zlist.data(), p.zlist.size() * sizeof(float));
 }
 
-// Stage 1 for the plan's z-values: fills C [nz][3][MF]; descriptors already on the device.
+// Stage 1 for the plan's z-values: fills C [nz][3][MF]; descriptors already on the device, or (d_desc null) with
+// the launches.
 static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_desc, float2* dC, char* cursor) {
     scw_ctx ctx = s->ctx;
     const int MF = s->MF, J = s->Jp;          // device row stride (even)
     const auto& groups = p.groups;
     const auto& ext = p.ext;
     const int max_nk = p.max_nk;
-    const PGroup* dg = (const PGroup*)d_desc;
-    const int2* de = (const int2*)(d_desc + p.off_e);
-    const float* dz = (const float*)(d_desc + p.off_z);
+    SepDesc desc;
+    desc.dev = d_desc;
+    if (!d_desc) sep_eval_desc(p, desc.here);
+    const int off_e = (int)p.off_e, off_z = (int)p.off_z;
     if (!groups.empty()) {
         if (J > 0) {
             const int nks = max_nk;            // a kernel per plane count: 5 planes cost 5, not 8
@@ -500,7 +503,7 @@ static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_d
             dim3 gp(((s->halves == 1 ? J : 2 * J) * nks + 127) / 128, (unsigned)groups.size());
             {
                 LaunchTimer lt(ctx, "sep_phase_kernel");
-                sep_phase_kernel<<<gp, 128, 0, ctx->stream>>>(dg, dz, s->dKz, s->halves == 1 ? s->dBeta : nullptr,
+                sep_phase_kernel<<<gp, 128, 0, ctx->stream>>>(desc, off_z, s->dKz, s->halves == 1 ? s->dBeta : nullptr,
                                                               s->dzb, J, nks, dPhi);
             }
             SCW_CUDA_TRY(cudaGetLastError());
@@ -512,7 +515,7 @@ static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_d
             LaunchTimer lt(ctx, "sep_contract_kernel");
             auto launch = [&](auto kernel, int rw, size_t smem) -> scw_status {
                 SCW_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-                kernel<<<grid_for(rw), kCtrWarps * 32, smem, ctx->stream>>>(dg, dPhi, s->dQ, MF, J, s->halves, dC);
+                kernel<<<grid_for(rw), kCtrWarps * 32, smem, ctx->stream>>>(desc, dPhi, s->dQ, MF, J, s->halves, dC);
                 return SCW_OK;
             };
             scw_status ls;
@@ -546,7 +549,7 @@ static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_d
     if (!ext.empty()) {
         const long long n = (long long)ext.size() * MF;
         LaunchTimer lt(ctx, "sep_exterior_kernel");
-        sep_exterior_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(de, (int)ext.size(), dz, s->dExt, MF,
+        sep_exterior_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(desc, off_e, (int)ext.size(), off_z, s->dExt, MF,
                                                                                  s->zb[0], s->zb[s->Z], dC);
         SCW_CUDA_TRY(cudaGetLastError());
         ctx->launches++;
@@ -714,6 +717,21 @@ scw_status sep_eval_record(scw_sep s, const SepEvalPlan& p, const char* d_desc, 
     return stage2_record(s, p, scratch, dE);
 }
 
+// The plan's launches with the context's scratch (reserved): the descriptors go with them, or up first (pinned
+// staging, guarded by the context's event) where there are too many.
+static scw_status sep_eval_launch(scw_sep s, const SepEvalPlan& p, float* dE) {
+    scw_ctx ctx = s->ctx;
+    if (p.desc_bytes <= kDescInline) return sep_eval_record(s, p, nullptr, (char*)ctx->sep_scratch.ptr, dE);
+    scw_status st;
+    SCW_CUDA_TRY(cudaEventSynchronize(ctx->desc_done));
+    if ((st = ctx->host_desc.reserve(p.desc_bytes)) != SCW_OK) return st;
+    if ((st = ctx->desc.reserve(p.desc_bytes)) != SCW_OK) return st;
+    sep_eval_desc(p, (char*)ctx->host_desc.ptr);
+    SCW_CUDA_TRY(cudaMemcpyAsync(ctx->desc.ptr, ctx->host_desc.ptr, p.desc_bytes, cudaMemcpyHostToDevice, ctx->stream));
+    SCW_CUDA_TRY(cudaEventRecord(ctx->desc_done, ctx->stream));
+    return sep_eval_record(s, p, (const char*)ctx->desc.ptr, (char*)ctx->sep_scratch.ptr, dE);
+}
+
 scw_status sep_eval(scw_sep s, int kind, float a0, float b0, float c, float da, float db, float dz, int Na, int Nb,
                     int Nz, float* dE, int method) {
     scw_ctx ctx = s->ctx;
@@ -722,14 +740,7 @@ scw_status sep_eval(scw_sep s, int kind, float a0, float b0, float c, float da, 
     scw_status st = sep_eval_plan(s, kind, a0, b0, c, da, db, dz, Na, Nb, Nz, method, p);
     if (st != SCW_OK) return st;
     if ((st = ctx->sep_scratch.reserve(p.scratch_bytes)) != SCW_OK) return st;
-    // descriptors to the device (pinned staging, guarded by the context's event)
-    SCW_CUDA_TRY(cudaEventSynchronize(ctx->desc_done));
-    if ((st = ctx->host_desc.reserve(p.desc_bytes)) != SCW_OK) return st;
-    if ((st = ctx->desc.reserve(p.desc_bytes)) != SCW_OK) return st;
-    sep_eval_desc(p, (char*)ctx->host_desc.ptr);
-    SCW_CUDA_TRY(cudaMemcpyAsync(ctx->desc.ptr, ctx->host_desc.ptr, p.desc_bytes, cudaMemcpyHostToDevice, ctx->stream));
-    SCW_CUDA_TRY(cudaEventRecord(ctx->desc_done, ctx->stream));
-    return sep_eval_record(s, p, (const char*)ctx->desc.ptr, (char*)ctx->sep_scratch.ptr, dE);
+    return sep_eval_launch(s, p, dE);
 }
 
 
@@ -753,12 +764,15 @@ static scw_status sep_eval_three(scw_sep s, const SepEvalPlan* plans, float* con
         if (!q) SCW_CUDA_TRY(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
     for (auto& e : s->plane_event)
         if (!e) SCW_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    SCW_CUDA_TRY(cudaEventSynchronize(ctx->desc_done));
-    if ((st = ctx->host_desc.reserve(desc_total)) != SCW_OK) return st;
-    if ((st = ctx->desc.reserve(desc_total)) != SCW_OK) return st;
-    for (int q = 0; q < 3; q++) sep_eval_desc(plans[q], (char*)ctx->host_desc.ptr + desc_off[q]);
-    SCW_CUDA_TRY(cudaMemcpyAsync(ctx->desc.ptr, ctx->host_desc.ptr, desc_total, cudaMemcpyHostToDevice, ctx->stream));
-    SCW_CUDA_TRY(cudaEventRecord(ctx->desc_done, ctx->stream));
+    const bool upload = plans[0].desc_bytes > kDescInline || plans[1].desc_bytes > kDescInline || plans[2].desc_bytes > kDescInline;
+    if (upload) {
+        SCW_CUDA_TRY(cudaEventSynchronize(ctx->desc_done));
+        if ((st = ctx->host_desc.reserve(desc_total)) != SCW_OK) return st;
+        if ((st = ctx->desc.reserve(desc_total)) != SCW_OK) return st;
+        for (int q = 0; q < 3; q++) sep_eval_desc(plans[q], (char*)ctx->host_desc.ptr + desc_off[q]);
+        SCW_CUDA_TRY(cudaMemcpyAsync(ctx->desc.ptr, ctx->host_desc.ptr, desc_total, cudaMemcpyHostToDevice, ctx->stream));
+        SCW_CUDA_TRY(cudaEventRecord(ctx->desc_done, ctx->stream));
+    }
     if ((st = ctx_tc_flag(ctx)) != SCW_OK) return st;      // cleared before any of the streams may raise it
     const cudaStream_t main_stream = ctx->stream;
     SCW_CUDA_TRY(cudaEventRecord(s->plane_event[0], main_stream));
@@ -768,7 +782,8 @@ static scw_status sep_eval_three(scw_sep s, const SepEvalPlan* plans, float* con
             ctx->stream = s->plane_stream[k - 1];
             SCW_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, s->plane_event[0], 0));
         }
-        st = sep_eval_record(s, plans[k], (const char*)ctx->desc.ptr + desc_off[k], (char*)ctx->sep_scratch.ptr + scratch_off[k], dE[k]);
+        st = sep_eval_record(s, plans[k], upload ? (const char*)ctx->desc.ptr + desc_off[k] : nullptr,
+                             (char*)ctx->sep_scratch.ptr + scratch_off[k], dE[k]);
         if (k) {
             // also after an error: the context's next work must not overtake what was launched
             const cudaError_t e = cudaEventRecord(s->plane_event[k], ctx->stream);
@@ -1000,13 +1015,7 @@ scw_status sep_eval_slab(scw_sep s, float x0, float y0, float z0, float dx, floa
     scw_status st = sep_eval_plan_planes(s, x0, y0, z0, dx, dy, dz, Nx, Ny, k_begin, k_end, method, p);
     if (st != SCW_OK) return st;
     if ((st = ctx->sep_scratch.reserve(p.scratch_bytes)) != SCW_OK) return st;
-    SCW_CUDA_TRY(cudaEventSynchronize(ctx->desc_done));
-    if ((st = ctx->host_desc.reserve(p.desc_bytes)) != SCW_OK) return st;
-    if ((st = ctx->desc.reserve(p.desc_bytes)) != SCW_OK) return st;
-    sep_eval_desc(p, (char*)ctx->host_desc.ptr);
-    SCW_CUDA_TRY(cudaMemcpyAsync(ctx->desc.ptr, ctx->host_desc.ptr, p.desc_bytes, cudaMemcpyHostToDevice, ctx->stream));
-    SCW_CUDA_TRY(cudaEventRecord(ctx->desc_done, ctx->stream));
-    return sep_eval_record(s, p, (const char*)ctx->desc.ptr, (char*)ctx->sep_scratch.ptr, dE);
+    return sep_eval_launch(s, p, dE);
 }
 
 }  // namespace scw

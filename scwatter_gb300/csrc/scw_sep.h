@@ -30,11 +30,20 @@ struct SepEvalPlan {
     int nrows = 0, ncols = 0, Mk = 0;
     size_t phi_bytes = 0, c_bytes = 0, t_bytes = 0, tab_bytes = 0, scratch_bytes = 0;
 };
+// A plan's descriptor block as stage 1's kernels get it: a device address, or (dev null) the block itself among the
+// kernel parameters.  Uploading it first cost a copy of 1 us that the host took 11 us to submit and the first kernel
+// waited 14 us for, as long as all of a small volume's kernels; a block that fits goes with the launches.
+constexpr size_t kDescInline = 3584;       // 64 groups and 256 planes; all parameters of a kernel below 4 KB
+struct SepDesc {
+    const char* dev;
+    alignas(16) char here[kDescInline];
+    __device__ __forceinline__ const char* base() const { return dev ? dev : here; }
+};
 // kind 0: Nz xy planes (a = x, b = y); 1: xz plane at y = c; 2: yz plane at x = c
 scw_status sep_eval_plan(const scw_sep_s* s, int kind, float a0, float b0, float c, float da, float db, float dz,
                          int Na, int Nb, int Nz, int method, SepEvalPlan& p);
 void sep_eval_desc(const SepEvalPlan& p, char* host);
-// launches only, on the set's context stream
+// launches only, on the set's context stream; d_desc null: the plan's block (at most kDescInline bytes) goes with them
 scw_status sep_eval_record(scw_sep_s* s, const SepEvalPlan& p, const char* d_desc, char* scratch, float* dE);
 
 // output GEMM of stage 2: E[r][col][c] = sum_m T[r][c][m] F[m][col]
