@@ -152,7 +152,7 @@ __device__ __forceinline__ bool window_deflates(const float2* T, int k, int ihi)
     if (tst == 0.f) return hqr_deflates<float2, false>(T, kLdn, k, ihi);
     const float ab = fmaxf(a1, u1), ba = fminf(a1, u1), aa = fmaxf(d1, dd), bb = fminf(d1, dd), is = __fdividef(1.f, aa + ab);
     const bool far = ba * (ab * is) <= fmaxf(small, ulp * (bb * (aa * is))) || ba * ab <= (ulp * d1) * (ulp * d1);
-    return a1 <= small || (fabsf(a.x) <= ulp * tst && far);
+    return a1 <= small || (a1 <= ulp * tst && far);
 }
 
 // The rotations of a sweep over columns l .. l + cnt - 1, in order, on row `row` of X from column ks on: a

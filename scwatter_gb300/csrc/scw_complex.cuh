@@ -138,7 +138,8 @@ __device__ __forceinline__ bool hqr_deflates(const C* H, int n, int k, int ihi) 
         if (k - 2 >= 0) tst += r_abs(hld<kCg>(H + (long long)(k - 1) * n + k - 2).x);
         if (k + 1 <= ihi) tst += r_abs(hld<kCg>(H + (long long)(k + 1) * n + k).x);
     }
-    if (r_abs(hkk1.x) > ulp * tst) return false;
+    // (zlahqr keeps its subdiagonals real and looks at the real part; these are not)
+    if (cabs1(hkk1) > ulp * tst) return false;
     // Ahues & Tisseur conservative deflation criterion (as in zlahqr)
     const C hk1k = hld<kCg>(H + (long long)(k - 1) * n + k);
     const C hkk = hld<kCg>(H + (long long)k * n + k);
