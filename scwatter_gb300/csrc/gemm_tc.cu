@@ -179,6 +179,10 @@ __device__ __forceinline__ void store_digits(const long long (&q)[8], unsigned c
     }
 }
 
+// 512 threads: bound by the latency of its loads (operands of two products of n = 648: 50 us with 256, 35 with 512 and with
+// 1024; of 20, with more blocks than SMs, 253, 234 and 245)
+constexpr int kSplitThreads = 512, kSplitK = kSplitThreads / 16;
+
 struct SplitArgs {
     const void *A, *B;
     long long rsA, ksA, rsB, ksB;      // element (row of A or column of B, inner index k) at row rs + k ks
@@ -196,7 +200,7 @@ struct SplitArgs {
 // the inner index, then the digits, a warp per stage of 16 inner indices (lane = 8 rows x 2 halves of
 // the stage x 2 row groups, so a warp stores 512 contiguous bytes per digit).
 template <int S, bool kA, typename T>
-__device__ __forceinline__ void split_group(const SplitArgs& p, int b, int g, int (*se)[17]) {
+__device__ __forceinline__ void split_group(const SplitArgs& p, int b, int g, int (*se)[kSplitK + 1]) {
     using C = Cfg<S>;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int per = kA ? p.gA : p.gB, r0 = g * 16, R = kA ? p.M : p.N;
@@ -204,13 +208,13 @@ __device__ __forceinline__ void split_group(const SplitArgs& p, int b, int g, in
     const long long rs = kA ? p.rsA : p.rsB, ks = kA ? p.ksA : p.ksB;
     const int* f = p.f + (long long)(kA ? b * p.fstep : b) * p.K;
     {
-        // 16 x 16 threads, the faster ones along the contiguous index
+        // 16 x kSplitK threads, the faster ones along the contiguous index
         const bool kfast = ks == 1;
-        const int r = kfast ? t >> 4 : t & 15, kr = kfast ? t & 15 : t >> 4;
+        const int r = kfast ? t / kSplitK : t & 15, kr = kfast ? t % kSplitK : t >> 4;
         int e = kNone;
         if (r0 + r < R) {
 #pragma unroll 4
-            for (int k = kr; k < p.K; k += 16) {
+            for (int k = kr; k < p.K; k += kSplitK) {
                 const int x = cexpo(src[(r0 + r) * rs + k * ks]);
                 if (x == kSpecial) e = kSpecial;
                 else if (x != kNone) e = max(e, kA ? x + f[k] : x - f[k]);
@@ -221,18 +225,18 @@ __device__ __forceinline__ void split_group(const SplitArgs& p, int b, int g, in
     __syncthreads();
     if (t < 16) {
         int e = kNone;
-        for (int q = 0; q < 16; q++) e = max(e, se[t][q]);
-        se[t][16] = e;
+        for (int q = 0; q < kSplitK; q++) e = max(e, se[t][q]);
+        se[t][kSplitK] = e;
         (kA ? p.eA : p.gN)[(long long)b * per * 16 + r0 + t] = e;
     }
     __syncthreads();
     const int rl = (lane & 7) + 8 * (lane >> 4), kh = (lane >> 3) & 1;
-    const int r = r0 + rl, e = se[rl][16];
+    const int r = r0 + rl, e = se[rl][kSplitK];
     const bool live = r < R && e > kNone / 2 && e < kSpecial;
     constexpr int TR = kA ? kTM : C::kTN, blkb = kA ? C::kABlk : C::kBBlk, dig = TR * kTK * 2;
     unsigned char* dst = (kA ? p.dA + (long long)b * p.mt * p.nk * C::kABlk : p.dB + (long long)b * p.nt * p.nk * C::kBBlk) +
                          (long long)(r0 / TR) * p.nk * blkb + (r0 % TR) * 32 + (lane >> 4) * 256 + kh * 128 + (lane & 7) * 16;
-    for (int st = warp; st < p.nk; st += 8) {
+    for (int st = warp; st < p.nk; st += kSplitThreads / 32) {
         const int k0 = st * kTK + kh * 8;
         long long qr[8], qi[8];
 #pragma unroll
@@ -254,8 +258,8 @@ __device__ __forceinline__ void split_group(const SplitArgs& p, int b, int g, in
 }
 
 template <int S, typename TA, typename TB>
-__global__ void __launch_bounds__(256) oz_split_kernel(SplitArgs p, const int* __restrict__ skip) {
-    __shared__ int se[16][17];
+__global__ void __launch_bounds__(kSplitThreads) oz_split_kernel(SplitArgs p, const int* __restrict__ skip) {
+    __shared__ int se[16][kSplitK + 1];
     const bool isA = (int)blockIdx.x < p.nA;
     const int blk = isA ? blockIdx.x : blockIdx.x - p.nA;
     const int per = isA ? p.gA : p.gB;
@@ -648,7 +652,7 @@ static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const
         }
         SplitArgs sp{Ab, Bb, rsA, ksA, rsB, ksB, sA, sB, opB == kOpC, M, N, K, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB,
                      na_ * sh.gA, f, eA, gN, dA, dB, b1 ? 0 : 1};
-        oz_split_kernel<S, TA, TB><<<na_ * sh.gA + nb_ * sh.gB, 256, 0, st>>>(sp, sk);
+        oz_split_kernel<S, TA, TB><<<na_ * sh.gA + nb_ * sh.gB, kSplitThreads, 0, st>>>(sp, sk);
         SCW_CUDA_TRY(cudaGetLastError());
         const long long tiles = (long long)sh.mt * sh.nt * nb;
         if (tiles > (1ll << 30)) return fail(SCW_ERR_ARG, "zgemm: too many tiles");
