@@ -14,6 +14,8 @@
 // The products of all panels, 20 matrices of n = 648: 5.5 ms, against 8.1 as digit products and 2.9 for their digits; 10
 // of n = 216: 0.50 against 0.63 + 0.29 ms; 4 of n = 50: 76 against 152 + 75 us.  A rank-32 update of 616 columns takes
 // 80 us (3 CTAs per SM; 88 with 2): the latency of its loads, two chunks and C is what bounds it.
+#include <algorithm>
+
 #include "scw_complex.cuh"
 #include "scw_dense.h"
 
@@ -43,11 +45,11 @@ struct CgArgs {
     float2* C;
     int M, N, K, lda, ldb, ldc;
     long long sA, sB, sC;
-    float alpha;
+    float alpha, conjA, conjB;         // conj: -1 for the conjugate
     int add;
 };
 
-// CA, CB: the conjugate transpose of the stored matrix.  KS groups of (TM / 4) (TN / 4) threads along the inner index.
+// CA, CB: the transpose of the stored matrix.  KS groups of (TM / 4) (TN / 4) threads along the inner index.
 // SHORT: at most two chunks, one set of sums.
 template <int TM, int TN, int KS, bool CA, bool CB, bool SHORT>
 __global__ void __launch_bounds__(TM / 4 * (TN / 4) * KS, SHORT ? 3 : 2)
@@ -93,14 +95,14 @@ cgemm_kernel(CgArgs p) {
 #pragma unroll
         for (int q = 0; q < nA; q++) {
             const int e = t + q * kG;
-            const float y = CA ? -ra[q].y : ra[q].y;
+            const float y = p.conjA * ra[q].y;
             sA[group][CA ? e / TM : e % kCgK][CA ? e % TM : e / kCgK] =
                 make_ulonglong2(cg_pair(ra[q].x, ra[q].x), cg_pair(y, y));
         }
 #pragma unroll
         for (int q = 0; q < nB; q++) {
             const int e = t + q * kG;
-            const float y = CB ? -rb[q].y : rb[q].y;
+            const float y = p.conjB * rb[q].y;
             sB[group][CB ? e % kCgK : e / TN][CB ? e / kCgK : e % TN] =
                 make_ulonglong2(cg_pair(rb[q].x, y), cg_pair(-y, rb[q].x));
         }
@@ -183,15 +185,15 @@ static scw_status cgemm_launch(cudaStream_t st, const CgArgs& p, bool ca, bool c
 scw_status cgemm(cudaStream_t st, int M, int N, int K, float alpha, const float2* A, int lda, long long sA, int opA,
                  const float2* B, int ldb, long long sB, int opB, bool add, float2* C, int ldc, long long sC, int batch) {
     if (M <= 0 || N <= 0 || batch <= 0) return SCW_OK;
-    const bool ca = opA == kOpC, cb = opB == kOpC;
+    const bool ca = opA != kOpN, cb = opB != kOpN;
+    const z::CgArgs p{A, B, C, M, N, K, lda, ldb, ldc, sA, sB, sC, alpha, opA == kOpC ? -1.f : 1.f, opB == kOpC ? -1.f : 1.f, add ? 1 : 0};
     // (a grid's z has 65 535 blocks at most)
-    const z::CgArgs p{A, B, C, M, N, K, lda, ldb, ldc, sA, sB, sC, alpha, add ? 1 : 0};
     for (int b0 = 0; b0 < batch; b0 += 65535) {
         z::CgArgs q = p;
         q.A += sA * b0;
         q.B += sB * b0;
         q.C += sC * b0;
-        const int nb = batch - b0 < 65535 ? batch - b0 : 65535;
+        const int nb = std::min(batch - b0, 65535);
         const scw_status s = M <= 32 ? z::cgemm_launch<32, 64, 2>(st, q, ca, cb, nb)
                            : N <= 32 ? z::cgemm_launch<64, 32, 2>(st, q, ca, cb, nb)
                            : K <= 2 * z::kCgK ? z::cgemm_launch<64, 64, 1, true>(st, q, ca, cb, nb)

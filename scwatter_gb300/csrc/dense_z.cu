@@ -1316,7 +1316,7 @@ scw_status trevc(cudaStream_t st, const C* T, C* X, int n, int batch, const int*
     return SCW_OK;
 }
 
-scw_status trtri32(cudaStream_t st, const float2* X, float2* Z, int n, int batch) {
+scw_status trtri_rows(cudaStream_t st, const float2* X, float2* Z, int n, int batch) {
     z::trtri_kernel<float2><<<dim3((n * 32 + 255) / 256, batch), 256, 0, st>>>(X, Z, n, (long long)n * n);
     SCW_CUDA_TRY(cudaGetLastError());
     return SCW_OK;
@@ -1369,7 +1369,7 @@ scw_status cgeev(cudaStream_t st, float2* A, float2* W, float2* V, int n, int ba
                  const GemmWs& ws, int share) {
     float2* Q = work;                        // batch * n * n: Schur vectors
     scw_status s = schur32(st, A, Q, W, n, batch, work + (long long)n * n * batch, status, ws, share);
-    if (s == SCW_OK) s = trevc<float2>(st, A, V, n, batch, nullptr);
+    if (s == SCW_OK) s = trevc32(st, A, V, n, batch);
     if (s != SCW_OK) return s;
     return gemm32(st, n, 1.0, Q, V, kOpT, 0.0, 0.0, V, batch, ws, nullptr);
 }

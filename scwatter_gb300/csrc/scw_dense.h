@@ -57,8 +57,7 @@ scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const doub
 template <typename TA, typename TB, typename TC>
 scw_status gemm32(cudaStream_t st, int n, double alpha, const TA* A, const TB* B, int opB, double beta, double diag, TC* C,
                   int batch, const GemmWs& ws, const int* skip);
-// FP32 product with a short side on the CUDA cores (cgemm32.cu): C = alpha op(A) op(B), added to C if add;
-// op = identity or conjugate transpose, alpha = +-1
+// FP32 product with a short side on the CUDA cores (cgemm32.cu): C = alpha op(A) op(B), added to C if add; alpha = +-1
 scw_status cgemm(cudaStream_t st, int M, int N, int K, float alpha, const float2* A, int lda, long long sA, int opA,
                  const float2* B, int ldb, long long sB, int opB, bool add, float2* C, int ldc, long long sC, int batch);
 
@@ -89,6 +88,9 @@ scw_status hqr32(cudaStream_t st, float2* H, float2* Z, int n, float2* W, int* s
 // triangular matrix whose columns those are
 template <typename C>
 scw_status trevc(cudaStream_t st, const C* T, C* X, int n, int batch, const int* skip);
+scw_status trtri_rows(cudaStream_t st, const float2* X, float2* Z, int n, int batch);
+// the same in FP32 in blocks (tri32.cu)
+scw_status trevc32(cudaStream_t st, const float2* T, float2* X, int n, int batch);
 scw_status trtri32(cudaStream_t st, const float2* X, float2* Z, int n, int batch);
 // eigenvalues W and right eigenvectors V (columns) of A (overwritten), FP64; work >= batch (n^2 + 3 n);
 // status[b] = 1 when the QR iteration did not converge.  wide: the Hessenberg reduction of
