@@ -49,10 +49,11 @@ CFG2 = dict(name="spheres[64,128,128] coef40x40 64 slices, grid 512x512x256", M0
 # the paired set (dram__bytes_read.sum + dram__bytes_write.sum = 985.03 MB + 4.47 MB for 984.27 MB of
 # V and C: 8 x 3 x 1600 x 3200 x 8 B + 32 x 3 x 1600 x 8 B)
 CONTRACT_TRAFFIC_RATIO = (985.032448e6 + 4.474368e6) / (8 * 3 * 1600 * 3200 * 8 + 32 * 3 * 1600 * 8)
-# XU (MUFU) thread instructions per point*mode of plain_eval_kernel on an xy plane, from ncu
-# (smsp__inst_executed_pipe_xu.sum x 32 / points*modes = 656e6 x 32 / 1.0486e10 on a 32 x 32 patch
-# of the [64,128,128] sphere set, 40 x 40 harmonics)
-PLAIN_XU_PER_PM = 2.0
+# tensor-core FLOP per point*mode of the plain summation: 3 components x 4 real products x 3 products
+# of high and low parts, two operations each
+PLAIN_FLOP_PER_PM = 72.0
+# tensor-core FLOP per FLOP of an FP64 product: 36 digit products
+DIGIT_PRODUCTS = 36.0
 PLAIN_PATCH = 128          # plain-form sample: PLAIN_PATCH x PLAIN_PATCH points of one interior xy plane
 CPU_SLICE = 3              # the slice the plain and CPU samples lie in
 
@@ -322,6 +323,14 @@ def link_peaks(torch, nbytes=2 << 30):
 
 
 _PEAKS = {}
+
+
+def bf16_peak():
+    """Measured bf16 tensor rate in TFLOP/s (burst)."""
+    try:
+        return float(json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["bf16_tflops"])
+    except Exception:
+        return 1900.0
 
 
 def measured_peaks(ctx):
@@ -594,13 +603,12 @@ def run_ours(args):
                 "plain": {"value": plain_v, "unit": UNIT, "ms": plain_ms,
                           "sample": f"{P}x{P} xy patch in slice {CPU_SLICE}, {len(W32)} waves/point",
                           "sm_count": sm_count,
-                          "roofline": {"bound": "mufu (sin, cos)", "achieved": PLAIN_XU_PER_PM * plain_v,
-                                       "peak": pk["sincos_ops_per_s"], "unit": "MUFU ops/s",
-                                       "frac": PLAIN_XU_PER_PM * plain_v / pk["sincos_ops_per_s"],
-                                       "count": f"{PLAIN_XU_PER_PM} XU instructions per point*mode (ncu "
-                                                "smsp__inst_executed_pipe_xu on an xy patch: one sin and one "
-                                                "cos; ex2 is skipped where the in-plane k is real); peak: "
-                                                "sin / cos rate measured by scw_measure_peaks",
+                          "roofline": {"bound": "tensor (f16)", "achieved": PLAIN_FLOP_PER_PM * plain_v / 1e12,
+                                       "peak": bf16_peak(), "unit": "TFLOP/s",
+                                       "frac": PLAIN_FLOP_PER_PM * plain_v / 1e12 / bf16_peak(),
+                                       "count": "36 tensor multiply-adds per point*mode: 3 components x 4 real products "
+                                                "x 3 products of high and low parts; peak: measured bf16 burst rate",
+                                       "sincos_ops_per_s": pk["sincos_ops_per_s"],
                                        "ex2_ops_per_s": pk["ex2_ops_per_s"]}},
                 "parity": parity,
                 "cpu_baseline": {"value": cpu_v, "unit": UNIT, "cores": cores, "kind": "port",
@@ -792,11 +800,12 @@ def solve_leg(ctx):
             "evaluators_vs_fp64_on_this_solve": parity,
             "evaluation_on_the_full_grid": grid,
             "eigen": eig,
-            "roofline": {"bound": "fp64", "achieved": 8 * macs / t_gpu / 1e12, "peak": fp64_peak,
-                         "unit": "TFLOP/s", "frac": 8 * macs / t_gpu / 1e12 / fp64_peak,
-                         "note": "FP64 GEMM/LU operation count of the solve over its wall time (the FP32 eigen "
-                                 "stage, one CTA per slice, runs beside it uncounted); peak: FP64 FMA rate "
-                                 "measured on this GPU (scw_measure_peaks)"}}
+            "roofline": {"bound": "tensor (bf16)", "achieved": DIGIT_PRODUCTS * 8 * macs / t_gpu / 1e12, "peak": bf16_peak(),
+                         "unit": "TFLOP/s", "frac": DIGIT_PRODUCTS * 8 * macs / t_gpu / 1e12 / bf16_peak(),
+                         "fp64_tflops": 8 * macs / t_gpu / 1e12, "fp64_fma_peak_tflops": fp64_peak,
+                         "note": "FP64 product / LU operation count of the solve over its wall time (the FP32 eigen "
+                                 "stage is not counted), each as 36 bf16 digit products; peaks: measured bf16 burst rate, "
+                                 "FP64 FMA rate measured on this GPU (scw_measure_peaks)"}}
 
 
 def solved_leg(args):
@@ -909,10 +918,12 @@ def batch_leg(args):
                                  "harmonics_layers": shapes},
                       "points_modes_per_s": pm / t, "graph": info, "create_s": t_create,
                       "item_status": st.tolist(), "eigen": eig,
-                      "roofline": {"bound": "fp64", "achieved": 8 * macs / t / 1e12, "peak": fp64_peak,
-                                   "unit": "TFLOP/s", "frac": 8 * macs / t / 1e12 / fp64_peak,
-                                   "note": "FP64 GEMM/LU operation count of all solves over the launch time; "
-                                           "peak: FP64 FMA rate measured on this GPU"}}))
+                      "roofline": {"bound": "tensor (bf16)", "achieved": DIGIT_PRODUCTS * 8 * macs / t / 1e12,
+                                   "peak": bf16_peak(), "unit": "TFLOP/s",
+                                   "frac": DIGIT_PRODUCTS * 8 * macs / t / 1e12 / bf16_peak(),
+                                   "fp64_tflops": 8 * macs / t / 1e12, "fp64_fma_peak_tflops": fp64_peak,
+                                   "note": "FP64 product / LU operation count of all solves over the launch time, each as 36 "
+                                           "bf16 digit products; peaks: measured bf16 burst rate, FP64 FMA rate"}}))
 
 
 def warm_leg(args):
