@@ -505,11 +505,16 @@ scw_status scw_batch_get(scw_batch b, int i, double* x, double* gamma, float* fi
     const Item& it = b->items[i];
     SCW_ON_DEVICE(b->ctx->device);
     if (x) SCW_CUDA_TRY(cudaMemcpy(x, it.out.x, sizeof(double2) * 6 * it.sp.MF, cudaMemcpyDeviceToHost));
-    if (gamma)
-        SCW_CUDA_TRY(cudaMemcpy(gamma, it.out.gam, sizeof(double2) * (size_t)it.sp.Z * it.sp.n, cudaMemcpyDeviceToHost));
-    if (field_host)
-        SCW_CUDA_TRY(cudaMemcpy(field_host, it.field, sizeof(float) * 6 * (size_t)it.Nx * it.Ny * it.Nz,
-                                cudaMemcpyDeviceToHost));
+    if (gamma) {
+        const size_t bytes = sizeof(double2) * (size_t)it.sp.Z * it.sp.n;
+        scw::touch_pages(gamma, bytes);
+        SCW_CUDA_TRY(cudaMemcpy(gamma, it.out.gam, bytes, cudaMemcpyDeviceToHost));
+    }
+    if (field_host) {
+        const size_t bytes = sizeof(float) * 6 * (size_t)it.Nx * it.Ny * it.Nz;
+        scw::touch_pages(field_host, bytes);
+        SCW_CUDA_TRY(cudaMemcpy(field_host, it.field, bytes, cudaMemcpyDeviceToHost));
+    }
     if (field_device) *field_device = it.field;
     return SCW_OK;
 }

