@@ -520,9 +520,12 @@ static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_d
             };
             scw_status ls;
             auto shapes = [&](auto nk) -> scw_status {
-                // rows per warp: 8 for one or two planes, 4 beyond; half as many in shape 1
+                // rows per warp: 8 for one or two planes, 4 beyond; half as many in shape 1 and where that leaves SMs
+                // without a CTA (104 harmonics, 5 groups, 60 CTAs: 5.7 -> 4.4 us; 126 harmonics, 15 groups, 180
+                // CTAs: 5.6 as it is, 6.0 with half)
                 constexpr int NK = decltype(nk)::value, RW = NK <= 2 ? 8 : 4;
-                if (s->ctr_shape == 0) return launch(sep_contract_kernel<NK, RW>, RW, CtrCfg<RW, NK>::kSmem);
+                const dim3 full = grid_for(RW);
+                if (s->ctr_shape == 0 && (int)(full.x * full.y) >= ctx->sm_count) return launch(sep_contract_kernel<NK, RW>, RW, CtrCfg<RW, NK>::kSmem);
                 return launch(sep_contract_kernel<NK, RW / 2>, RW / 2, CtrCfg<RW / 2, NK>::kSmem);
             };
             switch (nks) {
