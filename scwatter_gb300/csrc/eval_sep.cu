@@ -4,8 +4,8 @@
 // grid and kz per eigenmode j (sCWatter.cpp:904-952), so
 //     E_c(x, y, z) = sum_a e^{i kx_a x} sum_b e^{i ky_b y} C_c(a, b; z),
 //     C_c(p; z)   = sum_j Qdn_c(p, j) e^{i kzdn_j (z - z_l)} + sum_j Qup_c(p, j) e^{i kzup_j (z - z_{l+1})}.
-// Stage 1 (HBM-bound): C for every evaluated z-plane (sep_phase_kernel + sep_contract_kernel;
-//   sep_exterior_kernel for the incident/reflected and transmitted regions).
+// Stage 1 (HBM-bound): C for every evaluated z-plane (sep_prep_kernel: phases, and the planes of the
+//   incident/reflected and transmitted regions; sep_contract_kernel: the others).
 // Stage 2: T_c(row, a) = sum_b e^{i ky_b y_row} C_c(a, b; z_row) (sep_rows_kernel), then the
 //   output GEMM E_c(row, x) = sum_a T_c(row, a) e^{i kx_a x}: FP32 SIMT (sep_synth_kernel) or
 //   tcgen05 3xTF32 / split-BF16 (eval_sep_tc.cu).
@@ -37,6 +37,8 @@ __device__ __forceinline__ float2 phase_fp64(double kr, double ki, double dz) {
     return make_float2(m * c, m * s);
 }
 
+constexpr int kPrepThreads = 128;
+
 // Phase table of one group of planes, Phi[g][h][j][kk] (h = 0, 1; kk < nks; zero past g.nk):
 //   two-half sets: h = 0: exp(i kz_dn_j (z_kk - z_l)), h = 1: exp(i kz_up_j (z_kk - z_{l+1}));
 //   paired sets (beta != null): the mode amplitudes folded in, in FP64,
@@ -44,14 +46,13 @@ __device__ __forceinline__ float2 phase_fp64(double kr, double ki, double dz) {
 //     h = 1 (rows Ez):     beta_dn_j exp(i kz_dn_j (z - z_l)) - beta_up_j exp(i kz_up_j (z - z_{l+1}))
 // One thread per mode (and half, of a two-half set) and plane, planes fastest (consecutive stores): with one
 // thread per mode looping over the planes, the chain of FP64 phases took 20 us for 200 modes.
-__global__ void sep_phase_kernel(const __grid_constant__ SepDesc desc, int off_z, const double2* __restrict__ kz, const double2* __restrict__ beta,
-                                 const double* __restrict__ zb, int J, int nks, float2* __restrict__ Phi) {
-    const PGroup& g = reinterpret_cast<const PGroup*>(desc.base())[blockIdx.y];
-    const float* zlist = reinterpret_cast<const float*>(desc.base() + off_z);
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void phase_block(const PGroup& g, const float* zlist, int block, int group,
+                                            const double2* __restrict__ kz, const double2* __restrict__ beta,
+                                            const double* __restrict__ zb, int J, int nks, float2* __restrict__ Phi) {
+    const int e = block * kPrepThreads + threadIdx.x;
     const int j = e / nks, kk = e - j * nks;
     const int l = g.region - 1;
-    float2* out = Phi + (long long)blockIdx.y * 2 * J * nks + e;
+    float2* out = Phi + (long long)group * 2 * J * nks + e;
     const bool live = kk < g.nk;
     if (!beta) {
         // two-half set: j < 2 J runs over (half, mode)
@@ -212,14 +213,13 @@ sep_contract_kernel(const __grid_constant__ SepDesc desc, const float2* __restri
 // Exterior regions: region 0 = incident (referenced at the origin) + reflected (at z_0),
 // last region = transmitted (at z_Z).  One thread per (z entry, p), FP64; the phases serve all three
 // components.
-__global__ void sep_exterior_kernel(const __grid_constant__ SepDesc desc, int off_e, int n_ext, int off_z,
-                                    const double2* __restrict__ xd, int MF, double z0, double zZ,
-                                    float2* __restrict__ C) {
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void exterior_block(const int2* ext, int n_ext, const float* zlist, int block,
+                                               const double2* __restrict__ xd, int MF, double z0, double zZ,
+                                               float2* __restrict__ C) {
+    const long long idx = (long long)block * kPrepThreads + threadIdx.x;
     if (idx >= (long long)n_ext * MF) return;
     const int e = (int)(idx / MF), p = (int)(idx % MF);
-    const float* zlist = reinterpret_cast<const float*>(desc.base() + off_z);
-    const int2 ent = reinterpret_cast<const int2*>(desc.base() + off_e)[e];     // (zi, 0 = top exterior / 1 = bottom exterior)
+    const int2 ent = ext[e];     // (zi, 0 = top exterior / 1 = bottom exterior)
     const double z = (double)zlist[ent.x];
     // xd layout: inc[3][MF], refl[3][MF], trans[3][MF], kz_inc[MF], kz_refl[MF], kz_trans[MF]
     const double2* kzi = xd + 9 * MF;
@@ -239,7 +239,7 @@ __global__ void sep_exterior_kernel(const __grid_constant__ SepDesc desc, int of
     }
 }
 
-// The two phase tables of an evaluation in one launch (block row 0 or 1): tab[m][i] = exp(i k_m x_i),
+// A phase table of an evaluation: tab[m][i] = exp(i k_m x_i),
 // x_i = s + d * i in float (one rounding per operation)
 struct TableArgs {
     const double* k;
@@ -247,13 +247,49 @@ struct TableArgs {
     float s, d;
     float2* tab;
 };
-__global__ void sep_table_kernel(TableArgs t0, TableArgs t1) {
-    const TableArgs t = blockIdx.y == 0 ? t0 : t1;
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void table_block(const TableArgs& t, int block) {
+    const long long idx = (long long)block * kPrepThreads + threadIdx.x;
     if (idx >= (long long)t.M * t.N) return;
     const int m = (int)(idx / t.N), i = (int)(idx % t.N);
     const float x = __fadd_rn(t.s, __fmul_rn(t.d, (float)i));
     t.tab[idx] = phase_fp64(t.k[m], 0.0, (double)x);
+}
+
+// Everything that needs no contraction, in one launch: the groups' phase tables, the exterior planes of C, the two
+// tables of stage 2.  They are independent, short and bound by FP64, and a small evaluation is bound by its
+// launches (about 4 us of the host's time each).  In three launches / in one: 5 slices of 8x13 harmonics on
+// 65x71x33 points 31.8 / 27.7 us; 20 of 20x20 on 128x128x64 82.3 / 79.4 us; 3 of 20x20 on three 256x256 planes
+// 161 / 144 us.
+struct PrepArgs {
+    SepDesc desc;
+    int off_e, off_z;
+    int phase_blocks, groups, ext_blocks, t0_blocks;     // phase_blocks per group
+    const double2 *kz, *beta, *xd;
+    const double* zb;
+    int J, nks, n_ext, MF;
+    double z0, zZ;
+    float2 *Phi, *C;
+    TableArgs t0, t1;
+};
+static_assert(sizeof(PrepArgs) <= 4096, "kernel parameters");
+__global__ void __launch_bounds__(kPrepThreads) sep_prep_kernel(const __grid_constant__ PrepArgs a) {
+    const char* d = a.desc.base();
+    const float* zlist = reinterpret_cast<const float*>(d + a.off_z);
+    int b = blockIdx.x;
+    if (b < a.phase_blocks * a.groups) {
+        const int group = b / a.phase_blocks;
+        phase_block(reinterpret_cast<const PGroup*>(d)[group], zlist, b - group * a.phase_blocks, group, a.kz, a.beta, a.zb, a.J,
+                    a.nks, a.Phi);
+        return;
+    }
+    b -= a.phase_blocks * a.groups;
+    if (b < a.ext_blocks) {
+        exterior_block(reinterpret_cast<const int2*>(d + a.off_e), a.n_ext, zlist, b, a.xd, a.MF, a.z0, a.zZ, a.C);
+        return;
+    }
+    b -= a.ext_blocks;
+    if (b < a.t0_blocks) table_block(a.t0, b);
+    else table_block(a.t1, b - a.t0_blocks);
 }
 
 // Stage 2a: T[r][c][m] = sum_n R(r, n) * C[zi(r)][c][p(m, n)]
@@ -482,8 +518,8 @@ void sep_eval_desc(const SepEvalPlan& p, char* h) {
     std::memcpy(h + p.off_z, p.zlist.data(), p.zlist.size() * sizeof(float));
 }
 
-// Stage 1 for the plan's z-values: fills C [nz][3][MF]; descriptors already on the device, or (d_desc null) with
-// the launches.
+// Stage 1 for the plan's z-values: fills C [nz][3][MF], and stage 2's tables behind C and T; descriptors already
+// on the device, or (d_desc null) with the launches.
 static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_desc, float2* dC, char* cursor) {
     scw_ctx ctx = s->ctx;
     const int MF = s->MF, J = s->Jp;          // device row stride (even)
@@ -493,21 +529,54 @@ static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_d
     SepDesc desc;
     desc.dev = d_desc;
     if (!d_desc) sep_eval_desc(p, desc.here);
-    const int off_e = (int)p.off_e, off_z = (int)p.off_z;
+    PrepArgs a{};
+    a.desc = desc;
+    a.off_e = (int)p.off_e;
+    a.off_z = (int)p.off_z;
+    a.kz = s->dKz;
+    a.beta = s->halves == 1 ? s->dBeta : nullptr;
+    a.zb = s->dzb;
+    a.J = J;
+    a.nks = max_nk;                            // a contraction kernel per plane count: 5 planes cost 5, not 8
+    a.Phi = (float2*)cursor;
+    if (!groups.empty() && J > 0) {
+        a.groups = (int)groups.size();
+        // one thread per (half, mode, plane) for a two-half set, per (mode, plane) for a paired set
+        a.phase_blocks = ((s->halves == 1 ? J : 2 * J) * max_nk + kPrepThreads - 1) / kPrepThreads;
+    }
+    a.n_ext = (int)ext.size();
+    a.ext_blocks = (int)(((long long)ext.size() * MF + kPrepThreads - 1) / kPrepThreads);
+    a.xd = s->dExt;
+    a.MF = MF;
+    a.z0 = s->zb[0];
+    a.zZ = s->zb[s->Z];
+    a.C = dC;
+    // stage 2's tables: F along the columns, R along the rows (xz and yz planes: at the plane's coordinate)
+    float2* tabA = (float2*)((char*)dC + p.c_bytes + p.t_bytes);
+    float2* tabB = (float2*)((char*)tabA + p.tab_bytes);
+    if (p.kind == 0) {
+        a.t0 = {s->dkx, s->M0, p.Na, p.a0, p.da, tabA};
+        a.t1 = {s->dky, s->M1, p.Nb, p.b0, p.db, tabB};
+    } else if (p.kind == 1) {
+        a.t0 = {s->dkx, s->M0, p.Na, p.a0, p.da, tabA};
+        a.t1 = {s->dky, s->M1, 1, p.c, 0.f, tabB};
+    } else {
+        a.t0 = {s->dky, s->M1, p.Na, p.a0, p.da, tabA};
+        a.t1 = {s->dkx, s->M0, 1, p.c, 0.f, tabB};
+    }
+    auto blocks_of = [](const TableArgs& t) { return (int)(((long long)t.M * t.N + kPrepThreads - 1) / kPrepThreads); };
+    a.t0_blocks = blocks_of(a.t0);
+    {
+        LaunchTimer lt(ctx, "sep_prep_kernel");
+        sep_prep_kernel<<<(unsigned)(a.phase_blocks * a.groups + a.ext_blocks + a.t0_blocks + blocks_of(a.t1)), kPrepThreads, 0,
+                          ctx->stream>>>(a);
+        SCW_CUDA_TRY(cudaGetLastError());
+        ctx->launches++;
+    }
     if (!groups.empty()) {
         if (J > 0) {
-            const int nks = max_nk;            // a kernel per plane count: 5 planes cost 5, not 8
-            float2* dPhi = (float2*)cursor;
-            cursor += align256(groups.size() * 2 * (size_t)J * nks * sizeof(float2));
-            // one thread per (half, mode, plane) for a two-half set, per (mode, plane) for a paired set
-            dim3 gp(((s->halves == 1 ? J : 2 * J) * nks + 127) / 128, (unsigned)groups.size());
-            {
-                LaunchTimer lt(ctx, "sep_phase_kernel");
-                sep_phase_kernel<<<gp, 128, 0, ctx->stream>>>(desc, off_z, s->dKz, s->halves == 1 ? s->dBeta : nullptr,
-                                                              s->dzb, J, nks, dPhi);
-            }
-            SCW_CUDA_TRY(cudaGetLastError());
-            ctx->launches++;
+            const int nks = max_nk;
+            float2* dPhi = a.Phi;
             // per component c, ceil(MF / (warps x rows per warp)) CTAs
             auto grid_for = [&](int rw) {
                 return dim3(3 * ((MF + kCtrWarps * rw - 1) / (kCtrWarps * rw)), (unsigned)groups.size());
@@ -549,23 +618,6 @@ static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_d
                                                  ctx->stream));
         }
     }
-    if (!ext.empty()) {
-        const long long n = (long long)ext.size() * MF;
-        LaunchTimer lt(ctx, "sep_exterior_kernel");
-        sep_exterior_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(desc, off_e, (int)ext.size(), off_z, s->dExt, MF,
-                                                                                 s->zb[0], s->zb[s->Z], dC);
-        SCW_CUDA_TRY(cudaGetLastError());
-        ctx->launches++;
-    }
-    return SCW_OK;
-}
-
-static scw_status launch_tables(scw_ctx ctx, const TableArgs& a, const TableArgs& b) {
-    const long long n = std::max((long long)a.M * a.N, (long long)b.M * b.N);
-    LaunchTimer lt(ctx, "sep_table_kernel");
-    sep_table_kernel<<<dim3((unsigned)((n + 127) / 128), 2), 128, 0, ctx->stream>>>(a, b);
-    SCW_CUDA_TRY(cudaGetLastError());
-    ctx->launches++;
     return SCW_OK;
 }
 
@@ -683,11 +735,9 @@ static scw_status stage2_record(scw_sep s, const SepEvalPlan& p, char* scratch, 
     float2* tabB = (float2*)cursor;
     cursor += p.tab_bytes;
     scw_status st = SCW_OK;
-    const int nrows = p.nrows, ncols = p.ncols, Mk = p.Mk, Na = p.Na, Nb = p.Nb, Nz = p.Nz;
+    const int nrows = p.nrows, ncols = p.ncols, Mk = p.Mk, Nb = p.Nb, Nz = p.Nz;
     if (p.kind == 0) {
         // F = Ex table [a][x]; R = Ey table [b][y]
-        if ((st = launch_tables(ctx, {s->dkx, M0, Na, p.a0, p.da, tabA}, {s->dky, M1, Nb, p.b0, p.db, tabB})) != SCW_OK)
-            return st;
         {
             const size_t smem = (size_t)(rows_phase_off(M0, M1) + kRowsBlk * M1) * sizeof(float2);
             SCW_CUDA_TRY(cudaFuncSetAttribute(sep_rows_volume_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -701,12 +751,10 @@ static scw_status stage2_record(scw_sep s, const SepEvalPlan& p, char* scratch, 
         return sep_synth(ctx, dT, tabA, nrows, ncols, Mk, dE, p.method);
     } else if (p.kind == 1) {
         // xz plane at y = c: R = Ey(c) [b]; F = Ex table [a][x]
-        if ((st = launch_tables(ctx, {s->dkx, M0, Na, p.a0, p.da, tabA}, {s->dky, M1, 1, p.c, 0.f, tabB})) != SCW_OK) return st;
         if ((st = launch_rows(ctx, dC, tabB, 1, 1, 1, 0, nrows, 0, M0, M1, dT)) != SCW_OK) return st;
         return sep_synth(ctx, dT, tabA, nrows, ncols, Mk, dE, p.method);
     } else {
         // yz plane at x = c: R = Ex(c) [a]; F = Ey table [b][y]
-        if ((st = launch_tables(ctx, {s->dky, M1, Na, p.a0, p.da, tabA}, {s->dkx, M0, 1, p.c, 0.f, tabB})) != SCW_OK) return st;
         if ((st = launch_rows(ctx, dC, tabB, 1, 1, 1, 0, nrows, 1, M0, M1, dT)) != SCW_OK) return st;
         return sep_synth(ctx, dT, tabA, nrows, ncols, Mk, dE, p.method);
     }
