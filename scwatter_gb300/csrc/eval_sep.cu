@@ -144,6 +144,30 @@ sep_contract_kernel(const __grid_constant__ SepDesc desc, const float2* __restri
         }
         for (int j0 = 0; j0 < J; j0 += kCtrChunk) {
             const int nj = min(kCtrChunk, J - j0);
+            // lane iterations jp = lane + 32 it; the Q pairs of iteration it arrive through an
+            // S-deep cp.async ring (the slot refilled at iteration it is the one read at it - 1)
+            const int npair = nj / 2;
+            const int nit = lane < npair ? (npair - lane + 31) / 32 : 0;
+            auto start_ring = [&]() {
+#pragma unroll
+                for (int st = 0; st < S - 1; st++) {
+                    if (st < nit) {
+                        const int jp = lane + 32 * st;
+#pragma unroll
+                        for (int r = 0; r < RW; r++) cp_async16(qs + (st * RW + r) * 32, qrow[r] + j0 / 2 + jp);
+                    }
+                    cp_async_commit();
+                }
+            };
+            // The first chunk's ring starts before the phases are there: no kernel of the evaluation writes Q, and
+            // what did write it had ended before sep_prep_kernel let this one start (cp.async.cg reads L2).  In later
+            // chunks the ring waits for the staged phases: started ahead of them too, 3200 modes on 256 planes
+            // took 1823 us in place of 1805, 400 modes on 64 planes the same.
+            const bool first = half == 0 && j0 == 0;
+            if (first) {
+                start_ring();
+                chain_wait();
+            }
             __syncthreads();
             // consecutive threads fill consecutive pairs of one plane (conflict-free stores)
             for (int e = threadIdx.x; e < (nj / 2) * NK; e += blockDim.x) {
@@ -153,19 +177,7 @@ sep_contract_kernel(const __grid_constant__ SepDesc desc, const float2* __restri
                 ph[kk][jp] = make_float4(a.x, a.y, b.x, b.y);
             }
             __syncthreads();
-            // lane iterations jp = lane + 32 it; the Q pairs of iteration it arrive through an
-            // S-deep cp.async ring (the slot refilled at iteration it is the one read at it - 1)
-            const int npair = nj / 2;
-            const int nit = lane < npair ? (npair - lane + 31) / 32 : 0;
-#pragma unroll
-            for (int st = 0; st < S - 1; st++) {
-                if (st < nit) {
-                    const int jp = lane + 32 * st;
-#pragma unroll
-                    for (int r = 0; r < RW; r++) cp_async16(qs + (st * RW + r) * 32, qrow[r] + j0 / 2 + jp);
-                }
-                cp_async_commit();
-            }
+            if (!first) start_ring();
             for (int it = 0; it < nit; it++) {
                 const int nxt = it + S - 1;
                 if (nxt < nit) {
@@ -273,6 +285,8 @@ struct PrepArgs {
 };
 static_assert(sizeof(PrepArgs) <= 4096, "kernel parameters");
 __global__ void __launch_bounds__(kPrepThreads) sep_prep_kernel(const __grid_constant__ PrepArgs a) {
+    chain_wait();
+    chain_trigger();
     const char* d = a.desc.base();
     const float* zlist = reinterpret_cast<const float*>(d + a.off_z);
     int b = blockIdx.x;
@@ -298,6 +312,8 @@ __global__ void __launch_bounds__(kPrepThreads) sep_prep_kernel(const __grid_con
 // R(r, n) = Rtab[n * rld + r % rmod];  zi(r) = zoff + r / rdiv
 __global__ void sep_rows_kernel(const float2* __restrict__ C, const float2* __restrict__ Rtab, int rld, int rmod,
                                 int rdiv, int zoff, int nrows, int ctype, int M0, int M1, float2* __restrict__ T) {
+    chain_wait();
+    chain_trigger();
     const int Mk = ctype == 0 ? M0 : M1;
     const int Mn = ctype == 0 ? M1 : M0;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -340,15 +356,17 @@ sep_rows_volume_kernel(const float2* __restrict__ C, const float2* __restrict__ 
     const int j0 = blockIdx.x * kRowsBlk;
     const int MF = M0 * M1;
     const float2* Ck = C + (long long)k * 3 * MF;
+    chain_wait();
+    chain_trigger();
+    for (int e = threadIdx.x; e < kRowsBlk * M1; e += blockDim.x) {
+        const int b = e / kRowsBlk, r = e % kRowsBlk;
+        sR[e] = (j0 + r < Ny) ? tabY[(long long)b * Ny + j0 + r] : make_float2(0.f, 0.f);
+    }
     for (int e = threadIdx.x; e < 3 * MF; e += blockDim.x) {
         const int c = e / MF, p = e % MF, a = p / M1, b = p % M1;
         sC[(c * M1 + b) * M0 + a] = Ck[e];
     }
     if (threadIdx.x < 2) sC[3 * MF + threadIdx.x] = make_float2(0.f, 0.f);
-    for (int e = threadIdx.x; e < kRowsBlk * M1; e += blockDim.x) {
-        const int b = e / kRowsBlk, r = e % kRowsBlk;
-        sR[e] = (j0 + r < Ny) ? tabY[(long long)b * Ny + j0 + r] : make_float2(0.f, 0.f);
-    }
     __syncthreads();
     const int ncol = 3 * M0;
     const int npair = (ncol + 1) / 2;
@@ -405,13 +423,14 @@ sep_synth_kernel(const float2* __restrict__ T, const float2* __restrict__ F, int
     float2* sT = smem;                                  // [kSynRows][3][Mk]
     float2* sF = smem + kSynRows * 3 * kSynMaxK;        // [Mk][kSynCols]
     const int r0 = blockIdx.y * kSynRows, c0 = blockIdx.x * kSynCols;
-    for (int e = threadIdx.x; e < kSynRows * 3 * Mk; e += blockDim.x) {
-        const int rr = e / (3 * Mk);
-        sT[e] = (r0 + rr < nrows) ? T[(long long)r0 * 3 * Mk + e] : make_float2(0.f, 0.f);
-    }
+    chain_wait();
     for (int e = threadIdx.x; e < Mk * kSynCols; e += blockDim.x) {
         const int m = e / kSynCols, cc = e % kSynCols;
         sF[e] = (c0 + cc < ncols) ? F[(long long)m * ncols + c0 + cc] : make_float2(0.f, 0.f);
+    }
+    for (int e = threadIdx.x; e < kSynRows * 3 * Mk; e += blockDim.x) {
+        const int rr = e / (3 * Mk);
+        sT[e] = (r0 + rr < nrows) ? T[(long long)r0 * 3 * Mk + e] : make_float2(0.f, 0.f);
     }
     __syncthreads();
     const int tr = threadIdx.x / 16, tc = threadIdx.x % 16;
@@ -520,7 +539,8 @@ void sep_eval_desc(const SepEvalPlan& p, char* h) {
 
 // Stage 1 for the plan's z-values: fills C [nz][3][MF], and stage 2's tables behind C and T; descriptors already
 // on the device, or (d_desc null) with the launches.
-static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_desc, float2* dC, char* cursor) {
+static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_desc, float2* dC, char* cursor,
+                                bool chained) {
     scw_ctx ctx = s->ctx;
     const int MF = s->MF, J = s->Jp;          // device row stride (even)
     const auto& groups = p.groups;
@@ -568,9 +588,8 @@ static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_d
     a.t0_blocks = blocks_of(a.t0);
     {
         LaunchTimer lt(ctx, "sep_prep_kernel");
-        sep_prep_kernel<<<(unsigned)(a.phase_blocks * a.groups + a.ext_blocks + a.t0_blocks + blocks_of(a.t1)), kPrepThreads, 0,
-                          ctx->stream>>>(a);
-        SCW_CUDA_TRY(cudaGetLastError());
+        const int blocks = a.phase_blocks * a.groups + a.ext_blocks + a.t0_blocks + blocks_of(a.t1);
+        SCW_CUDA_TRY(launch_chained(chained, ctx->stream, dim3((unsigned)blocks), kPrepThreads, 0, sep_prep_kernel, a));
         ctx->launches++;
     }
     if (!groups.empty()) {
@@ -584,7 +603,8 @@ static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_d
             LaunchTimer lt(ctx, "sep_contract_kernel");
             auto launch = [&](auto kernel, int rw, size_t smem) -> scw_status {
                 SCW_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-                kernel<<<grid_for(rw), kCtrWarps * 32, smem, ctx->stream>>>(desc, dPhi, s->dQ, MF, J, s->halves, dC);
+                SCW_CUDA_TRY(launch_chained(chained, ctx->stream, grid_for(rw), kCtrWarps * 32, smem, kernel, desc, dPhi, s->dQ,
+                                            MF, J, s->halves, dC));
                 return SCW_OK;
             };
             scw_status ls;
@@ -622,24 +642,23 @@ static scw_status stage1_record(scw_sep s, const SepEvalPlan& p, const char* d_d
 }
 
 static scw_status launch_rows(scw_ctx ctx, const float2* C, const float2* Rtab, int rld, int rmod, int rdiv, int zoff,
-                              int nrows, int ctype, int M0, int M1, float2* T) {
+                              int nrows, int ctype, int M0, int M1, float2* T, bool chained) {
     const int Mk = ctype == 0 ? M0 : M1;
     const long long n = (long long)nrows * 3 * Mk;
     LaunchTimer lt(ctx, "sep_rows_kernel");
-    sep_rows_kernel<<<(unsigned)((n + 255) / 256), 256, 0, ctx->stream>>>(C, Rtab, rld, rmod, rdiv, zoff, nrows, ctype,
-                                                                          M0, M1, T);
-    SCW_CUDA_TRY(cudaGetLastError());
+    SCW_CUDA_TRY(launch_chained(chained, ctx->stream, dim3((unsigned)((n + 255) / 256)), 256, 0, sep_rows_kernel, C, Rtab, rld,
+                                rmod, rdiv, zoff, nrows, ctype, M0, M1, T));
     ctx->launches++;
     return SCW_OK;
 }
 
 scw_status sep_synth(scw_ctx ctx, const float2* T, const float2* F, int nrows, int ncols, int Mk, float* out,
-                     int method) {
+                     int method, bool chained) {
     if (method == SCW_SEP_TF32X3 || method == SCW_SEP_BF16X3) {
         // shapes whose operands do not fit the tensor-core kernel's shared and tensor memory (more
         // than 48 harmonics along the synthesis axis for 3xTF32, 80 for split-BF16) run the FP32
         // SIMT GEMM below, which is at least as accurate
-        scw_status st = sep_synth_tc(ctx, T, F, nrows, ncols, Mk, out, method);
+        scw_status st = sep_synth_tc(ctx, T, F, nrows, ncols, Mk, out, method, chained);
         if (st != SCW_ERR_UNSUPPORTED) return st;
     }
     if (Mk > kSynMaxK) return fail(SCW_ERR_UNSUPPORTED, "more than 64 harmonics along the synthesis axis");
@@ -651,8 +670,7 @@ scw_status sep_synth(scw_ctx ctx, const float2* T, const float2* F, int nrows, i
     }
     dim3 grid((ncols + kSynCols - 1) / kSynCols, (nrows + kSynRows - 1) / kSynRows);
     LaunchTimer lt(ctx, "sep_synth_kernel");
-    sep_synth_kernel<<<grid, 256, smem, ctx->stream>>>(T, F, nrows, ncols, Mk, out);
-    SCW_CUDA_TRY(cudaGetLastError());
+    SCW_CUDA_TRY(launch_chained(chained, ctx->stream, grid, 256, smem, sep_synth_kernel, T, F, nrows, ncols, Mk, out));
     ctx->launches++;
     return SCW_OK;
 }
@@ -722,7 +740,7 @@ scw_status sep_eval_slab(scw_sep s, float x0, float y0, float z0, float dx, floa
 
 // Stage 2 of one planned evaluation (tables, row products, output GEMM) on the context stream;
 // scratch laid out as in sep_eval_record (C, T, two tables, then stage 1's work).
-static scw_status stage2_record(scw_sep s, const SepEvalPlan& p, char* scratch, float* dE) {
+static scw_status stage2_record(scw_sep s, const SepEvalPlan& p, char* scratch, float* dE, bool chained) {
     scw_ctx ctx = s->ctx;
     const int M0 = s->M0, M1 = s->M1;
     char* cursor = scratch;
@@ -744,35 +762,34 @@ static scw_status stage2_record(scw_sep s, const SepEvalPlan& p, char* scratch, 
                                               (int)smem));
             dim3 grid((Nb + kRowsBlk - 1) / kRowsBlk, Nz);
             LaunchTimer lt(ctx, "sep_rows_volume_kernel");
-            sep_rows_volume_kernel<<<grid, 256, smem, ctx->stream>>>(dC, tabB, Nb, M0, M1, dT);
-            SCW_CUDA_TRY(cudaGetLastError());
+            SCW_CUDA_TRY(launch_chained(chained, ctx->stream, grid, 256, smem, sep_rows_volume_kernel, dC, tabB, Nb, M0, M1, dT));
             ctx->launches++;
         }
-        return sep_synth(ctx, dT, tabA, nrows, ncols, Mk, dE, p.method);
+        return sep_synth(ctx, dT, tabA, nrows, ncols, Mk, dE, p.method, chained);
     } else if (p.kind == 1) {
         // xz plane at y = c: R = Ey(c) [b]; F = Ex table [a][x]
-        if ((st = launch_rows(ctx, dC, tabB, 1, 1, 1, 0, nrows, 0, M0, M1, dT)) != SCW_OK) return st;
-        return sep_synth(ctx, dT, tabA, nrows, ncols, Mk, dE, p.method);
+        if ((st = launch_rows(ctx, dC, tabB, 1, 1, 1, 0, nrows, 0, M0, M1, dT, chained)) != SCW_OK) return st;
+        return sep_synth(ctx, dT, tabA, nrows, ncols, Mk, dE, p.method, chained);
     } else {
         // yz plane at x = c: R = Ex(c) [a]; F = Ey table [b][y]
-        if ((st = launch_rows(ctx, dC, tabB, 1, 1, 1, 0, nrows, 1, M0, M1, dT)) != SCW_OK) return st;
-        return sep_synth(ctx, dT, tabA, nrows, ncols, Mk, dE, p.method);
+        if ((st = launch_rows(ctx, dC, tabB, 1, 1, 1, 0, nrows, 1, M0, M1, dT, chained)) != SCW_OK) return st;
+        return sep_synth(ctx, dT, tabA, nrows, ncols, Mk, dE, p.method, chained);
     }
 }
 
 // Launches of one planned evaluation (no allocation, no host synchronisation).
-scw_status sep_eval_record(scw_sep s, const SepEvalPlan& p, const char* d_desc, char* scratch, float* dE) {
+scw_status sep_eval_record(scw_sep s, const SepEvalPlan& p, const char* d_desc, char* scratch, float* dE, bool chained) {
     const size_t head = p.c_bytes + p.t_bytes + 2 * p.tab_bytes;
-    scw_status st = stage1_record(s, p, d_desc, (float2*)scratch, scratch + head);
+    scw_status st = stage1_record(s, p, d_desc, (float2*)scratch, scratch + head, chained);
     if (st != SCW_OK) return st;
-    return stage2_record(s, p, scratch, dE);
+    return stage2_record(s, p, scratch, dE, chained);
 }
 
 // The plan's launches with the context's scratch (reserved): the descriptors go with them, or up first (pinned
 // staging, guarded by the context's event) where there are too many.
 static scw_status sep_eval_launch(scw_sep s, const SepEvalPlan& p, float* dE) {
     scw_ctx ctx = s->ctx;
-    if (p.desc_bytes <= kDescInline) return sep_eval_record(s, p, nullptr, (char*)ctx->sep_scratch.ptr, dE);
+    if (p.desc_bytes <= kDescInline) return sep_eval_record(s, p, nullptr, (char*)ctx->sep_scratch.ptr, dE, true);
     scw_status st;
     SCW_CUDA_TRY(cudaEventSynchronize(ctx->desc_done));
     if ((st = ctx->host_desc.reserve(p.desc_bytes)) != SCW_OK) return st;
@@ -1038,14 +1055,14 @@ static scw_status sep_eval_slab_pipelined(scw_sep s, float x0, float y0, float z
         char* buf = (char*)ctx->sep_scratch.ptr + (size_t)(c & 1) * scratch;
         if (c >= 2) SCW_CUDA_TRY(cudaStreamWaitEvent(main_stream, ev2[c - 2], 0));
         const size_t head = p.c_bytes + p.t_bytes + 2 * p.tab_bytes;
-        if ((st = stage1_record(s, p, (const char*)ctx->desc.ptr + desc_off[c], (float2*)buf, buf + head)) != SCW_OK)
+        if ((st = stage1_record(s, p, (const char*)ctx->desc.ptr + desc_off[c], (float2*)buf, buf + head, false)) != SCW_OK)
             return st;
         SCW_CUDA_TRY(cudaEventRecord(ev1[c], main_stream));
         SCW_CUDA_TRY(cudaStreamWaitEvent(s->hi_stream, ev1[c], 0));
         // stage 2 on the high-priority stream, its output GEMM on half the SMs
         ctx->stream = s->hi_stream;
         ctx->synth_ctas = std::max(1, ctx->sm_count / std::max(1, s->pipe_synth_div));
-        st = stage2_record(s, p, buf, dE + (size_t)(kb[c] - k_begin) * plane_floats);
+        st = stage2_record(s, p, buf, dE + (size_t)(kb[c] - k_begin) * plane_floats, false);
         ctx->stream = main_stream;
         ctx->synth_ctas = 0;
         if (st != SCW_OK) return st;

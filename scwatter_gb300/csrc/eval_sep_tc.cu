@@ -246,6 +246,7 @@ synth_tc_kernel(const float2* __restrict__ T, const float2* __restrict__ F, int 
     }
     __syncthreads();
     const uint32_t tmem = *tmem_slot;
+    chain_wait();
     // A: the phase tables of the CTA's x tiles into TMEM, lane x = x0 + 128 t + 32 w + lane (warps
     // 0-3), 8 columns per store: tf32 one element per column, bf16 elements 2c (low half) and 2c + 1
     // per column c
@@ -575,7 +576,7 @@ synth_tc_kernel(const float2* __restrict__ T, const float2* __restrict__ F, int 
 }  // namespace tc
 
 scw_status sep_synth_tc(scw_ctx ctx, const float2* T, const float2* F, int nrows, int ncols, int Mk, float* out,
-                        int method) {
+                        int method, bool chained) {
     const int kind = method == SCW_SEP_TF32X3 ? 0 : 1;
     const int EB = kind == 0 ? 4 : 2;
     const int kalign = kind == 0 ? 8 : 16;                  // K per MMA instruction
@@ -607,7 +608,8 @@ scw_status sep_synth_tc(scw_ctx ctx, const float2* T, const float2* F, int nrows
     LaunchTimer lt(ctx, kind == 0 ? "synth_tc_kernel<tf32x3>" : "synth_tc_kernel<bf16x3>");
     auto launch = [&](auto kernel) -> scw_status {
         SCW_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kernel<<<grid, tc::kWsThreads, smem, ctx->stream>>>(T, F, nrows, ncols, Mk, Kp, srows, out, ctx->tc_err);
+        SCW_CUDA_TRY(launch_chained(chained, ctx->stream, grid, tc::kWsThreads, smem, kernel, T, F, nrows, ncols, Mk, Kp,
+                                    srows, out, ctx->tc_err));
         return SCW_OK;
     };
     scw_status ls;

@@ -51,3 +51,35 @@ def test_volume_in_slabs(sets, planes):
             s.eval_slab_device(*grid, 9, 5, k, min(planes, k + 20), part[k:].data_ptr(), method=sp.FP32)
         ctx.synchronize()
         assert torch.equal(whole, part)
+
+
+@pytest.mark.parametrize("method", ["FP32", "TF32X3", "BF16X3"])
+@pytest.mark.parametrize("n,planes,z0", [(1, 1, 0.1), (65, 33, -1.6), (300, 9, -1.4), (70, 12, 40.0), (70, 12, -60.0), (33, 40, -4.0)])
+def test_queued_evaluations(sets, n, planes, z0, method):
+    """Evaluations queued one behind the other (their kernels' ends and starts overlap; planes inside the sample,
+    outside only, both) equal the same ones with the stream drained in between."""
+    import torch
+    from scwatter_gb300 import separable as sp
+    ctx, both = sets
+    m = getattr(sp, method)
+    jobs = []
+    for s in both:
+        for shift in (0.0, 0.21):
+            jobs.append(lambda o, s=s, f=shift: s.eval_volume_device(-2.0 + f, -1.0, z0, 0.03, 0.2, 0.1, n, 5, planes, o, method=m))
+            for axis in (1, 2):
+                jobs.append(lambda o, s=s, f=shift, a=axis: s.eval_plane_device(a, -2.0, z0, f, 0.1, n, o, method=m))
+    size = max(planes * 5 * n, n * n) * 3
+    one = torch.zeros((len(jobs), size), dtype=torch.complex64, device="cuda")
+    for o, job in zip(one, jobs):
+        ctx.synchronize()
+        torch.cuda.synchronize()
+        job(o.data_ptr())
+    ctx.synchronize()
+    for _ in range(3):
+        queued = torch.zeros_like(one)
+        torch.cuda.synchronize()
+        for o, job in zip(queued, jobs):
+            job(o.data_ptr())
+        ctx.synchronize()
+        assert torch.equal(queued, one)
+    assert int((one != 0).sum()) > 0
