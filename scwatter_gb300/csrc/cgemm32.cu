@@ -18,6 +18,7 @@
 
 #include "scw_complex.cuh"
 #include "scw_dense.h"
+#include "scw_launch.h"
 
 namespace scw {
 namespace z {
@@ -54,6 +55,7 @@ struct CgArgs {
 template <int TM, int TN, int KS, bool CA, bool CB, bool SHORT>
 __global__ void __launch_bounds__(TM / 4 * (TN / 4) * KS, SHORT ? 3 : 2)
 cgemm_kernel(CgArgs p) {
+    chain_wait();
     constexpr int kX = TN / 4, kG = TM / 4 * kX;         // threads along a row, of a group
     constexpr int nA = TM * kCgK / kG, nB = TN * kCgK / kG;
     extern __shared__ __align__(16) unsigned char cg_smem[];
@@ -175,8 +177,7 @@ static scw_status cgemm_launch(cudaStream_t st, const CgArgs& p, bool ca, bool c
     auto kernel = ca ? (cb ? cgemm_kernel<TM, TN, KS, true, true, SHORT> : cgemm_kernel<TM, TN, KS, true, false, SHORT>)
                      : (cb ? cgemm_kernel<TM, TN, KS, false, true, SHORT> : cgemm_kernel<TM, TN, KS, false, false, SHORT>);
     if (smem > 48 * 1024) SCW_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, threads, smem, st>>>(p);
-    SCW_CUDA_TRY(cudaGetLastError());
+    SCW_CUDA_TRY(launch_chained(true, st, grid, threads, smem, kernel, p));
     return SCW_OK;
 }
 

@@ -20,6 +20,7 @@
 #include <cooperative_groups.h>
 
 #include "scw_dense.h"
+#include "scw_launch.h"
 #include "scw_complex.cuh"
 
 namespace scw {
@@ -283,6 +284,7 @@ template <int C>
 __global__ void __launch_bounds__(256)
 lu_apply_kernel(double2* __restrict__ A, int ncols, int lda, long long sA, int k0, int nb, const int* __restrict__ piv,
                 long long sP, const int* __restrict__ skip) {
+    chain_wait();
     if (skipped(skip, blockIdx.y)) return;
     A += sA * blockIdx.y;
     piv += sP * blockIdx.y;
@@ -386,6 +388,7 @@ template <int C>
 __global__ void __launch_bounds__(256)
 trsm_block_kernel(const double2* __restrict__ LU, int lda, long long sA, int k0, int nb, double2* __restrict__ B, int ldb,
                   long long sB, int nrhs, int upper, const int* __restrict__ skip) {
+    chain_wait();
     if (skipped(skip, blockIdx.y)) return;
     LU += sA * blockIdx.y;
     B += sB * blockIdx.y;
@@ -1150,12 +1153,13 @@ scw_status gemm(cudaStream_t st, int M, int N, int K, C alpha, const C* A, int l
 // work (16 000 operations per column of 32 rows) then takes 20 us on one SM; 8 where 32 would leave SMs idle.
 static bool few_columns(int cols, int batch) { return (long long)((cols + 31) / 32) * batch < 152; }
 
-static void trsm_block(cudaStream_t st, const double2* LU, int lda, long long sA, int k0, int nb, double2* B, int ldb, long long sB,
+static cudaError_t trsm_block(cudaStream_t st, const double2* LU, int lda, long long sA, int k0, int nb, double2* B, int ldb, long long sB,
                        int nrhs, int upper, int batch, const int* skip) {
     if (few_columns(nrhs, batch))
-        z::trsm_block_kernel<8><<<dim3((nrhs + 7) / 8, batch), 256, 0, st>>>(LU, lda, sA, k0, nb, B, ldb, sB, nrhs, upper, skip);
-    else
-        z::trsm_block_kernel<32><<<dim3((nrhs + 31) / 32, batch), 256, 0, st>>>(LU, lda, sA, k0, nb, B, ldb, sB, nrhs, upper, skip);
+        return launch_chained(true, st, dim3((nrhs + 7) / 8, batch), 256, 0, z::trsm_block_kernel<8>, LU, lda, sA, k0, nb, B, ldb,
+                              sB, nrhs, upper, skip);
+    return launch_chained(true, st, dim3((nrhs + 31) / 32, batch), 256, 0, z::trsm_block_kernel<32>, LU, lda, sA, k0, nb, B, ldb,
+                          sB, nrhs, upper, skip);
 }
 
 scw_status zgetrf(cudaStream_t st, double2* A, int n, int ncols, int lda, long long sA, int* piv, long long sP, int* info,
@@ -1178,10 +1182,11 @@ scw_status zgetrf(cudaStream_t st, double2* A, int n, int ncols, int lda, long l
         SCW_CUDA_TRY(cudaGetLastError());
         if (ncols > nb) {
             if (few_columns(ncols, batch))
-                z::lu_apply_kernel<8><<<dim3((ncols + 7) / 8, batch), 256, 0, st>>>(A, ncols, lda, sA, k0, nb, piv, sP, skip);
+                SCW_CUDA_TRY(launch_chained(true, st, dim3((ncols + 7) / 8, batch), 256, 0, z::lu_apply_kernel<8>, A, ncols, lda, sA,
+                                            k0, nb, piv, sP, skip));
             else
-                z::lu_apply_kernel<32><<<dim3((ncols + 31) / 32, batch), 256, 0, st>>>(A, ncols, lda, sA, k0, nb, piv, sP, skip);
-            SCW_CUDA_TRY(cudaGetLastError());
+                SCW_CUDA_TRY(launch_chained(true, st, dim3((ncols + 31) / 32, batch), 256, 0, z::lu_apply_kernel<32>, A, ncols, lda,
+                                            sA, k0, nb, piv, sP, skip));
         }
         const int rem = n - k0 - nb;
         if (rem > 0) {
@@ -1203,8 +1208,7 @@ scw_status ztrsm_upper(cudaStream_t st, const double2* LU, int n, int lda, long 
     const double2 one = {1, 0}, minus = {-1, 0};
     for (int k0 = ((n - 1) / kTB) * kTB; k0 >= 0; k0 -= kTB) {
         const int nb = std::min(kTB, n - k0);
-        trsm_block(st, LU, lda, sA, k0, nb, B, ldb, sB, nrhs, 1, batch, skip);
-        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_CUDA_TRY(trsm_block(st, LU, lda, sA, k0, nb, B, ldb, sB, nrhs, 1, batch, skip));
         if (k0 > 0) {
             scw_status s = zgemm(st, k0, nrhs, nb, minus, LU + k0, lda, sA, B + (long long)k0 * ldb, ldb, sB, one, B, ldb,
                                  sB, batch, ws, skip);
@@ -1223,8 +1227,7 @@ scw_status zgetrs(cudaStream_t st, const double2* LU, int n, long long sA, const
     SCW_CUDA_TRY(cudaGetLastError());
     for (int k0 = 0; k0 < n; k0 += kTB) {
         const int nb = std::min(kTB, n - k0);
-        trsm_block(st, LU, n, sA, k0, nb, B, nrhs, sB, nrhs, 0, batch, skip);
-        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_CUDA_TRY(trsm_block(st, LU, n, sA, k0, nb, B, nrhs, sB, nrhs, 0, batch, skip));
         const int rem = n - k0 - nb;
         if (rem > 0) {
             scw_status s = zgemm(st, rem, nrhs, nb, minus, LU + (long long)(k0 + nb) * n + k0, n, sA,

@@ -46,6 +46,7 @@
 
 #include "scw_complex.cuh"
 #include "scw_dense.h"
+#include "scw_launch.h"
 #include "scw_tc.cuh"
 
 namespace scw {
@@ -109,6 +110,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 oz_inner_kernel(const T* __restrict__ B, long long ks, long long js, long long sB, int K, int N, int* __restrict__ f,
                 const int* __restrict__ skip) {
+    chain_wait();
     if (z::skipped(skip, blockIdx.y)) return;
     B += sB * blockIdx.y;
     f += (long long)blockIdx.y * K;
@@ -259,6 +261,7 @@ __device__ __forceinline__ void split_group(const SplitArgs& p, int b, int g, in
 
 template <int S, typename TA, typename TB>
 __global__ void __launch_bounds__(kSplitThreads) oz_split_kernel(SplitArgs p, const int* __restrict__ skip) {
+    chain_wait();
     __shared__ int se[16][kSplitK + 1];
     const bool isA = (int)blockIdx.x < p.nA;
     const int blk = isA ? blockIdx.x : blockIdx.x - p.nA;
@@ -331,6 +334,7 @@ __device__ __forceinline__ void put(float2* p, float x, float y) { *p = make_flo
 template <int S, typename TC>
 __global__ void __launch_bounds__(kThreads, 1)
 oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
+    chain_wait();
     using namespace tc;
     constexpr int kS = S, kTN = Cfg<S>::kTN, kABlk = Cfg<S>::kABlk, kBBlk = Cfg<S>::kBBlk, kStages = Cfg<S>::kStages;
     constexpr int kCols = kTN * 4 / kDrainWarps;  // columns of a drain warp
@@ -566,6 +570,7 @@ __global__ void __launch_bounds__(256)
 zgemv_kernel(int M, int K, double2 alpha, const double2* __restrict__ A, int lda, long long sA,
              const double2* __restrict__ x, int ldx, long long sX, double2 beta, double2* __restrict__ y, int ldy,
              long long sY, const int* __restrict__ skip) {
+    chain_wait();
     if (z::skipped(skip, blockIdx.y)) return;
     const int i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (i >= M) return;
@@ -644,22 +649,21 @@ static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const
         const bool scale = !(a1 && !b1);
         if (K > 0) {
             if (scale) {
-                oz_inner_kernel<TB><<<dim3((K + 7) / 8, nb_), 256, 0, st>>>(Bb, ksB, rsB, sB, K, N, f, sk);
-                SCW_CUDA_TRY(cudaGetLastError());
+                SCW_CUDA_TRY(launch_chained(true, st, dim3((K + 7) / 8, nb_), 256, 0, oz_inner_kernel<TB>, Bb, ksB, rsB, sB, K, N,
+                                            f, sk));
             } else {
                 SCW_CUDA_TRY(cudaMemsetAsync(f, 0, sizeof(int) * (size_t)K * nb_, st));
             }
         }
         SplitArgs sp{Ab, Bb, rsA, ksA, rsB, ksB, sA, sB, opB == kOpC, M, N, K, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB,
                      na_ * sh.gA, f, eA, gN, dA, dB, b1 ? 0 : 1};
-        oz_split_kernel<S, TA, TB><<<na_ * sh.gA + nb_ * sh.gB, kSplitThreads, 0, st>>>(sp, sk);
-        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_CUDA_TRY(launch_chained(true, st, dim3(na_ * sh.gA + nb_ * sh.gB), kSplitThreads, 0, oz_split_kernel<S, TA, TB>, sp, sk));
         const long long tiles = (long long)sh.mt * sh.nt * nb;
         if (tiles > (1ll << 30)) return fail(SCW_ERR_ARG, "zgemm: too many tiles");
         GemmArgs g{dA, dB, eA, gN, M, N, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB, a1, b1, alpha, beta, diag,
                    (void*)(C + sC * b0), ldc, sC, (int)tiles, ws.err};
-        oz_gemm_kernel<S, TC><<<(unsigned)std::min<long long>(tiles, sms), kThreads, smem, st>>>(g, sk);
-        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_CUDA_TRY(launch_chained(true, st, dim3((unsigned)std::min<long long>(tiles, sms)), kThreads, smem,
+                                    oz_gemm_kernel<S, TC>, g, sk));
     }
     return SCW_OK;
 }
@@ -692,9 +696,8 @@ scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const doub
                  const GemmWs& ws, const int* skip, double diag, int opB) {
     if (M <= 0 || N <= 0 || batch <= 0) return SCW_OK;
     if (N == 1 && diag == 0.0 && opB == kOpN) {
-        oz::zgemv_kernel<<<dim3((M + 7) / 8, batch), 256, 0, st>>>(M, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC,
-                                                                  skip);
-        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_CUDA_TRY(launch_chained(true, st, dim3((M + 7) / 8, batch), 256, 0, oz::zgemv_kernel, M, K, alpha, A, lda, sA, B,
+                                    ldb, sB, beta, C, ldc, sC, skip));
         return SCW_OK;
     }
     if (!ws.base && (diag != 0.0 || opB != kOpN)) return fail(SCW_ERR_ARG, "zgemm: this product needs a workspace");

@@ -229,6 +229,7 @@ __global__ void newton_gate_kernel(const double* __restrict__ worst, int n, int 
 //   mode 2 (Gc):             A1 <- E A1 + A2,    A2 <- E A1 - A2
 __global__ void mix_kernel(double2* __restrict__ A1, double2* __restrict__ A2, const double2* __restrict__ E, int n,
                            int ncol, int mode) {
+    chain_wait();
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long long)n * ncol) return;
     const int i = (int)(e / ncol);
@@ -911,8 +912,7 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
     for (int l = Zs - 1; l >= 0; l--) {
         const long long o = (long long)l * nn, half = (long long)n * nc;
         SCW_TRY(zgemm(st, n, nc, n, kOne, Uinv + o, n, Winv - Uinv, ws.X, nc, half, kZero, ws.A1, nc, half, 2, ws.gemm));
-        mix_kernel<<<nblk(half), 256, 0, st>>>(ws.A1, A2, ws.E + (size_t)l * n, n, nc, 0);
-        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_CUDA_TRY(launch_chained(true, st, nblk(half), 256, 0, mix_kernel, ws.A1, A2, ws.E + (size_t)l * n, n, nc, 0));
         SCW_TRY(zgemm(st, n, nc, n, kOne, ws.U + o, n, ws.W - ws.U, ws.A1, nc, half, kZero, ws.X, nc, half, 2, ws.gemm));
         L += 7;
     }
@@ -955,16 +955,14 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
             const double2* bp = ws.beta + (size_t)(l - 1) * N4;
             SCW_CUDA_TRY(cudaMemcpyAsync(ws.A1, bp, sizeof(double2) * n, cudaMemcpyDeviceToDevice, st));
             SCW_CUDA_TRY(cudaMemcpyAsync(A2, bp + n, sizeof(double2) * n, cudaMemcpyDeviceToDevice, st));
-            mix_kernel<<<nblk(n), 256, 0, st>>>(ws.A1, A2, ws.E + (size_t)(l - 1) * n, n, 1, 2);
-            SCW_CUDA_TRY(cudaGetLastError());
+            SCW_CUDA_TRY(launch_chained(true, st, nblk(n), 256, 0, mix_kernel, ws.A1, A2, ws.E + (size_t)(l - 1) * n, n, 1, 2));
             SCW_TRY(zgemm(st, n, 1, n, kOne, ws.U + o - nn, n, 0, ws.A1, 1, 0, kZero, ws.v, 1, 0, 1, ws.gemm));
             SCW_TRY(zgemm(st, n, 1, n, kOne, ws.W + o - nn, n, 0, A2, 1, 0, kZero, ws.v + n, 1, 0, 1, ws.gemm));
             L += 3;
         }
         SCW_TRY(zgemm(st, n, 1, n, kOne, Uinv + o, n, 0, ws.v, 1, 0, kZero, bl, 1, 0, 1, ws.gemm));
         SCW_TRY(zgemm(st, n, 1, n, kOne, Winv + o, n, 0, ws.v + n, 1, 0, kZero, bl + n, 1, 0, 1, ws.gemm));
-        mix_kernel<<<nblk(n), 256, 0, st>>>(bl, bl + n, ws.E + (size_t)l * n, n, 1, 1);
-        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_CUDA_TRY(launch_chained(true, st, nblk(n), 256, 0, mix_kernel, bl, bl + n, ws.E + (size_t)l * n, n, 1, 1));
         L += 3;
     }
     // Q_check / Q_hat with Ez from the magnetic field (sCWatter.cpp:781-871): Hm in P, Kn over U^-1, Ez

@@ -15,6 +15,7 @@
 
 #include "scw_complex.cuh"
 #include "scw_dense.h"
+#include "scw_launch.h"
 
 namespace scw {
 namespace z {
@@ -25,6 +26,7 @@ constexpr int kTriB = 32;
 // per vector, lane l: row i0 + l.
 __global__ void __launch_bounds__(256)
 trevc_block_kernel(const float2* __restrict__ T, float2* __restrict__ X, int n, int i0, int i1) {
+    chain_wait();
     T += (long long)n * n * blockIdx.y;
     X += (long long)n * n * blockIdx.y;
     __shared__ float2 B[kTriB][kTriB + 1];
@@ -78,6 +80,7 @@ trevc_block_kernel(const float2* __restrict__ T, float2* __restrict__ X, int n, 
 // lane l: column j0 + l.
 __global__ void __launch_bounds__(256)
 trtri_block_kernel(const float2* __restrict__ X, float2* __restrict__ Z, int n, int j0, int j1) {
+    chain_wait();
     X += (long long)n * n * blockIdx.y;
     Z += (long long)n * n * blockIdx.y;
     __shared__ float2 B[kTriB][kTriB + 1];           // column j0 + j of the matrix in row j
@@ -119,8 +122,7 @@ scw_status trevc32(cudaStream_t st, const float2* T, float2* X, int n, int batch
         const scw_status s = cgemm(st, below, i1 - i0, below, 1.f, X + (long long)i1 * n + i1, n, nn, kOpN, T + (long long)i0 * n + i1, n,
                                    nn, kOpT, false, X + (long long)i1 * n + i0, n, nn, batch);
         if (s != SCW_OK) return s;
-        z::trevc_block_kernel<<<dim3((n + 7) / 8, batch), 256, 0, st>>>(T, X, n, i0, i1);
-        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_CUDA_TRY(launch_chained(true, st, dim3((n + 7) / 8, batch), 256, 0, z::trevc_block_kernel, T, X, n, i0, i1));
     }
     return SCW_OK;
 }
@@ -132,8 +134,7 @@ scw_status trtri32(cudaStream_t st, const float2* X, float2* Z, int n, int batch
         const int j1 = std::min(n, j0 + z::kTriB);
         const scw_status s = cgemm(st, j0, j1 - j0, j0, 1.f, Z, n, nn, kOpN, X + (long long)j0 * n, n, nn, kOpT, false, Z + j0, n, nn, batch);
         if (s != SCW_OK) return s;
-        z::trtri_block_kernel<<<dim3((n + 7) / 8, batch), 256, 0, st>>>(X, Z, n, j0, j1);
-        SCW_CUDA_TRY(cudaGetLastError());
+        SCW_CUDA_TRY(launch_chained(true, st, dim3((n + 7) / 8, batch), 256, 0, z::trtri_block_kernel, X, Z, n, j0, j1));
     }
     return SCW_OK;
 }
