@@ -11,6 +11,7 @@
 
 #include "scw_complex.cuh"
 #include "scw_dense.h"
+#include "scw_launch.h"
 #include "scw_eigmix.h"
 
 namespace scw {
@@ -113,6 +114,7 @@ __global__ void to_f32_kernel(const double2* __restrict__ A, float2* __restrict_
 // FP32 eigenvalues -> FP64 starting point; state from the FP32 QR status
 __global__ void init_kernel(const float2* __restrict__ lam32, double2* __restrict__ lam, int n, const int* __restrict__ qr,
                             int* __restrict__ state, int* __restrict__ steps, double* __restrict__ res) {
+    chain_wait();
     const int b = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         const float2 l = lam32[(long long)n * b + i];
@@ -135,6 +137,7 @@ __global__ void __launch_bounds__(1024)
 cluster_kernel(const double2* __restrict__ lam, int n, const double* __restrict__ anorm, double tau_rel,
                int* __restrict__ label, int* __restrict__ member, int* __restrict__ cstart, int* __restrict__ ncl,
                int* __restrict__ state) {
+    chain_wait();
     const int b = blockIdx.x;
     extern __shared__ __align__(16) unsigned char smem[];
     double2* lm = reinterpret_cast<double2*>(smem);
@@ -230,6 +233,7 @@ cluster_kernel(const double2* __restrict__ lam, int n, const double* __restrict_
 __global__ void __launch_bounds__(256)
 resid_kernel(const double2* __restrict__ AX, const double2* __restrict__ X, const double2* __restrict__ lam, int n,
              float2* __restrict__ R32, double* __restrict__ rn, double* __restrict__ xn, const int* __restrict__ state) {
+    chain_wait();
     const int b = blockIdx.y;
     if (state[b] != kRefining) return;
     const long long nn = (long long)n * n;
@@ -269,6 +273,7 @@ resid_kernel(const double2* __restrict__ AX, const double2* __restrict__ X, cons
 __global__ void __launch_bounds__(256)
 gate_kernel(int n, const double* __restrict__ rn, const double* __restrict__ xn, const double* __restrict__ anorm,
             double tol, int step, int* __restrict__ state, int* __restrict__ steps, double* __restrict__ res) {
+    chain_wait();
     // tol: the stopping tolerance at early checks, the acceptance tolerance from step `steps` on
     const int b = blockIdx.x;
     if (state[b] != kRefining) return;
@@ -301,6 +306,7 @@ gate_kernel(int n, const double* __restrict__ rn, const double* __restrict__ xn,
 // lambda_i += E_ii for eigenvalues outside every cluster
 __global__ void singleton_kernel(const float2* __restrict__ E, const int* __restrict__ label, double2* __restrict__ lam,
                                  int n, int* __restrict__ state) {
+    chain_wait();
     const int b = blockIdx.y;
     if (state[b] != kRefining) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -324,6 +330,7 @@ __global__ void __launch_bounds__(kMaxCluster)
 cluster_eig_kernel(const float2* __restrict__ E, const int* __restrict__ member, const int* __restrict__ cstart,
                    const int* __restrict__ ncl, double2* __restrict__ lam, int n, const double* __restrict__ anorm,
                    double deg_rel, double2* __restrict__ Yout, float2* __restrict__ Yinv, int* __restrict__ state) {
+    chain_wait();
     const int b = blockIdx.y, c = blockIdx.x;
     if (state[b] != kRefining || c >= ncl[b]) return;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -563,6 +570,7 @@ __device__ __forceinline__ float2 divide32(float2 e, double2 d) {
 // F_ij = E_ij / (lambda_j - lambda_i) between different clusters / singletons, 0 within one
 __global__ void f_kernel(const float2* __restrict__ E, const double2* __restrict__ lam, const int* __restrict__ label,
                          int n, float2* __restrict__ F, const int* __restrict__ state) {
+    chain_wait();
     const int b = blockIdx.y;
     if (state[b] != kRefining) return;
     const long long nn = (long long)n * n;
@@ -589,6 +597,7 @@ __global__ void f_kernel(const float2* __restrict__ E, const double2* __restrict
 __global__ void __launch_bounds__(kMaxCluster)
 rotate_kernel(double2* __restrict__ X, const int* __restrict__ member, const int* __restrict__ cstart,
               const int* __restrict__ ncl, const double2* __restrict__ Yin, int n, const int* __restrict__ state) {
+    chain_wait();
     const int b = blockIdx.y, c = blockIdx.x;
     if (state[b] != kRefining || c >= ncl[b]) return;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -617,6 +626,7 @@ rotate_kernel(double2* __restrict__ X, const int* __restrict__ member, const int
 __global__ void __launch_bounds__(kMaxCluster)
 rotate_rows_kernel(float2* __restrict__ Yx, const int* __restrict__ member, const int* __restrict__ cstart,
                    const int* __restrict__ ncl, const float2* __restrict__ Yinv, int n, const int* __restrict__ state) {
+    chain_wait();
     const int b = blockIdx.y, c = blockIdx.x;
     if (state[b] != kRefining || c >= ncl[b]) return;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -640,6 +650,7 @@ rotate_rows_kernel(float2* __restrict__ Yx, const int* __restrict__ member, cons
 }
 
 __global__ void final_kernel(int* __restrict__ state, int* __restrict__ accepted, int Z) {
+    chain_wait();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= Z) return;
     if (state[b] == kRefining) state[b] = kNotConverged;
@@ -685,16 +696,19 @@ scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int
     MX_TRY(gemm32(st, n, 1.0, w.S1, w.S2, kOpT, 0.0, 0.0, V, Z, ws, nullptr));
     MX_TRY(gemm32(st, n, 1.0, w.S3, w.S1, kOpC, 0.0, 0.0, Yx, Z, ws, nullptr));
     if (launches) *launches += 10;
-    init_kernel<<<dim3(nblk(n), Z), 256, 0, st>>>(w.lam32, lam, n, w.qr, w.state, w.steps, w.res);
-    cluster_kernel<<<Z, 1024, cl_smem, st>>>(lam, n, w.anorm, prm.tau_rel, w.label, w.member, w.cstart, w.ncl, w.state);
+    SCW_CUDA_TRY(launch_chained(true, st, dim3(nblk(n), Z), 256, 0, init_kernel, w.lam32, lam, n, w.qr, w.state, w.steps,
+                                w.res));
+    SCW_CUDA_TRY(launch_chained(true, st, Z, 1024, cl_smem, cluster_kernel, lam, n, w.anorm, prm.tau_rel, w.label, w.member,
+                                w.cstart, w.ncl, w.state));
     MX_LAUNCHED(2);
     const int last = n >= EigMixParams::kLargeN ? std::max(prm.steps, prm.steps_large) : prm.steps;
     for (int s = 0; s <= last; s++) {
         // residual check (and right-hand side of the correction)
         MX_TRY(zgemm(st, n, n, n, d1, A, n, nn, V, n, nn, d0, AX, n, nn, Z, ws, w.state));
-        resid_kernel<<<dim3((n + 31) / 32, Z), 256, 0, st>>>(AX, V, lam, n, w.S3, w.rn, w.xn, w.state);
-        gate_kernel<<<Z, 256, 0, st>>>(n, w.rn, w.xn, w.anorm, s >= prm.steps ? prm.tol_accept : prm.tol, s, w.state,
-                                       w.steps, w.res);
+        SCW_CUDA_TRY(launch_chained(true, st, dim3((n + 31) / 32, Z), 256, 0, resid_kernel, AX, V, lam, n, w.S3, w.rn, w.xn,
+                                    w.state));
+        SCW_CUDA_TRY(launch_chained(true, st, Z, 256, 0, gate_kernel, n, w.rn, w.xn, w.anorm, s >= prm.steps ?
+                                    prm.tol_accept : prm.tol, s, w.state, w.steps, w.res));
         MX_LAUNCHED(5);
         if (s == last) break;
         if (s >= 2 && cap == cudaStreamCaptureStatusNone) {
@@ -704,23 +718,24 @@ scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int
         }
         // E = X^-1 R
         MX_TRY(gemm32(st, n, 1.0, Yx, w.S3, kOpN, 0.0, 0.0, w.S0, Z, ws, w.state));
-        singleton_kernel<<<dim3(nblk(n), Z), 256, 0, st>>>(w.S0, w.label, lam, n, w.state);
-        cluster_eig_kernel<<<dim3(maxcl, Z), kMaxCluster, eig_smem, st>>>(w.S0, w.member, w.cstart, w.ncl, lam, n,
-                                                                         w.anorm, prm.deg_rel, w.Y, w.Yi, w.state);
-        f_kernel<<<dim3(gZ, Z), 256, 0, st>>>(w.S0, lam, w.label, n, w.S1, w.state);
+        SCW_CUDA_TRY(launch_chained(true, st, dim3(nblk(n), Z), 256, 0, singleton_kernel, w.S0, w.label, lam, n, w.state));
+        SCW_CUDA_TRY(launch_chained(true, st, dim3(maxcl, Z), kMaxCluster, eig_smem, cluster_eig_kernel, w.S0, w.member,
+                                    w.cstart, w.ncl, lam, n, w.anorm, prm.deg_rel, w.Y, w.Yi, w.state));
+        SCW_CUDA_TRY(launch_chained(true, st, dim3(gZ, Z), 256, 0, f_kernel, w.S0, lam, w.label, n, w.S1, w.state));
         MX_LAUNCHED(6);
         // X += X F, then the cluster rotations; X^-1 follows by the inverse rotations and a Newton
         // step, Yx += Yx (I - X Yx), which squares the error F left in it
         MX_TRY(gemm32(st, n, 1.0, V, w.S1, kOpN, 1.0, 0.0, V, Z, ws, w.state));
-        rotate_kernel<<<dim3(maxcl, Z), kMaxCluster, rot_smem, st>>>(V, w.member, w.cstart, w.ncl, w.Y, n, w.state);
-        rotate_rows_kernel<<<dim3(maxcl, Z), kMaxCluster, rot_smem / 2, st>>>(Yx, w.member, w.cstart, w.ncl, w.Yi, n,
-                                                                             w.state);
+        SCW_CUDA_TRY(launch_chained(true, st, dim3(maxcl, Z), kMaxCluster, rot_smem, rotate_kernel, V, w.member, w.cstart,
+                                    w.ncl, w.Y, n, w.state));
+        SCW_CUDA_TRY(launch_chained(true, st, dim3(maxcl, Z), kMaxCluster, rot_smem / 2, rotate_rows_kernel, Yx, w.member,
+                                    w.cstart, w.ncl, w.Yi, n, w.state));
         MX_TRY(gemm32(st, n, -1.0, V, Yx, kOpN, 0.0, 1.0, w.S0, Z, ws, w.state));
         MX_TRY(gemm32(st, n, 1.0, Yx, w.S0, kOpN, 1.0, 0.0, Yx, Z, ws, w.state));
         MX_LAUNCHED(11);
     }
     // slices without convergence: the FP64 Householder + QR solver (qr[] reused as the skip mask)
-    final_kernel<<<nblk(Z), 256, 0, st>>>(w.state, w.qr, Z);
+    SCW_CUDA_TRY(launch_chained(true, st, nblk(Z), 256, 0, final_kernel, w.state, w.qr, Z));
     MX_LAUNCHED(1);
     MX_TRY(zgeev(st, A, lam, V, n, Z, fb_work, status, w.qr, prm.wide, ws));
     if (launches) *launches += 5;

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(256)
 oz_inner_kernel(const T* __restrict__ B, long long ks, long long js, long long sB, int K, int N, int* __restrict__ f,
                 const int* __restrict__ skip) {
     chain_wait();
+    chain_trigger();
     if (z::skipped(skip, blockIdx.y)) return;
     B += sB * blockIdx.y;
     f += (long long)blockIdx.y * K;
@@ -262,6 +263,7 @@ __device__ __forceinline__ void split_group(const SplitArgs& p, int b, int g, in
 template <int S, typename TA, typename TB>
 __global__ void __launch_bounds__(kSplitThreads) oz_split_kernel(SplitArgs p, const int* __restrict__ skip) {
     chain_wait();
+    chain_trigger();
     __shared__ int se[16][kSplitK + 1];
     const bool isA = (int)blockIdx.x < p.nA;
     const int blk = isA ? blockIdx.x : blockIdx.x - p.nA;
@@ -334,7 +336,6 @@ __device__ __forceinline__ void put(float2* p, float x, float y) { *p = make_flo
 template <int S, typename TC>
 __global__ void __launch_bounds__(kThreads, 1)
 oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
-    chain_wait();
     using namespace tc;
     constexpr int kS = S, kTN = Cfg<S>::kTN, kABlk = Cfg<S>::kABlk, kBBlk = Cfg<S>::kBBlk, kStages = Cfg<S>::kStages;
     constexpr int kCols = kTN * 4 / kDrainWarps;  // columns of a drain warp
@@ -368,6 +369,7 @@ oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     const int per = p.mt * p.nt;
+    chain_wait();
 
     if (warp == kDrainWarps) {
         // ---------------- copies ----------------
