@@ -93,7 +93,7 @@ struct scw_sep_s {
     cudaStream_t hi_stream = nullptr;
     // the viewer's second and third plane run beside the first (scw_sep_gpu_cw_evaluate)
     cudaStream_t plane_stream[2] = {nullptr, nullptr};
-    cudaEvent_t plane_event[3] = {nullptr, nullptr, nullptr};
+    cudaEvent_t plane_event[4] = {nullptr, nullptr, nullptr, nullptr};   // start, xz done, yz done, C of both
     std::vector<cudaEvent_t> pevents;
     int pipe_chunks = 0;                   // chunks of a pipelined slab (0 or 1: one pass)
     int pipe_synth_div = 2;                // the pipelined output GEMM runs on sm_count / pipe_synth_div SMs
