@@ -10,7 +10,8 @@
 //
 // Operands are built in shared memory, 32 waves (a chunk) at a time:
 //   * warps 20-22 take a wave per lane, every third chunk each: base phase at the tile centre reduced
-//     in FP64, amplitudes A' with that phase, scaled by the chunk's power of two, k in turns as two floats;
+//     in FP64, amplitudes A' with that phase, scaled by the chunk's power of two for each component (one for all three cut a
+//     component 2^-24 of the others to four digits), k in turns as two floats;
 //   * warps 8-19 build L and R, a wave per lane and eight columns (or rows) of points per warp: sine and cosine of
 //     the phase at columns 2 and 6 and of one step, phases in turns with both factors as two floats (an FP32
 //     product would lose 1e-6 at 30 radians), from the Taylor series on [-pi/4, pi/4]; the columns between are one
@@ -89,7 +90,7 @@ struct Wave {                                 // one staged wave
 
 struct Smem {
     Wave wave[kWaveSlots][kChunk];
-    float scale[kWaveSlots];                  // 2^e of the chunk's result
+    float scale[kWaveSlots][3];               // 2^e of the chunk's result, per component
     int cplx[kWaveSlots];
     F2 grid[kGroupsA + kGroupsB][5];          // per group of eight points, L's first: see eight()
     uint64_t wave_full[kWaveSlots], wave_empty[kWaveSlots], full[kBufs], empty[kBufs], acc_full[2], acc_empty[2];
@@ -326,19 +327,19 @@ plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items
             v.k = make_float4((float)kA, (float)(kA - (double)(float)kA), (float)kB, (float)(kB - (double)(float)kB));
             int cplx = (v.b.z != 0.f ? 1 : 0) | (v.b.w != 0.f ? 2 : 0);
             load(ch + kStage);
-            // the chunk's largest finite part below 2^e
+            // the chunk's largest finite part below 2^e, component by component: a weak one is not measured by the others
             auto part = [](float x) { return fabsf(x) <= 3.4e38f ? fabsf(x) : 0.f; };
-            const float big = fmaxf(fmaxf(fmaxf(part(v.a.x), part(v.a.y)), fmaxf(part(v.a.z), part(v.a.w))),
-                                    fmaxf(part(v.b.x), part(v.b.y)));
-            const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(big));
-            const int e = max(-100, min(128, (int)(top >> 23) - 126));
-            const float up = __int_as_float((12 - e + 127) << 23);
-            v.a.x *= up;
-            v.a.y *= up;
-            v.a.z *= up;
-            v.a.w *= up;
-            v.b.x *= up;
-            v.b.y *= up;
+            int e[3];
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                float& re = c == 0 ? v.a.x : c == 1 ? v.a.z : v.b.x;
+                float& im = c == 0 ? v.a.y : c == 1 ? v.a.w : v.b.y;
+                const unsigned top = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(part(re), part(im))));
+                e[c] = max(-100, min(128, (int)(top >> 23) - 126));
+                const float up = __int_as_float((12 - e[c] + 127) << 23);
+                re *= up;
+                im *= up;
+            }
             cplx = (int)__reduce_or_sync(0xffffffffu, (unsigned)cplx);
             int stop = S.abort;
             if (!stop && ch >= kWaveSlots && !mbar_wait(&S.wave_empty[s], (uint32_t)((ch / kWaveSlots - 1) & 1))) stop = 1;
@@ -348,7 +349,8 @@ plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items
             }
             S.wave[s][lane] = v;
             if (lane == 0) {
-                S.scale[s] = __int_as_float((e - 22 + 127) << 23);
+#pragma unroll
+                for (int c = 0; c < 3; c++) S.scale[s][c] = __int_as_float((e[c] - 22 + 127) << 23);
                 S.cplx[s] = cplx;
             }
             mbar_arrive(&S.wave_full[s]);
@@ -477,7 +479,7 @@ plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items
                 break;
             }
             tc_fence_after();
-            const F2 sc = both(S.scale[s]);
+            const F2 sc = both(S.scale[s][min(comp, 2)]);
             if (busy) {
 #pragma unroll
                 for (int c16 = 0; c16 < 32; c16 += 16) {
