@@ -24,10 +24,14 @@
 //     accumulator's rounding acts on the few last steps only.  R is kept as -im | re | im, so that re L x (re | im)
 //     and im L x (-im | re) are each one MMA of twice the columns: it reads L half as often, and the MMAs
 //     are bound by what they read from shared memory;
-//   * warps 0-7 add each chunk's sum, 2^e scaled, to FP32 registers, and every kMaxRun waves those to FP64
-//     partial sums; the partial sums of a tile's items meet in the reduce kernel, in a fixed order.
-// 409 600 waves x 3 planes of 200 x 200 points: 19.4 ms by the summation kernel, 4.3 ms here; 20 736 waves a layer on a
-// 101 x 77 x 50 volume: 5.10 -> 1.37 ms.  A chunk takes about 1600 clocks: 700 of them are MMA reads of shared memory and
+//   * warps 0-7 add each chunk's sum, 2^e scaled, to FP32 registers, every kRun chunks those to sums of two floats in
+//     the other half of tensor memory, and every kMaxRun waves these to FP64 partial sums, which meet in the reduce
+//     kernel, in a fixed order.  32 additions to a growing sum, not 1024: a run of 1024 waves loses less to rounding than the
+//     summation kernel's 256 additions (45 against 64 roundings of a sum of 256 waves, over 4096 waves that all add up).
+//     One FP32 sum of 4096 waves lost 1.5 times as much as that kernel.
+// 409 600 waves x 3 planes of 200 x 200 points: 19.4 ms by the summation kernel, 4.50 ms here; 20 736 waves a layer on a
+// 101 x 77 x 50 volume: 5.10 -> 1.39 ms (4.30 and 1.30 with one FP32 sum per 4096 waves, 4.45 and 1.33 with runs of 64 chunks:
+// tensor memory answers late, and sums that are late hold up the MMAs).  A chunk takes about 1600 clocks: 700 of them are MMA reads of shared memory and
 // 450 the stores of the operands, and the warps that build these issue half of the time.  Measured in the
 // second case on the way: K-major operands with a sine and cosine for every point and wave 2.9 ms, this
 // layout 1.55, operands in FP32 pairs with 9 and 12 warps 1.47 and 1.37 (7 warps 1.64).
@@ -50,7 +54,9 @@ constexpr uint32_t kGroup = kChunk * 16;              // bytes of a group of 8 p
 constexpr int kDrain = 8, kProd = 12, kStage = 3;      // warps
 constexpr int kWarps = kDrain + kProd + kStage + 1, kThreads = kWarps * 32;
 constexpr int kWaveSlots = 6;                 // staged chunks of waves
-constexpr uint32_t kCols = 256;               // TMEM: two accumulators of re | im, up to 64 columns each
+constexpr int kRun = 32;                      // chunks (1024 waves) added up in FP32
+constexpr uint32_t kCols = 512;               // TMEM: two accumulators of re | im, up to 64 columns each, and the runs' sums
+constexpr uint32_t kSumCol = 256, kSumLow = 128;      // their first column (re | im of all columns), and their low words
 constexpr int kGroupsA = kTileI / 8, kGroupsB = kTileJ / 8;
 
 // two floats per register pair: one issue slot for two results
@@ -81,6 +87,20 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
     return r;
 }
 __device__ __forceinline__ F2 neg2(F2 a) { return F2{a.v ^ 0x8000000080000000ull}; }
+// the same value in FP64, by integer operations but for subnormal and non-finite ones (a conversion takes 19 clocks of
+// the SM's FP64 pipe)
+__device__ __forceinline__ double widen(float x) {
+    const unsigned b = __float_as_uint(x), m = b & 0x7fffffffu;
+    if (m != 0u && m - 0x00800000u >= 0x7f000000u) return (double)x;
+    return __hiloint2double((int)(m ? (b & 0x80000000u) | ((m >> 3) + 0x38000000u) : b), (int)(b << 29));
+}
+// hi + x, its rounding error added to lo (Knuth's two-sum; what lo holds where hi is not finite means nothing)
+__device__ __forceinline__ void add_exact2(F2& hi, F2& lo, F2 x) {
+    const F2 m = both(-1.f), s = add2(hi, x), b = fma2(hi, m, s), t = fma2(b, m, s);
+    lo = add2(lo, add2(fma2(t, m, hi), fma2(b, m, x)));
+    hi = s;
+}
+__device__ __forceinline__ float low_word(float hi, float lo) { return isfinite(hi) ? lo : 0.f; }
 
 struct Wave {                                 // one staged wave
     float4 a;                                 // A'x re, im, A'y re, im (scaled)
@@ -95,6 +115,8 @@ struct Smem {
     F2 grid[kGroupsA + kGroupsB][5];          // per group of eight points, L's first: see eight()
     uint64_t wave_full[kWaveSlots], wave_empty[kWaveSlots], full[kBufs], empty[kBufs], acc_full[2], acc_empty[2];
     int task[kGroupsA + kGroupsB];            // of a chunk, in order: group of L, or 64 + group of R
+    Item item;                                // for the drain, which has no registers to spare for them
+    Plane plane;
     uint32_t tmem;
     volatile int abort;
 };
@@ -265,6 +287,8 @@ plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items
             mbar_init(&S.acc_empty[i], kDrain);
         }
         S.abort = 0;
+        S.item = it;
+        S.plane = g;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
@@ -461,12 +485,10 @@ plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items
         const int quarter = warp & 3, half = warp >> 2;
         const uint32_t tb = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 32);
         const bool busy = half * 32 < N;
-        const int r = quarter * 32 + lane, comp = r / kTileI, i = r - comp * kTileI;
-        const bool out = comp < 3 && i < ncol;
+        const int r = quarter * 32 + lane, comp = r / kTileI;
         F2 re[16], im[16];                    // columns 2 c and 2 c + 1
 #pragma unroll
         for (int c = 0; c < 16; c++) re[c].v = im[c].v = 0;
-        bool ok = true;
         for (int ch = 0; ch < nchunk; ch++) {
             const int buf = ch & 1, s = ch % kWaveSlots;
             int stop = S.abort;
@@ -475,26 +497,25 @@ plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items
                 stop = 1;
             if (__any_sync(0xffffffffu, stop)) {
                 S.abort = 1;
-                ok = false;
                 break;
             }
             tc_fence_after();
             const F2 sc = both(S.scale[s][min(comp, 2)]);
             if (busy) {
 #pragma unroll
-                for (int c16 = 0; c16 < 32; c16 += 16) {
-                    if (half * 32 + c16 < N) {
-                        uint32_t v[16];
-                        tmem_ld16(tb + (uint32_t)buf * 128u + c16, v);
-                        tmem_ld_wait();
+                for (int c8 = 0; c8 < 32; c8 += 8) {
+                    if (half * 32 + c8 < N) {
+                        uint32_t v[8];
+                        tmem_ld8(tb + (uint32_t)buf * 128u + c8, v);
+                        tmem_ld_wait8(v);
 #pragma unroll
-                        for (int c = 0; c < 8; c++)
-                            re[c16 / 2 + c] = fma2(pack(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1])), sc, re[c16 / 2 + c]);
-                        tmem_ld16(tb + (uint32_t)buf * 128u + (uint32_t)(N + c16), v);
-                        tmem_ld_wait();
+                        for (int c = 0; c < 4; c++)
+                            re[c8 / 2 + c] = fma2(pack(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1])), sc, re[c8 / 2 + c]);
+                        tmem_ld8(tb + (uint32_t)buf * 128u + (uint32_t)(N + c8), v);
+                        tmem_ld_wait8(v);
 #pragma unroll
-                        for (int c = 0; c < 8; c++)
-                            im[c16 / 2 + c] = fma2(pack(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1])), sc, im[c16 / 2 + c]);
+                        for (int c = 0; c < 4; c++)
+                            im[c8 / 2 + c] = fma2(pack(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1])), sc, im[c8 / 2 + c]);
                     }
                 }
             }
@@ -504,31 +525,87 @@ plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items
                 mbar_arrive(&S.acc_empty[buf]);
                 mbar_arrive(&S.wave_empty[s]);
             }
-            // the end of a run: into the item's FP64 partial sums, each element always by this thread
-            if (it.slot >= 0 && ((ch + 1) % (kMaxRun / kChunk) == 0 || ch + 1 == nchunk)) {
-                const bool first = ch < kMaxRun / kChunk;
+            // the end of a run: into the sums in tensor memory, and these at the end (and every kMaxRun waves) into
+            // the item's FP64 partial sums, each element always by this thread
+            const bool due = (ch + 1) % (kMaxRun / kChunk) == 0, end = ch + 1 == nchunk;
+            if (busy && (end || (ch + 1) % kRun == 0)) {
+                const bool first = ch % (kMaxRun / kChunk) < kRun;          // nothing in the sums yet
+                const uint32_t sum = tb + kSumCol;
 #pragma unroll
-                for (int c = 0; c < 32; c++) {
-                    const int j = half * 32 + c;
-                    if (j < nrow && out) {
-                        double2* o = partials + ((long long)it.slot * kTileJ + j) * (3 * kTileI) + r;
-                        double2 v = c & 1 ? make_double2((double)re[c / 2].y(), (double)im[c / 2].y())
-                                          : make_double2((double)re[c / 2].x(), (double)im[c / 2].x());
-                        if (!first) v = make_double2(o->x + v.x, o->y + v.y);
-                        *o = v;
+                for (int q = 0; q < 8; q++) {
+                    // columns c8 .. c8 + 7 of re (even q) or im
+                    const int c8 = q / 2 * 8, p = q & 1;
+                    if (half * 32 + c8 < N) {
+                        const uint32_t at = sum + (uint32_t)(c8 + 64 * p);
+                        uint32_t hv[8], lv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+                        if (!first) {
+                            tmem_ld8(at, hv);
+                            tmem_ld8(at + kSumLow, lv);
+                            tmem_ld_wait8(hv);
+                            tmem_ld_wait8(lv);
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; u++) {
+                            F2& x = p ? im[c8 / 2 + u] : re[c8 / 2 + u];
+                            F2 hi = x;
+                            if (!first) {
+                                hi = pack(__uint_as_float(hv[2 * u]), __uint_as_float(hv[2 * u + 1]));
+                                F2 lo = pack(__uint_as_float(lv[2 * u]), __uint_as_float(lv[2 * u + 1]));
+                                add_exact2(hi, lo, x);
+                                lv[2 * u] = __float_as_uint(lo.x());
+                                lv[2 * u + 1] = __float_as_uint(lo.y());
+                            }
+                            hv[2 * u] = __float_as_uint(hi.x());
+                            hv[2 * u + 1] = __float_as_uint(hi.y());
+                            x.v = 0;
+                        }
+                        tmem_st8(at, hv);
+                        tmem_st8(at + kSumLow, lv);
                     }
-                    if (c & 1) re[c / 2].v = im[c / 2].v = 0;
+                }
+                tmem_st_wait();
+                if (end || (due && S.item.slot >= 0)) {
+                    const bool add = ch >= kMaxRun / kChunk;
+                    const int slot = S.item.slot, jr0 = S.item.jr0, i0 = S.item.i0, rows = min(32, S.item.jr1 - jr0 - half * 32);
+                    const int Ni = S.plane.Ni;
+                    float2* const E = reinterpret_cast<float2*>(S.plane.out);
+                    const int i = r - comp * kTileI;
+                    const bool out = comp < 3 && i < min(kTileI, Ni - i0);
+#pragma unroll 1
+                    for (int c4 = 0; c4 < rows; c4 += 4) {
+                        uint32_t xh[4], xl[4], yh[4], yl[4];
+                        tmem_ld4(sum + c4, xh);
+                        tmem_ld4(sum + c4 + kSumLow, xl);
+                        tmem_ld4(sum + c4 + 64, yh);
+                        tmem_ld4(sum + c4 + 64 + kSumLow, yl);
+                        tmem_ld_wait4(xh);
+                        tmem_ld_wait4(xl);
+                        tmem_ld_wait4(yh);
+                        tmem_ld_wait4(yl);
+#pragma unroll
+                        for (int u = 0; u < 4; u++) {
+                            const int j = half * 32 + c4 + u;
+                            if (c4 + u >= rows || !out) continue;
+                            const float ah = __uint_as_float(xh[u]), al = low_word(ah, __uint_as_float(xl[u]));
+                            const float bh = __uint_as_float(yh[u]), bl = low_word(bh, __uint_as_float(yl[u]));
+                            if (slot < 0) {
+                                E[((long long)(jr0 + j) * Ni + i0 + i) * 3 + comp] = make_float2(ah + al, bh + bl);
+                            } else {
+                                double2* o = partials + ((long long)slot * kTileJ + j) * (3 * kTileI) + r;
+                                double2 v = make_double2(widen(ah), widen(bh));
+                                if (!first) v = make_double2(v.x + widen(al), v.y + widen(bl));
+                                if (add) v = make_double2(o->x + v.x, o->y + v.y);
+                                *o = v;
+                            }
+                        }
+                    }
                 }
             }
         }
-        if (ok && it.slot < 0 && out) {
-#pragma unroll
-            for (int c = 0; c < 32; c++) {
-                const int j = half * 32 + c;
-                if (j < nrow)
-                    reinterpret_cast<float2*>(g.out)[((long long)(it.jr0 + j) * g.Ni + it.i0 + i) * 3 + comp] =
-                        c & 1 ? make_float2(re[c / 2].y(), im[c / 2].y()) : make_float2(re[c / 2].x(), im[c / 2].x());
-            }
+        if (nchunk == 0 && comp < 3) {              // a region without waves: zeros
+            const int i = r - comp * kTileI;
+            for (int j = half * 32; j < min(nrow, half * 32 + 32); j++)
+                if (i < ncol) reinterpret_cast<float2*>(g.out)[((long long)(it.jr0 + j) * g.Ni + it.i0 + i) * 3 + comp] = make_float2(0.f, 0.f);
         }
     }
     __syncthreads();

@@ -10,7 +10,7 @@ namespace ptc {
 
 constexpr int kTileI = 40;        // columns of a tile: 3 components of five groups of eight in an MMA's 128 rows
 constexpr int kTileJ = 64;        // most rows
-constexpr int kMaxRun = 4096;     // waves added up in FP32 before they go to FP64 partial sums
+constexpr int kMaxRun = 4096;     // waves added up in two floats (1024 in one) before they go to FP64 partial sums
 
 struct Plane {
     float a0, b0, c;   // start along i (a) and j (b), fixed coordinate c
