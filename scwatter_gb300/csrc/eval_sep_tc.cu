@@ -526,7 +526,8 @@ synth_tc_kernel(const float2* __restrict__ T, const float2* __restrict__ F, int 
             uint32_t v[kEpiRows * 6];
 #pragma unroll
             for (int c16 = 0; c16 < kEpiRows * 6 / 16; c16++) tmem_ld16(tbase + (uint32_t)(16 * c16), &v[16 * c16]);
-            tmem_ld_wait();
+#pragma unroll
+            for (int c16 = 0; c16 < kEpiRows * 6 / 16; c16++) tmem_ld_wait16(&v[16 * c16]);
             tc_fence_before();
             mbar_arrive(&acc_empty[a]);
             for (int g0 = 0; g0 < kEpiRows; g0 += srows) {
