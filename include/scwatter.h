@@ -251,7 +251,9 @@ SCW_API scw_status scw_sep_gpu_cw_evaluate(scw_sep s, float* E_xy, float* E_xz, 
 /* MKL_multiply / MKL_linearsolve / MKL_eigensolve (third_Lapack.h:38-87).              */
 /* Complex values are (re, im) doubles.                                                 */
 /* ---------------------------------------------------------------------------------- */
-/* C = alpha A B + beta C; A: M x K, B: K x N, C: M x N per batch entry. */
+/* C = alpha A B + beta C; A: M x K, B: K x N, C: M x N per batch entry, C apart from A and B.  The error of each
+ * real and imaginary part is that of an FP64 sum of its products.  An entry that is not finite makes its
+ * row (of A) or column (of B) of the result NaN. */
 SCW_API scw_status scw_zgemm(scw_ctx ctx, int M, int N, int K, const double* alpha, const void* A, const void* B,
                              const double* beta, void* C, int batch);
 /* B := A^-1 B (A n x n overwritten by its LU factors, B n x nrhs); SCW_ERR_NUMERIC if singular;

@@ -1399,10 +1399,12 @@ scw_status scw_zgemm(scw_ctx ctx, int M, int N, int K, const double* alpha, cons
     // the workspace and the launches that use it go together: calls of several threads on one context
     // must not interleave
     std::lock_guard<std::mutex> lock(ctx->dense_mu);
-    ctx->launches += 3;
+    ctx->launches += 4;
     scw::GemmWs ws;
     scw_status st = scw::ctx_gemm_ws(ctx, scw::zgemm_ws_bytes(M, N, K, 1), scw::zgemm_ws_bytes(M, N, K, batch), ws);
-    if (st != SCW_OK) return st;
+    if (st == SCW_ERR_NOMEM) ws = scw::GemmWs{};          // no room for the digits: on the FP64 pipes
+    else if (st != SCW_OK) return st;
+    ws.parts = true;
     return scw::zgemm(ctx->stream, M, N, K, make_double2(alpha[0], alpha[1]), (const double2*)A, K, (long long)M * K,
                       (const double2*)B, N, (long long)K * N, make_double2(beta[0], beta[1]), (double2*)C, N,
                       (long long)M * N, batch, ws);

@@ -4,7 +4,7 @@
 // core, so an FP64 product is far cheaper as a sum of exact integer products (the error-free
 // splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59 (2012)):
 //   * the inner index is rescaled by powers of two, A'(i,k) = A(i,k) 2^f_k and B'(k,j) = B(k,j)
-//     2^-f_k with 2^f_k above row k of B, so that graded operands (the cascade's E^-1 rows) lose
+//     2^-f_k with 2^f_k above row k of B, so that operands graded along it (the cascade's E^-1 rows) lose
 //     nothing against a plain sum; then row i of A' gets the exponent e_i, column j of B' g_j;
 //   * every value becomes a 62-bit integer in units of 2^(e_i - 62) (2^(g_j - 62)), cut into kS = 8
 //     balanced base-256 digits, each in [-128, 128] and therefore exact in bf16;
@@ -15,8 +15,9 @@
 //     integers, and the final sum is rounded to FP64 once.
 // Diagonals d >= 8 are dropped: at most 2^-57 of the largest product per term.  Measured against
 // extended precision at n = 18 .. 1200 (random, constant, log-normal, diagonally dominant matrices,
-// eigenvectors): relative error 2e-17 .. 6.8e-16, where
-// a sequential FP64 sum has 9e-17 .. 1.7e-15.  With 7 digits (55 bits) the diagonally dominant and
+// eigenvectors): error against the largest |a'| |b'| of the row and column 2e-17 .. 6.8e-16, where
+// a sequential FP64 sum has 9e-17 .. 1.7e-15.  An entry more than 2^9 below its row's largest keeps fewer bits than
+// FP64: oz_parts_kernel is for callers to whom that matters.  With 7 digits (55 bits) the diagonally dominant and
 // eigenvector products came out 20 times less exact than an FP64 sum, so 8 it is (36 digit products
 // instead of 28).
 //
@@ -324,7 +325,12 @@ struct GemmArgs {
     long long sC;
     int tiles;
     int* err;
+    const unsigned* mask;              // a bit per element that oz_parts_kernel has written; null: none
 };
+
+__device__ __forceinline__ bool masked(const unsigned* mask, int M, int N, int b, int i, int j) {
+    return mask[((long long)b * M + i) * ((N + 31) / 32) + (j >> 5)] >> (j & 31) & 1u;
+}
 
 __device__ __forceinline__ double2 to_d(double2 v) { return v; }
 __device__ __forceinline__ double2 to_d(float2 v) { return make_double2(v.x, v.y); }
@@ -332,6 +338,154 @@ __device__ __forceinline__ void put(double2* p, double2 v) { *p = v; }
 __device__ __forceinline__ void put(float2* p, double2 v) { *p = make_float2((float)v.x, (float)v.y); }
 __device__ __forceinline__ void put(double2* p, float x, float y) { *p = make_double2(x, y); }
 __device__ __forceinline__ void put(float2* p, float x, float y) { *p = make_float2(x, y); }
+
+// The digits' error is at most 2 K 2^-59 R_i S_j per part (R, S: the row's and the column's powers of two), wherever the
+// sum of the |products| that make up the part lies.  So that sum is formed here, in FP32 and within 1e-5, and parts
+// where it is below R S max(2^-5, sqrt(K) 2^-7) are computed by FP64 operations: from 2^-6 on the digits' bound is
+// below that of an FP64 sum, (2 K + 1) 2^-53 of the sum; sqrt(K) 2^-7 is where their typical errors meet (digits 2^-62 a
+// product, a sequential sum K 2^-55 of the mean product).  A sum of zero is exact.  Rows of 10^10 and 1/3 times the identity had 1/3 to 9 digits.
+// Ordinary sums are large enough after one or two steps of 16 inner indices, where the tile is left: products of order 648 take
+// 132 us in place of 122, 20 of them 1680 in place of 1612, of order 3200 6.87 ms in place of 6.73.
+constexpr int kPT = 64, kPK = 16;                // as gemm_kernel: 64 x 64 tiles, 4 x 4 per thread, 16 inner indices at a time
+
+// |v| 2^s < 1 in FP32, rounded down to 21 bits; what is not zero at least 2^-60
+__device__ __forceinline__ float scaled_abs(double v, int s) {
+    const unsigned hi = (unsigned)__double2hiint(v) & 0x7fffffffu;
+    int ex = (int)(hi >> 20);
+    unsigned m = (hi & 0xfffffu) << 3;
+    if (ex == 0) {
+        if (v == 0.0) return 0.f;
+        const unsigned long long q = (unsigned long long)__double_as_longlong(v) << 12;       // subnormal: normalised
+        const int lz = __clzll((long long)q);
+        ex = -lz;
+        m = (unsigned)(q << lz << 1 >> 41);
+    }
+    ex += s - 1023;
+    if (ex < -60) return 0x1p-60f;
+    return __uint_as_float(((unsigned)(min(ex, 0) + 127) << 23) | m);
+}
+
+__global__ void __launch_bounds__(256)
+oz_parts_kernel(SplitArgs p, int a_shared, int b_shared, double2 alpha, double2 beta, double2* __restrict__ C, int ldc, long long sC,
+                unsigned* __restrict__ mask, const int* __restrict__ skip) {
+    using z::cfma;
+    chain_wait();
+    const int b = blockIdx.z;
+    if (z::skipped(skip, b)) return;
+    const double2* A = (const double2*)p.A + p.sA * b;
+    const double2* B = (const double2*)p.B + p.sB * b;
+    const int ba = a_shared ? 0 : b, bb = b_shared ? 0 : b;
+    const int *eA = p.eA + (long long)ba * p.gA * 16, *gN = p.gN + (long long)bb * p.gB * 16;
+    const int *fA = p.f + (long long)(ba * p.fstep) * p.K, *fB = p.f + (long long)bb * p.K;
+    const int i0 = blockIdx.y * kPT, j0 = blockIdx.x * kPT, tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    __shared__ __align__(16) double2 buf[2][kPK][kPT + 1];
+    __shared__ unsigned bits[kPT][2];
+    float2 (*As)[kPT + 1] = reinterpret_cast<float2(*)[kPT + 1]>(&buf[0][0][0]);
+    float2 (*Bs)[kPT + 1] = reinterpret_cast<float2(*)[kPT + 1]>(&buf[1][0][0]);
+    if (tid < 2 * kPT) bits[tid >> 1][tid & 1] = 0u;
+    float re[4][4] = {}, im[4][4] = {};
+    const float least = fmaxf(0x1p-5f, sqrtf((float)p.K) * 0x1p-7f);
+    auto inside = [&](int r, int q) { return i0 + ty + 16 * r < p.M && j0 + tx + 16 * q < p.N; };
+    const bool kfastA = p.ksA == 1, kfastB = p.ksB == 1;
+    for (int k0 = 0; k0 < p.K; k0 += kPK) {
+        for (int e = tid; e < kPK * kPT; e += 256) {
+            const int ra = kfastA ? e / kPK : e % kPT, ka = kfastA ? e % kPK : e / kPT;
+            const int rb = kfastB ? e / kPK : e % kPT, kb = kfastB ? e % kPK : e / kPT;
+            float2 a = make_float2(0.f, 0.f), c = a;
+            if (i0 + ra < p.M && k0 + ka < p.K) {
+                const int ex = eA[i0 + ra], s = fA[k0 + ka] - ex;
+                const double2 v = A[(i0 + ra) * p.rsA + (k0 + ka) * p.ksA];
+                if (ex > kNone / 2 && ex < kSpecial) a = make_float2(scaled_abs(v.x, s), scaled_abs(v.y, s));
+            }
+            if (j0 + rb < p.N && k0 + kb < p.K) {
+                const int ex = gN[j0 + rb], s = -fB[k0 + kb] - ex;
+                const double2 v = B[(j0 + rb) * p.rsB + (k0 + kb) * p.ksB];
+                if (ex > kNone / 2 && ex < kSpecial) c = make_float2(scaled_abs(v.x, s), scaled_abs(v.y, s));
+            }
+            As[ka][ra] = a;
+            Bs[kb][rb] = c;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < kPK; kk++) {
+            float2 a[4], c[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                a[q] = As[kk][ty + 16 * q];
+                c[q] = Bs[kk][tx + 16 * q];
+            }
+#pragma unroll
+            for (int r = 0; r < 4; r++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    re[r][q] = fmaf(a[r].x, c[q].x, fmaf(a[r].y, c[q].y, re[r][q]));
+                    im[r][q] = fmaf(a[r].x, c[q].y, fmaf(a[r].y, c[q].x, im[r][q]));
+                }
+        }
+        // no term is negative: enough is enough
+        float low = least;
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) low = fminf(low, inside(r, q) ? fminf(re[r][q], im[r][q]) : least);
+        if (__syncthreads_and(low >= least)) break;
+    }
+    unsigned weak = 0u;
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if ((re[r][q] > 0.f && re[r][q] < least) || (im[r][q] > 0.f && im[r][q] < least)) {
+                weak |= 1u << (4 * r + q);
+                const int c = tx + 16 * q;
+                atomicOr(&bits[ty + 16 * r][c >> 5], 1u << (c & 31));
+            }
+    const int any = __syncthreads_or((int)weak);
+    if (tid < 2 * kPT && i0 + (tid >> 1) < p.M && j0 + 32 * (tid & 1) < p.N)
+        mask[((long long)b * p.M + i0 + (tid >> 1)) * ((p.N + 31) / 32) + j0 / 32 + (tid & 1)] = bits[tid >> 1][tid & 1];
+    if (!any) return;
+    double2 acc[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) acc[r][q] = make_double2(0.0, 0.0);
+    for (int k0 = 0; k0 < p.K; k0 += kPK) {
+        for (int e = tid; e < kPK * kPT; e += 256) {
+            const int ra = kfastA ? e / kPK : e % kPT, ka = kfastA ? e % kPK : e / kPT;
+            const int rb = kfastB ? e / kPK : e % kPT, kb = kfastB ? e % kPK : e / kPT;
+            const double2 zero = make_double2(0.0, 0.0);
+            buf[0][ka][ra] = i0 + ra < p.M && k0 + ka < p.K ? A[(i0 + ra) * p.rsA + (k0 + ka) * p.ksA] : zero;
+            double2 v = j0 + rb < p.N && k0 + kb < p.K ? B[(j0 + rb) * p.rsB + (k0 + kb) * p.ksB] : zero;
+            if (p.conjB) v.y = -v.y;
+            buf[1][kb][rb] = v;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < kPK; kk++) {
+            double2 a[4], c[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                a[q] = buf[0][kk][ty + 16 * q];
+                c[q] = buf[1][kk][tx + 16 * q];
+            }
+#pragma unroll
+            for (int r = 0; r < 4; r++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) acc[r][q] = cfma(a[r], c[q], acc[r][q]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (!(weak >> (4 * r + q) & 1u)) continue;
+            double2* c = C + sC * b + (long long)(i0 + ty + 16 * r) * ldc + j0 + tx + 16 * q;
+            double2 v = z::cmul(alpha, acc[r][q]);
+            if (beta.x != 0.0 || beta.y != 0.0) v = cfma(beta, *c, v);
+            *c = v;
+        }
+}
 
 template <int S, typename TC>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -545,6 +699,7 @@ oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
                 for (int q = lane; q < 32 * kSeg; q += 32) {
                     const int r = q / kSeg, cc = q % kSeg;
                     if (row0 + r >= p.M || col0 + c0 + cc >= p.N) continue;
+                    if (p.mask && masked(p.mask, p.M, p.N, b, row0 + r, col0 + c0 + cc)) continue;
                     TC v = reinterpret_cast<const TC*>(stg + r * kStageRow)[cc];
                     TC* o = out + (long long)r * p.ldc + c0 + cc;
                     if (add1) {
@@ -597,7 +752,7 @@ static size_t al256(size_t x) { return (x + 255) / 256 * 256; }
 
 struct Shape {
     int nk, mt, nt, gA, gB;
-    size_t a, b, small_a, small_b;     // bytes per matrix: digits of A, of B, exponents
+    size_t a, b, small_a, small_b, m;  // bytes per matrix: digits of A, of B, exponents, a bit per element of C
     Shape(int S, int M, int N, int K) {
         const int tn = 256 / S;
         nk = (K + kTK - 1) / kTK;
@@ -609,8 +764,12 @@ struct Shape {
         b = (size_t)nt * nk * (2 * S * tn * kTK * 2);
         small_a = (size_t)gA * 16 * sizeof(int);
         small_b = ((size_t)gB * 16 + K) * sizeof(int);
+        m = (size_t)M * ((N + 31) / 32) * sizeof(unsigned);
     }
-    size_t bytes(int na, int nb) const { return al256(na * small_a) + al256(nb * small_b) + na * a + nb * b; }
+    // for na A, nb B and (nc > 0) the mask of nc C
+    size_t bytes(int na, int nb, int nc) const {
+        return al256(na * small_a) + al256(nb * small_b) + al256(nc * m) + na * a + nb * b;
+    }
 };
 
 // One product with S digits; element types double2 or float2 by operand.
@@ -631,8 +790,10 @@ static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const
     const long long ksB = opB == kOpN ? ldb : 1, rsB = opB == kOpN ? 1 : ldb;
     // as many matrices at a time as the workspace holds
     int step = batch;
-    while (step > 1 && sh.bytes(a1 ? 1 : step, b1 ? 1 : step) > ws.bytes) step = (step + 1) / 2;
-    if (sh.bytes(1, 1) > ws.bytes) return fail(SCW_ERR_NOMEM, "zgemm: workspace too small");
+    const bool parts = ws.parts && S == 8;
+    auto need = [&](int n) { return sh.bytes(a1 ? 1 : n, b1 ? 1 : n, parts ? n : 0); };
+    while (step > 1 && need(step) > ws.bytes) step = (step + 1) / 2;
+    if (need(1) > ws.bytes) return fail(SCW_ERR_NOMEM, "zgemm: workspace too small");
     for (int b0 = 0; b0 < batch; b0 += step) {
         const int nb = std::min(step, batch - b0);
         const int na_ = a1 ? 1 : nb, nb_ = b1 ? 1 : nb;
@@ -642,13 +803,15 @@ static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const
         int* gN = reinterpret_cast<int*>(cur);
         int* f = gN + (size_t)nb_ * sh.gB * 16;
         cur += al256(nb_ * sh.small_b);
+        unsigned* mask = parts ? reinterpret_cast<unsigned*>(cur) : nullptr;
+        if (parts) cur += al256(nb * sh.m);
         unsigned char* dA = reinterpret_cast<unsigned char*>(cur);
         unsigned char* dB = dA + na_ * sh.a;
         const TA* Ab = A + sA * b0;
         const TB* Bb = B + sB * b0;
         const int* sk = skip ? skip + b0 : nullptr;
         // with one A for several B the inner scaling would differ per matrix: none then
-        const bool scale = !(a1 && !b1);
+        const bool scale = !(a1 && !b1 && batch > 1);
         if (K > 0) {
             if (scale) {
                 SCW_CUDA_TRY(launch_chained(true, st, dim3((K + 7) / 8, nb_), 256, 0, oz_inner_kernel<TB>, Bb, ksB, rsB, sB, K, N,
@@ -660,10 +823,17 @@ static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const
         SplitArgs sp{Ab, Bb, rsA, ksA, rsB, ksB, sA, sB, opB == kOpC, M, N, K, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB,
                      na_ * sh.gA, f, eA, gN, dA, dB, b1 ? 0 : 1};
         SCW_CUDA_TRY(launch_chained(true, st, dim3(na_ * sh.gA + nb_ * sh.gB), kSplitThreads, 0, oz_split_kernel<S, TA, TB>, sp, sk));
+        if constexpr (S == 8) {
+            if (parts && K > 0)
+                SCW_CUDA_TRY(launch_chained(true, st, dim3((N + kPT - 1) / kPT, (M + kPT - 1) / kPT, nb), 256, 0, oz_parts_kernel, sp,
+                                            (int)a1, (int)b1, alpha, beta, C + sC * b0, ldc, sC, mask, sk));
+            else if (parts)
+                mask = nullptr;
+        }
         const long long tiles = (long long)sh.mt * sh.nt * nb;
         if (tiles > (1ll << 30)) return fail(SCW_ERR_ARG, "zgemm: too many tiles");
         GemmArgs g{dA, dB, eA, gN, M, N, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB, a1, b1, alpha, beta, diag,
-                   (void*)(C + sC * b0), ldc, sC, (int)tiles, ws.err};
+                   (void*)(C + sC * b0), ldc, sC, (int)tiles, ws.err, mask};
         SCW_CUDA_TRY(launch_chained(true, st, dim3((unsigned)std::min<long long>(tiles, sms)), kThreads, smem,
                                     oz_gemm_kernel<S, TC>, g, sk));
     }
@@ -691,7 +861,7 @@ scw_status ctx_gemm_ws(scw_ctx ctx, size_t one, size_t all, GemmWs& ws) {
     return st;
 }
 
-size_t zgemm_ws_bytes(int M, int N, int K, int batch) { return oz::Shape(8, M, N, K).bytes(batch, batch); }
+size_t zgemm_ws_bytes(int M, int N, int K, int batch) { return oz::Shape(8, M, N, K).bytes(batch, batch, batch); }
 
 scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const double2* A, int lda, long long sA,
                  const double2* B, int ldb, long long sB, double2 beta, double2* C, int ldc, long long sC, int batch,

@@ -35,6 +35,7 @@ struct GemmWs {
     char* base = nullptr;
     size_t bytes = 0;
     int* err = nullptr;
+    bool parts = false;                // every real and imaginary part as exact as an FP64 sum (see zgemm)
 };
 // cap on a workspace sized for a whole batch; larger batches go through it in parts
 constexpr size_t kGemmWsCap = 1024ull << 20;
@@ -46,8 +47,12 @@ scw_status ctx_gemm_ws(scw_ctx ctx, size_t one, size_t all, GemmWs& ws);
 // workspace that takes the whole batch in one pass
 size_t zgemm_ws_bytes(int M, int N, int K, int batch);
 // C = alpha A op(B) + beta C + diag I (row-major, batched by strides in elements), FP64 on the tensor
-// cores; op = identity, transpose or conjugate transpose.  C may be A or B.  Without a workspace
+// cores; op = identity, transpose or conjugate transpose.  Without a workspace
 // by gemm<double2> (plain products only).
+// The error is small against the largest |a_ik| |b_kj| of row i and column j (after the best scaling of the inner
+// index; none where one A, sA = 0, serves several B), not against the sum of all |a_ik| |b_kj|: what the solve needs.
+// With ws.parts it is small against the sums that make up each part of the result, as with FP64 arithmetic;
+// C must then not overlap A or B, which it may be otherwise.
 enum : int { kOpN = 0, kOpT = 1, kOpC = 2 };
 scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const double2* A, int lda, long long sA,
                  const double2* B, int ldb, long long sB, double2 beta, double2* C, int ldc, long long sC, int batch,
