@@ -1425,8 +1425,12 @@ scw_status scw_zgesv(scw_ctx ctx, int n, int nrhs, void* A, void* B, int batch, 
     scw::GemmWs ws;
     const size_t need = std::max(scw::zgemm_ws_bytes(n, n, 32, 1), scw::zgemm_ws_bytes(n, nrhs, 32, 1));
     scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, scw::kGemmWsCap)));
-    if (st == SCW_OK) st = scw::ctx_tc_flag(ctx);
-    ws = scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err};
+    if (st == SCW_ERR_NOMEM) {               // no room for the digits: on the FP64 pipes
+        st = SCW_OK;
+    } else if (st == SCW_OK) {
+        st = scw::ctx_tc_flag(ctx);
+        ws = scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err, true};
+    }
     if (st == SCW_OK) st = scw::zgetrf(ctx->stream, (double2*)A, n, n, n, nn, dpiv, n, dinfo, batch, ws, nullptr);
     if (st == SCW_OK)
         st = scw::zgetrs(ctx->stream, (const double2*)A, n, nn, dpiv, n, (double2*)B, nrhs, (long long)n * nrhs, batch,
