@@ -27,17 +27,17 @@ namespace scw {
 namespace z {
 
 // ------------------------------------------------------------------------------------
-// GEMM on the FP32 / FP64 pipes: C = alpha * op(A) * B + beta * C, op = identity.  64 x 64 tiles,
+// GEMM on the FP32 / FP64 pipes: C = alpha A B + beta C or alpha A B^T + beta C.  64 x 64 tiles,
 // 256 threads, each thread a 4 x 4 complex block; K staged 16 at a time through shared memory.
 // FP64 products run on the tensor cores (gemm_tc.cu, 20 to 35 times faster) and come here only
-// without a workspace: scw_zgemm while its stream is being captured.
+// without a workspace: while the stream of scw_zgemm is being captured, or where memory is short.
 // ------------------------------------------------------------------------------------
 constexpr int kGT = 64, kGK = 16;
 
 template <typename C>
 __global__ void __launch_bounds__(256)
 gemm_kernel(int M, int N, int K, C alpha, const C* __restrict__ A, int lda, long long sA, const C* __restrict__ B,
-            int ldb, long long sB, C beta, C* __restrict__ Cm, int ldc, long long sC, const int* __restrict__ skip) {
+            int ldb, long long sB, int tb, C beta, C* __restrict__ Cm, int ldc, long long sC, const int* __restrict__ skip) {
     if (skipped(skip, blockIdx.z)) return;
     __shared__ C As[kGK][kGT + 1];
     __shared__ C Bs[kGK][kGT + 1];
@@ -57,9 +57,9 @@ gemm_kernel(int M, int N, int K, C alpha, const C* __restrict__ A, int lda, long
             const int r = e / kGK, kk = e % kGK;         // A tile: rows i0 + r, cols k0 + kk
             const int gi = i0 + r, gk = k0 + kk;
             As[kk][r] = (gi < M && gk < K) ? A[(long long)gi * lda + gk] : zero;
-            const int kk2 = e / kGT, c = e % kGT;         // B tile: rows k0 + kk2, cols j0 + c
+            const int kk2 = tb ? e % kGK : e / kGT, c = tb ? e / kGK : e % kGT;         // B tile: rows k0 + kk2, cols j0 + c
             const int gk2 = k0 + kk2, gj = j0 + c;
-            Bs[kk2][c] = (gk2 < K && gj < N) ? B[(long long)gk2 * ldb + gj] : zero;
+            Bs[kk2][c] = (gk2 < K && gj < N) ? B[tb ? (long long)gj * ldb + gk2 : (long long)gk2 * ldb + gj] : zero;
         }
         __syncthreads();
 #pragma unroll
@@ -1110,6 +1110,16 @@ trevc_kernel(const C* __restrict__ T, C* __restrict__ X, int n, long long sA, co
     }
 }
 
+// copy of the batch entries that are not skipped
+__global__ void __launch_bounds__(256)
+copy_kernel(const double2* __restrict__ src, double2* __restrict__ dst, long long count, const int* __restrict__ skip) {
+    if (skipped(skip, blockIdx.y)) return;
+    src += count * blockIdx.y;
+    dst += count * blockIdx.y;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x)
+        dst[i] = src[i];
+}
+
 // Inverse Z of a unit upper triangular matrix given by its columns (column j = row j of X): row r of
 // Z X = I is z_r = 1, z_j = -sum_{i=r..j-1} z_i X_ij.  One warp per row.
 template <typename C>
@@ -1141,10 +1151,10 @@ trtri_kernel(const C* __restrict__ X, C* __restrict__ Z, int n, long long sA) {
 // ------------------------------------------------------------------------------------
 template <typename C>
 scw_status gemm(cudaStream_t st, int M, int N, int K, C alpha, const C* A, int lda, long long sA, const C* B, int ldb,
-                long long sB, C beta, C* Cm, int ldc, long long sC, int batch, const int* skip) {
+                long long sB, C beta, C* Cm, int ldc, long long sC, int batch, const int* skip, int opB) {
     if (M <= 0 || N <= 0 || batch <= 0) return SCW_OK;
     dim3 grid((N + z::kGT - 1) / z::kGT, (M + z::kGT - 1) / z::kGT, batch);
-    z::gemm_kernel<C><<<grid, 256, 0, st>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, Cm, ldc, sC, skip);
+    z::gemm_kernel<C><<<grid, 256, 0, st>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, opB == kOpT, beta, Cm, ldc, sC, skip);
     SCW_CUDA_TRY(cudaGetLastError());
     return SCW_OK;
 }
@@ -1354,11 +1364,16 @@ scw_status zgeev(cudaStream_t st, double2* A, double2* W, double2* V, int n, int
         SCW_CUDA_TRY(cudaGetLastError());
     }
     scw_status s = hqr_launch(st, A, Q, n, nn, W, status, skip, batch, active, wide);
-    // triangular eigenvectors as the rows of V, then V := Q V^T
+    // triangular eigenvectors as the rows of V, then Q V^T over A, copied to V
     if (s == SCW_OK) s = trevc<double2>(st, A, V, n, batch, skip);
+    GemmWs wp = ws;
+    wp.parts = true;
+    if (s == SCW_OK)
+        s = zgemm(st, n, n, n, make_double2(1, 0), Q, n, nn, V, n, nn, make_double2(0, 0), A, n, nn, batch, wp, skip, 0.0, kOpT);
     if (s != SCW_OK) return s;
-    return zgemm(st, n, n, n, make_double2(1, 0), Q, n, nn, V, n, nn, make_double2(0, 0), V, n, nn, batch, ws, skip, 0.0,
-                 kOpT);
+    z::copy_kernel<<<dim3((unsigned)std::min<long long>((nn + 255) / 256, 4096), batch), 256, 0, st>>>(A, V, nn, skip);
+    SCW_CUDA_TRY(cudaGetLastError());
+    return SCW_OK;
 }
 
 scw_status schur32(cudaStream_t st, float2* A, float2* Q, float2* W, int n, int batch, float2* work, int* status,
@@ -1378,7 +1393,7 @@ scw_status cgeev(cudaStream_t st, float2* A, float2* W, float2* V, int n, int ba
 }
 
 template scw_status gemm<double2>(cudaStream_t, int, int, int, double2, const double2*, int, long long, const double2*, int,
-                                  long long, double2, double2*, int, long long, int, const int*);
+                                  long long, double2, double2*, int, long long, int, const int*, int);
 template scw_status trevc<float2>(cudaStream_t, const float2*, float2*, int, int, const int*);
 
 }  // namespace scw
@@ -1466,10 +1481,15 @@ scw_status scw_zgeev(scw_ctx ctx, int n, void* A, void* W, void* V, int batch, i
     scw::DevBuf wbuf;
     const size_t need = scw::zgemm_ws_bytes(n, n, n, 1);
     scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, scw::kGemmWsCap)));
-    if (st == SCW_OK) st = scw::ctx_tc_flag(ctx);
+    scw::GemmWs ws;                          // without room for the digits: on the FP64 pipes
+    if (st == SCW_ERR_NOMEM) {
+        st = SCW_OK;
+    } else if (st == SCW_OK) {
+        st = scw::ctx_tc_flag(ctx);
+        ws = scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err};
+    }
     if (st == SCW_OK)
-        st = scw::zgeev(ctx->stream, (double2*)A, (double2*)W, (double2*)V, n, batch, work, dst, nullptr, true,
-                        scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err});
+        st = scw::zgeev(ctx->stream, (double2*)A, (double2*)W, (double2*)V, n, batch, work, dst, nullptr, true, ws);
     ctx->launches += 4;
     std::vector<int> status(batch, 0);
     if (st == SCW_OK) {

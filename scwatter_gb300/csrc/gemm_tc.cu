@@ -872,8 +872,8 @@ scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const doub
                                     ldb, sB, beta, C, ldc, sC, skip));
         return SCW_OK;
     }
-    if (!ws.base && (diag != 0.0 || opB != kOpN)) return fail(SCW_ERR_ARG, "zgemm: this product needs a workspace");
-    if (!ws.base) return gemm<double2>(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, skip);
+    if (!ws.base && (diag != 0.0 || opB == kOpC)) return fail(SCW_ERR_ARG, "zgemm: this product needs a workspace");
+    if (!ws.base) return gemm<double2>(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, skip, opB);
     return oz::run<8>(st, M, N, K, alpha, A, lda, sA, B, ldb, sB, opB, beta, diag, C, ldc, sC, batch, ws, skip);
 }
 

@@ -48,7 +48,7 @@ scw_status ctx_gemm_ws(scw_ctx ctx, size_t one, size_t all, GemmWs& ws);
 size_t zgemm_ws_bytes(int M, int N, int K, int batch);
 // C = alpha A op(B) + beta C + diag I (row-major, batched by strides in elements), FP64 on the tensor
 // cores; op = identity, transpose or conjugate transpose.  Without a workspace
-// by gemm<double2> (plain products only).
+// by gemm<double2> (no conjugate transpose, no diagonal).
 // The error is small against the largest |a_ik| |b_kj| of row i and column j (after the best scaling of the inner
 // index; none where one A, sA = 0, serves several B), not against the sum of all |a_ik| |b_kj|: what the solve needs.
 // With ws.parts it is small against the sums that make up each part of the result, as with FP64 arithmetic;
@@ -66,10 +66,10 @@ scw_status gemm32(cudaStream_t st, int n, double alpha, const TA* A, const TB* B
 scw_status cgemm(cudaStream_t st, int M, int N, int K, float alpha, const float2* A, int lda, long long sA, int opA,
                  const float2* B, int ldb, long long sB, int opB, bool add, float2* C, int ldc, long long sC, int batch);
 
-// C = alpha A B + beta C (row-major, batched by strides in elements)
+// C = alpha A op(B) + beta C, op = identity or transpose (row-major, batched by strides in elements)
 template <typename C>
 scw_status gemm(cudaStream_t st, int M, int N, int K, C alpha, const C* A, int lda, long long sA, const C* B, int ldb,
-                long long sB, C beta, C* Cm, int ldc, long long sC, int batch, const int* skip = nullptr);
+                long long sB, C beta, C* Cm, int ldc, long long sC, int batch, const int* skip = nullptr, int opB = kOpN);
 // in-place LU with partial pivoting of the first n columns of n x ncols matrices (leading dimension lda;
 // further columns are carried along as right-hand sides); info[b] = first zero pivot + 1
 scw_status zgetrf(cudaStream_t st, double2* A, int n, int ncols, int lda, long long sA, int* piv, long long sP, int* info,
