@@ -1376,20 +1376,23 @@ scw_status zgeev(cudaStream_t st, double2* A, double2* W, double2* V, int n, int
     return SCW_OK;
 }
 
-scw_status schur32(cudaStream_t st, float2* A, float2* Q, float2* W, int n, int batch, float2* work, int* status,
-                   const GemmWs& ws, int share) {
+scw_status schur32(cudaStream_t st, float2* A, float2* Q, float2* W, int n, int batch, float2* work, int* status, int share) {
     scw_status s = hess32(st, A, Q, n, batch, work, share);
     if (s == SCW_OK) s = hqr32(st, A, Q, n, W, status, batch, g_qr_cluster.load(), share);
     return s;
 }
 
-scw_status cgeev(cudaStream_t st, float2* A, float2* W, float2* V, int n, int batch, float2* work, int* status,
-                 const GemmWs& ws, int share) {
+// The product of Schur vectors and triangular eigenvectors on the CUDA cores: digit products of 30 bits would lose the
+// vectors' small entries (n = 300: 13.0 ms either way).
+scw_status cgeev(cudaStream_t st, float2* A, float2* W, float2* V, int n, int batch, float2* work, int* status, int share) {
+    const long long nn = (long long)n * n;
     float2* Q = work;                        // batch * n * n: Schur vectors
-    scw_status s = schur32(st, A, Q, W, n, batch, work + (long long)n * n * batch, status, ws, share);
+    scw_status s = schur32(st, A, Q, W, n, batch, work + nn * batch, status, share);
     if (s == SCW_OK) s = trevc32(st, A, V, n, batch);
+    if (s == SCW_OK) s = cgemm(st, n, n, n, 1.f, Q, n, nn, kOpN, V, n, nn, kOpT, false, A, n, nn, batch);
     if (s != SCW_OK) return s;
-    return gemm32(st, n, 1.0, Q, V, kOpT, 0.0, 0.0, V, batch, ws, nullptr);
+    SCW_CUDA_TRY(cudaMemcpyAsync(V, A, sizeof(float2) * nn * batch, cudaMemcpyDeviceToDevice, st));
+    return SCW_OK;
 }
 
 template scw_status gemm<double2>(cudaStream_t, int, int, int, double2, const double2*, int, long long, const double2*, int,
@@ -1519,13 +1522,7 @@ scw_status scw_cgeev(scw_ctx ctx, int n, void* A, void* W, void* V, int batch, i
         cudaFree(work);
         return fail(SCW_ERR_NOMEM, "scw_cgeev: workspace");
     }
-    scw::DevBuf wbuf;
-    const size_t need = scw::zgemm_ws_bytes(n, n, n, 1);
-    scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, scw::kGemmWsCap)));
-    if (st == SCW_OK) st = scw::ctx_tc_flag(ctx);
-    if (st == SCW_OK)
-        st = scw::cgeev(ctx->stream, (float2*)A, (float2*)W, (float2*)V, n, batch, work, dst,
-                        scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err}, 1);
+    scw_status st = scw::cgeev(ctx->stream, (float2*)A, (float2*)W, (float2*)V, n, batch, work, dst, 1);
     ctx->launches += 5;
     std::vector<int> status(batch, 0);
     if (st == SCW_OK) {

@@ -690,7 +690,7 @@ scw_status geev_mixed(cudaStream_t st, double2* A, double2* lam, double2* V, int
     MX_LAUNCHED(2);
     // FP32 Householder + QR: T in S0, Schur vectors Q in S1, eigenvalues lam32.  Triangular
     // eigenvectors Xt (rows of S2) and their inverse (S3): X = Q Xt, X^-1 = Xt^-1 Q^H
-    MX_TRY(schur32(st, w.S0, w.S1, w.lam32, n, Z, w.hp, w.qr, ws, prm.share));
+    MX_TRY(schur32(st, w.S0, w.S1, w.lam32, n, Z, w.hp, w.qr, prm.share));
     MX_TRY(trevc32(st, w.S0, w.S2, n, Z));
     MX_TRY(trtri32(st, w.S2, w.S3, n, Z));
     MX_TRY(gemm32(st, n, 1.0, w.S1, w.S2, kOpT, 0.0, 0.0, V, Z, ws, nullptr));

@@ -82,8 +82,7 @@ scw_status zgetrs(cudaStream_t st, const double2* LU, int n, long long sA, const
                   int nrhs, long long sB, int batch, const GemmWs& ws, const int* skip);
 // Schur form A = Q T Q^H in FP32 (T over A, eigenvalues W); work: hess32_ws_elems(n) per matrix; share:
 // solves of this size that run at the same time (lanes of a batch)
-scw_status schur32(cudaStream_t st, float2* A, float2* Q, float2* W, int n, int batch, float2* work, int* status,
-                   const GemmWs& ws, int share);
+scw_status schur32(cudaStream_t st, float2* A, float2* Q, float2* W, int n, int batch, float2* work, int* status, int share);
 // its stages: Hessenberg form of A with Q (hess32.cu), then the QR iteration with vectors accumulated into Z
 // (hqr32.cu; ctas: CTAs per matrix, 0 = chosen by size and batch)
 size_t hess32_ws_elems(int n);
@@ -106,8 +105,7 @@ constexpr int kWideMinN = 128;
 scw_status zgeev(cudaStream_t st, double2* A, double2* W, double2* V, int n, int batch, double2* work, int* status,
                  const int* skip, bool wide, const GemmWs& ws);
 // the same in FP32 (the first stage of the mixed solver); work >= batch (n^2 + hess32_ws_elems(n))
-scw_status cgeev(cudaStream_t st, float2* A, float2* W, float2* V, int n, int batch, float2* work, int* status,
-                 const GemmWs& ws, int share);
+scw_status cgeev(cudaStream_t st, float2* A, float2* W, float2* V, int n, int batch, float2* work, int* status, int share);
 // Hessenberg form of A (in place, n x n per batch entry) and the unitary Q (A = Q H Q^H);
 // work >= batch * 3 n
 scw_status zgehrd(cudaStream_t st, double2* A, double2* Q, int n, int batch, double2* work);

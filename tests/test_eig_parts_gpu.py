@@ -14,7 +14,7 @@ def ctx():
     return ev.Context(0)
 
 
-@pytest.mark.parametrize("entry,real,decades", [("scw_zgeev", np.float64, 24)])
+@pytest.mark.parametrize("entry,real,decades", [("scw_zgeev", np.float64, 24), ("scw_cgeev", np.float32, 9)])
 @pytest.mark.parametrize("n,batch", [(2, 1), (33, 2), (70, 1), (130, 2)])
 def test_triangular(ctx, entry, real, decades, n, batch):
     import torch
