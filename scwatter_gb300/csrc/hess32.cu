@@ -252,9 +252,7 @@ hess_panel_kernel(float2* __restrict__ A, int n, long long sA, int j0, int ib, i
             const float bt = -copysignf(sqrtf(alpha.x * alpha.x + alpha.y * alpha.y + x2), alpha.x);
             tau = make_float2((bt - alpha.x) / bt, -alpha.y / bt);
             beta = make_float2(bt, 0.f);
-            const float2 d = csub(alpha, beta);          // |d| >= |b|: no smaller than what x2 is made of
-            const float id = 1.f / cabs2(d);
-            scal = make_float2(d.x * id, -d.y * id);
+            scal = cdiv(make_float2(1.f, 0.f), csub(alpha, beta));     // (1 / |d|^2 would overflow below 5e-20)
         }
         const bool live = tau.x != 0.f || tau.y != 0.f;
         // column j of the Hessenberg form

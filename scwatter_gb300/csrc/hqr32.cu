@@ -71,28 +71,39 @@ __device__ __forceinline__ void rot32_rows(float c, float2 s, float2& x, float2&
 }
 __device__ __forceinline__ float2 conjf2(float2 s) { return make_float2(s.x, -s.y); }
 
-// rotation (c, s) with [c, s; -conj(s), c] [f; g] = [r; 0], from two reciprocal square roots
+// The power of two that brings a largest value `big` to [1, 2), and its inverse (within what a float can be scaled by).
+__device__ __forceinline__ void unit_scale(float big, float& up, float& back) {
+    const int e = min(max((int)(__float_as_uint(big) >> 23), 1), 253);
+    up = __uint_as_float((unsigned)(254 - e) << 23);
+    back = __uint_as_float((unsigned)e << 23);
+}
+
+// rotation (c, s) with [c, s; -conj(s), c] [f; g] = [r; 0], from two reciprocal square roots of scaled values: the squares
+// of values near the ends of the range would leave it, or lose the digits that make the rotation unitary
 __device__ __forceinline__ void givens32(float2 f, float2 g, float& c, float2& s, float2& r) {
-    const float gf = cabs2(g), ff = cabs2(f);
-    if (gf == 0.f) {
+    float up, back;
+    unit_scale(fmaxf(fmaxf(fabsf(f.x), fabsf(f.y)), fmaxf(fabsf(g.x), fabsf(g.y))), up, back);
+    const float2 fu = make_float2(f.x * up, f.y * up), gu = make_float2(g.x * up, g.y * up);
+    const float gf = cabs2(gu), ff = cabs2(fu);
+    if (gf < 1e-30f) {                        // |g| < 1e-15 |f|, or both zero
         c = 1.f;
         s = make_float2(0.f, 0.f);
         r = f;
         return;
     }
-    if (ff == 0.f) {
+    if (ff < 1e-30f) {
         const float ig = rsqrtf(gf);
         c = 0.f;
-        s = make_float2(g.x * ig, -g.y * ig);
-        r = make_float2(gf * ig, 0.f);
+        s = make_float2(gu.x * ig, -gu.y * ig);
+        r = make_float2(gf * ig * back, 0.f);
         return;
     }
     const float iaf = rsqrtf(ff), id = rsqrtf(ff + gf);
     c = ff * iaf * id;
-    const float2 fs = make_float2(f.x * iaf, f.y * iaf);
-    const float2 t = cmulc(g, fs);
+    const float2 fs = make_float2(fu.x * iaf, fu.y * iaf);
+    const float2 t = cmulc(gu, fs);
     s = make_float2(t.x * id, t.y * id);
-    const float d = (ff + gf) * id;
+    const float d = (ff + gf) * id * back;
     r = make_float2(fs.x * d, fs.y * d);
 }
 
@@ -103,17 +114,17 @@ __device__ __forceinline__ float rsqrt_fast(float x) {
     return r;
 }
 __device__ __forceinline__ void givens32_fast(float2 f, float2 g, float& c, float2& s, float2& r) {
-    const float gf = cabs2(g), ff = cabs2(f);
-    if (fminf(gf, ff) < 1e-36f) {
+    const float gf = cabs2(g), ff = cabs2(f), sum = ff + gf;
+    if (fminf(gf, ff) < 1e-30f || sum > 1e36f) {
         givens32(f, g, c, s, r);
         return;
     }
-    const float iaf = rsqrt_fast(ff), id = rsqrt_fast(ff + gf);
+    const float iaf = rsqrt_fast(ff), id = rsqrt_fast(sum);
     const float2 fs = make_float2(f.x * iaf, f.y * iaf);
     const float2 t = cmulc(g, fs);
     c = ff * iaf * id;
     s = make_float2(t.x * id, t.y * id);
-    const float d = (ff + gf) * id;
+    const float d = sum * id;
     r = make_float2(fs.x * d, fs.y * d);
 }
 
@@ -127,8 +138,14 @@ __device__ __forceinline__ float2 shift32(const float2* T, int ld, int l, int ih
         return make_float2(0.75f * fabsf(T[(l + 1) * ld + l].x) + a.x, a.y);
     }
     const float2 a = T[(ihi - 1) * ld + ihi - 1], b = T[(ihi - 1) * ld + ihi], c = T[ihi * ld + ihi - 1];
-    const float2 half = make_float2(0.5f * (a.x - d.x), 0.5f * (a.y - d.y));
-    const float2 bc = cmul(b, c);
+    // scaled by a power of two to about 1: the root is of the entries' fourth powers
+    const float2 h0 = make_float2(0.5f * (a.x - d.x), 0.5f * (a.y - d.y));
+    const float big = fmaxf(fmaxf(fmaxf(fabsf(h0.x), fabsf(h0.y)), fmaxf(fabsf(b.x), fabsf(b.y))), fmaxf(fabsf(c.x), fabsf(c.y)));
+    float up, back;
+    unit_scale(big, up, back);
+    auto scaled = [&](float2 v) { return make_float2(v.x * up, v.y * up); };
+    const float2 half = scaled(h0);
+    const float2 bc = cmul(scaled(b), scaled(c));
     const float2 q = cfma(half, half, bc);
     const float m2 = cabs2(q);
     float2 sq = make_float2(0.f, 0.f);
@@ -141,7 +158,7 @@ __device__ __forceinline__ float2 shift32(const float2* T, int ld, int l, int ih
     const float dd = cabs2(den);
     if (dd == 0.f) return d;
     const float2 x = cmulc(den, bc);                    // bc / den
-    return make_float2(d.x - __fdividef(x.x, dd), d.y - __fdividef(x.y, dd));
+    return make_float2(fmaf(-back, __fdividef(x.x, dd), d.x), fmaf(-back, __fdividef(x.y, dd), d.y));
 }
 
 // hqr_deflates of the window's entry (k, k - 1), all entries loaded at once and without exact divisions
@@ -185,19 +202,23 @@ __device__ __forceinline__ void sweep_columns(float2* X, int row, bool live, int
 // Householder vector of x (x_0 in lane 0 .., zero from lane cnt on): returns tau, beta in lane 0's terms; x
 // becomes w with w_0 = 1.  (I - tau w w^H)^H x = beta e_0.
 __device__ __forceinline__ void reflector32(float2& x, int lane, int cnt, float2& tau, float& beta, bool& none) {
+    float up, back;                            // (scaled, as in givens32)
+    unit_scale(__uint_as_float(__reduce_max_sync(0xffffffffu, lane < cnt ? __float_as_uint(fmaxf(fabsf(x.x), fabsf(x.y))) : 0u)), up, back);
+    x = make_float2(x.x * up, x.y * up);
     float n2 = (lane >= 1 && lane < cnt) ? cabs2(x) : 0.f;
     for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
     const float ax = __shfl_sync(0xffffffffu, x.x, 0), ay = __shfl_sync(0xffffffffu, x.y, 0);
     none = n2 == 0.f && ay == 0.f;
     if (none) {
         tau = make_float2(0.f, 0.f);
-        beta = ax;
+        beta = ax * back;
         return;
     }
     beta = -copysignf(sqrtf(ax * ax + ay * ay + n2), ax);
     tau = make_float2((beta - ax) / beta, -ay / beta);
     const float2 scal = cdiv(make_float2(1.f, 0.f), make_float2(ax - beta, ay));
     x = lane == 0 ? make_float2(1.f, 0.f) : lane < cnt ? cmul(x, scal) : make_float2(0.f, 0.f);
+    beta *= back;
 }
 
 __device__ __forceinline__ void pair_sync() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
