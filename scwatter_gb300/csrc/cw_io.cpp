@@ -39,6 +39,7 @@ scw_status DevBuf::reserve(size_t n) {
     size_t want = n + n / 4;
     cudaError_t e = cudaMalloc(&ptr, want);
     if (e != cudaSuccess) {
+        cudaGetLastError();                  // callers that go on without it check their launches with it
         ptr = nullptr;
         return fail(SCW_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
@@ -60,6 +61,7 @@ scw_status PinnedBuf::reserve(size_t n) {
     size_t want = n + n / 4;
     cudaError_t e = cudaMallocHost(&ptr, want);
     if (e != cudaSuccess) {
+        cudaGetLastError();
         ptr = nullptr;
         return fail(SCW_ERR_NOMEM, std::string("cudaMallocHost: ") + cudaGetErrorString(e));
     }
