@@ -850,6 +850,18 @@ static scw_status sep_eval_three(scw_sep s, const SepEvalPlan* plans, float* con
     }
     if ((st = ctx_tc_flag(ctx)) != SCW_OK) return st;      // cleared before any of the streams may raise it
     const cudaStream_t main_stream = ctx->stream;
+    // However this returns, the context is on its own stream again, and after an error nothing that was launched on
+    // the others still works on the shared buffers.
+    struct Restore {
+        scw_sep s;
+        cudaStream_t main;
+        bool failed = true;
+        ~Restore() {
+            s->ctx->stream = main;
+            if (failed)
+                for (cudaStream_t q : s->plane_stream) cudaStreamSynchronize(q);
+        }
+    } restore{s, main_stream};
     SCW_CUDA_TRY(cudaEventRecord(s->plane_event[0], main_stream));
     // xz and yz planes over the same z-values have the same C: one stage 1 for both, two launches and 28 us of the
     // device less (3 slices of 20x20 harmonics on three 256x256 planes: 143 -> 133 us, a smaller set 97 -> 92)
@@ -874,21 +886,20 @@ static scw_status sep_eval_three(scw_sep s, const SepEvalPlan* plans, float* con
     };
     // the main stream's plane first: its copy to the host, the first one, then waits for nothing while the others run
     // (256 x 256 planes: 127 us launched last, 119 first; 40 x 40: 83 and 69)
-    for (int k = 0; k < 3 && st == SCW_OK; k++) {
+    for (int k = 0; k < 3; k++) {
         if (k) {
             ctx->stream = s->plane_stream[k - 1];
             SCW_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, s->plane_event[0], 0));
         }
-        st = record(k);
+        if ((st = record(k)) != SCW_OK) return st;
         if (k) {
-            // also after an error: the context's next work must not overtake what was launched
-            const cudaError_t e = cudaEventRecord(s->plane_event[k], ctx->stream);
+            SCW_CUDA_TRY(cudaEventRecord(s->plane_event[k], ctx->stream));
             ctx->stream = main_stream;
-            SCW_CUDA_TRY(e);
             done[k] = s->plane_event[k];
         }
     }
-    return st;
+    restore.failed = false;
+    return SCW_OK;
 }
 
 // ------------------------------------------------------------------------------------
@@ -1405,17 +1416,17 @@ scw_status scw_sep_gpu_cw_evaluate(scw_sep s, float* E_xy, float* E_xz, float* E
     if ((st = scw::sep_eval_plan(s, 2, y_start, z_start, x, d, d, 0.f, N, N, 1, method, plans[2])) != SCW_OK) return st;
     cudaEvent_t done[3];
     st = scw::sep_eval_three(s, plans, dE, done);
-    const bool one_by_one = st == SCW_ERR_NOMEM && !done[1];      // no room for three: the planes in turn
-    if (one_by_one) {
+    if (st == SCW_ERR_NOMEM) {                // no room for three: the planes in turn
         st = SCW_OK;
+        for (auto& e : done) e = nullptr;
         const float a0[3] = {x_start, x_start, y_start}, b0[3] = {y_start, z_start, z_start}, c[3] = {z, y, x};
         for (int q = 0; q < 3 && st == SCW_OK; q++) st = scw::sep_eval(s, q, a0[q], b0[q], c[q], d, d, 0.f, N, N, 1, dE[q], method);
     }
+    if (st != SCW_OK) return st;
     for (int q = 0; q < 3; q++) {
         if (done[q]) SCW_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, done[q], 0));
-        if (st == SCW_OK) SCW_CUDA_TRY(cudaMemcpyAsync(out[q], dE[q], plane * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        SCW_CUDA_TRY(cudaMemcpyAsync(out[q], dE[q], plane * 4, cudaMemcpyDeviceToHost, ctx->stream));
     }
-    if (st != SCW_OK) return st;
     return scw_ctx_synchronize(ctx);
 }
 

@@ -87,3 +87,22 @@ def test_product_without_room_for_its_digits(shim):
     ctx.synchronize()
     assert (C - A @ B).abs().max().item() < 1e-12
     """)
+
+
+@pytest.mark.parametrize("at", range(3))
+def test_planes_leave_the_context_on_its_stream(shim, at):
+    _child(shim, """
+    ref = planes(new_set())
+    s = new_set()
+    planes(s)
+    mine = stream()
+    shim.shim_wait(%d)                 # of the waits of the second and third plane
+    try:
+        planes(s)
+        raise SystemExit("no error")
+    except _lib.ScwError as e:
+        assert e.status == 4
+    assert stream() == mine
+    del s
+    assert same(planes(new_set()), ref)
+    """ % at)
