@@ -517,8 +517,8 @@ static scw_status launch_planes_tc(scw_waves w, const std::vector<PlaneGeom>& pl
     char* d = (char*)ctx->desc.ptr;
     const ptc::Waves waves{w->kre, w->kim, w->zref, w->amp, (long long)w->n};
     return ptc::launch(ctx, (const ptc::Plane*)d, (const ptc::Item*)(d + items_off), (int)P.items.size(),
-                       (const ptc::Tile*)(d + tiles_off), (int)P.tiles.size(), P.max_rows, waves,
-                       (double2*)ctx->scratch.ptr);
+                       (const ptc::Tile*)(d + tiles_off), (int)P.tiles.size(), P.max_rows,
+                       P.items.front().w1 - P.items.front().w0, waves, (double2*)ctx->scratch.ptr);      // longest first
 }
 
 static scw_status launch_planes(scw_waves w, std::vector<PlaneGeom>& planes) {

@@ -29,8 +29,8 @@
 //     kernel, in a fixed order.  32 additions to a growing sum, not 1024: a run of 1024 waves loses less to rounding than the
 //     summation kernel's 256 additions (45 against 64 roundings of a sum of 256 waves, over 4096 waves that all add up).
 //     One FP32 sum of 4096 waves lost 1.5 times as much as that kernel.
-// 409 600 waves x 3 planes of 200 x 200 points: 19.4 ms by the summation kernel, 4.50 ms here; 20 736 waves a layer on a
-// 101 x 77 x 50 volume: 5.10 -> 1.39 ms (4.30 and 1.30 with one FP32 sum per 4096 waves, 4.45 and 1.33 with runs of 64 chunks:
+// 409 600 waves x 3 planes of 200 x 200 points: 19.4 ms by the summation kernel, 4.45 ms here; 20 736 waves a layer on a
+// 101 x 77 x 50 volume: 5.10 -> 1.39 ms (4.30 and 1.30 with one FP32 sum per 4096 waves:
 // tensor memory answers late, and sums that are late hold up the MMAs).  A chunk takes about 1600 clocks: 700 of them are MMA reads of shared memory and
 // 450 the stores of the operands, and the warps that build these issue half of the time.  Measured in the
 // second case on the way: K-major operands with a sine and cosine for every point and wave 2.9 ms, this
@@ -87,13 +87,6 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
     return r;
 }
 __device__ __forceinline__ F2 neg2(F2 a) { return F2{a.v ^ 0x8000000080000000ull}; }
-// the same value in FP64, by integer operations but for subnormal and non-finite ones (a conversion takes 19 clocks of
-// the SM's FP64 pipe)
-__device__ __forceinline__ double widen(float x) {
-    const unsigned b = __float_as_uint(x), m = b & 0x7fffffffu;
-    if (m != 0u && m - 0x00800000u >= 0x7f000000u) return (double)x;
-    return __hiloint2double((int)(m ? (b & 0x80000000u) | ((m >> 3) + 0x38000000u) : b), (int)(b << 29));
-}
 // hi + x, its rounding error added to lo (Knuth's two-sum; what lo holds where hi is not finite means nothing)
 __device__ __forceinline__ void add_exact2(F2& hi, F2& lo, F2 x) {
     const F2 m = both(-1.f), s = add2(hi, x), b = fma2(hi, m, s), t = fma2(b, m, s);
@@ -239,6 +232,8 @@ __device__ __forceinline__ void split8(const F2 (&v)[4], uint4& h, uint4& l) {
     l = make_uint4(half2(lo[0].x(), lo[1].x()), half2(lo[2].x(), lo[3].x()), half2(lo[0].y(), lo[1].y()), half2(lo[2].y(), lo[3].y()));
 }
 
+// kLong: items of more than kRun chunks among them
+template <bool kLong>
 __global__ void __launch_bounds__(kThreads, 1)
 plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items, Waves W, double2* __restrict__ partials,
                 int* __restrict__ err) {
@@ -292,7 +287,7 @@ plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        tmem_alloc(&S.tmem, kCols);
+        tmem_alloc(&S.tmem, kLong ? kCols : kSumCol);
         tmem_relinquish();
     }
     fence_proxy_async();
@@ -525,6 +520,7 @@ plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items
                 mbar_arrive(&S.acc_empty[buf]);
                 mbar_arrive(&S.wave_empty[s]);
             }
+            if (!kLong) continue;
             // the end of a run: into the sums in tensor memory, and these at the end (and every kMaxRun waves) into
             // the item's FP64 partial sums, each element always by this thread
             const bool due = (ch + 1) % (kMaxRun / kChunk) == 0, end = ch + 1 == nchunk;
@@ -568,11 +564,12 @@ plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items
                     const bool add = ch >= kMaxRun / kChunk;
                     const int slot = S.item.slot, jr0 = S.item.jr0, i0 = S.item.i0, rows = min(32, S.item.jr1 - jr0 - half * 32);
                     const int Ni = S.plane.Ni;
-                    float2* const E = reinterpret_cast<float2*>(S.plane.out);
                     const int i = r - comp * kTileI;
                     const bool out = comp < 3 && i < min(kTileI, Ni - i0);
+                    float2* E = reinterpret_cast<float2*>(S.plane.out) + ((long long)(jr0 + half * 32) * Ni + i0 + i) * 3 + comp;
+                    double2* o = partials + ((long long)slot * kTileJ + half * 32) * (3 * kTileI) + r;
 #pragma unroll 1
-                    for (int c4 = 0; c4 < rows; c4 += 4) {
+                    for (int c4 = 0; c4 < rows; c4 += 4, E += 12 * Ni, o += 4 * 3 * kTileI) {
                         uint32_t xh[4], xl[4], yh[4], yl[4];
                         tmem_ld4(sum + c4, xh);
                         tmem_ld4(sum + c4 + kSumLow, xl);
@@ -584,35 +581,44 @@ plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items
                         tmem_ld_wait4(yl);
 #pragma unroll
                         for (int u = 0; u < 4; u++) {
-                            const int j = half * 32 + c4 + u;
                             if (c4 + u >= rows || !out) continue;
                             const float ah = __uint_as_float(xh[u]), al = low_word(ah, __uint_as_float(xl[u]));
                             const float bh = __uint_as_float(yh[u]), bl = low_word(bh, __uint_as_float(yl[u]));
                             if (slot < 0) {
-                                E[((long long)(jr0 + j) * Ni + i0 + i) * 3 + comp] = make_float2(ah + al, bh + bl);
+                                E[(long long)u * 3 * Ni] = make_float2(ah + al, bh + bl);
                             } else {
-                                double2* o = partials + ((long long)slot * kTileJ + j) * (3 * kTileI) + r;
-                                double2 v = make_double2(widen(ah), widen(bh));
-                                if (!first) v = make_double2(v.x + widen(al), v.y + widen(bl));
-                                if (add) v = make_double2(o->x + v.x, o->y + v.y);
-                                *o = v;
+                                double2* q = o + u * 3 * kTileI;
+                                double2 v = make_double2((double)ah, (double)bh);
+                                if (!first) v = make_double2(v.x + (double)al, v.y + (double)bl);
+                                if (add) v = make_double2(q->x + v.x, q->y + v.y);
+                                *q = v;
                             }
                         }
                     }
                 }
             }
         }
-        if (nchunk == 0 && comp < 3) {              // a region without waves: zeros
-            const int i = r - comp * kTileI;
-            for (int j = half * 32; j < min(nrow, half * 32 + 32); j++)
-                if (i < ncol) reinterpret_cast<float2*>(g.out)[((long long)(it.jr0 + j) * g.Ni + it.i0 + i) * 3 + comp] = make_float2(0.f, 0.f);
+        const int i = r - comp * kTileI;
+        if ((!kLong || nchunk == 0) && comp < 3 && i < ncol && !S.abort) {
+            // one run (or no wave at all): from the registers
+#pragma unroll
+            for (int c = 0; c < 32; c++) {
+                const int j = half * 32 + c;
+                if (j < nrow) {
+                    const float x = c & 1 ? re[c / 2].y() : re[c / 2].x(), y = c & 1 ? im[c / 2].y() : im[c / 2].x();
+                    if (it.slot >= 0)
+                        partials[((long long)it.slot * kTileJ + j) * (3 * kTileI) + r] = make_double2((double)x, (double)y);
+                    else
+                        reinterpret_cast<float2*>(g.out)[((long long)(it.jr0 + j) * g.Ni + it.i0 + i) * 3 + comp] = make_float2(x, y);
+                }
+            }
         }
     }
     __syncthreads();
     if (tid == 0 && S.abort) atomicExch(err, 1);
     if (warp == 0) {
         tc_fence_after();
-        tmem_dealloc(tmem, kCols);
+        tmem_dealloc(tmem, kLong ? kCols : kSumCol);
     }
 }
 
@@ -635,15 +641,18 @@ plain_tc_reduce_kernel(const Plane* __restrict__ planes, const Tile* __restrict_
 }
 
 scw_status launch(scw_ctx ctx, const Plane* planes, const Item* items, int nitems, const Tile* tiles, int ntiles, int max_rows,
-                  const Waves& W, double2* partials) {
+                  long long longest, const Waves& W, double2* partials) {
     constexpr size_t smem = kBufs * kBufBytes + sizeof(Smem);
     static_assert(smem <= 227 * 1024, "shared memory of the plain evaluator");
-    SCW_CUDA_TRY(cudaFuncSetAttribute(plain_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // items of one run each, as small evaluations have, go from registers to memory: 9604 waves on 30 x 60 x 10 points, 750 items,
+    // take 94 us, by the kernel for long ones 121
+    auto kernel = longest > kRun * kChunk ? plain_tc_kernel<true> : plain_tc_kernel<false>;
+    SCW_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     scw_status st = ctx_tc_flag(ctx);
     if (st != SCW_OK) return st;
     {
         LaunchTimer lt(ctx, "plain_tc_kernel");
-        plain_tc_kernel<<<nitems, kThreads, smem, ctx->stream>>>(planes, items, W, partials, ctx->tc_err);
+        kernel<<<nitems, kThreads, smem, ctx->stream>>>(planes, items, W, partials, ctx->tc_err);
     }
     SCW_CUDA_TRY(cudaGetLastError());
     ctx->launches++;

@@ -40,9 +40,9 @@ struct Waves {
     long long n;
 };
 
-// partials: kTileJ x 3 kTileI double2 per slot
+// longest: the most waves of an item; partials: kTileJ x 3 kTileI double2 per slot
 scw_status launch(scw_ctx ctx, const Plane* planes, const Item* items, int nitems, const Tile* tiles, int ntiles, int max_rows,
-                  const Waves& W, double2* partials);
+                  long long longest, const Waves& W, double2* partials);
 
 }  // namespace ptc
 }  // namespace scw
