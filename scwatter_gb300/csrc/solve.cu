@@ -551,7 +551,6 @@ scw_status plan_solve(const scw_solve_params* prm, int Zs, int Y, int X, SolvePl
     p.n1 = n1r;
     p.external = prm->external != 0;
     p.pz = prm->pz != 0;
-    p.eig_mixed = prm->eig_fp64 == 0 && 2 * (long long)p.MF <= mx::kMaxN;
     p.zb.resize(ZL);
     p.zb[0] = prm->z - prm->size[2] / 2.0;
     for (int i = 1; i < ZL; i++) p.zb[i] = p.zb[i - 1] + prm->size[2] / Zs;
@@ -588,6 +587,7 @@ scw_status plan_solve(const scw_solve_params* prm, int Zs, int Y, int X, SolvePl
     p.M1 = M1;
     p.MF = MF;
     p.n = 2 * MF;
+    p.eig_mixed = prm->eig_fp64 == 0 && p.n <= mx::kMaxN;
     // k grids (FourierWave.h:319-334): integer series -(M/2) .. (M-1)/2
     p.ps.resize(M0);
     p.qs.resize(M1);
