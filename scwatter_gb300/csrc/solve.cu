@@ -249,127 +249,56 @@ __global__ void mix_kernel(double2* __restrict__ A1, double2* __restrict__ A2, c
     }
 }
 
-// f3 (4MF x 3MF, sCWatter.cpp:372-389)
-__global__ void f3_kernel(const double* __restrict__ Sx, const double* __restrict__ Sy, const double2* __restrict__ Sz1,
-                          int MF, double2* __restrict__ F) {
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int ncol = 3 * MF;
-    if (e >= 4LL * MF * ncol) return;
-    const int r = (int)(e / ncol), c = (int)(e % ncol);
-    const int blk = r / MF, m = r % MF;
-    double2 v = make_double2(0, 0);
-    if (blk == 0 && c == m) v = make_double2(-1, 0);
-    else if (blk == 1 && c == MF + m) v = make_double2(-1, 0);
-    else if (blk == 2 && c == MF + m) v = Sz1[m];
-    else if (blk == 2 && c == 2 * MF + m) v = make_double2(-Sy[m], 0);
-    else if (blk == 3 && c == m) v = make_double2(-Sz1[m].x, -Sz1[m].y);
-    else if (blk == 3 && c == 2 * MF + m) v = make_double2(Sx[m], 0);
-    F[e] = v;
-}
-
-// f3 with the z columns eliminated by the divergence rows, Tz = -(Sx Tx + Sy Ty) / Sz1 (4MF x 2MF)
-__global__ void f3_reduced_kernel(const double* __restrict__ Sx, const double* __restrict__ Sy,
-                                  const double2* __restrict__ Sz1, int MF, double2* __restrict__ F) {
+// f3 (sCWatter.cpp:372-389) on two of T's components per harmonic: 4MF x 2MF, columns m and MF + m
+__global__ void f3_kernel(const BcPair* __restrict__ bc, int MF, double2* __restrict__ F) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int n = 2 * MF;
     if (e >= 4LL * MF * n) return;
     const int r = (int)(e / n), c = (int)(e % n);
     const int blk = r / MF, m = r % MF;
-    double2 v = make_double2(0, 0);
-    if (c % MF == m) {
-        const double2 i1 = cinv(Sz1[m]);
-        const double sx = Sx[m], sy = Sy[m];
-        const bool y = c >= MF;
-        if (blk == 0 && !y) v = make_double2(-1, 0);
-        else if (blk == 1 && y) v = make_double2(-1, 0);
-        else if (blk == 2 && !y) v = make_double2(sx * sy * i1.x, sx * sy * i1.y);
-        else if (blk == 2) v = make_double2(Sz1[m].x + sy * sy * i1.x, Sz1[m].y + sy * sy * i1.y);
-        else if (blk == 3 && !y) v = make_double2(-Sz1[m].x - sx * sx * i1.x, -Sz1[m].y - sx * sx * i1.y);
-        else if (blk == 3) v = make_double2(-sx * sy * i1.x, -sx * sy * i1.y);
-    }
-    F[e] = v;
+    F[e] = c % MF == m ? bc[m].L[2 * blk + c / MF] : make_double2(0, 0);
 }
 
-// The boundary system with Rz (divergence rows), Rx and Ry (first 2MF matching rows) eliminated: the
-// 2MF x 2MF matrix for (Tx, Ty) and its right-hand side as column 2MF.  T3: 4MF x 2MF, f: f1 EF.
-//   Rx = -f0 - t0 T, Ry = -f1 - t1 T, Rz = (Sx Rx + Sy Ry) / Sz0,
-//   row m: (t2 - a t0 - b t1) T = -f2 + a f0 + b f1,  a = Sx Sy / Sz0,  b = Sz0 + Sy^2 / Sz0
-//   row MF + m: (t3 - c t0 - d t1) T = -f3 + c f0 + d f1,  c = -Sz0 - Sx^2 / Sz0,  d = -a
-__global__ void bc_reduced_kernel(const double* __restrict__ Sx, const double* __restrict__ Sy,
-                                  const double2* __restrict__ Sz0, const double2* __restrict__ T3,
-                                  const double2* __restrict__ f, int MF, double2* __restrict__ A) {
+// The boundary system (divergence rows and matching rows [f2 | T3] x = -f1 EF, sCWatter.cpp:143-146, 393-461) with R
+// eliminated: the 2MF x 2MF matrix for T's pairs and its right-hand side as column 2MF.  T3 = Gd_0 Gc_static^-1 f3: 4MF x
+// 2MF, f: f1 EF.  Row k MF + m: t_q[k] - M[k] (t_p[0], t_p[1]) with t the harmonic's four rows of [T3 | -f].
+__global__ void bc_matrix_kernel(const BcPair* __restrict__ bc, const double2* __restrict__ T3, const double2* __restrict__ f, int MF,
+                                 double2* __restrict__ A) {
     const int n = 2 * MF, ld = n + 1;
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long long)MF * ld) return;
     const int m = (int)(e / ld), j = (int)(e % ld);
-    const double2 s0 = Sz0[m], i0 = cinv(s0);
-    const double sx = Sx[m], sy = Sy[m];
-    const double2 a = make_double2(sx * sy * i0.x, sx * sy * i0.y);
-    const double2 b = make_double2(s0.x + sy * sy * i0.x, s0.y + sy * sy * i0.y);
-    const double2 c = make_double2(-s0.x - sx * sx * i0.x, -s0.y - sx * sx * i0.y);
-    double2 t[4];
-    for (int q = 0; q < 4; q++) {
-        t[q] = j < n ? T3[((long long)q * MF + m) * n + j] : f[q * MF + m];
-        if (j == n) t[q] = make_double2(-t[q].x, -t[q].y);
-    }
-    A[(long long)m * ld + j] = csub(csub(t[2], cmul(a, t[0])), cmul(b, t[1]));
-    A[(long long)(MF + m) * ld + j] = cadd(csub(t[3], cmul(c, t[0])), cmul(a, t[1]));
+    auto row = [&](int q) {
+        if (j < n) return T3[((long long)q * MF + m) * n + j];
+        const double2 v = f[q * MF + m];
+        return make_double2(-v.x, -v.y);
+    };
+    const BcPair& h = bc[m];
+    const double2 t0 = row(h.p[0]), t1 = row(h.p[1]);
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+        A[(long long)(k * MF + m) * ld + j] = csub(csub(row(h.q[k]), cmul(h.M[2 * k], t0)), cmul(h.M[2 * k + 1], t1));
 }
 
-// x (6MF) from (Tx, Ty) = column 2MF of A and r = [t0; t1] T
-__global__ void bc_expand_kernel(const double* __restrict__ Sx, const double* __restrict__ Sy,
-                                 const double2* __restrict__ Sz0, const double2* __restrict__ Sz1,
-                                 const double2* __restrict__ f, const double2* __restrict__ A,
+// x (6MF) from T's pairs, column 2MF of A, and r = T3 of them (4MF)
+__global__ void bc_expand_kernel(const BcPair* __restrict__ bc, const double2* __restrict__ f, const double2* __restrict__ A,
                                  const double2* __restrict__ r, int MF, double2* __restrict__ x) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x, n = 2 * MF, ld = n + 1;
     if (m >= MF) return;
-    const double2 tx = A[(long long)m * ld + n], ty = A[(long long)(MF + m) * ld + n];
-    const double2 rx = make_double2(-f[m].x - r[m].x, -f[m].y - r[m].y);
-    const double2 ry = make_double2(-f[MF + m].x - r[MF + m].x, -f[MF + m].y - r[MF + m].y);
-    const double sx = Sx[m], sy = Sy[m];
-    x[m] = rx;
-    x[MF + m] = ry;
-    x[2 * MF + m] = cmul(make_double2(sx * rx.x + sy * ry.x, sx * rx.y + sy * ry.y), cinv(Sz0[m]));
-    x[3 * MF + m] = tx;
-    x[4 * MF + m] = ty;
-    x[5 * MF + m] = cmul(make_double2(-sx * tx.x - sy * ty.x, -sx * tx.y - sy * ty.y), cinv(Sz1[m]));
-}
-
-// the 6MF x 6MF boundary matrix (sCWatter.cpp:143-146, 393-461): divergence constraints,
-// then [f2 | T3] with T3 = Gd_0 Gc_static^-1 f3 (4MF x 3MF)
-__global__ void bc_matrix_kernel(const double* __restrict__ Sx, const double* __restrict__ Sy,
-                                 const double2* __restrict__ Sz0, const double2* __restrict__ Sz1,
-                                 const double2* __restrict__ T3, int MF, double2* __restrict__ A) {
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int N6 = 6 * MF;
-    if (e >= (long long)N6 * N6) return;
-    const int r = (int)(e / N6), c = (int)(e % N6);
-    double2 v = make_double2(0, 0);
-    if (r < MF) {
-        const int m = r;
-        if (c == m) v = make_double2(Sx[m], 0);
-        else if (c == MF + m) v = make_double2(Sy[m], 0);
-        else if (c == 2 * MF + m) v = make_double2(-Sz0[m].x, -Sz0[m].y);
-    } else if (r < 2 * MF) {
-        const int m = r - MF;
-        if (c == 3 * MF + m) v = make_double2(Sx[m], 0);
-        else if (c == 4 * MF + m) v = make_double2(Sy[m], 0);
-        else if (c == 5 * MF + m) v = Sz1[m];
-    } else {
-        const int rr = r - 2 * MF;
-        if (c >= 3 * MF) {
-            v = T3[(long long)rr * 3 * MF + (c - 3 * MF)];
-        } else {
-            const int blk = rr / MF, m = rr % MF;
-            if (blk == 0 && c == m) v = make_double2(1, 0);
-            else if (blk == 1 && c == MF + m) v = make_double2(1, 0);
-            else if (blk == 2 && c == MF + m) v = Sz0[m];
-            else if (blk == 2 && c == 2 * MF + m) v = make_double2(Sy[m], 0);
-            else if (blk == 3 && c == m) v = make_double2(-Sz0[m].x, -Sz0[m].y);
-            else if (blk == 3 && c == 2 * MF + m) v = make_double2(-Sx[m], 0);
-        }
+    const BcPair& h = bc[m];
+    auto put = [&](double2* out, const double2* ratio, int third, double2 u, double2 v) {
+        const int a = third == 0 ? 1 : 0, b = third == 2 ? 1 : 2;
+        out[a * MF + m] = u;
+        out[b * MF + m] = v;
+        out[third * MF + m] = cadd(cmul(ratio[0], u), cmul(ratio[1], v));
+    };
+    put(x + 3 * MF, h.r1, h.c1, A[(long long)m * ld + n], A[(long long)(MF + m) * ld + n]);
+    double2 g[2];
+    for (int k = 0; k < 2; k++) {
+        const int q = h.p[k] * MF + m;
+        g[k] = make_double2(-f[q].x - r[q].x, -f[q].y - r[q].y);
     }
-    A[e] = v;
+    put(x, h.r0, h.c0, cadd(cmul(h.Fi[0], g[0]), cmul(h.Fi[1], g[1])), cadd(cmul(h.Fi[2], g[0]), cmul(h.Fi[3], g[1])));
 }
 
 // Kn[l][m_i][m_j] = scale * NIf[lin] with lin the wrapped difference index read column-major
@@ -436,12 +365,6 @@ __global__ void to_c64_kernel(const double2* __restrict__ a, float2* __restrict_
 }
 
 // b = [0 (2MF); -f1 EF (4MF)]  (sCWatter.cpp:459-460)
-__global__ void bc_rhs_kernel(const double2* __restrict__ f1EF, int MF, double2* __restrict__ b) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= 6 * MF) return;
-    b[e] = e < 2 * MF ? make_double2(0.0, 0.0) : make_double2(-f1EF[e - 2 * MF].x, -f1EF[e - 2 * MF].y);
-}
-
 // v = f1 EF + f2 R with R = x[0, 3MF)  (sCWatter.cpp:745-747)
 __global__ void beta_init_kernel(const double2* __restrict__ f1EF, const double2* __restrict__ x,
                                  const double* __restrict__ Sx, const double* __restrict__ Sy,
@@ -506,6 +429,69 @@ static void fft_shift_index(int m, int n, std::vector<int>& indx, std::vector<in
         if (n % 2 == 1) indy[i] = i < n - q - 1 ? (n - q) + i : i - (n - q - 1);
         else indy[i] = i < n - q ? q + i : i - (n - q);
     }
+}
+
+// The pair of one harmonic (see BcPair).
+static BcPair bc_pair(double Sx, double Sy, cd Sz0, cd Sz1) {
+    auto d2 = [](cd v) { return make_double2(v.real(), v.imag()); };
+    BcPair h{};
+    // the component that follows from the other two, and its ratios; all zero where s is (no medium)
+    auto third = [](const cd* s, cd* ratio) {
+        int c = 2;
+        for (int i = 1; i >= 0; i--)
+            if (std::abs(s[i]) > std::abs(s[c])) c = i;
+        const int a = c == 0 ? 1 : 0, b = c == 2 ? 1 : 2;
+        const bool none = s[c] == cd(0, 0);
+        ratio[0] = none ? cd(0, 0) : -s[a] / s[c];
+        ratio[1] = none ? cd(0, 0) : -s[b] / s[c];
+        return c;
+    };
+    // a 4 x 3 matrix on the pair
+    auto on_pair = [](const cd (*f)[3], int c, const cd* ratio, cd (*out)[2]) {
+        const int a = c == 0 ? 1 : 0, b = c == 2 ? 1 : 2;
+        for (int q = 0; q < 4; q++) {
+            out[q][0] = f[q][a] + f[q][c] * ratio[0];
+            out[q][1] = f[q][b] + f[q][c] * ratio[1];
+        }
+    };
+    const cd s1[3] = {Sx, Sy, Sz1}, s0[3] = {Sx, Sy, -Sz0};
+    cd r1[2], r0[2], L[4][2], F[4][2];
+    h.c1 = third(s1, r1);
+    h.c0 = third(s0, r0);
+    const cd f3[4][3] = {{-1, 0, 0}, {0, -1, 0}, {0, Sz1, -Sy}, {-Sz1, 0, Sx}};
+    const cd f2[4][3] = {{1, 0, 0}, {0, 1, 0}, {0, Sz0, Sy}, {-Sz0, 0, -Sx}};
+    on_pair(f3, h.c1, r1, L);
+    on_pair(f2, h.c0, r0, F);
+    double best = -1.0;
+    cd det = 1;
+    for (int i = 0; i < 4; i++)
+        for (int j = i + 1; j < 4; j++) {
+            const cd d = F[i][0] * F[j][1] - F[i][1] * F[j][0];
+            if (std::abs(d) > best) {
+                best = std::abs(d);
+                det = d;
+                h.p[0] = i;
+                h.p[1] = j;
+            }
+        }
+    for (int i = 0, k = 0; i < 4; i++)
+        if (i != h.p[0] && i != h.p[1]) h.q[k++] = i;
+    const cd* a = F[h.p[0]];
+    const cd* b = F[h.p[1]];
+    const cd Fi[4] = {b[1] / det, -a[1] / det, -b[0] / det, a[0] / det};
+    for (int k = 0; k < 2; k++) {
+        const cd* g = F[h.q[k]];
+        h.M[2 * k] = d2(g[0] * Fi[0] + g[1] * Fi[2]);
+        h.M[2 * k + 1] = d2(g[0] * Fi[1] + g[1] * Fi[3]);
+        h.r1[k] = d2(r1[k]);
+        h.r0[k] = d2(r0[k]);
+    }
+    for (int k = 0; k < 4; k++) h.Fi[k] = d2(Fi[k]);
+    // without a medium below there is no T: zero columns, which the factorisation reports
+    const bool none = s1[h.c1] == cd(0, 0);
+    for (int q = 0; q < 4; q++)
+        for (int c = 0; c < 2; c++) h.L[2 * q + c] = none ? make_double2(0, 0) : d2(L[q][c]);
+    return h;
 }
 
 #define SCW_TRY(expr)                          \
@@ -618,10 +604,8 @@ scw_status plan_solve(const scw_solve_params* prm, int Zs, int Y, int X, SolvePl
         p.Sz0[f] = std::sqrt(ni0 * ni0 - cd(sx * sx) - cd(sy * sy));
         p.Sz1[f] = std::sqrt(ni1 * ni1 - cd(sx * sx) - cd(sy * sy));
     }
-    // no harmonic grazes an outer medium: the boundary system can divide by every Sz
-    p.reduced_bc = true;
-    for (int f = 0; f < MF; f++)
-        p.reduced_bc = p.reduced_bc && std::abs(p.Sz0[f]) >= 0.02 && std::abs(p.Sz1[f]) >= 0.02;
+    p.bc.resize(MF);
+    for (int f = 0; f < MF; f++) p.bc[f] = bc_pair(p.Sx[f], p.Sy[f], p.Sz0[f], p.Sz1[f]);
     // the DFT rows / columns that land in the centred crop after the shift
     std::vector<int> ix, iy;
     fft_shift_index(Y, X, ix, iy);
@@ -670,6 +654,7 @@ void carve_in(const SolvePlan& p, Carver& c, SolveIn& in) {
     in.Sz1 = c.take<double2>(MF);
     in.f1EF = c.take<double2>(4 * MF);
     in.EF = c.take<double2>(3 * MF);
+    in.bc = c.take<BcPair>(MF);
     in.qs = c.take<int>(p.M1);
     in.ps = c.take<int>(p.M0);
     in.up = c.take<double>(p.M0);
@@ -682,7 +667,7 @@ void carve_in(const SolvePlan& p, Carver& c, SolveIn& in) {
 }
 
 void carve_ws(const SolvePlan& p, Carver& c, SolveWs& ws) {
-    const size_t Z = p.Z, MF = p.MF, n = p.n, nn = n * n, N4 = 4 * MF, M3 = 3 * MF, M6 = 6 * MF;
+    const size_t Z = p.Z, MF = p.MF, n = p.n, nn = n * n, N4 = 4 * MF;
     ws.coef = c.take<double2>(Z * 2 * MF);
     ws.P = c.take<double2>(Z * (nn + 3 * n));     // P, then eigen-solver work, then the inverses' scratch
     ws.Q = c.take<double2>(Z * nn);               // Q, then W^-1
@@ -693,7 +678,7 @@ void carve_ws(const SolvePlan& p, Carver& c, SolveWs& ws) {
     ws.E = c.take<double2>(Z * n);
     ws.beta = c.take<double2>(Z * N4);
     ws.v = c.take<double2>(N4);
-    ws.piv = c.take<int>(std::max(Z * n, M6));
+    ws.piv = c.take<int>(Z * n);
     ws.worst = c.take<double>(2 * Z);
     ws.good = c.take<int>(2 * Z);
     // mixed eigen-solver: small buffers of its own; S0, S1 (adjacent) inside P, S2, S3 inside W
@@ -708,7 +693,7 @@ void carve_ws(const SolvePlan& p, Carver& c, SolveWs& ws) {
         ws.mix.S3 = Wf + Z * nn;
     }
     // operands of the FP64 products: the largest of them for one matrix, a whole batch up to the cap
-    const size_t one = std::max({zgemm_ws_bytes((int)n, (int)M3, (int)n, 1), zgemm_ws_bytes((int)M6, (int)M6, 32, 1),
+    const size_t one = std::max({zgemm_ws_bytes((int)n, (int)n, (int)n, 1), zgemm_ws_bytes((int)n, (int)n + 1, 32, 1),
                                  zgemm_ws_bytes(p.X, p.M1, p.Y, 1), zgemm_ws_bytes(p.M0, p.M1, p.X, 1)});
     ws.gemm.bytes = std::max(one, std::min(one * Z, kGemmWsCap));
     ws.gemm.base = c.take<char>(ws.gemm.bytes);
@@ -718,12 +703,11 @@ void carve_ws(const SolvePlan& p, Carver& c, SolveWs& ws) {
     ws.F = ca.take<double2>(2 * Z * (size_t)p.Y * p.X);
     ws.T = ca.take<double2>(2 * Z * (size_t)p.X * p.M1);
     Carver cc{c.base, t0};
-    // columns of the cascade: (Tx, Ty), or all three components where a harmonic grazes
-    const size_t nc = p.reduced_bc ? n : M3, nb = p.reduced_bc ? n : M6;
-    ws.X = cc.take<double2>(N4 * nc);
-    ws.A1 = cc.take<double2>(2 * n * nc);
-    ws.A = cc.take<double2>(nb * (nb + 1));
-    ws.b = cc.take<double2>(nb);
+    // columns of the cascade: two components of T per harmonic
+    ws.X = cc.take<double2>(N4 * n);
+    ws.A1 = cc.take<double2>(2 * n * n);
+    ws.A = cc.take<double2>(n * (n + 1));
+    ws.b = cc.take<double2>(N4);
     c.off = std::max(ca.off, cc.off);
 }
 
@@ -769,6 +753,7 @@ scw_status upload_inputs(const SolvePlan& p, const double* sample, const SolveIn
     SCW_TRY(up(in.Sz1, p.Sz1.data(), sizeof(double2) * MF));
     SCW_TRY(up(in.f1EF, p.f1EF.data(), sizeof(double2) * 4 * MF));
     SCW_TRY(up(in.EF, p.EF.data(), sizeof(double2) * 3 * MF));
+    SCW_TRY(up(in.bc, p.bc.data(), sizeof(BcPair) * MF));
     SCW_TRY(up(in.qs, p.qs.data(), sizeof(int) * p.M1));
     SCW_TRY(up(in.ps, p.ps.data(), sizeof(int) * p.M0));
     SCW_TRY(up(in.up, p.up.data(), sizeof(double) * p.M0));
@@ -901,11 +886,8 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
     double2* Winv = ws.Q;
     SCW_TRY(record_inverses(p, in, ws, out, Uinv, Winv, st, &L));
     // T3 = Gd_0 Gc_static^-1 f3 = prod_l V_l diag(E_l^-1, E_l) V_l^-1 f3
-    const int nc = p.reduced_bc ? n : M3;
-    if (p.reduced_bc)
-        f3_reduced_kernel<<<nblk((long long)N4 * nc), 256, 0, st>>>(in.Sx, in.Sy, in.Sz1, MF, ws.X);
-    else
-        f3_kernel<<<nblk((long long)N4 * nc), 256, 0, st>>>(in.Sx, in.Sy, in.Sz1, MF, ws.X);
+    const int nc = n;
+    f3_kernel<<<nblk((long long)N4 * nc), 256, 0, st>>>(in.bc, MF, ws.X);
     SCW_CUDA_TRY(cudaGetLastError());
     // the two products of each half-step (U^-1 and W^-1, then U and W) run as one batch of two
     double2* A2 = ws.A1 + (size_t)n * nc;
@@ -917,25 +899,14 @@ scw_status record_solve(const SolvePlan& p, const SolveIn& in, const SolveWs& ws
         L += 7;
     }
     // boundary system and its solve (sCWatter.cpp:393-461, 722)
-    if (p.reduced_bc) {
-        bc_reduced_kernel<<<nblk((long long)MF * (n + 1)), 256, 0, st>>>(in.Sx, in.Sy, in.Sz0, ws.X, in.f1EF, MF, ws.A);
-        SCW_CUDA_TRY(cudaGetLastError());
-        SCW_TRY(zgetrf(st, ws.A, n, n + 1, n + 1, 0, ws.piv, 0, out.status + 3 * Zs, 1, ws.gemm, nullptr));
-        SCW_TRY(ztrsm_upper(st, ws.A, n, n + 1, 0, ws.A + n, 1, n + 1, 0, 1, ws.gemm, nullptr));
-        SCW_TRY(zgemm(st, n, 1, n, kOne, ws.X, n, 0, ws.A + n, n + 1, 0, kZero, ws.b, 1, 0, 1, ws.gemm));
-        bc_expand_kernel<<<nblk(MF), 256, 0, st>>>(in.Sx, in.Sy, in.Sz0, in.Sz1, in.f1EF, ws.A, ws.b, MF, out.x);
-        SCW_CUDA_TRY(cudaGetLastError());
-        L += 4 + 7 * ((n + 31) / 32);
-    } else {
-        bc_matrix_kernel<<<nblk((long long)M6 * M6), 256, 0, st>>>(in.Sx, in.Sy, in.Sz0, in.Sz1, ws.X, MF, ws.A);
-        SCW_CUDA_TRY(cudaGetLastError());
-        bc_rhs_kernel<<<nblk(M6), 256, 0, st>>>(in.f1EF, MF, ws.b);
-        SCW_CUDA_TRY(cudaGetLastError());
-        SCW_TRY(zgetrf(st, ws.A, M6, M6, M6, 0, ws.piv, 0, out.status + 3 * Zs, 1, ws.gemm, nullptr));
-        SCW_TRY(zgetrs(st, ws.A, M6, 0, ws.piv, 0, ws.b, 1, 0, 1, ws.gemm, nullptr));
-        SCW_CUDA_TRY(cudaMemcpyAsync(out.x, ws.b, sizeof(double2) * M6, cudaMemcpyDeviceToDevice, st));
-        L += 4 + 9 * ((M6 + 31) / 32);
-    }
+    bc_matrix_kernel<<<nblk((long long)MF * (n + 1)), 256, 0, st>>>(in.bc, ws.X, in.f1EF, MF, ws.A);
+    SCW_CUDA_TRY(cudaGetLastError());
+    SCW_TRY(zgetrf(st, ws.A, n, n + 1, n + 1, 0, ws.piv, 0, out.status + 3 * Zs, 1, ws.gemm, nullptr));
+    SCW_TRY(ztrsm_upper(st, ws.A, n, n + 1, 0, ws.A + n, 1, n + 1, 0, 1, ws.gemm, nullptr));
+    SCW_TRY(zgemm(st, N4, 1, n, kOne, ws.X, n, 0, ws.A + n, n + 1, 0, kZero, ws.b, 1, 0, 1, ws.gemm));
+    bc_expand_kernel<<<nblk(MF), 256, 0, st>>>(in.bc, in.f1EF, ws.A, ws.b, MF, out.x);
+    SCW_CUDA_TRY(cudaGetLastError());
+    L += 4 + 7 * ((n + 31) / 32);
     if (out.sepExt) {
         sep_ext_kernel<<<nblk(M3), 256, 0, st>>>(in.EF, out.x, in.Sz0, in.Sz1, MF, k, p.n0, p.n1, out.sepExt);
         SCW_CUDA_TRY(cudaGetLastError());

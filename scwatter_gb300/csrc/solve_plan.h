@@ -22,13 +22,26 @@ namespace sv {
 
 using cd = std::complex<double>;
 
+// How one harmonic's reflected wave R and transmitted wave T enter the boundary system.  Each is divergence free, s . R = 0 with
+// s = (Sx, Sy, -Sz0) and s . T = 0 with s = (Sx, Sy, Sz1), so one component follows from two: the one with the
+// largest |s|, whose ratios are at most 1 (the z component alone would be divided by Sz, which vanishes where a harmonic grazes).
+// Of the four matching rows two determine R's pair, those with the largest determinant; the other two are left for T.
+struct BcPair {
+    double2 L[8];          // f3 (4 x 3) on T's pair: row q, column c at 2 q + c
+    double2 M[4];          // f2's other rows times the inverse of its rows p, both on R's pair
+    double2 Fi[4];         // that inverse
+    double2 r1[2], r0[2];  // T's and R's third component from the pair
+    int c1, c0;            // which that is
+    int p[2], q[2];        // matching rows for R, and the others
+    int pad[2];
+};
+
 struct SolvePlan {
     int Z = 0, Y = 0, X = 0;
     int M0 = 0, M1 = 0, MF = 0, n = 0;      // n = 2 MF
     double k = 0, n0 = 1, n1 = 1;
     bool external = false, pz = true;
     bool eig_mixed = true;                  // FP32 QR + FP64 refinement (else FP64 QR throughout)
-    bool reduced_bc = true;                 // boundary system of order 2MF (no |Sz| near zero), else 6MF
     bool wide_hess = false;                 // Hessenberg reductions over the whole GPU (single solves)
     int share = 1;                          // solves recorded to run at the same time (lanes of a batch)
     std::vector<double> zb, dz;             // Z + 1 boundaries, Z thicknesses
@@ -37,6 +50,7 @@ struct SolvePlan {
     std::vector<double> up_pz, wq_pz;       // per harmonic m = q M0 + p (M_PI), Ez step
     std::vector<double> Sx, Sy;             // flattened meshes (column-major, sCWatter.cpp:677-680)
     std::vector<cd> Sz0, Sz1, EF, f1EF;     // MF, MF, 3MF, 4MF
+    std::vector<BcPair> bc;                 // per harmonic
     std::vector<cd> tw1, tw2;               // DFT twiddles of the cropped bins: [Y][M1], [M0][X]
 };
 
@@ -55,6 +69,7 @@ struct Carver {
 
 struct SolveIn {                            // uploaded once
     double2 *data, *tw1, *tw2, *Sz0, *Sz1, *f1EF, *EF;
+    BcPair* bc;
     int *qs, *ps;
     double *up, *wq, *dz, *Sx, *Sy, *uppz, *wqpz;
 };
