@@ -14,6 +14,7 @@
 // the slices of a sample.
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 #include <cmath>
 #include <vector>
 
@@ -151,6 +152,8 @@ __device__ __forceinline__ double2 lu_sub(double2 x, double2 l, double2 p) {    
     return make_double2(fma(-l.x, p.x, fma(l.y, p.y, x.x)), fma(-l.x, p.y, fma(-l.y, p.x, x.y)));
 }
 
+// kFar: where a CTA's rows do not fit into shared memory the panel stays in A
+template <bool kFar>
 __global__ void __cluster_dims__(kLuCtas, 1, 1) __launch_bounds__(kLuThreads)
 lu_panel_kernel(double2* __restrict__ A, int n, int lda, long long sA, int k0, int nb, int rows, int* __restrict__ piv,
                 long long sP, int* __restrict__ info, const int* __restrict__ skip) {
@@ -163,18 +166,19 @@ lu_panel_kernel(double2* __restrict__ A, int n, int lda, long long sA, int k0, i
     extern __shared__ __align__(16) unsigned char lu_smem[];
     LuSlot* slot = reinterpret_cast<LuSlot*>(lu_smem);   // [2][kLuCtas]: candidates of column parity
     LuSlot* krow = slot + 2 * kLuCtas;                   // [2]: row k
-    double2* P = reinterpret_cast<double2*>(krow + 2);   // [rows][nb + 1]
-    const int ld = nb + 1;
+    const int g0 = k0 + rank * rows;                     // this CTA's rows g0 .. g0 + nr - 1
+    const int nr = max(0, min(rows, n - g0));
+    double2* const P = kFar ? A + (long long)g0 * lda + k0 : reinterpret_cast<double2*>(krow + 2);   // [rows][ld]
+    const std::conditional_t<kFar, long long, int> ld = kFar ? lda : nb + 1;
     constexpr int kWarps = kLuThreads / 32;
     __shared__ LuKey red[kWarps], mine;
     __shared__ double2 mine_inv;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int g0 = k0 + rank * rows;                     // this CTA's rows g0 .. g0 + nr - 1
-    const int nr = max(0, min(rows, n - g0));
-    for (int e = tid; e < nr * nb; e += kLuThreads) {
-        const int r = e / nb, c = e - r * nb;
-        P[r * ld + c] = A[(long long)(g0 + r) * lda + k0 + c];
-    }
+    if (!kFar)
+        for (int e = tid; e < nr * nb; e += kLuThreads) {
+            const int r = e / nb, c = e - r * nb;
+            P[r * ld + c] = A[(long long)(g0 + r) * lda + k0 + c];
+        }
     __syncthreads();
     const LuKey nothing{-1, 0x7fffffff, 0u};
     auto better = [](const LuKey& x, const LuKey& y) {
@@ -270,10 +274,11 @@ lu_panel_kernel(double2* __restrict__ A, int n, int lda, long long sA, int k0, i
         if (lane == 0) red[warp] = best;
         __syncthreads();
     }
-    for (int e = tid; e < nr * nb; e += kLuThreads) {
-        const int r = e / nb, c = e - r * nb;
-        A[(long long)(g0 + r) * lda + k0 + c] = P[r * ld + c];
-    }
+    if (!kFar)
+        for (int e = tid; e < nr * nb; e += kLuThreads) {
+            const int r = e / nb, c = e - r * nb;
+            A[(long long)(g0 + r) * lda + k0 + c] = P[r * ld + c];
+        }
 }
 
 // The panel's row interchanges on the columns outside it, then L11 U12 = A12 on the columns right of
@@ -1176,19 +1181,20 @@ scw_status zgetrf(cudaStream_t st, double2* A, int n, int ncols, int lda, long l
                   int batch, const GemmWs& ws, const int* skip) {
     if (n <= 0 || batch <= 0) return SCW_OK;
     SCW_CUDA_TRY(cudaMemsetAsync(info, 0, sizeof(int) * batch, st));
-    // panel width: as many columns as the cluster's shared memory holds of the first panel
+    // the panel in the cluster's shared memory where 32 columns of it fit (up to 3264 rows), else in A, by way of L2.  (Narrower panels
+    // in shared memory end at 53 872 rows and are no faster before: order 4096 78 ms with 16 columns, 80 here; 6400 375 with 8, 230 here.)
     constexpr size_t kLimit = 220 * 1024, kSlots = sizeof(z::LuSlot) * (2 * z::kLuCtas + 2);
     auto smem_of = [](int rows, int nb) { return kSlots + sizeof(double2) * (size_t)rows * (nb + 1); };
-    auto rows_of = [&](int k0) { return (n - k0 + z::kLuCtas - 1) / z::kLuCtas; };
-    int width = z::kNB;
-    while (width > 1 && smem_of(rows_of(0), width) > kLimit) width /= 2;
-    if (smem_of(rows_of(0), width) > kLimit) return fail(SCW_ERR_ARG, "getrf: matrix too large");
-    SCW_CUDA_TRY(cudaFuncSetAttribute(z::lu_panel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLimit));
+    SCW_CUDA_TRY(cudaFuncSetAttribute(z::lu_panel_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLimit));
     const double2 one = {1, 0}, minus = {-1, 0};
+    constexpr int width = z::kNB;
     for (int k0 = 0; k0 < n; k0 += width) {
-        const int nb = std::min(width, n - k0), rows = rows_of(k0);
-        z::lu_panel_kernel<<<z::kLuCtas * batch, z::kLuThreads, smem_of(rows, nb), st>>>(A, n, lda, sA, k0, nb, rows, piv,
-                                                                                      sP, info, skip);
+        const int nb = std::min(width, n - k0), rows = (n - k0 + z::kLuCtas - 1) / z::kLuCtas;
+        if (smem_of(rows, nb) <= kLimit)
+            z::lu_panel_kernel<false><<<z::kLuCtas * batch, z::kLuThreads, smem_of(rows, nb), st>>>(A, n, lda, sA, k0, nb, rows, piv,
+                                                                                                 sP, info, skip);
+        else
+            z::lu_panel_kernel<true><<<z::kLuCtas * batch, z::kLuThreads, kSlots, st>>>(A, n, lda, sA, k0, nb, rows, piv, sP, info, skip);
         SCW_CUDA_TRY(cudaGetLastError());
         if (ncols > nb) {
             if (few_columns(ncols, batch))
