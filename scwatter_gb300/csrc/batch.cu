@@ -371,9 +371,21 @@ scw_status scw_batch_create(scw_ctx ctx, const scw_batch_item* items, int count,
     std::iota(all.begin(), all.end(), 0);
     size_t free_b = 0, total_b = 0;
     SCW_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-    size_t max_ws = 0;
-    for (const auto& it : b->items) max_ws = std::max(max_ws, it.ws_bytes);
-    const int max_lanes = (int)std::max<size_t>(1, std::min<size_t>(16, (size_t)(0.8 * free_b) / std::max<size_t>(max_ws, 1)));
+    auto fitting_lanes = [&]() {
+        size_t max_ws = 0;
+        for (const auto& it : b->items) max_ws = std::max(max_ws, it.ws_bytes);
+        return (int)std::max<size_t>(1, std::min<size_t>(16, (size_t)(0.8 * free_b) / std::max<size_t>(max_ws, 1)));
+    };
+    int max_lanes = fitting_lanes();
+    if (max_lanes < (lanes > 0 ? lanes : 16)) {
+        // memory limits the lanes: they matter more than whole batches of digits (a slice's product at a time fills the GPU
+        // where arenas are that large)
+        for (auto& it : b->items) {
+            it.sp.gemm_cap = 0;
+            it.ws_bytes = lane_need(it);
+        }
+        max_lanes = fitting_lanes();
+    }
     const auto t0 = std::chrono::steady_clock::now();
     if (lanes == 0 || method == 0) {
         // calibration subset: 8 items spread over the cheaper half by cost, so tuning costs a

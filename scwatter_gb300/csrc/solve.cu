@@ -695,7 +695,7 @@ void carve_ws(const SolvePlan& p, Carver& c, SolveWs& ws) {
     // operands of the FP64 products: the largest of them for one matrix, a whole batch up to the cap
     const size_t one = std::max({zgemm_ws_bytes((int)n, (int)n, (int)n, 1), zgemm_ws_bytes((int)n, (int)n + 1, 32, 1),
                                  zgemm_ws_bytes(p.X, p.M1, p.Y, 1), zgemm_ws_bytes(p.M0, p.M1, p.X, 1)});
-    ws.gemm.bytes = std::max(one, std::min(one * Z, kGemmWsCap));
+    ws.gemm.bytes = std::max(one, std::min(one * Z, p.gemm_cap));
     ws.gemm.base = c.take<char>(ws.gemm.bytes);
     // temporary region, two overlays
     const size_t t0 = (c.off + 255) / 256 * 256;

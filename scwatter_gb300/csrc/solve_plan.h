@@ -44,6 +44,7 @@ struct SolvePlan {
     bool eig_mixed = true;                  // FP32 QR + FP64 refinement (else FP64 QR throughout)
     bool wide_hess = false;                 // Hessenberg reductions over the whole GPU (single solves)
     int share = 1;                          // solves recorded to run at the same time (lanes of a batch)
+    size_t gemm_cap = kGemmWsCap;           // digits of a product beyond what one matrix needs (batched products go in parts)
     std::vector<double> zb, dz;             // Z + 1 boundaries, Z thicknesses
     std::vector<int> ps, qs;                // integer harmonic series
     std::vector<double> up, wq;             // k grids (reference PI)

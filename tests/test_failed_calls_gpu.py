@@ -1,5 +1,5 @@
 """CUDA calls that fail, made to by a library loaded before the runtime (host side only: an allocation that cannot be had, an
-error code in place of a call): what can go on without it does, and an error leaves the context as it was."""
+error code in place of a call, little memory left): what can go on without it does, and an error leaves the context as it was."""
 import os
 import subprocess
 import sys
@@ -15,13 +15,20 @@ SHIM = r"""
 #include <dlfcn.h>
 #include <stddef.h>
 static int malloc_at = -1, wait_at = -1;          /* calls until the one that fails */
+static size_t free_bytes;                         /* what cudaMemGetInfo says, unless zero */
 void shim_malloc(int at) { malloc_at = at; }
 void shim_wait(int at) { wait_at = at; }
+void shim_free(size_t n) { free_bytes = n; }
 static void* runtime(const char* name) { return dlsym(dlopen("libcudart.so.13", RTLD_LAZY | RTLD_NOLOAD), name); }
 int cudaMalloc(void** p, size_t n) {
     static int (*next)(void**, size_t);
     if (!next) next = (int (*)(void**, size_t))runtime("cudaMalloc");
     return next(p, malloc_at >= 0 && malloc_at-- == 0 ? (size_t)1 << 50 : n);
+}
+int cudaMemGetInfo(size_t* f, size_t* t) {
+    int r = ((int (*)(size_t*, size_t*))runtime("cudaMemGetInfo"))(f, t);
+    if (free_bytes) *f = free_bytes;
+    return r;
 }
 int cudaStreamWaitEvent(void* s, void* e, unsigned f) {
     static int (*next)(void*, void*, unsigned);
@@ -106,3 +113,27 @@ def test_planes_leave_the_context_on_its_stream(shim, at):
     del s
     assert same(planes(new_set()), ref)
     """ % at)
+
+
+def test_batch_lanes_where_memory_is_short(shim):
+    """Digits of whole batches of slices give way to lanes.  30 slices of order 98: arenas of about 40 MB, 65 with them."""
+    _child(shim, """
+    from scwatter_gb300 import batch as bt, samples
+    def batch(lanes):
+        items = [bt.BatchItem(sample=samples.spheres((30, 16, 16), n_spheres=3, radius=(2, 5), seed=i),
+                              grid=(-8, -8, -20, 1.0, 1.0, 4.0, 16, 15, 10), lam=1.0, direction=(0, 0, 1), ex=(1, 0), ey=(0, 0),
+                              size=(16.0, 16.0, 30.0), coef=(7, 7)) for i in range(4)]
+        return bt.Batch(ctx, items, lanes=lanes, method=2)
+    shim.shim_free(ctypes.c_size_t(210 << 20))
+    b = batch(4)
+    shim.shim_free(ctypes.c_size_t(0))
+    assert b.info()["lanes"] == 4, b.info()["lanes"]
+    b.run()
+    assert not b.wait().any()
+    ref = batch(4)
+    ref.run()
+    assert not ref.wait().any()
+    for i in range(4):
+        for u, v in zip(b.result(i), ref.result(i)):
+            assert np.abs(u - v).max() <= 1e-5 * np.abs(v).max()
+    """)
