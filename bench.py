@@ -633,16 +633,16 @@ CPU_SOLVE_SLICES = 2       # slices of the [20,64,64] sphere sample the CPU orac
 
 
 def fp64_solve_macs(M0, M1, Z, Y, X, checks, pz=True):
-    """Complex multiply-adds of the FP64 GEMM / LU work of one coupled-wave solve, the operation
-    counts of the products the solver issues: per slice the two DFT crops, PQ, W = Q U, the LU
-    inverses of U and W (n^3 / 3 + n^3 each), the cascade (4 products n x n x 3MF), the Ez rows
-    (2 x MF x MF x 2MF) and, per sample, the boundary LU ((6MF)^3 / 3); plus the eigen-solver's
-    FP64 residual products (``checks`` of n^3).  The FP32 eigen stage is not counted."""
+    """Complex multiply-adds of the FP64 products and the LU of one coupled-wave solve whose slices the mixed
+    eigen-solver takes, as the solver issues them: per slice the two DFT crops, PQ, W = Q U, U^-1 (two residuals
+    I - U Y of n^3), W^-1 (its start U^-1 P and one residual), the cascade (4 products n x n x n), the Ez rows
+    (MF x MF x 2MF) and, per sample, the boundary LU of order 2MF (n^3 / 3); plus the eigen-solver's
+    FP64 residual products (``checks`` of n^3).  Corrections in 30 bits, the FP32 eigen stage and what slices that
+    fall back to the FP64 solver add are not counted."""
     MF = M0 * M1
     n = 2 * MF
-    per_slice = (2 * (X * Y * M1 + M0 * M1 * X) + n ** 3 + n ** 3 + 2 * (n ** 3 / 3 + n ** 3)
-                 + 4 * n * n * 3 * MF + (2 * MF * MF * n if pz else 0))
-    return Z * per_slice + (6 * MF) ** 3 / 3 + checks * n ** 3
+    per_slice = 2 * (X * Y * M1 + M0 * M1 * X) + 10 * n ** 3 + (MF * MF * n if pz else 0)
+    return Z * per_slice + n ** 3 / 3 + checks * n ** 3
 
 
 def solved_parity(ctx, sol, slices, N=24, pin_every=9):

@@ -135,7 +135,7 @@ SCW_API scw_status scw_eval_plane_device(scw_waves waves, int axis, float a_star
 SCW_API scw_status scw_eval_volume_device(scw_waves waves, float x_start, float y_start, float z_start,
                                           float dx, float dy, float dz, int Nx, int Ny, int Nz, float* dE);
 /* Allocation-free variant of scw_eval_plane_device (no counterpart in the reference).
- * Same arguments, output and stream behaviour, for callers that must not allocate GPU memory
+ * Same arguments, output (to rounding: another kernel, slower on large planes) and stream behaviour, for callers that must not allocate GPU memory
  * while they run: applications that pre-size one device pool and count any other cudaMalloc
  * as a leak, frame loops that may not stall on the allocator, plug-in hosts that forbid device
  * allocation.  It calls no cudaMalloc, cudaMallocHost, cudaFree or allocating library routine:
@@ -232,8 +232,8 @@ SCW_API scw_status scw_sep_eval_slab_host(scw_sep s, const void* Q_host, float x
  * slabs are kept on the device).  0 restores a default. */
 SCW_API scw_status scw_sep_set_streaming(scw_sep s, int64_t chunk_bytes, int64_t slab_bytes);
 /* Tile shape of the coefficient contraction: 0 (default) = 8 mode rows per warp for launches of 1 or 2
- * planes per group, 4 for 3 to 8; 1 = half as many.  Results are bit-identical; the
- * batch autotuner picks it for its items. */
+ * planes per group, 4 for 3 to 8, half as many where that gives fewer CTAs than the GPU has SMs; 1 = half as many
+ * always.  Results are bit-identical; the batch autotuner picks it for its items. */
 SCW_API scw_status scw_sep_set_tiles(scw_sep s, int ctr_shape);
 /* Device slabs of >= 32 planes in `chunks` chunks whose stages overlap on two streams (stage 1 of
  * a chunk beside stage 2 of the previous, its output GEMM on SM count / synth_sm_div SMs);

@@ -1166,7 +1166,11 @@ scw_status gemm(cudaStream_t st, int M, int N, int K, C alpha, const C* A, int l
 
 // Columns per CTA of the triangular kernels: 32 reuse the block of L or U for more columns, but their FP64
 // work (16 000 operations per column of 32 rows) then takes 20 us on one SM; 8 where 32 would leave SMs idle.
-static bool few_columns(int cols, int batch) { return (long long)((cols + 31) / 32) * batch < 152; }
+static bool few_columns(int cols, int batch) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
+    return (long long)((cols + 31) / 32) * batch < sms;
+}
 
 static cudaError_t trsm_block(cudaStream_t st, const double2* LU, int lda, long long sA, int k0, int nb, double2* B, int ldb, long long sB,
                        int nrhs, int upper, int batch, const int* skip) {

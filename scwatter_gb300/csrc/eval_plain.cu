@@ -590,7 +590,8 @@ scw_status waves_upload(scw_waves w, const std::vector<double>& kre, const std::
     scw_ctx ctx = w->ctx;
     SCW_ON_DEVICE(ctx->device);
     const size_t n = (size_t)w->n;
-    // largest |Re k| and |Im k| per axis and region (NaN stays: no bound holds then)
+    // largest |Re k| and |Im k| per axis and region (NaN stays: no bound holds then), one more pass over the waves:
+    // about 5 % of a plain set's preparation
     w->kmax.assign(6 * w->begin.size(), 0.0);
     for (size_t r = 0; r < w->begin.size(); r++)
         for (int c = 0; c < 3; c++) {
@@ -814,7 +815,8 @@ scw_status scw_gpu_cw_evaluate(scw_waves w, float* E_xy, float* E_xz, float* E_y
 // sub-allocates one pre-sized pool for everything and treats any other cudaMalloc as a
 // leak, a real-time viewer that may not stall on the allocator in its frame loop, or a
 // plug-in host that forbids its plug-ins from allocating device memory.  The entry point
-// below evaluates one plane like scw_eval_plane_device but takes its split-K scratch from
+// below evaluates the plane that scw_eval_plane_device evaluates, by the summation kernel (the tensor-core form, about
+// four times as fast, plans on the host and takes its scratch from the context), with its split-K scratch from
 // a fixed array compiled into this library, passes its tiny descriptor tables as kernel
 // parameters, and calls no cudaMalloc, cudaMallocHost, cudaFree or allocating library
 // routine.

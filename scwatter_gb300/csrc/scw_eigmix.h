@@ -1,7 +1,7 @@
 // Mixed-precision eigen-solver of batched dense complex matrices (eig_mixed.cu).
 //
 // GB300 issues FP64 at about 1/64 of its FP32 rate, and the Householder + QR eigen-solve of a
-// layer matrix is inherently one CTA per matrix.  So the O(n^3) factorisation runs in FP32,
+// layer matrix is a chain of steps on a few CTAs.  So the O(n^3) factorisation runs in FP32,
 // and FP64 accuracy comes back through Newton refinement of all eigenpairs at once, which
 // costs one FP64 GEMM per step spread over every SM:
 //   R = A X - X diag(lambda)          (FP64 GEMM)

@@ -78,8 +78,8 @@ struct scw_sep_s {
     //     over (Ex, Ey, Ez) -- the structure of the solver's modes, whose E rows are the same
     //     eigenvector for the two roots +-gamma and whose H rows (hence Ez) change sign.
     int halves = 2;
-    // contraction tile shape: 0 = the default rows per warp for the launch's planes per group
-    // (8, 8, 4, 2 for 1, 2, 4, 8 planes), 1 = half as many rows per warp (twice the CTAs);
+    // contraction tile shape: 0 = the default rows per warp for the launch's planes per group (8 for one or two
+    // planes, 4 for 3 to 8; half as many where that leaves SMs without a CTA), 1 = half as many always;
     // chosen by the batch autotuner
     int ctr_shape = 0;
     float2* dQ = nullptr;
