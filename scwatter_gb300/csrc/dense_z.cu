@@ -1451,14 +1451,10 @@ scw_status scw_zgesv(scw_ctx ctx, int n, int nrhs, void* A, void* B, int batch, 
     const long long nn = (long long)n * n;
     scw::DevBuf wbuf;
     scw::GemmWs ws;
-    const size_t need = std::max(scw::zgemm_ws_bytes(n, n, 32, 1), scw::zgemm_ws_bytes(n, nrhs, 32, 1));
-    scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, scw::kGemmWsCap)));
-    if (st == SCW_ERR_NOMEM) {               // no room for the digits: on the FP64 pipes
-        st = SCW_OK;
-    } else if (st == SCW_OK) {
-        st = scw::ctx_tc_flag(ctx);
-        ws = scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err, true};
-    }
+    scw_status st = scw::reserve_gemm_ws(
+        ctx, wbuf, std::max(scw::zgemm_ws_bytes(n, n, 32, 1), scw::zgemm_ws_bytes(n, nrhs, 32, 1)), batch, ws);
+    if (st == SCW_ERR_NOMEM) st = SCW_OK;    // no room for the digits: on the FP64 pipes
+    ws.parts = true;
     if (st == SCW_OK) st = scw::zgetrf(ctx->stream, (double2*)A, n, n, n, nn, dpiv, n, dinfo, batch, ws, nullptr);
     if (st == SCW_OK)
         st = scw::zgetrs(ctx->stream, (const double2*)A, n, nn, dpiv, n, (double2*)B, nrhs, (long long)n * nrhs, batch,
@@ -1492,15 +1488,9 @@ scw_status scw_zgeev(scw_ctx ctx, int n, void* A, void* W, void* V, int batch, i
         return fail(SCW_ERR_NOMEM, "scw_zgeev: workspace");
     }
     scw::DevBuf wbuf;
-    const size_t need = scw::zgemm_ws_bytes(n, n, n, 1);
-    scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, scw::kGemmWsCap)));
-    scw::GemmWs ws;                          // without room for the digits: on the FP64 pipes
-    if (st == SCW_ERR_NOMEM) {
-        st = SCW_OK;
-    } else if (st == SCW_OK) {
-        st = scw::ctx_tc_flag(ctx);
-        ws = scw::GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err};
-    }
+    scw::GemmWs ws;
+    scw_status st = scw::reserve_gemm_ws(ctx, wbuf, scw::zgemm_ws_bytes(n, n, n, 1), batch, ws);
+    if (st == SCW_ERR_NOMEM) st = SCW_OK;    // no room for the digits: on the FP64 pipes
     if (st == SCW_OK)
         st = scw::zgeev(ctx->stream, (double2*)A, (double2*)W, (double2*)V, n, batch, work, dst, nullptr, true, ws);
     ctx->launches += 4;

@@ -780,13 +780,11 @@ extern "C" scw_status scw_zgeev_mixed(scw_ctx ctx, int n, void* A, void* W, void
     mx::EigMixParams prm;
     prm.wide = true;
     DevBuf wbuf;
-    const size_t need = zgemm_ws_bytes(n, n, n, 1);
-    scw_status st = wbuf.reserve(std::max(need, std::min(need * batch, kGemmWsCap)));
-    if (st == SCW_OK) st = ctx_tc_flag(ctx);
+    GemmWs ws;
+    scw_status st = reserve_gemm_ws(ctx, wbuf, zgemm_ws_bytes(n, n, n, 1), batch, ws);
     if (st == SCW_OK)
         st = mx::geev_mixed(ctx->stream, (double2*)A, (double2*)W, (double2*)V, n, batch, w,
-                            reinterpret_cast<double2*>(blk), dst, prm, GemmWs{(char*)wbuf.ptr, wbuf.bytes, ctx->tc_err},
-                            &L);
+                            reinterpret_cast<double2*>(blk), dst, prm, ws, &L);
     ctx->launches += L;
     std::vector<int> status(batch, 0), state(batch, 0), steps(batch, 0);
     std::vector<double> res(batch, 0.0);

@@ -861,6 +861,14 @@ scw_status ctx_gemm_ws(scw_ctx ctx, size_t one, size_t all, GemmWs& ws) {
     return st;
 }
 
+scw_status reserve_gemm_ws(scw_ctx ctx, DevBuf& buf, size_t one, int batch, GemmWs& ws) {
+    scw_status st = buf.reserve(std::max(one, std::min(one * batch, kGemmWsCap)));
+    if (st == SCW_ERR_NOMEM && batch > 1) st = buf.reserve(one);
+    if (st == SCW_OK) st = ctx_tc_flag(ctx);
+    ws = st == SCW_OK ? GemmWs{(char*)buf.ptr, buf.bytes, ctx->tc_err} : GemmWs{};
+    return st;
+}
+
 size_t zgemm_ws_bytes(int M, int N, int K, int batch) { return oz::Shape(8, M, N, K).bytes(batch, batch, batch); }
 
 scw_status zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const double2* A, int lda, long long sA,

@@ -16,8 +16,7 @@
 //     window needs and goes on chasing; the other CTAs of the cluster do the rest meanwhile.
 // What bounds it: at n = 648 half of the time is the serial QR of the deflation windows (44 of them, 0.18 ms
 // each) and a third the leader's chase (290 windows of 512 rotations, 18 us each).  Measured: 18.2 ms for
-// 20 matrices of n = 648 on clusters of 6 CTAs, 3.76 ms for 10 of n = 216, 0.58 ms for 4 of n = 50 (of which 0.6 and 0.1 ms by
-// keeping imaginary parts of subdiagonals and values far from unit scale); with the deflation
+// 20 matrices of n = 648 on clusters of 6 CTAs, 3.76 ms for 10 of n = 216, 0.58 ms for 4 of n = 50; with the deflation
 // window's column operations after each sweep 2.2, 0.7 and 0.14 more; a chase of one bulge at a time (800 clocks per
 // rotation, no deflation windows) took 316 and 23.6 ms.
 // H and Z are read through L2 (ld.global.cg): other CTAs of the cluster write them between barriers.

@@ -46,6 +46,9 @@ scw_status ctx_tc_flag(scw_ctx ctx);
 scw_status ctx_gemm_ws(scw_ctx ctx, size_t one, size_t all, GemmWs& ws);
 // workspace that takes the whole batch in one pass
 size_t zgemm_ws_bytes(int M, int N, int K, int batch);
+// buf as a workspace for products of `one` bytes of operands a matrix: for the whole batch up to the cap, or for one
+// matrix at a time where memory is short
+scw_status reserve_gemm_ws(scw_ctx ctx, DevBuf& buf, size_t one, int batch, GemmWs& ws);
 // C = alpha A op(B) + beta C + diag I (row-major, batched by strides in elements), FP64 on the tensor
 // cores; op = identity, transpose or conjugate transpose.  Without a workspace
 // by gemm<double2> (no conjugate transpose, no diagonal).

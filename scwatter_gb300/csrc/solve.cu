@@ -1018,14 +1018,17 @@ scw_status scw_solve(scw_ctx ctx, const double* sample, int Zs, int Y, int X, co
     SolveIn in{};
     SolveWs ws{};
     SolveOut o{};
-    Carver sz;
-    carve_in(p, sz, in);
-    carve_ws(p, sz, ws);
-    carve_out(p, sz, o, false, false);
     char* blk = nullptr;
-    if (cudaMalloc(&blk, sz.off) != cudaSuccess) {
+    for (bool small : {false, true}) {
+        if (small) p.gemm_cap = 0;           // where memory is short, with the digits of one slice's product
+        Carver sz;
+        carve_in(p, sz, in);
+        carve_ws(p, sz, ws);
+        carve_out(p, sz, o, false, false);
+        if (cudaMalloc(&blk, sz.off) == cudaSuccess) break;
         cudaGetLastError();
-        return fail(SCW_ERR_NOMEM, "scw_solve: cudaMalloc of " + std::to_string(sz.off >> 20) + " MiB");
+        blk = nullptr;
+        if (small) return fail(SCW_ERR_NOMEM, "scw_solve: cudaMalloc of " + std::to_string(sz.off >> 20) + " MiB");
     }
     std::unique_ptr<char, void (*)(char*)> blk_guard(blk, [](char* q) { cudaFree(q); });
     Carver c{blk, 0};
@@ -1095,13 +1098,16 @@ scw_status scw_layer_problem(scw_ctx ctx, const double* sample, int Zs, int Y, i
     SCW_ON_DEVICE(ctx->device);
     SolveIn in{};
     SolveWs ws{};
-    Carver sz;
-    carve_in(p, sz, in);
-    carve_ws(p, sz, ws);
     char* blk = nullptr;
-    if (cudaMalloc(&blk, sz.off) != cudaSuccess) {
+    for (bool small : {false, true}) {
+        if (small) p.gemm_cap = 0;
+        Carver sz;
+        carve_in(p, sz, in);
+        carve_ws(p, sz, ws);
+        if (cudaMalloc(&blk, sz.off) == cudaSuccess) break;
         cudaGetLastError();
-        return fail(SCW_ERR_NOMEM, "scw_layer_problem: cudaMalloc");
+        blk = nullptr;
+        if (small) return fail(SCW_ERR_NOMEM, "scw_layer_problem: cudaMalloc");
     }
     std::unique_ptr<char, void (*)(char*)> guard(blk, [](char* q) { cudaFree(q); });
     Carver c{blk, 0};

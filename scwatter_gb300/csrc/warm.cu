@@ -355,10 +355,9 @@ scw_status scw_eig_warm(scw_ctx ctx, int n, const void* A_, int batch, const voi
     int* rep_excl = (int*)take(sizeof(int) * kMaxExcl * (size_t)n * batch);
     // workspace of the FP64 products
     scw::DevBuf gbuf;
-    const size_t gneed = scw::zgemm_ws_bytes(n, n, n, 1);
-    if ((s = gbuf.reserve(std::max(gneed, std::min(gneed * batch, scw::kGemmWsCap)))) != SCW_OK) return s;
-    if ((s = scw::ctx_tc_flag(ctx)) != SCW_OK) return s;
-    const scw::GemmWs gws{(char*)gbuf.ptr, gbuf.bytes, ctx->tc_err};
+    scw::GemmWs gws;
+    s = scw::reserve_gemm_ws(ctx, gbuf, scw::zgemm_ws_bytes(n, n, n, 1), batch, gws);
+    if (s != SCW_OK && s != SCW_ERR_NOMEM) return s;         // (without room for the digits: on the FP64 pipes)
     // Hessenberg form and its norm
     SCW_CUDA_TRY(cudaMemcpyAsync(Hm, A, sizeof(double2) * nn * batch, cudaMemcpyDeviceToDevice, st));
     s = scw::zgehrd(st, Hm, Qm, n, batch, hw);

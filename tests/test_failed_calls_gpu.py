@@ -137,3 +137,31 @@ def test_batch_lanes_where_memory_is_short(shim):
         for u, v in zip(b.result(i), ref.result(i)):
             assert np.abs(u - v).max() <= 1e-5 * np.abs(v).max()
     """)
+
+
+def test_solve_without_room_for_a_batch_of_digits(shim):
+    _child(shim, """
+    from scwatter_gb300 import solver, samples
+    kw = dict(lam=1.0, direction=(0, 0, 1), ex=(1, 0), ey=(0, 0), size=(16.0, 16.0, 6.0), coef=(5, 5))
+    s = samples.spheres((6, 16, 16), n_spheres=3, radius=(2, 5), seed=1)
+    ref = solver.solve(s, ctx=ctx, **kw).x
+    shim.shim_malloc(0)                # the solve's arena
+    x = solver.solve(s, ctx=ctx, **kw).x
+    assert np.abs(x - ref).max() <= 1e-11 * np.abs(ref).max()
+    """)
+
+
+def test_eigen_solvers_without_room_for_digits(shim):
+    _child(shim, """
+    import torch
+    A0 = torch.randn(3, 40, 40, dtype=torch.complex128, device="cuda")
+    for name, at in (("scw_zgeev_mixed", 2), ("scw_zgeev", 2)):        # work, status, digits
+        A, V = A0.clone(), torch.zeros_like(A0)
+        W = torch.zeros(3, 40, dtype=torch.complex128, device="cuda")
+        torch.cuda.synchronize()
+        shim.shim_malloc(at)
+        more = (None, None, None) if name == "scw_zgeev_mixed" else (None,)
+        _lib.call(name, ctx.handle, 40, *(ctypes.c_void_p(t.data_ptr()) for t in (A, W, V)), 3, *more)
+        R = A0 @ V - V * W[:, None, :]
+        assert (torch.linalg.norm(R) / torch.linalg.norm(A0) / torch.linalg.norm(V)).item() < 1e-12
+    """)
