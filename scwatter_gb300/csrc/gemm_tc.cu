@@ -487,7 +487,8 @@ oz_parts_kernel(SplitArgs p, int a_shared, int b_shared, double2 alpha, double2 
         }
 }
 
-template <int S, typename TC>
+// kMask: elements whose bit p.mask has set are left as they are
+template <int S, typename TC, bool kMask>
 __global__ void __launch_bounds__(kThreads, 1)
 oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
     using namespace tc;
@@ -699,7 +700,7 @@ oz_gemm_kernel(GemmArgs p, const int* __restrict__ skip) {
                 for (int q = lane; q < 32 * kSeg; q += 32) {
                     const int r = q / kSeg, cc = q % kSeg;
                     if (row0 + r >= p.M || col0 + c0 + cc >= p.N) continue;
-                    if (p.mask && masked(p.mask, p.M, p.N, b, row0 + r, col0 + c0 + cc)) continue;
+                    if (kMask && masked(p.mask, p.M, p.N, b, row0 + r, col0 + c0 + cc)) continue;
                     TC v = reinterpret_cast<const TC*>(stg + r * kStageRow)[cc];
                     TC* o = out + (long long)r * p.ldc + c0 + cc;
                     if (add1) {
@@ -782,7 +783,6 @@ static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const
     SCW_CUDA_TRY(cudaGetDevice(&dev));
     SCW_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     constexpr size_t smem = Cfg<S>::kSmem;
-    SCW_CUDA_TRY(cudaFuncSetAttribute(oz_gemm_kernel<S, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const Shape sh(S, M, N, K);
     const bool a1 = sA == 0 && !skip, b1 = sB == 0 && !skip;     // one operand for the whole batch
     // element (i, k) of op(A) at i rsA + k ksA, (k, j) of op(B) at k ksB + j rsB
@@ -834,8 +834,15 @@ static scw_status run(cudaStream_t st, int M, int N, int K, double2 alpha, const
         if (tiles > (1ll << 30)) return fail(SCW_ERR_ARG, "zgemm: too many tiles");
         GemmArgs g{dA, dB, eA, gN, M, N, sh.nk, sh.mt, sh.nt, sh.gA, sh.gB, a1, b1, alpha, beta, diag,
                    (void*)(C + sC * b0), ldc, sC, (int)tiles, ws.err, mask};
-        SCW_CUDA_TRY(launch_chained(true, st, dim3((unsigned)std::min<long long>(tiles, sms)), kThreads, smem,
-                                    oz_gemm_kernel<S, TC>, g, sk));
+        auto product = [&](auto kernel) -> scw_status {
+            SCW_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            SCW_CUDA_TRY(launch_chained(true, st, dim3((unsigned)std::min<long long>(tiles, sms)), kThreads, smem, kernel, g, sk));
+            return SCW_OK;
+        };
+        scw_status ps;
+        if constexpr (S == 8) ps = mask ? product(oz_gemm_kernel<S, TC, true>) : product(oz_gemm_kernel<S, TC, false>);
+        else ps = product(oz_gemm_kernel<S, TC, false>);
+        if (ps != SCW_OK) return ps;
     }
     return SCW_OK;
 }
