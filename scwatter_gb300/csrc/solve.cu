@@ -433,25 +433,31 @@ static void fft_shift_index(int m, int n, std::vector<int>& indx, std::vector<in
 
 // The pair of one harmonic (see BcPair).
 static BcPair bc_pair(double Sx, double Sy, cd Sz0, cd Sz1) {
+    // (without std::complex's product, quotient and modulus, which look for infinities and are calls: the host plans every solve)
     auto d2 = [](cd v) { return make_double2(v.real(), v.imag()); };
+    auto mul = [](cd a, cd b) { return cd(a.real() * b.real() - a.imag() * b.imag(), a.real() * b.imag() + a.imag() * b.real()); };
+    auto inv = [](cd a) {
+        const double d = 1.0 / std::norm(a);
+        return cd(a.real() * d, -a.imag() * d);
+    };
     BcPair h{};
     // the component that follows from the other two, and its ratios; all zero where s is (no medium)
-    auto third = [](const cd* s, cd* ratio) {
+    auto third = [&](const cd* s, cd* ratio) {
         int c = 2;
         for (int i = 1; i >= 0; i--)
-            if (std::abs(s[i]) > std::abs(s[c])) c = i;
+            if (std::norm(s[i]) > std::norm(s[c])) c = i;
         const int a = c == 0 ? 1 : 0, b = c == 2 ? 1 : 2;
-        const bool none = s[c] == cd(0, 0);
-        ratio[0] = none ? cd(0, 0) : -s[a] / s[c];
-        ratio[1] = none ? cd(0, 0) : -s[b] / s[c];
+        const cd r = s[c] == cd(0, 0) ? cd(0, 0) : -inv(s[c]);
+        ratio[0] = mul(s[a], r);
+        ratio[1] = mul(s[b], r);
         return c;
     };
     // a 4 x 3 matrix on the pair
-    auto on_pair = [](const cd (*f)[3], int c, const cd* ratio, cd (*out)[2]) {
+    auto on_pair = [&](const cd (*f)[3], int c, const cd* ratio, cd (*out)[2]) {
         const int a = c == 0 ? 1 : 0, b = c == 2 ? 1 : 2;
         for (int q = 0; q < 4; q++) {
-            out[q][0] = f[q][a] + f[q][c] * ratio[0];
-            out[q][1] = f[q][b] + f[q][c] * ratio[1];
+            out[q][0] = f[q][a] + mul(f[q][c], ratio[0]);
+            out[q][1] = f[q][b] + mul(f[q][c], ratio[1]);
         }
     };
     const cd s1[3] = {Sx, Sy, Sz1}, s0[3] = {Sx, Sy, -Sz0};
@@ -466,9 +472,9 @@ static BcPair bc_pair(double Sx, double Sy, cd Sz0, cd Sz1) {
     cd det = 1;
     for (int i = 0; i < 4; i++)
         for (int j = i + 1; j < 4; j++) {
-            const cd d = F[i][0] * F[j][1] - F[i][1] * F[j][0];
-            if (std::abs(d) > best) {
-                best = std::abs(d);
+            const cd d = mul(F[i][0], F[j][1]) - mul(F[i][1], F[j][0]);
+            if (std::norm(d) > best) {
+                best = std::norm(d);
                 det = d;
                 h.p[0] = i;
                 h.p[1] = j;
@@ -476,13 +482,12 @@ static BcPair bc_pair(double Sx, double Sy, cd Sz0, cd Sz1) {
         }
     for (int i = 0, k = 0; i < 4; i++)
         if (i != h.p[0] && i != h.p[1]) h.q[k++] = i;
-    const cd* a = F[h.p[0]];
-    const cd* b = F[h.p[1]];
-    const cd Fi[4] = {b[1] / det, -a[1] / det, -b[0] / det, a[0] / det};
+    const cd *a = F[h.p[0]], *b = F[h.p[1]], id = inv(det);
+    const cd Fi[4] = {mul(b[1], id), -mul(a[1], id), -mul(b[0], id), mul(a[0], id)};
     for (int k = 0; k < 2; k++) {
         const cd* g = F[h.q[k]];
-        h.M[2 * k] = d2(g[0] * Fi[0] + g[1] * Fi[2]);
-        h.M[2 * k + 1] = d2(g[0] * Fi[1] + g[1] * Fi[3]);
+        h.M[2 * k] = d2(mul(g[0], Fi[0]) + mul(g[1], Fi[2]));
+        h.M[2 * k + 1] = d2(mul(g[0], Fi[1]) + mul(g[1], Fi[3]));
         h.r1[k] = d2(r1[k]);
         h.r0[k] = d2(r0[k]);
     }
