@@ -677,8 +677,10 @@ hqr32_kernel(float2* __restrict__ H, float2* __restrict__ Z, int n, long long sA
     int ihi = n - 1, idle = 0, rounds = 0;              // rank 0's state
     int sweep_l = 0, sweep_hi = -1, sweep_ms = 0;       // rank 0: a sweep is due
     const int limit = 30 * max(10, n);
-    // larger windows deflate more at a time, but their QR grows with the square (measured with 16, 20, 24, 28, 32: n =
-    // 216 4.08, 3.79, 3.72, 3.95, 3.99 ms; n = 648 21.3, 19.4, 18.4, 17.7, 17.8 ms)
+    // larger windows deflate more at a time, but their QR grows with the square (measured with 16, 20, 24, 28, 32 on layers: n =
+    // 216 4.08, 3.79, 3.72, 3.95, 3.99 ms; n = 648 21.3, 19.4, 18.4, 17.7, 17.8 ms; between them on graded random matrices, 24 and 32:
+    // n = 100 1.9, 2.1; 216 5.1, 5.3; 288 7.1, 7.5; 350 9.4, 9.8; 450 13.5, 14.1; 576 19.9, 20.8; 648 24.2, 25.0 ms.  Up to 400 both
+    // kinds want 24; beyond, layers, which gain from more shifts, decide.)
     const int window = n < 400 ? 24 : kNW;
     while (true) {
         if (rank == 0) {
