@@ -62,6 +62,7 @@ struct Graph {
 
 struct scw_batch_s {
     scw_ctx ctx = nullptr;
+    int device = -1;                        // the context's: it may be gone when this is freed
     std::vector<Item> items;
     int lanes = 0, method = 0;
     std::vector<scw_ctx> lane_ctx;
@@ -79,7 +80,7 @@ struct scw_batch_s {
     std::vector<double> tune_log;  // lanes, method, contraction tile shape, ms per candidate
     int ctr_shape = 0;             // chosen contraction tile shape (scw_sep_s::ctr_shape)
     ~scw_batch_s() {
-        ::scw::DeviceScope dev_scope_(ctx ? ctx->device : -1);
+        ::scw::DeviceScope dev_scope_(device);
         g.reset();
         for (auto c : lane_ctx) scw_ctx_destroy(c);
         for (auto s : lane_stream) cudaStreamDestroy(s);
@@ -281,6 +282,7 @@ scw_status scw_batch_create(scw_ctx ctx, const scw_batch_item* items, int count,
     std::unique_ptr<scw_batch_s> b(new (std::nothrow) scw_batch_s());
     if (!b) return fail(SCW_ERR_NOMEM, "host allocation");
     b->ctx = ctx;
+    b->device = ctx->device;
     b->items.resize(count);
     // ---- plans ----
     size_t in_bytes = 0, out_bytes = 0, field_bytes = 0;

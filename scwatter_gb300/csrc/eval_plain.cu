@@ -624,7 +624,7 @@ using scw::fail;
 
 static void free_waves(scw_waves w) {
     if (!w) return;
-    ::scw::DeviceScope dev_scope_(w->ctx ? w->ctx->device : -1);
+    ::scw::DeviceScope dev_scope_(w->device);
     if (w->kre) cudaFree(w->kre);
     if (w->kim) cudaFree(w->kim);
     if (w->zref) cudaFree(w->zref);
@@ -647,6 +647,7 @@ scw_status scw_gpu_initialize(scw_ctx ctx, int layers, const float* z_layers, co
     scw_waves w = new (std::nothrow) scw_waves_s();
     if (!w) return fail(SCW_ERR_NOMEM, "host allocation");
     w->ctx = ctx;
+    w->device = ctx->device;
     w->layers = layers;
     w->n = n_waves;
     w->z_layers.assign(z_layers, z_layers + layers);
@@ -682,6 +683,7 @@ scw_status scw_gpu_initialize_cw(scw_ctx ctx, scw_cw cw, scw_waves* out) {
     scw_waves w = new (std::nothrow) scw_waves_s();
     if (!w) return fail(SCW_ERR_NOMEM, "host allocation");
     w->ctx = ctx;
+    w->device = ctx->device;
     w->layers = layers;
     w->n = total;
     const size_t n = (size_t)total;

@@ -1134,7 +1134,7 @@ using scw::fail;
 // ------------------------------------------------------------------------------------
 static void sep_free(scw_sep s) {
     if (!s) return;
-    ::scw::DeviceScope dev_scope_(s->ctx ? s->ctx->device : -1);
+    ::scw::DeviceScope dev_scope_(s->device);
     if (s->dQ && s->own_Q) cudaFree(s->dQ);
     if (s->dKz) cudaFree(s->dKz);
     if (s->dExt) cudaFree(s->dExt);
@@ -1164,6 +1164,7 @@ static scw_status sep_create(scw_ctx ctx, int M0, int M1, int n_slices, int mode
     scw_sep s = new (std::nothrow) scw_sep_s();
     if (!s) return fail(SCW_ERR_NOMEM, "host allocation");
     s->ctx = ctx;
+    s->device = ctx->device;
     s->M0 = M0;
     s->M1 = M1;
     s->MF = M0 * M1;

@@ -133,6 +133,7 @@ using scw::fail;
 
 struct scw_mlp_s {
     scw_ctx ctx = nullptr;
+    int device = -1;                        // the context's: it may be gone when this is freed
     int n_in = 0, width = 0, n_out = 0;
     long long n_par = 0;
     long long off[6] = {};          // W1 b1 W2 b2 W3 b3 offsets in the parameter vector
@@ -146,7 +147,7 @@ struct scw_mlp_s {
     float *H1 = nullptr, *H2 = nullptr, *Y = nullptr, *dY = nullptr, *dH2 = nullptr, *dH1 = nullptr;
     double* sums = nullptr;
     ~scw_mlp_s() {
-        ::scw::DeviceScope dev_scope_(ctx ? ctx->device : -1);
+        ::scw::DeviceScope dev_scope_(device);
         for (void* p : {(void*)P, (void*)G, (void*)Mv, (void*)Vv, (void*)H1, (void*)H2, (void*)Y, (void*)dY,
                         (void*)dH2, (void*)dH1, (void*)sums})
             cudaFree(p);
@@ -256,6 +257,7 @@ scw_status scw_mlp_create(scw_ctx ctx, int n_in, int width, int n_out, uint64_t 
     scw_mlp m = new (std::nothrow) scw_mlp_s();
     if (!m) return fail(SCW_ERR_NOMEM, "host allocation");
     m->ctx = ctx;
+    m->device = ctx->device;
     m->n_in = n_in;
     m->width = width;
     m->n_out = n_out;

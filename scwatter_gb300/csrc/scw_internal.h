@@ -152,6 +152,7 @@ struct scw_cw_s {
 
 struct scw_waves_s {
     scw_ctx ctx = nullptr;
+    int device = -1;                        // the context's: it may be gone when this is freed
     int layers = 0;
     int64_t n = 0;
     int rule = 0;                           // 0: z >= z_l - 0.001, 1: z >= z_l

@@ -61,6 +61,7 @@ scw_status sep_synth_tc(scw_ctx ctx, const float2* T, const float2* F, int nrows
 
 struct scw_sep_s {
     scw_ctx ctx = nullptr;
+    int device = -1;                        // the context's: it may be gone when this is freed
     int M0 = 0, M1 = 0, MF = 0, Z = 0, J = 0;
     int Jp = 0;                            // J rounded up to even: row stride of Q / kz on the device (zero padded)
     int rule = 0;

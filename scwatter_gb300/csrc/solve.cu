@@ -40,6 +40,7 @@ using cd = std::complex<double>;
 
 struct scw_solution_s {
     scw_ctx ctx = nullptr;
+    int device = -1;                        // the context's: it may be gone when this is freed
     int M0 = 0, M1 = 0, MF = 0, Z = 0;
     double k = 0, n0 = 1, n1 = 1;
     bool external = false;
@@ -56,7 +57,7 @@ struct scw_solution_s {
     std::vector<double> eig_res;
     ~scw_solution_s() {
         if (dQ || dV || dBeta) {
-            ::scw::DeviceScope dev_scope_(ctx->device);
+            ::scw::DeviceScope dev_scope_(device);
             if (dQ) cudaFree(dQ);
             if (dV) cudaFree(dV);
             if (dBeta) cudaFree(dBeta);
@@ -1004,6 +1005,7 @@ scw_status scw_solve(scw_ctx ctx, const double* sample, int Zs, int Y, int X, co
     std::unique_ptr<scw_solution_s> sol(new (std::nothrow) scw_solution_s());
     if (!sol) return fail(SCW_ERR_NOMEM, "host allocation");
     sol->ctx = ctx;
+    sol->device = ctx->device;
     sol->M0 = p.M0;
     sol->M1 = p.M1;
     sol->MF = p.MF;
