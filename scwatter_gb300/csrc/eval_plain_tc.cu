@@ -16,7 +16,7 @@
 //     the phase at columns 2 and 6 and of one step, phases in turns with both factors as two floats (an FP32
 //     product would lose 1e-6 at 30 radians), from the Taylor series on [-pi/4, pi/4]; the columns between are one
 //     or two steps away, times 1 + i k delta for delta, the rounding of that grid coordinate.  Values are split into
-//     fp16 hi + lo (22 bits; L is scaled to 2^12 and R to 2^10, which leaves room for growth inside a tile
+//     fp16 hi + lo (22 bits, 23 in R; L is scaled to 2^12 and R to 2^10, which leaves room for growth inside a tile
 //     and keeps lo far above fp16's smallest values even for waves 2^-12 below the chunk's largest) and stored
 //     as 16 bytes of eight points of one wave, the MN-major core-matrix row: lanes store side by side, where
 //     rows of eight waves (K-major) had four lanes on the same banks;
@@ -29,7 +29,7 @@
 //     kernel, in a fixed order.  32 additions to a growing sum, not 1024: a run of 1024 waves loses less to rounding than the
 //     summation kernel's 256 additions (45 against 64 roundings of a sum of 256 waves, over 4096 waves that all add up).
 //     One FP32 sum of 4096 waves lost 1.5 times as much as that kernel.
-// 409 600 waves x 3 planes of 200 x 200 points: 19.4 ms by the summation kernel, 4.45 ms here; 20 736 waves a layer on a
+// 409 600 waves x 3 planes of 200 x 200 points: 19.4 ms by the summation kernel, 4.47 ms here; 20 736 waves a layer on a
 // 101 x 77 x 50 volume: 5.10 -> 1.39 ms (4.30 and 1.30 with one FP32 sum per 4096 waves:
 // tensor memory answers late, and sums that are late hold up the MMAs).  A chunk takes about 1600 clocks: 700 of them are MMA reads of shared memory and
 // 450 the stores of the operands, and the warps that build these issue half of the time.  Measured in the
@@ -216,13 +216,24 @@ __device__ __forceinline__ void eight(float kh, float kl, float G, bool lossy, c
     }
 }
 
-// eight values as fp16 hi (the upper 11 bits of each) and lo (the rest, rounded)
+// Eight values as fp16 hi and lo (the rest, rounded).  kNear: hi is the nearest value of 11 bits, so that lo has either
+// sign and half the size; else the upper 11 bits.  Nothing adds the product of two lo, and of two cut ones it leans one way:
+// with both operands cut, sums of 600 random waves on grids of a hundredth of a wavelength were 2.9e-7 to 3.1e-7 off, where
+// the summation kernel has 2.3e-7 to 3.1e-7; with R nearest they are 1.5e-7 to 2.1e-7 off on grids of every extent.  409 600
+// waves on three 200 x 200 planes: 4.45 ms both cut, 4.47 R nearest, 4.73 L nearest, 4.73 both (1.2e-7 to 1.9e-7).
+template <bool kNear>
 __device__ __forceinline__ void split8(const F2 (&v)[4], uint4& h, uint4& l) {
     F2 hi[4], lo[4];
 #pragma unroll
     for (int u = 0; u < 4; u++) {
-        hi[u].v = v[u].v & 0xffffe000ffffe000ull;
-        lo[u] = add2(v[u], neg2(hi[u]));
+        if (kNear) {
+            const F2 m = both(-1.f), t = mul2(v[u], both(8193.f));
+            hi[u] = fma2(fma2(v[u], m, t), m, t);
+            lo[u] = fma2(hi[u], m, v[u]);
+        } else {
+            hi[u].v = v[u].v & 0xffffe000ffffe000ull;
+            lo[u] = add2(v[u], neg2(hi[u]));
+        }
     }
     auto half2 = [](float x, float y) {
         const __half2 q = __floats2half2_rn(x, y);
@@ -407,12 +418,12 @@ plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items
                     F2 v[4];
 #pragma unroll
                     for (int u = 0; u < 4; u++) v[u] = fma2(both(ar), re[u], mul2(both(-ai), im[u]));
-                    split8(v, h, l);
+                    split8<false>(v, h, l);
                     *reinterpret_cast<uint4*>(pc) = h;
                     *reinterpret_cast<uint4*>(pc + kPartA) = l;
 #pragma unroll
                     for (int u = 0; u < 4; u++) v[u] = fma2(both(ar), im[u], mul2(both(ai), re[u]));
-                    split8(v, h, l);
+                    split8<false>(v, h, l);
                     *reinterpret_cast<uint4*>(pc + 2 * kPartA) = h;
                     *reinterpret_cast<uint4*>(pc + 3 * kPartA) = l;
                 }
@@ -420,10 +431,10 @@ plain_tc_kernel(const Plane* __restrict__ planes, const Item* __restrict__ items
                 const int gr = task - 64;
                 eight(k.z, k.w, b.w, cplx & 2, S.grid[kGroupsA + gr], g.db, 1024.f, re, im);
                 unsigned char* pb = p + 4 * kPartA + gr * kGroup;
-                split8(re, h, l);
+                split8<true>(re, h, l);
                 *reinterpret_cast<uint4*>(pb + nB * kGroup) = h;
                 *reinterpret_cast<uint4*>(pb + nB * kGroup + kPartB) = l;
-                split8(im, h, l);
+                split8<true>(im, h, l);
                 *reinterpret_cast<uint4*>(pb + 2 * nB * kGroup) = h;
                 *reinterpret_cast<uint4*>(pb + 2 * nB * kGroup + kPartB) = l;
                 constexpr uint32_t neg = 0x80008000u;
